@@ -41,20 +41,18 @@ WORKLOAD = "droplet512"
 METRIC = "cell-updates/s/step plain FP64 vs mixed at stated error; adjoint/forward cost"
 UNIT = "cell-updates/s"
 
-# The dominant kernel's counters per interior cell of one launch (k_weno2, one
-# velocity level: the advection of (u, v, w); the (uo, vo, wo) level is carried
-# over from the previous step).  DRAM bytes read + written from the ncu capture of
-# one one-level launch at 256x128x128 (113.5 MB + 68.7 MB over 4,194,304 cells;
-# python bench.py --profile --workload couette256 --warmup 2 --steps 1 under
-# ncu --set full -k regex:k_weno2 -s 1 -c 1 --clock-control none).  FP64
-# instructions (DADD + DMUL + DFMA thread instructions; flops count an FMA twice):
-# half of a two-level launch's (955.7 M + 1219.5 M + 1885.8 M at 256x128x128),
-# both levels running the same loop body.
-WENO_CAPTURE = ("ncu --set full of one one-level k_weno2 launch, couette256 256x128x128 (DRAM bytes); "
-                "FP64 instruction counts: half of a two-level launch's at the same size")
-WENO_TRAFFIC_PER_CELL = (113.540352e6 + 68.679168e6) / 4194304
-WENO_FP64_INST_PER_CELL = (955711488 + 1219493888 + 1885798400) / 2 / 4194304
-WENO_FP64_FLOPS_PER_CELL = (955711488 + 1219493888 + 2 * 1885798400) / 2 / 4194304
+# The dominant kernel's counters per interior cell of one velocity level (k_weno_line,
+# its three launches: the advection of (u, v, w); the (uo, vo, wo) level is carried
+# over from the previous step), from ncu captures of one level at 256x128x128
+# (4,194,304 cells, walks of 32 points, as at the benchmark's size): DRAM bytes read +
+# written, and FP64 instructions (DADD + DMUL + DFMA thread instructions; flops count
+# an FMA twice).
+WENO_CAPTURE = ("ncu of the three k_weno_line launches of one level at 256x128x128: DRAM bytes, DADD + DMUL + DFMA "
+                "thread instructions")
+WENO_TRAFFIC_PER_CELL = (192.281088e6 + 94.842624e6 + 238.377984e6 + 71.68256e6 + 244.354048e6 + 57.25312e6) / 4194304
+WENO_DADD, WENO_DMUL, WENO_DFMA = 3 * 93978624, 140771328 + 2 * 128188416, 188743680 + 2 * 201326592
+WENO_FP64_INST_PER_CELL = (WENO_DADD + WENO_DMUL + WENO_DFMA) / 4194304
+WENO_FP64_FLOPS_PER_CELL = (WENO_DADD + WENO_DMUL + 2 * WENO_DFMA) / 4194304
 # weno5.h's own formula (both one-sided reconstructions) per cell and level
 WENO_REFERENCE_FLOPS_PER_CELL = 1383.0
 
@@ -607,7 +605,7 @@ def main():
     del pinned, host
 
     # ---- rooflines ------------------------------------------------------------
-    # Dominant kernel: WENO5 advection of (u, v, w) (k_weno2, one level: stage 4),
+    # Dominant kernel: WENO5 advection of (u, v, w) (k_weno_line, one level: stage 4),
     # FP64-pipe bound.  Executed FP64 instructions per second (ncu DADD + DMUL +
     # DFMA per cell of one launch, WENO_FP64_INST_PER_CELL) against the FP64 pipe's
     # instruction rate, half the FMA-chain flop rate fmf_measure_fma_rate measures
@@ -630,7 +628,7 @@ def main():
     roofline = {"bound": "fp64", "achieved": inst_rate, "peak": inst_peak, "unit": "T FP64 instructions/s",
                 "frac": inst_rate / inst_peak,
                 "traffic": WENO_TRAFFIC_PER_CELL * cfg.cells,
-                "kernel": "k_weno2, one level (the step's cal_advu_weno5 of u, v, w)", "kernel_ms": ms_stage.value,
+                "kernel": "k_weno_line, one level in three launches (the step's cal_advu_weno5 of u, v, w)", "kernel_ms": ms_stage.value,
                 "kernel_ms_both_levels": ms_stage2.value,
                 "fp64_inst_per_cell": WENO_FP64_INST_PER_CELL,
                 "counters_source": WENO_CAPTURE + ", scaled to the workload by its cell count",

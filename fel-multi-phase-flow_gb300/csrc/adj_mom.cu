@@ -11,7 +11,7 @@ namespace fmf {
 namespace adj {
 
 namespace {
-// The forward derivative is fused_weno.cu's wdir: the five differences e taken
+// The forward derivative (fused_weno.cu) in its one-stencil form: the five differences e taken
 // walking from the upwind end of the stencil, and R(e) = num / den with
 //   s_k/3 = (13/3) t1^2 + t2^2,  x = s2 s3, y = s1 s3, z = s1 s2,
 //   X = x^2, Y = y^2 + 1e-80/486, Z = z^2,

@@ -5,10 +5,10 @@
 //
 // weno5.h forms both one-sided reconstructions and multiplies the unused one by
 // vel-|vel| = 0 (or vel+|vel| = 0); here only the upwind side is evaluated, which
-// gives the same value and halves the FP64 work, in a rearranged form of the same
-// quotient (wdir) that needs about two thirds of the remaining FP64 operations.
-// The grid has one thread per interior cell (x fastest, 32 x 4 block, one k plane
-// per grid z).
+// gives the same value and halves the work, in a rearranged form of the same
+// quotient.  FP64: a thread walks part of a line (k_weno_line, one launch per axis).
+// FP32 and FP32 pairs: one thread per interior cell (x fastest, 32 x 4 block, one k
+// plane per grid z).
 #include <cstring>
 
 #include "../../include/fmf_capi.h"
@@ -21,53 +21,21 @@ namespace fused {
 
 namespace {
 // One directional derivative of weno5.h:2-70 times dxi, from the upwind side
-// only (the reference multiplies the other side by vel -/+ |vel| = 0).
+// only (the reference multiplies the other side by vel -/+ |vel| = 0):
 //  * vsum = 4 vel exactly: the reference's ((a+b)*0.5 + (c+d)*0.5)*0.5 scales
 //    (a+b) + (c+d) by powers of two only, so vsum = (a+b) + (c+d) and the term
 //    (vel + |vel|)/12 * dxi (or vel - |vel|) is |vsum| * dxi/24 on the side used.
-//  * The five differences are taken walking from the upwind end, q[c-3S]..q[c+2S]
-//    for vel > 0 (dfm5, dfm3, dfm1, dfp1, dfp3) and q[c+3S]..q[c-2S] for vel < 0,
-//    where they are -(dfp5, dfp3, dfp1, dfm1, dfm3); the reconstruction is odd in
-//    its inputs, so the sign of vel cancels and one formula serves both sides.
+//  * The five differences a5, a3, a1, b1, b3 are taken walking from the upwind end,
+//    q[c-3S]..q[c+2S] for vel > 0 (dfm5, dfm3, dfm1, dfp1, dfp3) and q[c+3S]..q[c-2S]
+//    for vel < 0, where they are -(dfp5, dfp3, dfp1, dfm1, dfm3); the reconstruction
+//    is odd in its inputs, so the sign of vel cancels and one formula serves both.
 //  * Weights: with the reference's m1 = (s2 s3)^2, m2 = 6 (s1 s3)^2,
 //    m3 = 3 (s1 s2)^2, w1 = m1 / (m1 + m2 + m3 + 1e-80), w3 likewise and
 //    w2 = 1 - w1 - w3, its sum w1 d1 + w2 d2 + w3 d3 equals
-//    (m1 d1 + m2 d2 + m3 d3 + 1e-80 d2) / (m1 + m2 + m3 + 1e-80).  That quotient
-//    is formed here with every s divided by 3 and every m by 486 (the factors 6
-//    and 3 moved onto d1/6 and d3/2), the 1e-80 divided by 486 and added to m2:
-//    the same value with fewer FP64 operations.
-// kx = dxi / 24.
-__device__ __forceinline__ double wdir(const double* __restrict__ q, long c, long S, double vsum, double kx) {
-  // zero and sign tested on the bits (a double comparison would take an FP64-pipe
-  // slot): +-0 return 0; a positive sign bit walks from c - 3S
-  const long long vb = __double_as_longlong(vsum);
-  if ((vb << 1) == 0) return 0.0;
-  const long st = vb > 0 ? S : -S;
-  const double* p = q + c - 3 * st;
-  const double q0 = __ldg(p), q1 = __ldg(p + st), q2 = __ldg(p + 2 * st), q3 = __ldg(p + 3 * st),
-               q4 = __ldg(p + 4 * st), q5 = __ldg(p + 5 * st);
-  const double a5 = q1 - q0, a3 = q2 - q1, a1 = q3 - q2, b1 = q4 - q3, b3 = q5 - q4;
-  constexpr double c13 = 13.0 / 3.0;
-  // s/3 = (13/3) t1^2 + t2^2 (weno5.h's 13 t1^2 + 3 t2^2)
-  double t1 = fma(a3, -2.0, a5 + a1), t2 = fma(a3, -4.0, fma(a1, 3.0, a5));
-  const double s1 = fma(t1 * c13, t1, t2 * t2);
-  t1 = fma(a1, -2.0, a3 + b1);
-  t2 = a3 - b1;
-  const double s2 = fma(t1 * c13, t1, t2 * t2);
-  t1 = fma(b1, -2.0, a1 + b3);
-  t2 = fma(b1, -4.0, fma(a1, 3.0, b3));
-  const double s3 = fma(t1 * c13, t1, t2 * t2);
-  const double x = s2 * s3, y = s1 * s3, z = s1 * s2;
-  const double X = x * x, Y = fma(y, y, 1.0e-80 / 486.0), Z = z * z;
-  // d1/6, d2, d3/2 of weno5.h (d1 = 2 a5 - 7 a3 + 11 a1, d2 = -a3 + 5 a1 + 2 b1,
-  // d3 = 2 a1 + 5 b1 - b3)
-  const double d1 = fma(a1, 11.0 / 6.0, fma(a3, -7.0 / 6.0, a5 * (1.0 / 3.0)));
-  const double d2 = fma(b1, 2.0, fma(a1, 5.0, -a3));
-  const double d3 = fma(b1, 2.5, fma(b3, -0.5, a1));
-  const double num = fma(Z, d3, fma(Y, d2, X * d1));
-  const double den = fma(X, 1.0 / 6.0, fma(Z, 0.5, Y));
-  return (fabs(vsum) * kx) * (num * recip_nr(den));
-}
+//    (m1 d1 + m2 d2 + m3 d3 + 1e-80 d2) / (m1 + m2 + m3 + 1e-80).  The FP32 and
+//    FP32-pair forms take that quotient with every s divided by 3 and every m by 486
+//    (the factors 6 and 3 moved onto d1/6 and d3/2), the 1e-80 divided by 486 and
+//    added to m2; the FP64 form (k_weno_line) takes it about d2.
 
 // FP32 variant for the mixed-precision step.
 //
@@ -78,11 +46,11 @@ __device__ __forceinline__ double wdir(const double* __restrict__ q, long c, lon
 // on the FP32 pipe (converting each double where a stencil reads it put about
 // thirteen conversions per point on GB300's FP64 pipe).
 //
-// The derivative is wdir's rearranged quotient in float.  The product-form
+// The derivative is that quotient in float.  The product-form
 // weights scale like the 8th power of the differences, so float would underflow
 // for smooth fields: the five differences are divided by their largest magnitude
 // s first (the quotient is unchanged by a common scale; the result is multiplied
-// back by s), and wdir's additive 1e-80/486 becomes 1e-80/486/s^8 in scaled
+// back by s), and the additive 1e-80/486 becomes 1e-80/486/s^8 in scaled
 // units, evaluated as a power of two and clamped to [2^-126, 2^100].  The lower
 // clamp keeps the denominator a normal float where all three smoothness
 // indicators are 0 (data exactly linear in float: the quotient is then d2, the
@@ -210,7 +178,7 @@ __device__ __forceinline__ df::D wdir_df(const float2* __restrict__ q, long c, l
   }
   return df::wdir_core(w, vsum, kx);
 }
-// The FP64-accurate step's WENO5 of one or both levels (as k_weno2) in FP32-pair
+// The FP64-accurate step's WENO5 of one or both levels in FP32-pair
 // arithmetic: sp holds the split pairs of u, v, w (then uo, vo, wo); each velocity
 // sum and derivative is a pair, the three derivatives of a component are summed as
 // pairs and the sum is rounded to a double once.  The nine (component, direction)
@@ -258,47 +226,112 @@ __global__ void __launch_bounds__(128) k_weno2_df(Grid g, int nlev, const int* _
   }
 }
 
-__global__ void __launch_bounds__(128) k_weno2(Grid g, int nlev, const int* __restrict__ keep, double dxi,
-                                               double dyi, double dzi,
-                                               const double* __restrict__ u,
-                                               const double* __restrict__ v, const double* __restrict__ w,
-                                               const double* __restrict__ uo, const double* __restrict__ vo,
-                                               const double* __restrict__ wo, double* __restrict__ au,
-                                               double* __restrict__ av, double* __restrict__ aw,
-                                               double* __restrict__ auo, double* __restrict__ avo,
-                                               double* __restrict__ awo) {
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int k = 1 + (int)blockIdx.z;
-  if (i > g.ni || j > g.nj) return;
-  const long X = 1, Y = g.sy, Z = g.sz;
-  const long c = g.at(i, j, k);
-  const double kx = dxi * (1.0 / 24.0), ky = dyi * (1.0 / 24.0), kz = dzi * (1.0 / 24.0);
+// FP64: the derivatives along one axis (DIR) of the three components, written to
+// (DIR 0) or added to adv.  A thread walks m consecutive points of a line of one
+// component.  With D the differences of q between neighbours, E those of D, T those
+// of E and U those of T, every term of the quotient but the weights' products belongs
+// to a point or half point of the line, not to the stencil, and is formed once:
+//   the smoothness indicators (weno5.h's divided by 12; 13 t1^2 + 3 t2^2 with
+//   t1 = T1 and t2 = 3 E2 - E1 = 2 E2 + T1, ...) are
+//     s1 = (4/3) T1^2 + E2 (2 E2 - E1),  s2 = (4/3) T2^2 + E2 E3,
+//     s3 = (4/3) T3^2 + E3 (2 E3 - E4);
+//   d2 - d1 = 2 U1, d2 - d3 = U2 and d2 = 6 a1 + E2 + 2 E3, so the quotient is
+//     d2 - (2/3 X U1 + Z U2) / (X/3 + 2 Y + Z),
+//   X = (s2 s3)^2, Y = (s1 s3)^2 + 1e-80/124416, Z = (s1 s2)^2.
+// For vel < 0 the window is walked from the other end: E and U keep their sign there,
+// a1 and T change theirs, so each term is a choice between two values of the line, and
+// E3 and U2 are the same on both sides.
+// Bound by the FP64 pipe, which takes 64 cycles per warp instruction in each quarter
+// of an SM: everything else (choices, shifts, the strided accesses of the x lines,
+// whose lanes lie along j, the second and third pass over adv) hides behind it.  32
+// FP64 operations per derivative, 288 per cell, against 484 with one thread per cell
+// and its nine stencils: 30.85 -> 19.3 ms at 512x256x256, 3.86 -> 2.51 at 256x128x128,
+// 0.488 -> 0.344 at 128x64x64, the pipe 86 % busy either way.
+template <int DIR>
+__global__ void __launch_bounds__(32) k_weno_line(Grid g, int m, const int* __restrict__ keep, double kd,
+                                                   const double* __restrict__ u, const double* __restrict__ v,
+                                                   const double* __restrict__ w, double* __restrict__ au,
+                                                   double* __restrict__ av, double* __restrict__ aw) {
+  if (keep && *keep) return;
+  const int nl = DIR == 0 ? g.nj : g.ni, nr = DIR == 2 ? g.nj : g.nk;
+  const int nm = DIR == 0 ? g.ni : (DIR == 1 ? g.nj : g.nk);
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= nl * nr) return;
+  const int r = t / nl, l = t - r * nl;
+  const int m0 = (int)blockIdx.y * m, m1 = min(nm, m0 + m);
+  const long S = DIR == 0 ? 1 : (DIR == 1 ? g.sy : g.sz);
+  long c = DIR == 0 ? g.at(1 + m0, 1 + l, 1 + r) : (DIR == 1 ? g.at(1 + l, 1 + m0, 1 + r) : g.at(1 + l, 1 + r, 1 + m0));
+  const int comp = (int)blockIdx.z;
+  const double* q = comp == 0 ? u : (comp == 1 ? v : w);
+  const double* a = DIR == 0 ? u : (DIR == 1 ? v : w);  // the advecting component
+  double* out = comp == 0 ? au : (comp == 1 ? av : aw);
+  const long Sq = comp == 0 ? 1 : (comp == 1 ? g.sy : g.sz);
+  constexpr double c43 = 4.0 / 3.0;
+  // the line up to the first point: D(-1/2..3/2), E(-2..1), T(-1/2, 1/2), Q = (4/3) T^2, U(-1), U(0)
+  double qp = __ldg(q + c + 2 * S);
+  const double qm3 = __ldg(q + c - 3 * S), qm2 = __ldg(q + c - 2 * S), qm1 = __ldg(q + c - S), q0 = __ldg(q + c),
+               q1 = __ldg(q + c + S);
+  double dm = q0 - qm1, dp = q1 - q0, dn = qp - q1;
+  double e0, e1, e2, e3, Q0, Q1, Q2, u0, u1, tn;
+  {
+    const double d5 = qm2 - qm3, d3 = qm1 - qm2;
+    e0 = d3 - d5;
+    e1 = dm - d3;
+    e2 = dp - dm;
+    e3 = dn - dp;
+    const double ta = e1 - e0, tb = e2 - e1;
+    tn = e3 - e2;
+    Q0 = (ta * c43) * ta;
+    Q1 = (tb * c43) * tb;
+    Q2 = (tn * c43) * tn;
+    u0 = tb - ta;
+    u1 = tn - tb;
+  }
+  double pm = __ldg(a + c - S) + __ldg(a + c - S + Sq);
+  double qn = __ldg(q + c + 3 * S), an = __ldg(a + c), as = __ldg(a + c + Sq);
 #pragma unroll 1
-  for (int lev = 0; lev < nlev; ++lev) {
-    if (lev == 1 && keep && *keep) break;
-    const double* U = lev ? uo : u;
-    const double* V = lev ? vo : v;
-    const double* W = lev ? wo : w;
-    const double u0 = __ldg(U + c), uxm = __ldg(U + c - X), uxp = __ldg(U + c + X);
-    const double v0 = __ldg(V + c), vym = __ldg(V + c - Y), vyp = __ldg(V + c + Y);
-    const double w0 = __ldg(W + c), wzm = __ldg(W + c - Z), wzp = __ldg(W + c + Z);
-    double a;
-    // u (cal_advu_weno5.f:80-120); each vsum is 4 times the reference's vel
-    a = wdir(U, c, X, (uxm + u0) + (u0 + uxp), kx);
-    a += wdir(U, c, Y, (vym + __ldg(V + c + X - Y)) + (v0 + __ldg(V + c + X)), ky);
-    a += wdir(U, c, Z, (wzm + __ldg(W + c + X - Z)) + (w0 + __ldg(W + c + X)), kz);
-    (lev ? auo : au)[c] = a;
-    // v (:147-187)
-    a = wdir(V, c, X, (uxm + __ldg(U + c - X + Y)) + (u0 + __ldg(U + c + Y)), kx);
-    a += wdir(V, c, Y, (vym + v0) + (v0 + vyp), ky);
-    a += wdir(V, c, Z, (wzm + __ldg(W + c + Y - Z)) + (w0 + __ldg(W + c + Y)), kz);
-    (lev ? avo : av)[c] = a;
-    // w (:214-254)
-    a = wdir(W, c, X, (uxm + __ldg(U + c - X + Z)) + (u0 + __ldg(U + c + Z)), kx);
-    a += wdir(W, c, Y, (vym + __ldg(V + c - Y + Z)) + (v0 + __ldg(V + c + Z)), ky);
-    a += wdir(W, c, Z, (wzm + w0) + (w0 + wzp), kz);
-    (lev ? awo : aw)[c] = a;
+  for (int k = m0; k < m1; ++k, c += S) {
+    // the window's leading terms: D(5/2), E(2), T(3/2), U(1)
+    const double df = qn - qp, e4 = df - dn, tf = e4 - e3, Q3 = (tf * c43) * tf, u2 = tf - tn;
+    const double pp = an + as, vsum = pm + pp;
+    qp = qn;
+    const double prev = DIR == 0 ? 0.0 : out[c];
+    if (k + 1 < m1) {
+      qn = __ldg(q + c + 4 * S);
+      an = __ldg(a + c + S);
+      as = __ldg(a + c + S + Sq);
+    }
+    // sign and zero of vsum from its bits (a double comparison takes an FP64-pipe slot)
+    const long long vb = __double_as_longlong(vsum);
+    const bool pos = vb >= 0;
+    const double E1 = pos ? e0 : e4, E2 = pos ? e1 : e3, E4 = pos ? e3 : e1, U1 = pos ? u0 : u2;
+    const double a1 = pos ? dm : -dp;
+    const double s1 = fma(E2, fma(E2, 2.0, -E1), pos ? Q0 : Q3), s2 = fma(E2, e2, pos ? Q1 : Q2),
+                 s3 = fma(e2, fma(e2, 2.0, -E4), pos ? Q2 : Q1);
+    const double x = s2 * s3, y = s1 * s3, z = s1 * s2;
+    const double X = x * x, Y = fma(y, y, 1.0e-80 / 124416.0), Z = z * z;
+    const double num = fma(Z, u1, X * (U1 * (2.0 / 3.0))), den = fma(X, 1.0 / 3.0, fma(Y, 2.0, Z));
+    const double d2 = fma(a1, 6.0, fma(e2, 2.0, E2));
+    const double f = fma(-num, recip_h(den), d2), vk = fabs(vsum) * kd;
+    const bool still = (vb << 1) == 0;
+    if (DIR == 0)
+      out[c] = still ? 0.0 : vk * f;
+    else
+      out[c] = still ? prev : fma(vk, f, prev);
+    pm = pp;
+    dm = dp;
+    dp = dn;
+    dn = df;
+    e0 = e1;
+    e1 = e2;
+    e2 = e3;
+    e3 = e4;
+    Q0 = Q1;
+    Q1 = Q2;
+    Q2 = Q3;
+    u0 = u1;
+    u1 = u2;
+    tn = tf;
   }
 }
 }  // namespace
@@ -339,9 +372,26 @@ static void weno5_levels(cudaStream_t s, const Grid& g, int nlev, double dxi, do
     set_status(FMF_ERR_ARG);
     return;
   }
-  k_weno2<<<gr, b, 0, s>>>(g, nlev, keep, dxi, dyi, dzi, u, v, w, uo, vo, wo, adv[0], adv[1], adv[2], ao[0], ao[1],
-                           ao[2]);
-  count_launch();
+  // Points per walk: the first point of a walk costs about 28 operations more, so as
+  // many as leave a warp for each of the 608 quarter SMs (768: three components' lines
+  // of a power-of-two grid come in steps), 32 at most.  One-warp blocks spread a small
+  // grid over all of them.  Measured, us: 32x32x16 m = 1 31, 2 25, 4 31; 64x32x32 m = 2
+  // 68, 4 62, 16 79; 128x64x64 m = 8 356, 32 344, 64 375; 512x256x256 m = 16 19690, 32
+  // 19320, 64 19150.
+  int m = 1;
+  while (m < 32 && g.cells() * 3 >= 2L * m * 768 * 32) m *= 2;
+  auto grid = [&](int nl, int nr, int nm) {
+    return dim3((unsigned)(((long)nl * nr + 31) / 32), (unsigned)((nm + m - 1) / m), 3);
+  };
+  for (int lev = 0; lev < nlev; ++lev) {
+    const double *U = lev ? uo : u, *V = lev ? vo : v, *W = lev ? wo : w;
+    double* const* o = lev ? ao : adv;
+    const int* kp = lev ? keep : nullptr;
+    k_weno_line<0><<<grid(g.nj, g.nk, g.ni), 32, 0, s>>>(g, m, kp, dxi * (1.0 / 24.0), U, V, W, o[0], o[1], o[2]);
+    k_weno_line<1><<<grid(g.ni, g.nk, g.nj), 32, 0, s>>>(g, m, kp, dyi * (1.0 / 24.0), U, V, W, o[0], o[1], o[2]);
+    k_weno_line<2><<<grid(g.ni, g.nj, g.nk), 32, 0, s>>>(g, m, kp, dzi * (1.0 / 24.0), U, V, W, o[0], o[1], o[2]);
+    count_launch(3);
+  }
 }
 
 void weno5_both(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, const double* u,

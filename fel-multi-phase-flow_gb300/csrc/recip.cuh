@@ -17,6 +17,17 @@ __device__ __forceinline__ double recip_nr(double x) {
   return fma(r, fma(-x, r, 1.0), r);
 }
 
+// 1/x by one third-order step, r <- r + r (e + e^2) with e = 1 - x r (the series
+// 1/(1 - e) = 1 + e + e^2 + ..., E. Schroeder, Math. Ann. 2 (1870) 317-365): the
+// approximate reciprocal's error 2^-23 cubes to 2^-69, so three FP64 operations
+// give what recip_nr's four do.  Inputs as recip_nr.
+__device__ __forceinline__ double recip_h(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
 // 1/sqrt(s): Newton-Raphson on f(y) = y^-2 - s, y <- y (3 - s y^2)/2, whose
 // relative error squares per step, seeded with the PTX approximate reciprocal
 // square root rsqrt.approx.ftz.f64; two steps reach FP64 rounding.  Seven FP64
