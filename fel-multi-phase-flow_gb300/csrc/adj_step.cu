@@ -510,11 +510,12 @@ int record_step(fmf_adj* a, bool graphs) {
     // :545-573 (the fused kernel where the grid tiles; csf_T differentiates the same
     // sequence of reference subroutines either way)
     if (csf_fused) {
+      double* const work[4] = {a->csfwork, a->csfwork + 3 * n, a->csfwork + 6 * n, a->csfwork + 9 * n};
       if (!carry)
         fused::csf_force(s, g, dxi, dyi, dzi, P.rhol, P.rhog, P.sigma, phi1, a->sfst[0], a->sfst[1], a->sfst[2],
-                         a->mixed);
+                         a->mixed, work);
       fused::csf_force(s, g, dxi, dyi, dzi, P.rhol, P.rhog, P.sigma, phn1, a->sfstn[0], a->sfstn[1], a->sfstn[2],
-                       a->mixed);
+                       a->mixed, work);
     } else {
       if (!carry) csf_fwd(a, phi1, a->sfst);
       csf_fwd(a, phn1, a->sfstn);

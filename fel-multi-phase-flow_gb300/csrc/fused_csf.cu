@@ -11,20 +11,21 @@
 //   n23 at (i,j+1/2,k+1/2) = N(mean over i-1/2, i+1/2),
 // N(v) = v/(|v| + 1e-30*|dxinv|) and vertex gradients from cal_grad_p2a.f:46-60.
 //
-// A block owns a 32 x 8 tile of (i,j) columns and marches over a chunk of k planes.
-// Vertex gradients G of planes k, k+1 and the normals of planes k-1..k+1 live in
-// shared memory; H(k+1) = G(k)+G(k+1) gives both n12(k+1) and, summed over the
-// four surrounding (i,j), npp(k+1).  Each normal is formed once per block.
+// FP64 (the FP64 step): three kernels over the whole grid, k_csf_grad (the vertex
+// gradients G), k_csf_normals (the four families) and k_csf_force, with G and the nine
+// normal components used in device memory (12 n doubles of workspace).
 //
-// Three instantiations: R = double (the FP64 step; phi read straight from global
-// memory), R = float (the mixed-precision step; each phi plane is converted once
-// into a shared-memory ring of three planes, everything after that is FP32 and the
-// three forces are widened to double on the store) and R = Pr, an FP32 pair (the
-// FP64-accurate step FMF_FP64E: phi planes split into pairs in the same ring, the
-// arithmetic in FP32-pair operations on the FP32 pipe, the forces rounded to double).
+// FP32 (R = float, the mixed-precision step) and FP32 pairs (R = Pr, the FP64-accurate
+// step FMF_FP64E): one kernel, k_csf.  A block owns a 32 x 8 tile of (i,j) columns and
+// marches over a chunk of k planes; each phi plane is converted once into a
+// shared-memory ring of three planes.  Vertex gradients G of planes k, k+1 and the
+// normals of planes k-1..k+1 live in shared memory; H(k+1) = G(k)+G(k+1) gives both
+// n12(k+1) and, summed over the four surrounding (i,j), npp(k+1).  Each normal is
+// formed once per block, and the forces are widened or rounded to double on the store.
 #include <algorithm>
 #include <type_traits>
 
+#include "../../include/fmf_capi.h"
 #include "df64.cuh"
 #include "fused.cuh"
 #include "recip.cuh"
@@ -54,9 +55,6 @@ __host__ __device__ __forceinline__ Pr operator*(Pr a, Pr b) { return df::mul(a.
 __host__ __device__ __forceinline__ Pr operator-(Pr a) { return df::neg(a.v); }
 
 template <class R>
-constexpr bool kStaged = !std::is_same<R, double>::value;
-
-template <class R>
 struct CsfP {
   R dxi, dyi, dzi, gx, gy, gz, vs2, vs8;  // vs2 = 2 vs, vs8 = 8 vs
   R fx, fy, fz;                           // -(2 sigma/(rho_l + rho_g)) dxinv etc. (calfst.f:40-42)
@@ -70,23 +68,11 @@ struct Smem {
   R a12[2][2][NP];  // n12 (x, y), planes k and k+1; region i in [I0-1, I0+TX-1], j in [J0-1, J0+TY-1]
   R a13[2][2][NP];  // n13 (x, z), planes k-1 and k; same region
   R a23[2][2][NP];  // n23 (y, z), planes k-1 and k; same region
-  R Q[kStaged<R> ? 3 : 1][kStaged<R> ? QP : 1];  // staged phi planes, slot = plane % 3
+  R Q[3][QP];       // staged phi planes, slot = plane % 3
 };
 
-// N(v) = v/(|v| + vs).  Where |v| exceeds vs by more than 1e12 the relative
-// correction vs/|v| is below 1e-12 and 1/|v| is used; smaller |v| (including zero
-// gradients) takes the exact expression.  Callers pass v scaled by 1/c (a sum
-// instead of a mean) with vs scaled by 1/c: N(c w) = w/(|w| + vs/c).
-__device__ __forceinline__ void unit(double x, double y, double z, double vs, double* o) {
-  const double s = x * x + y * y + z * z;
-  const double big = vs * 1.0e12;
-  // s > big^2 compared on the bit patterns (both non-negative; no FP64-pipe compare)
-  const bool far = __double_as_longlong(s) > __double_as_longlong(big * big);
-  const double inv = far ? rsqrt_nr(s) : 1.0 / (sqrt(s) + vs);
-  o[0] = x * inv;
-  o[1] = y * inv;
-  o[2] = z * inv;
-}
+// N(v) = v/(|v| + vs).  Callers pass v scaled by 1/c (a sum instead of a mean) with
+// vs scaled by 1/c: N(c w) = w/(|w| + vs/c).
 // FP32: where |v| < 1e-15 the squares would leave the normal range, so numerator
 // and denominator are both scaled by 2^64 first (an exact power-of-two scaling).
 __device__ __forceinline__ void unit(float x, float y, float z, float vs, float* o) {
@@ -133,29 +119,8 @@ __device__ __forceinline__ void unit(Pr x, Pr y, Pr z, Pr vs, Pr* o) {
   o[2] = mul(Z, inv);
 }
 
-// vertex gradient at (i+1/2, j+1/2, k+1/2), straight from phi in global memory
-__device__ void grad_plane(const Grid& g, const CsfP<double>& p, const double* __restrict__ phi, int I0, int J0,
-                           int k, double (*G)[GP]) {
-  const long X = 1, Y = g.sy, Z = g.sz;
-  for (int e = threadIdx.x; e < GP; e += blockDim.x) {
-    const int a = e % GX, b = e / GX;
-    const int i = I0 - 1 + a, j = J0 - 1 + b;
-    const long c = g.at(i, j, k);
-    const double q000 = __ldg(phi + c), qp00 = __ldg(phi + c + X), q0p0 = __ldg(phi + c + Y),
-                 qpp0 = __ldg(phi + c + X + Y), q00p = __ldg(phi + c + Z), qp0p = __ldg(phi + c + X + Z),
-                 q0pp = __ldg(phi + c + Y + Z), qppp = __ldg(phi + c + X + Y + Z);
-    // per (i, j) corner the sum and the difference of the two k planes; with
-    // ta = s(+,+) - s(0,0) and tb = s(+,0) - s(0,+), the x sum is ta + tb, the y sum ta - tb
-    // and the z sum the four differences (18 operations instead of 24)
-    const double s00 = q000 + q00p, sp0 = qp00 + qp0p, s0p = q0p0 + q0pp, spp = qpp0 + qppp;
-    const double d00 = q00p - q000, dp0 = qp0p - qp00, d0p = q0pp - q0p0, dpp = qppp - qpp0;
-    const double ta = spp - s00, tb = sp0 - s0p;
-    G[0][e] = (ta + tb) * p.gx;
-    G[1][e] = (ta - tb) * p.gy;
-    G[2][e] = ((d00 + dp0) + (d0p + dpp)) * p.gz;
-  }
-}
-// the same from two staged planes (Qa = plane k, Qb = plane k+1)
+// vertex gradient at (i+1/2, j+1/2, k+1/2) from two staged planes (Qa = plane k, Qb =
+// plane k+1)
 template <class R>
 __device__ void grad_staged(const CsfP<R>& p, const R* Qa, const R* Qb, R (*G)[GP]) {
   for (int e = threadIdx.x; e < GP; e += blockDim.x) {
@@ -239,8 +204,7 @@ __device__ void centre_normals(const CsfP<R>& p, Smem<R>& S, int gk, int gk1, in
 template <class R>
 __global__ void __launch_bounds__(256) k_csf(Grid g, CsfP<R> p, int kchunk, const double* __restrict__ phi,
                                              double* __restrict__ fu, double* __restrict__ fv,
-                                             double* __restrict__ fw, double* __restrict__ kap,
-                                             const int* __restrict__ skip) {
+                                             double* __restrict__ fw, const int* __restrict__ skip) {
   if (skip && *skip) return;  // the whole block leaves before any barrier
   extern __shared__ double smraw[];
   Smem<R>& S = *reinterpret_cast<Smem<R>*>(smraw);
@@ -250,15 +214,10 @@ __global__ void __launch_bounds__(256) k_csf(Grid g, CsfP<R> p, int kchunk, cons
   int sp = 0;          // pp/n12 slot of plane k
   int sm = 0;          // n13/n23 slot of plane k-1
   // warm-up: G(kb-1) -> gB, G(kb) -> gA; n13/n23(kb-1) from gB; npp/n12(kb) from both
-  if constexpr (kStaged<R>) {
-    for (int q = kb - 1; q <= kb + 1; ++q) stage_plane(g, phi, I0, J0, q, S.Q[q % 3]);
-    __syncthreads();
-    grad_staged(p, S.Q[(kb - 1) % 3], S.Q[kb % 3], S.G[gB]);
-    grad_staged(p, S.Q[kb % 3], S.Q[(kb + 1) % 3], S.G[gA]);
-  } else {
-    grad_plane(g, p, phi, I0, J0, kb - 1, S.G[gB]);
-    grad_plane(g, p, phi, I0, J0, kb, S.G[gA]);
-  }
+  for (int q = kb - 1; q <= kb + 1; ++q) stage_plane(g, phi, I0, J0, q, S.Q[q % 3]);
+  __syncthreads();
+  grad_staged(p, S.Q[(kb - 1) % 3], S.Q[kb % 3], S.G[gB]);
+  grad_staged(p, S.Q[kb % 3], S.Q[(kb + 1) % 3], S.G[gA]);
   __syncthreads();
   side_normals(p, S, gB, sm);
   centre_normals(p, S, gB, gA, sp);
@@ -267,13 +226,9 @@ __global__ void __launch_bounds__(256) k_csf(Grid g, CsfP<R> p, int kchunk, cons
   const int i = I0 + tx, j = J0 + ty;
   for (int k = kb; k <= ke; ++k) {
     // G(k+1) -> gB; n13/n23(k) from gA; npp/n12(k+1)
-    if constexpr (kStaged<R>) {
-      stage_plane(g, phi, I0, J0, k + 2, S.Q[(k + 2) % 3]);  // the slot of plane k-1, unused from here on
-      __syncthreads();
-      grad_staged(p, S.Q[(k + 1) % 3], S.Q[(k + 2) % 3], S.G[gB]);
-    } else {
-      grad_plane(g, p, phi, I0, J0, k + 1, S.G[gB]);
-    }
+    stage_plane(g, phi, I0, J0, k + 2, S.Q[(k + 2) % 3]);  // the slot of plane k-1, unused from here on
+    __syncthreads();
+    grad_staged(p, S.Q[(k + 1) % 3], S.Q[(k + 2) % 3], S.G[gB]);
     __syncthreads();
     side_normals(p, S, gA, sm ^ 1);
     centre_normals(p, S, gA, gB, sp ^ 1);
@@ -288,28 +243,12 @@ __global__ void __launch_bounds__(256) k_csf(Grid g, CsfP<R> p, int kchunk, cons
                    (S.a23[sm ^ 1][1][f] - S.a23[sm][1][f]) * p.dzi;
       const R kw = (S.a13[sm ^ 1][0][f] - S.a13[sm ^ 1][0][f - 1]) * p.dxi +
                    (S.a23[sm ^ 1][0][f] - S.a23[sm ^ 1][0][f - NX]) * p.dyi + (S.pp[sp ^ 1][2][e] - S.pp[sp][2][e]) * p.dzi;
-      R ph, px, py, pz;
-      if constexpr (kStaged<R>) {
-        const int cq = (ty + 1) * QX + tx + 1;
-        const R* Qk = S.Q[k % 3];
-        ph = Qk[cq];
-        px = Qk[cq + 1];
-        py = Qk[cq + QX];
-        pz = S.Q[(k + 1) % 3][cq];
-      } else {
-        ph = __ldg(phi + c);
-        px = __ldg(phi + c + 1);
-        py = __ldg(phi + c + g.sy);
-        pz = __ldg(phi + c + g.sz);
-      }
+      const int cq = (ty + 1) * QX + tx + 1;
+      const R* Qk = S.Q[k % 3];
+      const R ph = Qk[cq], px = Qk[cq + 1], py = Qk[cq + QX], pz = S.Q[(k + 1) % 3][cq];
       fu[c] = (double)(ku * (px - ph) * p.fx);
       fv[c] = (double)(kv * (py - ph) * p.fy);
       fw[c] = (double)(kw * (pz - ph) * p.fz);
-      if (kap) {  // the curvatures at the u, v, w points, kept for the adjoint
-        kap[c] = (double)ku;
-        kap[c + g.n] = (double)kv;
-        kap[c + 2 * g.n] = (double)kw;
-      }
     }
     __syncthreads();
     gA ^= 1;
@@ -354,7 +293,7 @@ int csf_chunk(const Grid& g, const void* fn, size_t smem) {
 
 template <class R>
 void launch_csf(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double rhol, double rhog,
-                double sigma, const double* phi, double* fu, double* fv, double* fw, double* kap, const int* skip) {
+                double sigma, const double* phi, double* fu, double* fv, double* fw, const int* skip) {
   CsfP<R> p;
   p.dxi = (R)dxinv;
   p.dyi = (R)dyinv;
@@ -373,22 +312,248 @@ void launch_csf(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doubl
   cudaFuncSetAttribute(k_csf<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const int kchunk = csf_chunk(g, (const void*)k_csf<R>, smem);
   dim3 gr((unsigned)(g.ni / TX), (unsigned)(g.nj / TY), (unsigned)((g.nk + kchunk - 1) / kchunk));
-  k_csf<R><<<gr, 256, smem, s>>>(g, p, kchunk, phi, fu, fv, fw, kap, skip);
+  k_csf<R><<<gr, 256, smem, s>>>(g, p, kchunk, phi, fu, fv, fw, skip);
   count_launch();
+}
+
+// ---- FP64 ------------------------------------------------------------------------
+// Bound by the FP64 pipe (64 cycles per warp instruction and quarter SM), so the three
+// kernels trade device memory for operations: each vertex gradient and each normal is
+// formed once (one tiled kernel formed 1.4 and 1.25 of each, with five barriers per
+// plane), the sums the families share are formed once, and warps whose points all lie
+// where phi is constant store the zeros that the arithmetic would give without doing
+// it: away from the interface phi is exactly 0 or 1 (solphi_mthinc3's snap).  At
+// 512x256x256 (sessile drop) 11.9 -> 1.2 ms, at 256x128x128 1.59 -> 0.30, at 128x64x256
+// with a profile that varies nearly everywhere 0.92 -> 0.33, at 32x32x16 0.068 -> 0.017.
+struct CsfD {
+  double gx, gy, gz;      // 0.25 dxinv ...
+  double dxi, dyi, dzi;
+  double vs2, vs8;        // 2 vs, 8 vs
+  double big2, big8;      // (1e12 vs2)^2, (1e12 vs8)^2
+  double fx, fy, fz;      // -(2 sigma/(rho_l + rho_g)) dxinv etc. (calfst.f:40-42)
+};
+__device__ __forceinline__ unsigned long long mag(double x) {  // 0 for +-0 only
+  return (unsigned long long)__double_as_longlong(x) << 1;
+}
+// 1/(sqrt(s) + vs) for s = |v|^2.  Where |v| exceeds vs by more than 1e12 the relative
+// correction vs/|v| is below 1e-12 and 1/|v| is used (the comparisons are on the bit
+// patterns: all are non-negative); s = 0 gives 0 (the components it multiplies are 0 or
+// their squares underflowed), other small s the exact expression.
+__device__ __forceinline__ double inv_norm(double s, double vs, double big) {
+  if (__double_as_longlong(s) > __double_as_longlong(big)) return rsqrt_h(s);
+  return mag(s) == 0 ? 0.0 : 1.0 / (sqrt(s) + vs);
+}
+
+// G at (i+1/2, j+1/2, k+1/2) for i, j, k in -1..n+1 into G[0..2] (n apart); threads
+// over the flattened (i, j) plane so that every warp is full
+__global__ void __launch_bounds__(128) k_csf_grad(Grid g, CsfD p, const double* __restrict__ phi,
+                                                  double* __restrict__ G, const int* __restrict__ skip) {
+  if (skip && *skip) return;
+  const int W = g.ni + 3;
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= W * (g.nj + 3)) return;
+  const int b = t / W, a = t - b * W;
+  const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
+  const long c = g.at(a - 1, b - 1, (int)blockIdx.y - 1);
+  const double q000 = __ldg(phi + c), qp00 = __ldg(phi + c + X), q0p0 = __ldg(phi + c + Y),
+               qpp0 = __ldg(phi + c + X + Y), q00p = __ldg(phi + c + Z), qp0p = __ldg(phi + c + X + Z),
+               q0pp = __ldg(phi + c + Y + Z), qppp = __ldg(phi + c + X + Y + Z);
+  // all eight equal in every bit and finite: the gradient is 0
+  const long long r = __double_as_longlong(q000);
+  auto df = [&](double x) { return (unsigned long long)(__double_as_longlong(x) ^ r); };
+  const bool varies = (df(qp00) | df(q0p0) | df(qpp0) | df(q00p) | df(qp0p) | df(q0pp) | df(qppp)) != 0 ||
+                      ((r >> 52) & 0x7ff) == 0x7ff;
+  if (!__any_sync(__activemask(), varies)) {
+    G[c] = 0.0;
+    G[c + n] = 0.0;
+    G[c + 2 * n] = 0.0;
+    return;
+  }
+  // per (i, j) corner the sum and the difference of the two k planes; with
+  // ta = s(+,+) - s(0,0) and tb = s(+,0) - s(0,+), the x sum is ta + tb, the y sum ta - tb
+  // and the z sum the four differences (18 operations instead of 24)
+  const double s00 = q000 + q00p, sp0 = qp00 + qp0p, s0p = q0p0 + q0pp, spp = qpp0 + qppp;
+  const double d00 = q00p - q000, dp0 = qp0p - qp00, d0p = q0pp - q0p0, dpp = qppp - qpp0;
+  const double ta = spp - s00, tb = sp0 - s0p;
+  G[c] = (ta + tb) * p.gx;
+  G[c + n] = (ta - tb) * p.gy;
+  G[c + 2 * n] = ((d00 + dp0) + (d0p + dpp)) * p.gz;
+}
+
+// The normals at i, j, k in 0..n+1 from G, arrays n apart: npp in pp; n12 (x, y) and the
+// x of n13 in n12; the z of n13 and n23 (y, z) in nside.  A thread walks m planes of its (i, j)
+// column: P, the sum of G over the four vertices around the column, and G itself are
+// kept from plane to plane, so the means take 18 additions per point.
+__global__ void __launch_bounds__(128) k_csf_normals(Grid g, CsfD p, int m, const double* __restrict__ G,
+                                                     double* __restrict__ pp, double* __restrict__ n12,
+                                                     double* __restrict__ nside, const int* __restrict__ skip) {
+  if (skip && *skip) return;
+  const int W = g.ni + 2;
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= W * (g.nj + 2)) return;
+  const int b = t / W, a = t - b * W;
+  const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
+  const int k0 = (int)blockIdx.y * m, k1 = min(g.nk + 2, k0 + m);
+  long c = g.at(a, b, k0 - 1);  // the plane below the first
+  double g0[3], P0[3];
+  unsigned long long any0 = 0;
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const double* Gq = G + q * n + c;
+    const double gc = __ldg(Gq), gx = __ldg(Gq - X), gy = __ldg(Gq - Y), gxy = __ldg(Gq - X - Y);
+    any0 |= mag(gc) | mag(gx) | mag(gy) | mag(gxy);
+    g0[q] = gc;
+    P0[q] = (gx + gc) + (gxy + gy);
+  }
+  c += Z;
+#pragma unroll 1
+  for (int k = k0; k < k1; ++k, c += Z) {
+    double gc[3], gx[3], gy[3], gxy[3];
+    unsigned long long any1 = 0;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double* Gq = G + q * n + c;
+      gc[q] = __ldg(Gq);
+      gx[q] = __ldg(Gq - X);
+      gy[q] = __ldg(Gq - Y);
+      gxy[q] = __ldg(Gq - X - Y);
+      any1 |= mag(gc[q]) | mag(gx[q]) | mag(gy[q]) | mag(gxy[q]);
+    }
+    if (!__any_sync(__activemask(), (any0 | any1) != 0)) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        pp[c + q * n] = 0.0;
+        n12[c + q * n] = 0.0;
+        nside[c + q * n] = 0.0;
+        g0[q] = 0.0;
+        P0[q] = 0.0;
+      }
+      any0 = 0;
+      continue;
+    }
+    double sx[3], sy[3], P[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      sx[q] = gx[q] + gc[q];
+      sy[q] = gy[q] + gc[q];
+      P[q] = sx[q] + (gxy[q] + gy[q]);
+    }
+    auto norm = [&](double x, double y, double z, double vs, double big) {
+      return inv_norm(fma(z, z, fma(y, y, x * x)), vs, big);
+    };
+    {  // npp: the 8 vertices around the cell, with 8 vs
+      const double x = P0[0] + P[0], y = P0[1] + P[1], z = P0[2] + P[2], r = norm(x, y, z, p.vs8, p.big8);
+      pp[c] = x * r;
+      pp[c + n] = y * r;
+      pp[c + 2 * n] = z * r;
+    }
+    {  // n12: G of this plane and the one below
+      const double x = g0[0] + gc[0], y = g0[1] + gc[1], z = g0[2] + gc[2], r = norm(x, y, z, p.vs2, p.big2);
+      n12[c] = x * r;
+      n12[c + n] = y * r;
+    }
+    {  // n13: G(j-1) and G(j)
+      const double r = norm(sy[0], sy[1], sy[2], p.vs2, p.big2);
+      n12[c + 2 * n] = sy[0] * r;
+      nside[c] = sy[2] * r;
+    }
+    {  // n23: G(i-1) and G(i)
+      const double r = norm(sx[0], sx[1], sx[2], p.vs2, p.big2);
+      nside[c + n] = sx[1] * r;
+      nside[c + 2 * n] = sx[2] * r;
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      g0[q] = gc[q];
+      P0[q] = P[q];
+    }
+    any0 = any1;
+  }
+}
+
+// the curvatures (calrkap.f:45-98) and the force on the interior u, v, w points; where
+// phi does not differ from its three upper neighbours the force is 0
+__global__ void __launch_bounds__(256) k_csf_force(Grid g, CsfD p, const double* __restrict__ phi,
+                                                   const double* __restrict__ pp, const double* __restrict__ n12,
+                                                   const double* __restrict__ nside, double* __restrict__ fu,
+                                                   double* __restrict__ fv, double* __restrict__ fw,
+                                                   const int* __restrict__ skip) {
+  if (skip && *skip) return;
+  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
+  if (i > g.ni || j > g.nj) return;
+  const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
+  const long c = g.at(i, j, 1 + (int)blockIdx.z);
+  const double ph = __ldg(phi + c), px = __ldg(phi + c + X), py = __ldg(phi + c + Y), pz = __ldg(phi + c + Z);
+  const long long r = __double_as_longlong(ph);
+  const bool varies = ((__double_as_longlong(px) ^ r) | (__double_as_longlong(py) ^ r) |
+                       (__double_as_longlong(pz) ^ r)) != 0 || ((r >> 52) & 0x7ff) == 0x7ff;
+  if (!__any_sync(__activemask(), varies)) {
+    fu[c] = 0.0;
+    fv[c] = 0.0;
+    fw[c] = 0.0;
+    return;
+  }
+  const double *ax = n12, *ay = n12 + n, *bx = n12 + 2 * n, *bz = nside, *ey = nside + n, *ez = nside + 2 * n;
+  const double ku = (__ldg(pp + c + X) - __ldg(pp + c)) * p.dxi + (__ldg(ay + c) - __ldg(ay + c - Y)) * p.dyi +
+                    (__ldg(bz + c) - __ldg(bz + c - Z)) * p.dzi;
+  const double kv = (__ldg(ax + c) - __ldg(ax + c - X)) * p.dxi + (__ldg(pp + n + c + Y) - __ldg(pp + n + c)) * p.dyi +
+                    (__ldg(ez + c) - __ldg(ez + c - Z)) * p.dzi;
+  const double kw = (__ldg(bx + c) - __ldg(bx + c - X)) * p.dxi + (__ldg(ey + c) - __ldg(ey + c - Y)) * p.dyi +
+                    (__ldg(pp + 2 * n + c + Z) - __ldg(pp + 2 * n + c)) * p.dzi;
+  fu[c] = ku * (px - ph) * p.fx;
+  fv[c] = kv * (py - ph) * p.fy;
+  fw[c] = kw * (pz - ph) * p.fz;
+}
+
+void csf_fp64(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double rhol, double rhog,
+              double sigma, const double* phi, double* fu, double* fv, double* fw, double* const* work,
+              const int* skip) {
+  CsfD p;
+  p.dxi = dxinv;
+  p.dyi = dyinv;
+  p.dzi = dzinv;
+  p.gx = 0.25 * dxinv;
+  p.gy = 0.25 * dyinv;
+  p.gz = 0.25 * dzinv;
+  const double vs = std::sqrt(dxinv * dxinv + dyinv * dyinv + dzinv * dzinv) * 1.0e-30;
+  p.vs2 = 2.0 * vs;
+  p.vs8 = 8.0 * vs;
+  p.big2 = p.vs2 * 1.0e12 * (p.vs2 * 1.0e12);
+  p.big8 = p.vs8 * 1.0e12 * (p.vs8 * 1.0e12);
+  const double st = 2.0 * sigma / (rhol + rhog);
+  p.fx = -st * dxinv;
+  p.fy = -st * dyinv;
+  p.fz = -st * dzinv;
+  double *G = work[0], *pp = work[1], *n12 = work[2], *nside = work[3];
+  k_csf_grad<<<dim3((unsigned)(((long)(g.ni + 3) * (g.nj + 3) + 127) / 128), (unsigned)(g.nk + 3)), 128, 0, s>>>(
+      g, p, phi, G, skip);
+  // planes per walk: the first costs 9 additions more; as many as leave a warp for each
+  // of the 608 quarter SMs, 8 at most
+  const long cols = (long)(g.ni + 2) * (g.nj + 2);
+  int m = 1;
+  while (m < 8 && cols * (g.nk + 2) >= 2L * m * 768 * 32) m *= 2;
+  k_csf_normals<<<dim3((unsigned)((cols + 127) / 128), (unsigned)((g.nk + 2 + m - 1) / m)), 128, 0, s>>>(
+      g, p, m, G, pp, n12, nside, skip);
+  k_csf_force<<<dim3((unsigned)(g.ni / TX), (unsigned)(g.nj / TY), (unsigned)g.nk), dim3(TX, TY), 0, s>>>(
+      g, p, phi, pp, n12, nside, fu, fv, fw, skip);
+  count_launch(3);
 }
 }  // namespace
 
 bool csf_supported(const Grid& g) { return g.ni % TX == 0 && g.nj % TY == 0; }
 
 void csf_force(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double rhol, double rhog,
-               double sigma, const double* phi, double* fu, double* fv, double* fw, int prec, double* kap,
+               double sigma, const double* phi, double* fu, double* fv, double* fw, int prec, double* const* work,
                const int* skip) {
   if (prec == 1)
-    launch_csf<float>(s, g, dxinv, dyinv, dzinv, rhol, rhog, sigma, phi, fu, fv, fw, kap, skip);
+    launch_csf<float>(s, g, dxinv, dyinv, dzinv, rhol, rhog, sigma, phi, fu, fv, fw, skip);
   else if (prec == 2)
-    launch_csf<Pr>(s, g, dxinv, dyinv, dzinv, rhol, rhog, sigma, phi, fu, fv, fw, kap, skip);
+    launch_csf<Pr>(s, g, dxinv, dyinv, dzinv, rhol, rhog, sigma, phi, fu, fv, fw, skip);
+  else if (!work)
+    set_status(FMF_ERR_ARG);
   else
-    launch_csf<double>(s, g, dxinv, dyinv, dzinv, rhol, rhog, sigma, phi, fu, fv, fw, kap, skip);
+    csf_fp64(s, g, dxinv, dyinv, dzinv, rhol, rhog, sigma, phi, fu, fv, fw, work, skip);
 }
 
 }  // namespace fused

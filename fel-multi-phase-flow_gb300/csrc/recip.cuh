@@ -42,4 +42,14 @@ __device__ __forceinline__ double rsqrt_nr(double s) {
   return y;
 }
 
+// 1/sqrt(s) by one third-order step from the same seed y (relative error 2^-22):
+// with e = 1 - s y^2, 1/sqrt(s) = y (1 - e)^(-1/2) = y (1 + e/2 + 3/8 e^2 + ...), whose
+// next term is below 2^-63.  Five FP64 operations.  Inputs as rsqrt_nr.
+__device__ __forceinline__ double rsqrt_h(double s) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+  const double e = fma(-(s * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
 }  // namespace fmf
