@@ -481,23 +481,22 @@ int record_step(fmf_adj* a, bool graphs) {
       fused::mthinc_fluxes(s, g, dxi, dyi, dzi, dt, P.bet_mthinc, phi1, a->gx1[0], a->gx1[1], a->gx1[2], S[SU],
                            S[SV], S[SW], a->fl[0], a->fl[1], a->fl[2], a->band, a->band + nb, a->mixed, a->newton);
     }
-    op::solphi_mthinc2(s, g, dxi, dyi, dzi, dt, S[SU], S[SV], S[SW], a->fl[0], a->fl[1], a->fl[2], phi1, phn1);
+    fused::mthinc_advance(s, g, dxi, dyi, dzi, dt, S[SU], S[SV], S[SW], a->fl[0], a->fl[1], a->fl[2], phi1, phn1);
     dcopy(a, phn1, a->pa, n);
-    fused::vertex_gradient(s, g, dxi, dyi, dzi, phn1, a->gxn[0], a->gxn[1], a->gxn[2]);
+    fused::vertex_gradient(s, g, dxi, dyi, dzi, phn1, a->gxn[0], a->gxn[1], a->gxn[2], true);
     adj::mthinc3_record(s, g, dxi, dyi, dzi, P.bet_mthinc, a->gxn[0], a->gxn[1], a->gxn[2], a->pa, a->pb, a->pass);
-    op::solphi_mthinc3(s, g, dxi, dyi, dzi, P.bet_mthinc, a->gxn[0], a->gxn[1], a->gxn[2], phi1, phn1, a->sums);
+    fused::mthinc_volume_fix(s, g, dxi, dyi, dzi, P.bet_mthinc, a->gxn[0], a->gxn[1], a->gxn[2], phi1, phn1, phn0,
+                             a->sums);
     dcopy(a, phn1, a->pc, n);
     op::gnbc(s, g, S[SU], S[SW], P.uwall, a->theta0, P.sigma, a->zeta, a->theta);
     op::bnd_contact_angle(s, g, phn1, a->theta, P.dx, P.dy, P.dz);
-    op::bnd_periodic(s, g, phn1);
+    fused::halo_periodic(s, g, phn1);
     dcopy(a, phn1, a->phn1f, n);
-    // :509-517
-    op::summation(s, g, phn0, phn1);
-    op::bnd_neumann(s, g, phn0);
+    // :510-517 (:509 with the volume fix)
     op::bnd_contact_angle(s, g, phi0, a->theta, P.dx, P.dy, P.dz);
-    op::bnd_periodic(s, g, phn0);
+    fused::halo_neumann_periodic(s, g, phn0);
     // :526-541
-    op::mixture_means(s, g, phi0, phn0, P.rhol, P.rhog, P.rmul, P.rmug, a->rho, a->rhon, a->rmu, a->rmun);
+    fused::mixture_means(s, g, phi0, phn0, P.rhol, P.rhog, P.rmul, P.rmug, a->rho, a->rhon, a->rmu, a->rmun);
     if (carry)
       fused::weno5_one(s, g, dxi, dyi, dzi, S[SU], S[SV], S[SW], a->adv, a->mixed, a->wsplit);
     else
@@ -586,14 +585,12 @@ int record_step(fmf_adj* a, bool graphs) {
     op::caldiv(s, g, dxi, dyi, dzi, dt, a->un[0], a->un[1], a->un[2], a->div, nullptr);
     fused::pressure_half(s, g, P.rhog, dxi, dzi, a->as_f, a->an_f, a->ap_f, a->div, a->pr, a->pi, a->dp, a->tdma);
     op::bnd_avzero(s, g, a->dp);
-    op::bnd_neumann(s, g, a->dp);
-    op::bnd_periodic(s, g, a->dp);
+    fused::halo_neumann_periodic(s, g, a->dp);
     fused::project(s, g, P.rhog, dxi, dyi, dzi, dt, a->dp, a->phat, a->un[0], a->un[1], a->un[2], a->pn);
     for (int q = 0; q < 3; ++q) dcopy(a, a->un[q], a->un2[q], n);
     fused::wall_halo(s, g, 7, P.uwall, a->wallc, a->un[0], a->un[1], a->un[2]);
     op::bnd_avzero(s, g, a->pn);
-    op::bnd_neumann(s, g, a->pn);
-    op::bnd_periodic(s, g, a->pn);
+    fused::halo_neumann_periodic(s, g, a->pn);
     // :686-697 rotation (copies: the record keeps the step's inputs in the arrays above)
     for (int q = 0; q < 3; ++q) {
       dcopy(a, S[SU + q], S[SUO + q], n);

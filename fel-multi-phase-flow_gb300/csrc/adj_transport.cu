@@ -401,7 +401,7 @@ void phin_stale_T(cudaStream_t s, const Grid& g, const double* pass, double* lph
   });
 }
 
-// sums[0..2] = (sum phi, sum pb, sum pb^2 (1-pb)) as left by op::solphi_mthinc3;
+// sums[0..2] = (sum phi, sum pb, sum pb^2 (1-pb)) as left by fused::mthinc_volume_fix;
 // scal: device scratch of >= 4 doubles
 void mthinc3_T(cudaStream_t s, const Grid& g, const double* pb, const double* pass, const double* sums,
                double* lphin, double* lphi, double* scal) {

@@ -27,9 +27,29 @@ void weno5_keep(cudaStream_t s, const Grid& g, double dxi, double dyi, double dz
                 double* const* advo, const int* keep, int prec = 0, float2* split = nullptr);
 
 // cal_grad_p2a (the vertex gradients of q at (i+1/2, j+1/2, k+1/2), i, j, k in
-// -2..n+2) in fewer FP64 operations than the reference's order
+// -2..n+2) in fewer FP64 operations than the reference's order.  near1: values within
+// 64 units in the last place below 1 count as 1 (for the band test of the volume fix)
 void vertex_gradient(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const double* q,
-                     double* qx, double* qy, double* qz);
+                     double* qx, double* qy, double* qz, bool near1 = false);
+// solphi_mthinc2 on the interior
+void mthinc_advance(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt,
+                    const double* u, const double* v, const double* w, const double* fx, const double* fy,
+                    const double* fz, const double* phi, double* phin);
+// the snap and clip of solphi_mthinc3 (:61-120) of phin by its vertex gradients
+void mthinc_snap(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double bet,
+                 const double* gx, const double* gy, const double* gz, double* phin);
+// solphi_mthinc3 of phin from its vertex gradients gx, gy, gz; the interior of phin0 =
+// the result (summation for one bubble).  sums: 3 doubles, (sum phi, sum phin, sum
+// phin^2 (1 - phin)) after the snap.
+void mthinc_volume_fix(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double bet,
+                       const double* gx, const double* gy, const double* gz, const double* phi, double* phin,
+                       double* phin0, double* sums);
+// bnd_periodic; bnd_neumann followed by bnd_periodic
+void halo_periodic(cudaStream_t s, const Grid& g, double* q);
+void halo_neumann_periodic(cudaStream_t s, const Grid& g, double* q);
+// the four cal_arith_mean of main.f90:526-529
+void mixture_means(cudaStream_t s, const Grid& g, const double* phi0, const double* phin0, double rhol, double rhog,
+                   double rmul, double rmug, double* rho, double* rhon, double* rmu, double* rmun);
 
 // solphi_mthinc1 for the faces solphi_mthinc2 reads (every face of rows 1..n in
 // the two directions normal to it, faces 0..n along it); list/count: device scratch

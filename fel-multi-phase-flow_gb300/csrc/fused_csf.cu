@@ -26,6 +26,7 @@
 #include <type_traits>
 
 #include "../../include/fmf_capi.h"
+#include "bits.cuh"
 #include "df64.cuh"
 #include "fused.cuh"
 #include "recip.cuh"
@@ -332,9 +333,6 @@ struct CsfD {
   double big2, big8;      // (1e12 vs2)^2, (1e12 vs8)^2
   double fx, fy, fz;      // -(2 sigma/(rho_l + rho_g)) dxinv etc. (calfst.f:40-42)
 };
-__device__ __forceinline__ unsigned long long mag(double x) {  // 0 for +-0 only
-  return (unsigned long long)__double_as_longlong(x) << 1;
-}
 // 1/(sqrt(s) + vs) for s = |v|^2.  Where |v| exceeds vs by more than 1e12 the relative
 // correction vs/|v| is below 1e-12 and 1/|v| is used (the comparisons are on the bit
 // patterns: all are non-negative); s = 0 gives 0 (the components it multiplies are 0 or
@@ -362,7 +360,7 @@ __global__ void __launch_bounds__(128) k_csf_grad(Grid g, CsfD p, const double* 
   const long long r = __double_as_longlong(q000);
   auto df = [&](double x) { return (unsigned long long)(__double_as_longlong(x) ^ r); };
   const bool varies = (df(qp00) | df(q0p0) | df(qpp0) | df(q00p) | df(qp0p) | df(q0pp) | df(qppp)) != 0 ||
-                      ((r >> 52) & 0x7ff) == 0x7ff;
+                      !finite_bits(r);
   if (!__any_sync(__activemask(), varies)) {
     G[c] = 0.0;
     G[c + n] = 0.0;
@@ -487,7 +485,7 @@ __global__ void __launch_bounds__(256) k_csf_force(Grid g, CsfD p, const double*
   const double ph = __ldg(phi + c), px = __ldg(phi + c + X), py = __ldg(phi + c + Y), pz = __ldg(phi + c + Z);
   const long long r = __double_as_longlong(ph);
   const bool varies = ((__double_as_longlong(px) ^ r) | (__double_as_longlong(py) ^ r) |
-                       (__double_as_longlong(pz) ^ r)) != 0 || ((r >> 52) & 0x7ff) == 0x7ff;
+                       (__double_as_longlong(pz) ^ r)) != 0 || !finite_bits(r);
   if (!__any_sync(__activemask(), varies)) {
     fu[c] = 0.0;
     fv[c] = 0.0;

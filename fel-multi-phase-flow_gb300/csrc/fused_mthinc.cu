@@ -1,6 +1,14 @@
-// fused_mthinc.cu -- MTHINC fluxes (solphi_mthinc1.f) for the fused step.
+// fused_mthinc.cu -- the vertex gradients (cal_grad_p2a.f), MTHINC fluxes
+// (solphi_mthinc1.f) and snap (solphi_mthinc3.f:61-120) for the fused step; the rest of
+// the transport is in k_transport.cu.
 //
-// Two kernels instead of one thread per cell on the full 0..n+1 range:
+// Away from the interface phi is exactly 0 or 1 (solphi_mthinc3's snap), and there
+// these kernels' FP64 operations give zeros or the value they were given: a warp
+// whose points are all such takes that result from the bits of what it read and does
+// no arithmetic.  The FP64 pipe, 64 cycles per warp instruction, bounds every kernel
+// here otherwise.
+//
+// Fluxes: two kernels instead of one thread per cell on the full 0..n+1 range:
 //   k_classify: every cell forms its normal from the 8 vertex gradients; cells
 //     outside the interface band write their truncated upwind fluxes at once,
 //     band cells are appended to a compact list;
@@ -15,6 +23,10 @@
 // and their west/south/bottom face when u<0, so every face in 0..n of every
 // interior row gets exactly one writer (solphi_mthinc1.f:121-130 zeroes first;
 // faces nobody donates through hold the zero written by k_classify's owner).
+#include <cmath>
+#include <cstring>
+
+#include "bits.cuh"
 #include "fused.cuh"
 #include "recip.cuh"
 
@@ -23,10 +35,71 @@ namespace fused {
 
 namespace {
 struct MC {
-  double gp1, gp2, lim, eps_trunc, bet, dt, dxi, dyi, dzi;
+  double gp1, gp2, lim, bet, dt, dxi, dyi, dzi;
   double lim2lo, lim2hi;  // lim^2 (1 -/+ 1e-12)
   double dtdx, dtdy, dtdz;  // dt dxinv etc.
+  long long eps, one_eps;   // eps_trunc and the smallest t with 1 - t <= eps_trunc, as bits
 };
+// the constants of solphi_mthinc1.f and solphi_mthinc3.f (dt = 0 for the latter)
+MC make_mc(double dxinv, double dyinv, double dzinv, double dt, double bet) {
+  MC m;
+  const double dx = 1.0 / dxinv, dy = 1.0 / dyinv, dz = 1.0 / dzinv;
+  m.gp1 = -0.5 / std::sqrt(3.0);
+  m.gp2 = 0.5 / std::sqrt(3.0);
+  const double dcellinv = 1.0 / std::sqrt((dx * dx + dy * dy + dz * dz) / 3.0);
+  const double ch = std::cosh(-bet * 1.5);
+  m.lim = bet / (2.0 * (ch * ch)) * dcellinv;
+  m.lim2lo = m.lim * m.lim * (1.0 - 1.0e-12);
+  m.lim2hi = m.lim * m.lim * (1.0 + 1.0e-12);
+  const double eps = 0.5 * (std::tanh(-bet * 2.5) + 1.0);
+  double t = 1.0 - eps;
+  while (1.0 - t > eps) t = std::nextafter(t, 2.0);
+  while (1.0 - std::nextafter(t, 0.0) <= eps) t = std::nextafter(t, 0.0);
+  std::memcpy(&m.eps, &eps, sizeof(double));
+  std::memcpy(&m.one_eps, &t, sizeof(double));
+  m.bet = bet;
+  m.dt = dt;
+  m.dxi = dxinv;
+  m.dyi = dyinv;
+  m.dzi = dzinv;
+  m.dtdx = dt * dxinv;
+  m.dtdy = dt * dyinv;
+  m.dtdz = dt * dzinv;
+  return m;
+}
+
+// The 8 vertex gradients around a cell, and whether any of them is not 0
+struct G8 {
+  double v[8];
+  __device__ __forceinline__ unsigned long long load(const double* __restrict__ p, long c, long X, long Y, long Z) {
+    v[0] = __ldg(p + c - X - Y - Z);
+    v[1] = __ldg(p + c - Y - Z);
+    v[2] = __ldg(p + c - X - Z);
+    v[3] = __ldg(p + c - Z);
+    v[4] = __ldg(p + c - X - Y);
+    v[5] = __ldg(p + c - Y);
+    v[6] = __ldg(p + c - X);
+    v[7] = __ldg(p + c);
+    unsigned long long z = 0;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) z |= mag(v[t]);
+    return z;
+  }
+  __device__ __forceinline__ double mean() const {
+    return (v[0] + v[1] + v[2] + v[3] + v[4] + v[5] + v[6] + v[7]) * 0.125;
+  }
+};
+// The band test sqrt(q2) <= lim of the reference for the squared norm q2 of the mean
+// gradient: decided on q2 against lim^2 where q2 is clearly on one side (compared as
+// bit patterns: all three are non-negative), with the square root only within 1e-12 of
+// it.  q2 is rounded operation by operation, as the adjoint's record of the snap does.
+__device__ __forceinline__ bool outside_band(const G8& gx, const G8& gy, const G8& gz, const MC& m) {
+  const double x = gx.mean(), y = gy.mean(), z = gz.mean();
+  const double q2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
+  const long long qb = __double_as_longlong(q2);
+  return qb < __double_as_longlong(m.lim2lo) ? true
+                                             : (qb > __double_as_longlong(m.lim2hi) ? false : sqrt(q2) <= m.lim);
+}
 
 __device__ __forceinline__ double avg8(const double* __restrict__ p, long c, long X, long Y, long Z) {
   return (__ldg(p + c - X - Y - Z) + __ldg(p + c - Y - Z) + __ldg(p + c - X - Z) + __ldg(p + c - Z) +
@@ -41,7 +114,7 @@ __device__ __forceinline__ float ex(float x) { return expf(fminf(x, 80.0f)); }
 // exactly 0, as the quotient does; NaN stays NaN), the quotient in float
 __device__ __forceinline__ double inv1p(double e) {
   const double a = 1.0 + e;
-  return (__double2hiint(a) == 0x7ff00000 && __double2loint(a) == 0) ? 0.0 : recip_nr(a);
+  return (__double2hiint(a) == 0x7ff00000 && __double2loint(a) == 0) ? 0.0 : recip_h(a);
 }
 __device__ __forceinline__ float inv1p(float e) { return 1.0f / (1.0f + e); }
 
@@ -92,42 +165,42 @@ __global__ void __launch_bounds__(256) k_classify(Grid g, MC m, const double* __
   if (i > g.ni + 1 || j > g.nj + 1) return;
   const long X = 1, Y = g.sy, Z = g.sz;
   const long c = g.at(i, j, k);
-  const double rnx = avg8(gx, c, X, Y, Z), rny = avg8(gy, c, X, Y, Z), rnz = avg8(gz, c, X, Y, Z);
-  const double q2 = rnx * rnx + rny * rny + rnz * rnz;
+  G8 ax, ay, az;
+  const bool graded = (ax.load(gx, c, X, Y, Z) | ay.load(gy, c, X, Y, Z) | az.load(gz, c, X, Y, Z)) != 0;
   const double uw = __ldg(u + c - X), ue = __ldg(u + c), vs = __ldg(v + c - Y), vn = __ldg(v + c),
                wb = __ldg(w + c - Z), wt = __ldg(w + c);
-  // the band test sqrt(q2) <= lim of the reference: decided on q2 against lim^2
-  // where q2 is clearly on one side (compared as bit patterns: all three are
-  // non-negative), with the square root only within 1e-12 of it
-  const long long qb = __double_as_longlong(q2);
-  const bool band = qb < __double_as_longlong(m.lim2lo)
-                        ? false
-                        : (qb > __double_as_longlong(m.lim2hi) ? true : !(sqrt(q2) <= m.lim));
+  const unsigned warp = __activemask();
+  const bool band = __any_sync(warp, graded) && !outside_band(ax, ay, az, m);
   if (band) {
     const int slot = atomicAdd(count, 1);
     list[slot] = (int)c;
   }
-  double phi00 = 0.0;
-  if (!band) {
-    phi00 = __ldg(phi + c);
-    if (phi00 <= m.eps_trunc) phi00 = 0.0;
-    if (1.0 - phi00 <= m.eps_trunc) phi00 = 1.0;
-  }
+  const double phi00 = band ? 0.0 : snap01(__ldg(phi + c), m.eps, m.one_eps);
   // owned faces: east/north/top when the velocity there is >= 0 (this cell donates or
   // the flux is zero), west/south/bottom when < 0; band cells leave the donated
   // faces to k_band but still zero the owned faces they do not donate through.
-  // Signs are read from the bits: nonneg(v) is v >= 0 (so true for -0 as well; it
-  // differs from the comparison only for NaN).  Fluxes are v phi dt/dx with dt/dx
-  // formed once.
-  auto nonneg = [](double v) { return __double_as_longlong(v) >= 0 || (__double_as_longlong(v) << 1) == 0; };
-  const double pdx = phi00 * m.dtdx, pdy = phi00 * m.dtdy, pdz = phi00 * m.dtdz;
+  // Fluxes are v phi dt/dx with phi dt/dx formed first.
+  const long long pb = __double_as_longlong(phi00);
+  double pdx = 0.0, pdy = 0.0, pdz = 0.0;
+  if (__any_sync(warp, pb != 0)) {
+    if (__any_sync(warp, pb != 0 && pb != kOneBits)) {
+      pdx = phi00 * m.dtdx;
+      pdy = phi00 * m.dtdy;
+      pdz = phi00 * m.dtdz;
+    } else if (pb != 0) {
+      pdx = m.dtdx;
+      pdy = m.dtdy;
+      pdz = m.dtdz;
+    }
+  }
   const bool e_ = nonneg(ue), w_ = nonneg(uw), n_ = nonneg(vn), s_ = nonneg(vs), t_ = nonneg(wt), b_ = nonneg(wb);
-  if (e_) fx[c] = band ? 0.0 : ue * pdx;
-  if (!w_) fx[c - X] = band ? 0.0 : uw * pdx;
-  if (n_) fy[c] = band ? 0.0 : vn * pdy;
-  if (!s_) fy[c - Y] = band ? 0.0 : vs * pdy;
-  if (t_) fz[c] = band ? 0.0 : wt * pdz;
-  if (!b_) fz[c - Z] = band ? 0.0 : wb * pdz;
+  auto flux = [&](double vel, double pd) { return __any_sync(__activemask(), pb != 0) ? vel * pd : 0.0; };
+  if (e_) fx[c] = flux(ue, pdx);
+  if (!w_) fx[c - X] = flux(uw, pdx);
+  if (n_) fy[c] = flux(vn, pdy);
+  if (!s_) fy[c - Y] = flux(vs, pdy);
+  if (t_) fz[c] = flux(wt, pdz);
+  if (!b_) fz[c - Z] = flux(wb, pdz);
   // west/south/bottom faces of the first cells with no in-range donor stay zero
   if (i == 0 && w_) fx[c - X] = 0.0;
   if (j == 0 && s_) fy[c - Y] = 0.0;
@@ -173,7 +246,7 @@ __global__ void __launch_bounds__(128) k_band(Grid g, MC m, const double* __rest
       const R f = sig8f<R>(E, (R)0.125, ex(m2b * ddd), &sd) - ph;
       // df = 0.5 bet sum 0.125/cosh^2 = 0.5 bet * 0.125 * 4 * sum s(1-s)
       const R df = (R)0.25 * bet * sd;
-      step = sizeof(R) == 8 ? (R)((double)(f * df) * recip_nr((double)(df * df + reg))) : f * df / (df * df + reg);
+      step = sizeof(R) == 8 ? (R)((double)(f * df) * recip_h((double)(df * df + reg))) : f * df / (df * df + reg);
       const R dn = ddd - step;
       // once d no longer changes, every remaining iteration recomputes the same
       // f, df and step: stopping here is the ten-step result bit for bit.  In
@@ -210,34 +283,84 @@ __global__ void __launch_bounds__(128) k_band(Grid g, MC m, const double* __rest
   }
 }
 // cal_grad_p2a.f:46-60 for the fused step: the vertex gradient at (i+1/2, j+1/2,
-// k+1/2), i, j, k in -2..n+2, from the 8 surrounding points.  Per (i, j) corner the
-// sum s and difference d of the two k planes; with ta = s(+,+) - s(0,0) and
-// tb = s(+,0) - s(0,+) the x sum is ta + tb, the y sum ta - tb and the z sum the
-// four differences: 18 FP64 operations per point instead of the reference's 27.
-__global__ void __launch_bounds__(256) k_vertex_grad(Grid g, double cx, double cy, double cz,
+// k+1/2), i, j, k in -2..n+2, from the 8 surrounding points (threads over the flattened
+// (i, j) plane, so that every warp is full).  Per (i, j) corner the sum s and difference
+// d of the two k planes; with ta = s(+,+) - s(0,0) and tb = s(+,0) - s(0,+) the x sum is
+// ta + tb, the y sum ta - tb and the z sum the four differences: 18 FP64 operations per
+// point instead of the reference's 27, none in a warp whose points are all flat.
+// NEAR1 (phin before its snap, for the band test alone): eight values within 64 units in
+// the last place below 1 count as flat.  There phin is 1 but for the roundings of
+// solphi_mthinc2; a gradient of 2^-47 dxinv is 1e-12 of the band test's limit, inside
+// which the test falls back on the square root.
+template <bool NEAR1>
+__global__ void __launch_bounds__(128) k_vertex_grad(Grid g, double cx, double cy, double cz,
                                                      const double* __restrict__ q, double* __restrict__ qx,
                                                      double* __restrict__ qy, double* __restrict__ qz) {
-  const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int k = -2 + (int)blockIdx.z;
-  if (i > g.ni + 2 || j > g.nj + 2) return;
+  const int W = g.ni + 5;
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= W * (g.nj + 5)) return;
+  const int b = t / W, a = t - b * W;
   const long X = 1, Y = g.sy, Z = g.sz;
-  const long c = g.at(i, j, k);
+  const long c = g.at(a - 2, b - 2, (int)blockIdx.y - 2);
   const double q000 = __ldg(q + c), qp00 = __ldg(q + c + X), q0p0 = __ldg(q + c + Y), qpp0 = __ldg(q + c + X + Y),
                q00p = __ldg(q + c + Z), qp0p = __ldg(q + c + X + Z), q0pp = __ldg(q + c + Y + Z),
                qppp = __ldg(q + c + X + Y + Z);
-  const double s00 = q000 + q00p, sp0 = qp00 + qp0p, s0p = q0p0 + q0pp, spp = qpp0 + qppp;
-  const double ta = spp - s00, tb = sp0 - s0p;
-  qx[c] = (ta + tb) * cx;
-  qy[c] = (ta - tb) * cy;
-  qz[c] = ((q00p - q000) + (qp0p - qp00) + ((q0pp - q0p0) + (qppp - qpp0))) * cz;
+  const long long r = __double_as_longlong(q000);
+  auto df = [&](double x) { return (unsigned long long)(__double_as_longlong(x) ^ r); };
+  bool flat = (df(qp00) | df(q0p0) | df(qpp0) | df(q00p) | df(qp0p) | df(q0pp) | df(qppp)) == 0 && finite_bits(r);
+  if (NEAR1) {
+    auto below = [&](double x) { return (unsigned long long)(kOneBits - __double_as_longlong(x)); };
+    flat = flat || (below(q000) | below(qp00) | below(q0p0) | below(qpp0) | below(q00p) | below(qp0p) | below(q0pp) |
+                    below(qppp)) < 64;
+  }
+  double gx = 0.0, gy = 0.0, gz = 0.0;
+  if (!flat) {
+    const double s00 = q000 + q00p, sp0 = qp00 + qp0p, s0p = q0p0 + q0pp, spp = qpp0 + qppp;
+    const double ta = spp - s00, tb = sp0 - s0p;
+    gx = (ta + tb) * cx;
+    gy = (ta - tb) * cy;
+    gz = ((q00p - q000) + (qp0p - qp00) + ((q0pp - q0p0) + (qppp - qpp0))) * cz;
+  }
+  qx[c] = gx;
+  qy[c] = gy;
+  qz[c] = gz;
+}
+
+// solphi_mthinc3.f:61-120: the snap over 0..n+1 of cells outside the band (by the vertex
+// gradients of phin) and the clip of the interior, in one pass (each touches its point
+// alone).
+__global__ void __launch_bounds__(256) k_snap(Grid g, MC m, const double* __restrict__ gx,
+                                              const double* __restrict__ gy, const double* __restrict__ gz,
+                                              double* __restrict__ phin) {
+  const int W = g.ni + 2;
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= W * (g.nj + 2)) return;
+  const int j = t / W, i = t - j * W, k = (int)blockIdx.y;
+  const long X = 1, Y = g.sy, Z = g.sz;
+  const long c = g.at(i, j, k);
+  G8 ax, ay, az;
+  const bool graded = (ax.load(gx, c, X, Y, Z) | ay.load(gy, c, X, Y, Z) | az.load(gz, c, X, Y, Z)) != 0;
+  double p = phin[c];
+  if (!__any_sync(__activemask(), graded) || outside_band(ax, ay, az, m)) p = snap01(p, m.eps, m.one_eps);
+  if (i >= 1 && i <= g.ni && j >= 1 && j <= g.nj && k >= 1 && k <= g.nk) p = clip01(p);
+  phin[c] = p;
 }
 }  // namespace
 
 void vertex_gradient(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const double* q,
-                     double* qx, double* qy, double* qz) {
-  const dim3 b(32, 8, 1), gr((unsigned)((g.ni + 5 + 31) / 32), (unsigned)((g.nj + 5 + 7) / 8), (unsigned)(g.nk + 5));
-  k_vertex_grad<<<gr, b, 0, s>>>(g, 0.25 * dxinv, 0.25 * dyinv, 0.25 * dzinv, q, qx, qy, qz);
+                     double* qx, double* qy, double* qz, bool near1) {
+  const dim3 gr((unsigned)(((long)(g.ni + 5) * (g.nj + 5) + 127) / 128), (unsigned)(g.nk + 5));
+  if (near1)
+    k_vertex_grad<true><<<gr, 128, 0, s>>>(g, 0.25 * dxinv, 0.25 * dyinv, 0.25 * dzinv, q, qx, qy, qz);
+  else
+    k_vertex_grad<false><<<gr, 128, 0, s>>>(g, 0.25 * dxinv, 0.25 * dyinv, 0.25 * dzinv, q, qx, qy, qz);
+  count_launch();
+}
+
+void mthinc_snap(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double bet,
+                 const double* gx, const double* gy, const double* gz, double* phin) {
+  const dim3 gr((unsigned)(((long)(g.ni + 2) * (g.nj + 2) + 255) / 256), (unsigned)(g.nk + 2));
+  k_snap<<<gr, 256, 0, s>>>(g, make_mc(dxinv, dyinv, dzinv, 0.0, bet), gx, gy, gz, phin);
   count_launch();
 }
 
@@ -245,24 +368,7 @@ void mthinc_fluxes(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
                    const double* phi, const double* gx, const double* gy, const double* gz, const double* u,
                    const double* v, const double* w, double* fx, double* fy, double* fz, int* list, int* count,
                    bool fp32, double* newton) {
-  MC m;
-  const double dx = 1.0 / dxinv, dy = 1.0 / dyinv, dz = 1.0 / dzinv;
-  m.gp1 = -0.5 / std::sqrt(3.0);
-  m.gp2 = 0.5 / std::sqrt(3.0);
-  const double dcellinv = 1.0 / std::sqrt((dx * dx + dy * dy + dz * dz) / 3.0);
-  const double ch = std::cosh(-bet * 1.5);
-  m.lim = bet / (2.0 * (ch * ch)) * dcellinv;
-  m.lim2lo = m.lim * m.lim * (1.0 - 1.0e-12);
-  m.lim2hi = m.lim * m.lim * (1.0 + 1.0e-12);
-  m.eps_trunc = 0.5 * (std::tanh(-bet * 2.5) + 1.0);
-  m.bet = bet;
-  m.dt = dt;
-  m.dxi = dxinv;
-  m.dyi = dyinv;
-  m.dzi = dzinv;
-  m.dtdx = dt * dxinv;
-  m.dtdy = dt * dyinv;
-  m.dtdz = dt * dzinv;
+  const MC m = make_mc(dxinv, dyinv, dzinv, dt, bet);
   FMF_CUDA(cudaMemsetAsync(count, 0, sizeof(int), s));
   dim3 b(32, 8, 1);
   dim3 gr((unsigned)((g.ni + 2 + 31) / 32), (unsigned)((g.nj + 2 + 7) / 8), (unsigned)(g.nk + 2));

@@ -9,39 +9,6 @@ namespace op {
 void cal_arith_mean(cudaStream_t s, const Grid& g, const double* phi, double ql, double qg, double* q) {
   flat(s, g.n, [=] __device__(long t) { q[t] = ql * (1.0 - phi[t]) + qg * phi[t]; });
 }
-// The four cal_arith_mean calls of main.f90:526-529 in one pass: rho, rhon from
-// (rhol, rhog) and rmu, rmun from (rmul, rmug) over phi0 and phin0 -- the same
-// expression per point, two points per thread per pass so that four loads are in
-// flight (the single-field pass keeps one and runs at a third of HBM's rate).
-namespace {
-__global__ void __launch_bounds__(256) k_means4(long n, const double* __restrict__ p0, const double* __restrict__ p1,
-                                                double rl, double rg, double ml, double mg, double* __restrict__ rho,
-                                                double* __restrict__ rhon, double* __restrict__ rmu,
-                                                double* __restrict__ rmun) {
-  const long stride = (long)gridDim.x * blockDim.x;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += 2 * stride) {
-    const long t2 = t + stride;
-    const bool two = t2 < n;
-    const double a = p0[t], b = p1[t];
-    const double a2 = two ? p0[t2] : 0.0, b2 = two ? p1[t2] : 0.0;
-    rho[t] = rl * (1.0 - a) + rg * a;
-    rhon[t] = rl * (1.0 - b) + rg * b;
-    rmu[t] = ml * (1.0 - a) + mg * a;
-    rmun[t] = ml * (1.0 - b) + mg * b;
-    if (two) {
-      rho[t2] = rl * (1.0 - a2) + rg * a2;
-      rhon[t2] = rl * (1.0 - b2) + rg * b2;
-      rmu[t2] = ml * (1.0 - a2) + mg * a2;
-      rmun[t2] = ml * (1.0 - b2) + mg * b2;
-    }
-  }
-}
-}  // namespace
-void mixture_means(cudaStream_t s, const Grid& g, const double* phi0, const double* phin0, double rhol, double rhog,
-                   double rmul, double rmug, double* rho, double* rhon, double* rmu, double* rmun) {
-  k_means4<<<152 * 8, 256, 0, s>>>(g.n, phi0, phin0, rhol, rhog, rmul, rmug, rho, rhon, rmu, rmun);
-  count_launch();
-}
 // cal_harm_mean.f:42-56
 void cal_harm_mean(cudaStream_t s, const Grid& g, const double* phi, double ql, double qg, double* q) {
   flat(s, g.n, [=] __device__(long t) { q[t] = 1.0 / ((1.0 - phi[t]) / ql + phi[t] / qg); });

@@ -511,17 +511,17 @@ static void seg_pre_b(fmf_ctx* c) {
     fused::mthinc_fluxes(s, g, dxinv, dyinv, dzinv, dt, P.bet_mthinc, phi1, c->phix, c->phiy, c->phiz, c->u, c->v,
                          c->w, c->flx, c->fly, c->flz, c->band, c->band + nb, P.precision == FMF_MIXED);
   }
-  op::solphi_mthinc2(s, g, dxinv, dyinv, dzinv, dt, c->u, c->v, c->w, c->flx, c->fly, c->flz, phi1, phin1);
-  fused::vertex_gradient(s, g, dxinv, dyinv, dzinv, phin1, c->phix, c->phiy, c->phiz);
-  op::solphi_mthinc3(s, g, dxinv, dyinv, dzinv, P.bet_mthinc, c->phix, c->phiy, c->phiz, phi1, phin1, c->red);
+  fused::mthinc_advance(s, g, dxinv, dyinv, dzinv, dt, c->u, c->v, c->w, c->flx, c->fly, c->flz, phi1, phin1);
+  fused::vertex_gradient(s, g, dxinv, dyinv, dzinv, phin1, c->phix, c->phiy, c->phiz, true);
+  // with the interior of phin(0) (summation, :509)
+  fused::mthinc_volume_fix(s, g, dxinv, dyinv, dzinv, P.bet_mthinc, c->phix, c->phiy, c->phiz, phi1, phin1, phin0,
+                           c->red);
   op::gnbc(s, g, c->u, c->w, P.uwall, c->theta0, P.sigma, c->zeta, c->theta);
   op::bnd_contact_angle(s, g, phin1, c->theta, P.dx, P.dy, P.dz);
-  op::bnd_periodic(s, g, phin1);
-  // :509-517 on phin (the contact-angle pass on phi(0) of :515, independent of
+  fused::halo_periodic(s, g, phin1);
+  // :510-517 on phin (the contact-angle pass on phi(0) of :515, independent of
   // these, follows in part c)
-  op::summation(s, g, phin0, phin1);
-  op::bnd_neumann(s, g, phin0);
-  op::bnd_periodic(s, g, phin0);
+  fused::halo_neumann_periodic(s, g, phin0);
 }
 static void seg_pre_c(fmf_ctx* c) {
   const fmf_params& P = c->prm;
@@ -529,7 +529,7 @@ static void seg_pre_c(fmf_ctx* c) {
   double* phi0 = c->phi;
   op::bnd_contact_angle(c->s, g, phi0, c->theta, P.dx, P.dy, P.dz);  // gnbc result unchanged since :498
   // :526-529
-  op::mixture_means(c->s, g, phi0, c->phin, P.rhol, P.rhog, P.rmul, P.rmug, c->rho, c->rhon, c->rmu, c->rmun);
+  fused::mixture_means(c->s, g, phi0, c->phin, P.rhol, P.rhog, P.rmul, P.rmug, c->rho, c->rhon, c->rmu, c->rmun);
 }
 static void seg_pre(fmf_ctx* c) {
   seg_pre_a(c);
@@ -726,14 +726,12 @@ static void seg_post(fmf_ctx* c) {
   fused::pressure_half(s, g, P.rhog, dxinv, dzinv, c->as_f, c->an_f, c->ap_f, c->div, c->pr, c->pi, c->dp,
                         c->tdma);
   op::bnd_avzero(s, g, c->dp);
-  op::bnd_neumann(s, g, c->dp);
-  op::bnd_periodic(s, g, c->dp);
+  fused::halo_neumann_periodic(s, g, c->dp);
   // :648-661
   fused::project(s, g, P.rhog, dxinv, dyinv, dzinv, dt, c->dp, c->phat, c->un, c->vn, c->wn, c->pn);
   fused::wall_halo(s, g, 7, P.uwall, c->wallc, c->un, c->vn, c->wn);
   op::bnd_avzero(s, g, c->pn);
-  op::bnd_neumann(s, g, c->pn);
-  op::bnd_periodic(s, g, c->pn);
+  fused::halo_neumann_periodic(s, g, c->pn);
   // :695-697 phi(l) = phin(l); phin keeps its values (cpy leaves the source intact),
   // so after the pointer swap below the new phin must equal the new phi
   op::copy(s, 2 * n, c->phin, c->phi);
