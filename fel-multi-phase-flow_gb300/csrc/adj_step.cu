@@ -522,19 +522,19 @@ int record_step(fmf_adj* a, bool graphs) {
     // :579-623
     const double* advp[3] = {a->adv[0], a->adv[1], a->adv[2]};
     const double* advop[3] = {a->advo[0], a->advo[1], a->advo[2]};
-    const double* prsp[3] = {a->prs[0], a->prs[1], a->prs[2]};
+    const fused::Fluids fl{P.rhol, P.rhog, P.rmul, P.rmug};
     const double* visp[3] = {a->vis[0], a->vis[1], a->vis[2]};
     const double* fstp[3] = {a->sfst[0], a->sfst[1], a->sfst[2]};
     const double* fstnp[3] = {a->sfstn[0], a->sfstn[1], a->sfstn[2]};
     // the FP64 factors A, B the reverse differentiates (the viscous solve's fixed
     // point is un* = A visn(un*) + B in either precision)
-    fused::src_visc_prep(s, g, dxi, dyi, dzi, dt, P.harmonic, P.grvb, P.grvp, S[SU], S[SV], S[SW], advp, advop, prsp,
-                         visp, fstp, fstnp, a->rmun, a->rho, a->rhon, a->E, a->AB, a->l1, a->l2, phi1, P.dy, a->wallc);
+    fused::src_visc_prep(s, g, dxi, dyi, dzi, dt, P.harmonic, P.grvb, P.grvp, S[SU], S[SV], S[SW], advp, advop,
+                         a->phat, visp, fstp, fstnp, fl, a->rmun, a->rho, a->rhon, a->E, a->AB, a->l1, a->l2, phi1, P.dy, a->wallc);
     if (a->mixed)
       // the mixed solve's FP64 first-sweep residual, FP32 factors and wall/halo
       // constants; un = u through zero corrections
-      fused::refine_prep(s, g, dxi, dyi, dzi, dt, P.harmonic, P.grvb, P.grvp, S[SU], S[SV], S[SW], advp, advop, prsp,
-                         visp, fstp, fstnp, a->rmun, a->rho, a->rhon, a->E, a->l1, a->l2, phi1, P.dy, P.uwall,
+      fused::refine_prep(s, g, dxi, dyi, dzi, dt, P.harmonic, P.grvb, P.grvp, S[SU], S[SV], S[SW], advp, advop,
+                         a->phat, visp, fstp, fstnp, fl, a->rmun, a->rho, a->rhon, a->E, a->l1, a->l2, phi1, P.dy, P.uwall,
                          a->wallc, a->rb);
     else
       for (int q = 0; q < 3; ++q) dcopy(a, S[SU + q], a->un[q], n);

@@ -81,15 +81,20 @@ void explicit_viscous(cudaStream_t s, const Grid& g, double dxinv, double dyinv,
                       const double* v, const double* w, const double* mu, double* tau, double* const* vis,
                       double* sk = nullptr, bool pairs = false);
 
+// the densities and viscosities of the two fluids (phi = 0 and phi = 1)
+struct Fluids {
+  double rhol, rhog, rmul, rmug;
+};
 // Viscous solve.  src_visc_prep: edge viscosities E[0..2] (xy, xz, yz edges, i,j,k in
 // 0..n), per-component A/B (AB[0..5] = Au Bu Av Bv Aw Bw) with the momentum
-// right-hand side of cal_srcu formed in registers, and the Navier-slip wall
+// right-hand side of cal_srcu formed in registers (its pressure gradient from phat =
+// 2 p - po), and the Navier-slip wall
 // coefficients wallc (2*(nk+6)*(ni+6)*2 doubles) from phi, l1, l2.
 void src_visc_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt, int harmonic,
                    double grvb, double grvp, const double* u, const double* v, const double* w,
-                   const double* const* adv, const double* const* advo, const double* const* prs,
-                   const double* const* vis, const double* const* fst, const double* const* fstn, const double* mu,
-                   const double* rho, const double* rhon, double* const* E, double* const* AB, const double* l1,
+                   const double* const* adv, const double* const* advo, const double* phat,
+                   const double* const* vis, const double* const* fst, const double* const* fstn, const Fluids& fl,
+                   const double* mu, const double* rho, const double* rhon, double* const* E, double* const* AB, const double* l1,
                    const double* l2, const double* phi, double dy, double* wallc, bool pairs = false);
 // the Navier-slip coefficients wallc alone (as src_visc_prep computes them)
 void wall_coef(cudaStream_t s, const Grid& g, double dy, const double* l1, const double* l2, const double* phi,
@@ -138,9 +143,9 @@ long refine_floats(const Grid& g, int part);
 // from u, v, w, and zero corrections
 void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt, int harmonic,
                  double grvb, double grvp, const double* u, const double* v, const double* w,
-                 const double* const* adv, const double* const* advo, const double* const* prs,
-                 const double* const* vis, const double* const* fst, const double* const* fstn, const double* mu,
-                 const double* rho, const double* rhon, double* const* E, const double* l1, const double* l2,
+                 const double* const* adv, const double* const* advo, const double* phat,
+                 const double* const* vis, const double* const* fst, const double* const* fstn, const Fluids& fl,
+                 const double* mu, const double* rho, const double* rhon, double* const* E, const double* l1, const double* l2,
                  const double* phi, double dy, double uwall, double* wallc, const RefineBufs& rb);
 // one outer iteration on the corrections; errsum[0] = sum of squared increments
 void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv,

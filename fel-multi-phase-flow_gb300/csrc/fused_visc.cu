@@ -19,6 +19,7 @@
 // sweeps run in FP32 on the correction d = un - u (FP32 storage and arithmetic),
 // and un = u + d is formed in FP64 at the end.
 #include <cstdlib>
+#include <cstring>
 
 #include "df64.cuh"
 #include "fused.cuh"
@@ -30,10 +31,16 @@ namespace fused {
 
 namespace {
 struct VP {
-  double dtinv, dx2, dy2, dz2, dxy, dxz, dyz;
+  double dxi, dyi, dzi, dtinv, dx2, dy2, dz2, dxy, dxz, dyz;
   int harmonic;
 };
 
+// whether five doubles have the same bits
+__device__ __forceinline__ bool same_bits(double a, double b, double c, double d, double e) {
+  const long long r = __double_as_longlong(a);
+  return ((__double_as_longlong(b) ^ r) | (__double_as_longlong(c) ^ r) | (__double_as_longlong(d) ^ r) |
+          (__double_as_longlong(e) ^ r)) == 0;
+}
 __device__ __forceinline__ double mean4(double a, double b, double c, double d, int harm) {
   if (!harm) return 0.25 * (a + b + c + d);
   return 4.0 / (1.0 / a + 1.0 / b + 1.0 / c + 1.0 / d);
@@ -44,18 +51,26 @@ __device__ __forceinline__ double mean4(double a, double b, double c, double d, 
 struct F3 {
   float* f[3];
 };
-__global__ void __launch_bounds__(256) k_edges(Grid g, VP p, const double* __restrict__ mu, double* __restrict__ exy,
+// Where the seven viscosities are equal bits their arithmetic means are that value (2a
+// is exact, 3a within one unit of a's last place, so 3a + a rounds to 4a), and a warp of
+// such points takes it without the arithmetic.  Threads over the flattened (i, j) plane.
+__global__ void __launch_bounds__(128) k_edges(Grid g, VP p, const double* __restrict__ mu, double* __restrict__ exy,
                                                double* __restrict__ exz, double* __restrict__ eyz, F3 f) {
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int k = (int)blockIdx.z;
-  if (i > g.ni || j > g.nj) return;
+  const int W = g.ni + 1;
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= W * (g.nj + 1)) return;
+  const int j = t / W, i = t - j * W, k = (int)blockIdx.y;
   const long X = 1, Y = g.sy, Z = g.sz;
   const long c = g.at(i, j, k);
-  const double m0 = __ldg(mu + c), mx = __ldg(mu + c + X), my = __ldg(mu + c + Y), mz = __ldg(mu + c + Z);
-  const double a = mean4(m0, mx, my, __ldg(mu + c + X + Y), p.harmonic);
-  const double b = mean4(m0, mx, mz, __ldg(mu + c + X + Z), p.harmonic);
-  const double d = mean4(m0, my, mz, __ldg(mu + c + Y + Z), p.harmonic);
+  const double m0 = __ldg(mu + c), mx = __ldg(mu + c + X), my = __ldg(mu + c + Y), mz = __ldg(mu + c + Z),
+               mxy = __ldg(mu + c + X + Y), mxz = __ldg(mu + c + X + Z), myz = __ldg(mu + c + Y + Z);
+  const bool flat = same_bits(m0, mx, my, mz, mxy) && same_bits(m0, mxz, myz, m0, m0) && !p.harmonic;
+  double a = m0, b = m0, d = m0;
+  if (__any_sync(__activemask(), !flat)) {
+    a = mean4(m0, mx, my, mxy, p.harmonic);
+    b = mean4(m0, mx, mz, mxz, p.harmonic);
+    d = mean4(m0, my, mz, myz, p.harmonic);
+  }
   exy[c] = a;
   exz[c] = b;
   eyz[c] = d;
@@ -67,11 +82,11 @@ __global__ void __launch_bounds__(256) k_edges(Grid g, VP p, const double* __res
 }
 
 // cal_srcu.f:53-137 fused with the update factors: src is formed in registers and
-// only A = 0.5/(rho00*D), B = src/D are stored.  With T = 1/(rho00/dt + a_p/2)
-// these are A = T/2 and B = (rho00*(explicit terms) - prs + vis/2)*T: one
-// reciprocal per component (recip_nr: Newton-Raphson, no division).
+// only A = 0.5/(rho00*D), B = src/D are stored, and the pressure gradient of
+// cal_grad_prs.f is taken from phat = 2 p - po.  With T = 1/(rho00/dt + a_p/2) these are
+// A = T/2 and B = (rho00*(explicit terms) - prs + vis/2)*T.
 struct SrcIn {
-  const double *u, *v, *w, *rho, *rhon, *adv[3], *advo[3], *prs[3], *vis[3], *fst[3], *fstn[3];
+  const double *u, *v, *w, *rho, *rhon, *adv[3], *advo[3], *phat, *vis[3], *fst[3], *fstn[3];
   double grvb, grvp;
 };
 // Outputs: FP64 A and B per component, or (REFINE) FP32 A and the FP64 first-sweep
@@ -85,8 +100,22 @@ template <int COMP, class T>
 __device__ __forceinline__ T visn_at(const Grid& g, const VP& p, long c, const T* __restrict__ mu,
                                      const T* __restrict__ exy, const T* __restrict__ exz,
                                      const T* __restrict__ eyz, const T* un, const T* vn, const T* wn);
-template <bool REFINE>
-__global__ void __launch_bounds__(256) k_src_ab(Grid g, VP p, SrcIn in, const double* __restrict__ mu,
+// FP64 (the FP64 step).  With s = the sum of the four densities (4 rho00), T's
+// denominator doubled is 1/A = s/(2 dt) + a_p, one reciprocal (recip_h), and
+// B = A (s (explicit terms)/2 - 2 prs + vis), the constants folded on the host: 70 FP64
+// operations per cell against 84 and 6 for the gradient's own kernel.  Where the
+// densities and viscosities a point reads are one fluid's own (hd: its A per component,
+// from the host), a warp of such points skips the denominators: 31 operations.
+struct SrcK {
+  double hdt;                      // 1/(2 dt)
+  double dx2, dy2, dz2;            // dxinv^2 ...
+  double tx2, ty2, tz2;            // 2 dxinv^2 ...
+  double px, py, pz;               // -2 dxinv ...
+  double hg[3];                    // half the body force per component
+  long long rb[2], mb[2];          // the two fluids' density and viscosity, as bits
+  double s[2], a[2][3];            // 4 rho and A of each
+};
+__global__ void __launch_bounds__(256) k_src_ab(Grid g, SrcK K, SrcIn in, const double* __restrict__ mu,
                                                 const double* __restrict__ exy, const double* __restrict__ exz,
                                                 const double* __restrict__ eyz, ABOut out) {
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -95,54 +124,50 @@ __global__ void __launch_bounds__(256) k_src_ab(Grid g, VP p, SrcIn in, const do
   if (i > g.ni || j > g.nj) return;
   const long X = 1, Y = g.sy, Z = g.sz;
   const long c = g.at(i, j, k);
-  const double r0 = __ldg(in.rho + c), n0 = __ldg(in.rhon + c);
-  // rho00 * src
-  auto rsrc = [&](int q, const double* vel, double r, double grav) {
-    return r * (__ldg(vel + c) * p.dtinv - __ldg(in.adv[q] + c) * 1.5 + __ldg(in.advo[q] + c) * 0.5 +
-                __ldg(in.fst[q] + c) * 0.5 + __ldg(in.fstn[q] + c) * 0.5 + grav) -
-           __ldg(in.prs[q] + c) + __ldg(in.vis[q] + c) * 0.5;
+  auto L = [&](const double* a, long o) { return __ldg(a + c + o); };
+  const double r0 = L(in.rho, 0), rx = L(in.rho, X), ry = L(in.rho, Y), rz = L(in.rho, Z);
+  const double n0 = L(in.rhon, 0), nx = L(in.rhon, X), ny = L(in.rhon, Y), nz = L(in.rhon, Z);
+  const double m0 = L(mu, 0), mx = L(mu, X), my = L(mu, Y), mz = L(mu, Z);
+  const double xy0 = L(exy, 0), xyx = L(exy, -X), xyy = L(exy, -Y), xz0 = L(exz, 0), xzx = L(exz, -X),
+               xzz = L(exz, -Z), yz0 = L(eyz, 0), yzy = L(eyz, -Y), yzz = L(eyz, -Z);
+  const long long rb = __double_as_longlong(r0), mb = __double_as_longlong(m0);
+  const bool flat = same_bits(r0, rx, ry, rz, n0) && same_bits(r0, nx, ny, nz, r0) && same_bits(m0, mx, my, mz, xy0) &&
+                    same_bits(m0, xyx, xyy, xz0, xzx) && same_bits(m0, xzz, yz0, yzy, yzz);
+  const int f = flat && rb == K.rb[0] && mb == K.mb[0] ? 0 : (flat && rb == K.rb[1] && mb == K.mb[1] ? 1 : -1);
+  double su, sv, sw, Au, Av, Aw;
+  if (__any_sync(__activemask(), f < 0)) {
+    const double s0 = r0 + n0;
+    su = s0 + (rx + nx);
+    sv = s0 + (ry + ny);
+    sw = s0 + (rz + nz);
+    Au = recip_h(fma(K.dz2, xzz + xz0, fma(K.dy2, xyy + xy0, fma(K.tx2, m0 + mx, su * K.hdt))));
+    Av = recip_h(fma(K.dz2, yzz + yz0, fma(K.ty2, m0 + my, fma(K.dx2, xyx + xy0, sv * K.hdt))));
+    Aw = recip_h(fma(K.tz2, m0 + mz, fma(K.dy2, yzy + yz0, fma(K.dx2, xzx + xz0, sw * K.hdt))));
+  } else {
+    su = sv = sw = f ? K.s[1] : K.s[0];
+    Au = f ? K.a[1][0] : K.a[0][0];
+    Av = f ? K.a[1][1] : K.a[0][1];
+    Aw = f ? K.a[1][2] : K.a[0][2];
+  }
+  const double p0 = L(in.phat, 0);
+  // B = A (s (vel/dt - 1.5 adv + 0.5 (advo + fst + fstn) + grav)/2 - 2 prs + vis)
+  auto store = [&](int q, const double* vel, double s, double A, double pd, double pk) {
+    const double t = (L(in.fst[q], 0) + L(in.fstn[q], 0)) + L(in.advo[q], 0);
+    const double e = fma(t, 0.25, fma(L(in.adv[q], 0), -0.75, fma(L(vel, 0), K.hdt, K.hg[q])));
+    out.a[q][c] = A;
+    out.b[q][c] = A * fma(pd, pk, fma(s, e, L(in.vis[q], 0)));
   };
-  auto store = [&](int q, double A, double B, double visn, const double* vel) {
-    if (REFINE) {
-      out.af[q][c] = (float)A;
-      out.rf[q][c] = (float)(A * visn + B - __ldg(vel + c));
-    } else {
-      out.a[q][c] = A;
-      out.b[q][c] = B;
-    }
-  };
-  {
-    const double r = (r0 + __ldg(in.rho + c + X) + n0 + __ldg(in.rhon + c + X)) * 0.25;
-    const double ap = p.dz2 * __ldg(exz + c - Z) + p.dy2 * __ldg(exy + c - Y) + p.dx2 * __ldg(mu + c) * 2.0 +
-                      p.dx2 * __ldg(mu + c + X) * 2.0 + p.dy2 * __ldg(exy + c) + p.dz2 * __ldg(exz + c);
-    const double T = recip_nr(r * p.dtinv + ap * 0.5);
-    const double vn = REFINE ? visn_at<0, double>(g, p, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
-    store(0, 0.5 * T, rsrc(0, in.u, r, in.grvb) * T, vn, in.u);
-  }
-  if (j <= g.nj - 1) {
-    const double r = (r0 + __ldg(in.rho + c + Y) + n0 + __ldg(in.rhon + c + Y)) * 0.25;
-    const double ap = p.dz2 * __ldg(eyz + c - Z) + p.dy2 * __ldg(mu + c) * 2.0 + p.dx2 * __ldg(exy + c - X) +
-                      p.dx2 * __ldg(exy + c) + p.dy2 * __ldg(mu + c + Y) * 2.0 + p.dz2 * __ldg(eyz + c);
-    const double T = recip_nr(r * p.dtinv + ap * 0.5);
-    const double vn = REFINE ? visn_at<1, double>(g, p, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
-    store(1, 0.5 * T, rsrc(1, in.v, r, in.grvp) * T, vn, in.v);
-  }
-  {
-    const double r = (r0 + __ldg(in.rho + c + Z) + n0 + __ldg(in.rhon + c + Z)) * 0.25;
-    const double ap = p.dz2 * __ldg(mu + c) * 2.0 + p.dy2 * __ldg(eyz + c - Y) + p.dx2 * __ldg(exz + c - X) +
-                      p.dx2 * __ldg(exz + c) + p.dy2 * __ldg(eyz + c) + p.dz2 * __ldg(mu + c + Z) * 2.0;
-    const double T = recip_nr(r * p.dtinv + ap * 0.5);
-    const double vn = REFINE ? visn_at<2, double>(g, p, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
-    store(2, 0.5 * T, rsrc(2, in.w, r, 0.0) * T, vn, in.w);
-  }
+  store(0, in.u, su, Au, L(in.phat, X) - p0, K.px);
+  if (j <= g.nj - 1) store(1, in.v, sv, Av, L(in.phat, Y) - p0, K.py);
+  store(2, in.w, sw, Aw, L(in.phat, Z) - p0, K.pz);
 }
 
 // k_src_ab with A and B in FP32-pair arithmetic (each double read split into a
 // pair, A and B rounded to doubles once).  The FP64-accurate step (FMF_FP64E, REFINE
 // false) stores them.  The mixed-precision step (REFINE true) forms the first-sweep
-// residual R = A visn(u) + B - u from them in FP64, as k_src_ab<true> does: the
+// residual R = A visn(u) + B - u from them in FP64: the
 // viscous sum visn reads 20 doubles for about 25 operations, and with it in pairs
-// as well the kernel measured 10.2 ms against 9.7 for k_src_ab<true> at
+// as well the kernel measured 10.2 ms against 9.7 for an all-FP64 kernel at
 // 512x256x256 (the splits cost more than the FP64 operations they replace); in
 // this form, 6.7 ms.  The momentum-factor denominator is
 // grouped as dz2 (e(-Z) + e(0)) + dy2 (e(-Y) + e(0)) + 2 dx2 (mu(0) + mu(X)) (and
@@ -163,12 +188,14 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pd, SrcIn in
   const long c = g.at(i, j, k);
   auto L = [&](const double* a, long o) { return split_double(__ldg(a + c + o)); };
   const D r0n0 = add(L(in.rho, 0), L(in.rhon, 0)), mu0 = L(mu, 0);
-  // rho00 * src
-  auto rsrc = [&](int q, const double* vel, D r, D grav) {
+  // rho00 * src; the pressure gradient as cal_grad_prs rounds it
+  const double p0 = __ldg(in.phat + c);
+  auto rsrc = [&](int q, const double* vel, D r, D grav, long S, double di) {
+    const D prs = split_double(__dmul_rn(__dsub_rn(__ldg(in.phat + c + S), p0), di));
     D t = sub(mul(L(vel, 0), p.dtinv), mulf(L(in.adv[q], 0), 1.5f));
     t = add(t, scale(add(add(L(in.advo[q], 0), L(in.fst[q], 0)), L(in.fstn[q], 0)), 0.5f));
     t = add(t, grav);
-    return add(sub(mul(r, t), L(in.prs[q], 0)), scale(L(in.vis[q], 0), 0.5f));
+    return add(sub(mul(r, t), prs), scale(L(in.vis[q], 0), 0.5f));
   };
   // A = T/2, B = rs T; REFINE: A and R = A visn + B - u (FP64) as floats
   auto store = [&](int q, D r, D ap, D rs, double vn, const double* vel) {
@@ -189,7 +216,7 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pd, SrcIn in
     ap = add(ap, mul(p.dy2, add(L(exy, -Y), L(exy, 0))));
     ap = add(ap, mul(p.dx2x2, add(mu0, L(mu, X))));
     const double vn = REFINE ? visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
-    store(0, r, ap, rsrc(0, in.u, r, p.grvb), vn, in.u);
+    store(0, r, ap, rsrc(0, in.u, r, p.grvb, X, pd.dxi), vn, in.u);
   }
   if (j <= g.nj - 1) {
     const D r = scale(add(r0n0, add(L(in.rho, Y), L(in.rhon, Y))), 0.25f);
@@ -197,7 +224,7 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pd, SrcIn in
     ap = add(ap, mul(p.dy2x2, add(mu0, L(mu, Y))));
     ap = add(ap, mul(p.dx2, add(L(exy, -X), L(exy, 0))));
     const double vn = REFINE ? visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
-    store(1, r, ap, rsrc(1, in.v, r, p.grvp), vn, in.v);
+    store(1, r, ap, rsrc(1, in.v, r, p.grvp, Y, pd.dyi), vn, in.v);
   }
   {
     const D r = scale(add(r0n0, add(L(in.rho, Z), L(in.rhon, Z))), 0.25f);
@@ -205,53 +232,72 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pd, SrcIn in
     ap = add(ap, mul(p.dy2, add(L(eyz, -Y), L(eyz, 0))));
     ap = add(ap, mul(p.dx2, add(L(exz, -X), L(exz, 0))));
     const double vn = REFINE ? visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
-    store(2, r, ap, rsrc(2, in.w, r, zero), vn, in.w);
+    store(2, r, ap, rsrc(2, in.w, r, zero, Z, pd.dzi), vn, in.w);
   }
 }
 
 // The explicit viscous term 2 div(mu S) of main.f90:538-541 (calsij, cal_arith_tau,
 // cal_div_tensor) for the interior u, v, w points, which are all the step reads.
-// k_stress forms the six stresses over i, j, k in 0..n+1 (the points the interior
-// divergence reads) straight from u, v, w and mu: tau_ii = 2 mu S_ii and, on the
-// edges, tau_ij = 2 (mean of 4 mu) S_ij with S_ij = (du_i/dx_j + du_j/dx_i)/2,
-// the factors 2, 1/2 and 1/4 folded into the constants; the strain never goes
-// through memory.  k_div_stress takes its divergence on the interior.
+// k_stress forms six stresses over i, j, k in 0..n+1 (the points the interior divergence
+// reads) straight from u, v, w and mu, each without its constant factor:
+//   t_xx = mu du (tau_xx = 2 mu du dxinv),
+//   t_xy = (sum of 4 mu) (du_y + (dyinv/dxinv)^-1 dv_x) (tau_xy = t_xy dyinv / 4), ...
+// and k_div_stress takes their divergence on the interior with the factors folded into
+// its own: 26 + 18 FP64 operations per cell against 33 + 21; where the viscosities are
+// equal bits, their sum is 4 mu exactly (see k_edges) and the first 18.  The strain never
+// goes through memory.
 // (sk, optional: the six strain components of calsij.f:28-139 at the same points,
 // kept by the adjoint's record of the step)
-__global__ void __launch_bounds__(256) k_stress(Grid g, double dxi, double dyi, double dzi,
-                                                const double* __restrict__ u, const double* __restrict__ v,
-                                                const double* __restrict__ w, const double* __restrict__ mu,
-                                                double* __restrict__ tau, double* __restrict__ sk) {
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int k = (int)blockIdx.z;
-  if (i > g.ni + 1 || j > g.nj + 1) return;
+struct StressK {
+  double dxi, dyi, dzi;
+  double rxy, rxz, ryz;        // dxinv/dyinv, dxinv/dzinv, dyinv/dzinv
+  double xx, yy, zz;           // 2 dxinv^2 ...
+  double qyy, qzz, qxy, qxz, qyz;  // dyinv^2/4, dzinv^2/4, dxinv dyinv/4, dxinv dzinv/4, dyinv dzinv/4
+};
+__global__ void __launch_bounds__(128) k_stress(Grid g, StressK K, const double* __restrict__ u,
+                                                const double* __restrict__ v, const double* __restrict__ w,
+                                                const double* __restrict__ mu, double* __restrict__ tau,
+                                                double* __restrict__ sk) {
+  const int W = g.ni + 2;
+  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  if (t >= W * (g.nj + 2)) return;
+  const int j = t / W, i = t - j * W, k = (int)blockIdx.y;
   const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
   const long c = g.at(i, j, k);
-  const double m0 = __ldg(mu + c), mx = __ldg(mu + c + X), my = __ldg(mu + c + Y), mz = __ldg(mu + c + Z);
+  const double m0 = __ldg(mu + c), mx = __ldg(mu + c + X), my = __ldg(mu + c + Y), mz = __ldg(mu + c + Z),
+               mxy = __ldg(mu + c + X + Y), mxz = __ldg(mu + c + X + Z), myz = __ldg(mu + c + Y + Z);
   const double u0 = __ldg(u + c), v0 = __ldg(v + c), w0 = __ldg(w + c);
-  const double hx = 0.25 * dxi, hy = 0.25 * dyi, hz = 0.25 * dzi;
-  tau[c] = (u0 - __ldg(u + c - X)) * m0 * (2.0 * dxi);
-  tau[c + n] = (v0 - __ldg(v + c - Y)) * m0 * (2.0 * dyi);
-  tau[c + 2 * n] = (w0 - __ldg(w + c - Z)) * m0 * (2.0 * dzi);
-  tau[c + 3 * n] = ((__ldg(u + c + Y) - u0) * hy + (__ldg(v + c + X) - v0) * hx) *
-                   ((m0 + mx) + (my + __ldg(mu + c + X + Y)));
-  tau[c + 4 * n] = ((__ldg(u + c + Z) - u0) * hz + (__ldg(w + c + X) - w0) * hx) *
-                   ((m0 + mx) + (mz + __ldg(mu + c + X + Z)));
-  tau[c + 5 * n] = ((__ldg(v + c + Z) - v0) * hz + (__ldg(w + c + Y) - w0) * hy) *
-                   ((m0 + my) + (mz + __ldg(mu + c + Y + Z)));
+  const double dux = u0 - __ldg(u + c - X), dvy = v0 - __ldg(v + c - Y), dwz = w0 - __ldg(w + c - Z);
+  const double duy = __ldg(u + c + Y) - u0, dvx = __ldg(v + c + X) - v0, duz = __ldg(u + c + Z) - u0,
+               dwx = __ldg(w + c + X) - w0, dvz = __ldg(v + c + Z) - v0, dwy = __ldg(w + c + Y) - w0;
+  const bool flat = same_bits(m0, mx, my, mz, mxy) && same_bits(m0, mxz, myz, m0, m0);
+  double sxy, sxz, syz;
+  if (__any_sync(__activemask(), !flat)) {
+    const double mx0 = m0 + mx, my0 = m0 + my;
+    sxy = mx0 + (my + mxy);
+    sxz = mx0 + (mz + mxz);
+    syz = my0 + (mz + myz);
+  } else {
+    sxy = sxz = syz = 4.0 * m0;
+  }
+  tau[c] = dux * m0;
+  tau[c + n] = dvy * m0;
+  tau[c + 2 * n] = dwz * m0;
+  tau[c + 3 * n] = fma(dvx, K.rxy, duy) * sxy;
+  tau[c + 4 * n] = fma(dwx, K.rxz, duz) * sxz;
+  tau[c + 5 * n] = fma(dwy, K.ryz, dvz) * syz;
   if (sk) {
-    sk[c] = (u0 - __ldg(u + c - X)) * dxi;
-    sk[c + n] = (v0 - __ldg(v + c - Y)) * dyi;
-    sk[c + 2 * n] = (w0 - __ldg(w + c - Z)) * dzi;
-    sk[c + 3 * n] = ((__ldg(u + c + Y) - u0) * dyi + (__ldg(v + c + X) - v0) * dxi) * 0.5;
-    sk[c + 4 * n] = ((__ldg(u + c + Z) - u0) * dzi + (__ldg(w + c + X) - w0) * dxi) * 0.5;
-    sk[c + 5 * n] = ((__ldg(v + c + Z) - v0) * dzi + (__ldg(w + c + Y) - w0) * dyi) * 0.5;
+    sk[c] = dux * K.dxi;
+    sk[c + n] = dvy * K.dyi;
+    sk[c + 2 * n] = dwz * K.dzi;
+    sk[c + 3 * n] = (duy * K.dyi + dvx * K.dxi) * 0.5;
+    sk[c + 4 * n] = (duz * K.dzi + dwx * K.dxi) * 0.5;
+    sk[c + 5 * n] = (dvz * K.dzi + dwy * K.dyi) * 0.5;
   }
 }
-__global__ void __launch_bounds__(256) k_div_stress(Grid g, double dxi, double dyi, double dzi,
-                                                    const double* __restrict__ t, double* __restrict__ vu,
-                                                    double* __restrict__ vv, double* __restrict__ vw) {
+__global__ void __launch_bounds__(256) k_div_stress(Grid g, StressK K, const double* __restrict__ t,
+                                                    double* __restrict__ vu, double* __restrict__ vv,
+                                                    double* __restrict__ vw) {
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   const int k = 1 + (int)blockIdx.z;
@@ -265,14 +311,14 @@ __global__ void __launch_bounds__(256) k_div_stress(Grid g, double dxi, double d
   const double* t5 = t + 4 * n;
   const double* t6 = t + 5 * n;
   const double a4 = __ldg(t4 + c), a5 = __ldg(t5 + c), a6 = __ldg(t6 + c);
-  vu[c] = (__ldg(t1 + c + X) - __ldg(t1 + c)) * dxi + (a4 - __ldg(t4 + c - Y)) * dyi + (a5 - __ldg(t5 + c - Z)) * dzi;
-  vv[c] = (a4 - __ldg(t4 + c - X)) * dxi + (__ldg(t2 + c + Y) - __ldg(t2 + c)) * dyi + (a6 - __ldg(t6 + c - Z)) * dzi;
-  vw[c] = (a5 - __ldg(t5 + c - X)) * dxi + (a6 - __ldg(t6 + c - Y)) * dyi + (__ldg(t3 + c + Z) - __ldg(t3 + c)) * dzi;
+  vu[c] = (__ldg(t1 + c + X) - __ldg(t1 + c)) * K.xx + (a4 - __ldg(t4 + c - Y)) * K.qyy + (a5 - __ldg(t5 + c - Z)) * K.qzz;
+  vv[c] = (a4 - __ldg(t4 + c - X)) * K.qxy + (__ldg(t2 + c + Y) - __ldg(t2 + c)) * K.yy + (a6 - __ldg(t6 + c - Z)) * K.qzz;
+  vw[c] = (a5 - __ldg(t5 + c - X)) * K.qxz + (a6 - __ldg(t6 + c - Y)) * K.qyz + (__ldg(t3 + c + Z) - __ldg(t3 + c)) * K.zz;
 }
 
-// The FP64-accurate and mixed-precision steps: k_stress and k_div_stress in
-// FP32-pair arithmetic (each double read split into a pair, each output rounded to
-// a double once); the same sums in the same grouping.
+// The FP64-accurate and mixed-precision steps: the stresses themselves and their
+// divergence in FP32-pair arithmetic (each double read split into a pair, each output
+// rounded to a double once).
 // With sk (the adjoint's record of a mixed-precision step) the strain components
 // are written as well, in FP64 as k_stress forms them.
 struct VPT {
@@ -1076,6 +1122,9 @@ bool one_pass_refresh(const Grid& g) {
 
 VP make_vp(double dxinv, double dyinv, double dzinv, double dt, int harmonic) {
   VP p;
+  p.dxi = dxinv;
+  p.dyi = dyinv;
+  p.dzi = dzinv;
   p.dtinv = dt > 0.0 ? 1.0 / dt : 0.0;
   p.dx2 = dxinv * dxinv;
   p.dy2 = dyinv * dyinv;
@@ -1099,11 +1148,11 @@ const int kPi[4] = {1, 1, 1, 2}, kPj[4] = {1, 1, 2, 1}, kPk[4] = {1, 2, 1, 1};
 // k_edges + k_src_ab<REFINE> + k_wall_coef
 template <bool REFINE>
 void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const double* v, const double* w,
-              const double* const* adv, const double* const* advo, const double* const* prs,
+              const double* const* adv, const double* const* advo, const double* phat,
               const double* const* vis, const double* const* fst, const double* const* fstn, double grvb,
-              double grvp, const double* mu, const double* rho, const double* rhon, double* const* E, F3 ef,
-              ABOut out, const double* l1, const double* l2, const double* phi, double dy, double* wallc,
-              bool pairs = false) {
+              double grvp, const Fluids& fl, const double* mu, const double* rho, const double* rhon, double* const* E,
+              F3 ef, ABOut out, const double* l1, const double* l2, const double* phi, double dy, double* wallc,
+              bool pairs) {
   SrcIn in;
   in.u = u;
   in.v = v;
@@ -1113,14 +1162,15 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
   for (int q = 0; q < 3; ++q) {
     in.adv[q] = adv[q];
     in.advo[q] = advo[q];
-    in.prs[q] = prs[q];
     in.vis[q] = vis[q];
     in.fst[q] = fst[q];
     in.fstn[q] = fstn[q];
   }
+  in.phat = phat;
   in.grvb = grvb;
   in.grvp = grvp;
-  k_edges<<<dim3((g.ni + 1 + 31) / 32, (g.nj + 1 + 7) / 8, g.nk + 1), kB, 0, s>>>(g, p, mu, E[0], E[1], E[2], ef);
+  k_edges<<<dim3((unsigned)(((long)(g.ni + 1) * (g.nj + 1) + 127) / 128), (unsigned)(g.nk + 1)), 128, 0, s>>>(
+      g, p, mu, E[0], E[1], E[2], ef);
   if (pairs) {
     using df::split_double;
     VPS ps;
@@ -1136,7 +1186,31 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
     k_src_ab_e<REFINE><<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, ps, p, in, mu, E[0], E[1],
                                                                                  E[2], out);
   } else {
-    k_src_ab<REFINE><<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, p, in, mu, E[0], E[1], E[2], out);
+    SrcK K;
+    K.hdt = 0.5 * p.dtinv;
+    K.dx2 = p.dx2;
+    K.dy2 = p.dy2;
+    K.dz2 = p.dz2;
+    K.tx2 = 2.0 * p.dx2;
+    K.ty2 = 2.0 * p.dy2;
+    K.tz2 = 2.0 * p.dz2;
+    K.px = -2.0 * p.dxi;
+    K.py = -2.0 * p.dyi;
+    K.pz = -2.0 * p.dzi;
+    K.hg[0] = 0.5 * grvb;
+    K.hg[1] = 0.5 * grvp;
+    K.hg[2] = 0.0;
+    const double rf[2] = {fl.rhol, fl.rhog}, mf[2] = {fl.rmul, fl.rmug};
+    for (int q = 0; q < 2; ++q) {
+      std::memcpy(&K.rb[q], &rf[q], sizeof(double));
+      std::memcpy(&K.mb[q], &mf[q], sizeof(double));
+      K.s[q] = 4.0 * rf[q];
+      const double xx = 2.0 * mf[q] * p.dx2, yy = 2.0 * mf[q] * p.dy2, zz = 2.0 * mf[q] * p.dz2;
+      K.a[q][0] = 1.0 / (2.0 * rf[q] * p.dtinv + 2.0 * xx + yy + zz);
+      K.a[q][1] = 1.0 / (2.0 * rf[q] * p.dtinv + xx + 2.0 * yy + zz);
+      K.a[q][2] = 1.0 / (2.0 * rf[q] * p.dtinv + xx + yy + 2.0 * zz);
+    }
+    k_src_ab<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, K, in, mu, E[0], E[1], E[2], out);
   }
   k_wall_coef<<<wall_grid(g), kB, 0, s>>>(g, dy, l1, l2, phi, wallc);
   count_launch(3);
@@ -1161,17 +1235,17 @@ void sweep_all(cudaStream_t s, const Grid& g, double* part, double* errsum, Pair
 
 void src_visc_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt, int harmonic,
                    double grvb, double grvp, const double* u, const double* v, const double* w,
-                   const double* const* adv, const double* const* advo, const double* const* prs,
-                   const double* const* vis, const double* const* fst, const double* const* fstn, const double* mu,
-                   const double* rho, const double* rhon, double* const* E, double* const* AB, const double* l1,
+                   const double* const* adv, const double* const* advo, const double* phat,
+                   const double* const* vis, const double* const* fst, const double* const* fstn, const Fluids& fl,
+                   const double* mu, const double* rho, const double* rhon, double* const* E, double* const* AB, const double* l1,
                    const double* l2, const double* phi, double dy, double* wallc, bool pairs) {
   ABOut out{};
   for (int q = 0; q < 3; ++q) {
     out.a[q] = AB[2 * q];
     out.b[q] = AB[2 * q + 1];
   }
-  src_prep<false>(s, g, make_vp(dxinv, dyinv, dzinv, dt, harmonic), u, v, w, adv, advo, prs, vis, fst, fstn, grvb,
-                  grvp, mu, rho, rhon, E, F3{{nullptr, nullptr, nullptr}}, out, l1, l2, phi, dy, wallc, pairs);
+  src_prep<false>(s, g, make_vp(dxinv, dyinv, dzinv, dt, harmonic), u, v, w, adv, advo, phat, vis, fst, fstn, grvb,
+                  grvp, fl, mu, rho, rhon, E, F3{{nullptr, nullptr, nullptr}}, out, l1, l2, phi, dy, wallc, pairs);
 }
 
 void wall_coef(cudaStream_t s, const Grid& g, double dy, const double* l1, const double* l2, const double* phi,
@@ -1204,10 +1278,12 @@ void explicit_viscous(cudaStream_t s, const Grid& g, double dxinv, double dyinv,
     count_launch(2);
     return;
   }
-  k_stress<<<dim3((g.ni + 2 + 31) / 32, (g.nj + 2 + 7) / 8, g.nk + 2), kB, 0, s>>>(g, dxinv, dyinv, dzinv, u, v, w,
-                                                                               mu, tau, sk);
-  k_div_stress<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, dxinv, dyinv, dzinv, tau, vis[0],
-                                                                         vis[1], vis[2]);
+  const StressK K{dxinv, dyinv, dzinv, dxinv / dyinv, dxinv / dzinv, dyinv / dzinv, 2.0 * dxinv * dxinv,
+                  2.0 * dyinv * dyinv, 2.0 * dzinv * dzinv, 0.25 * dyinv * dyinv, 0.25 * dzinv * dzinv,
+                  0.25 * dxinv * dyinv, 0.25 * dxinv * dzinv, 0.25 * dyinv * dzinv};
+  k_stress<<<dim3((unsigned)(((long)(g.ni + 2) * (g.nj + 2) + 127) / 128), (unsigned)(g.nk + 2)), 128, 0, s>>>(
+      g, K, u, v, w, mu, tau, sk);
+  k_div_stress<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, K, tau, vis[0], vis[1], vis[2]);
   count_launch(2);
 }
 
@@ -1257,9 +1333,9 @@ long refine_floats(const Grid& g, int part) {
 
 void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt, int harmonic,
                  double grvb, double grvp, const double* u, const double* v, const double* w,
-                 const double* const* adv, const double* const* advo, const double* const* prs,
-                 const double* const* vis, const double* const* fst, const double* const* fstn, const double* mu,
-                 const double* rho, const double* rhon, double* const* E, const double* l1, const double* l2,
+                 const double* const* adv, const double* const* advo, const double* phat,
+                 const double* const* vis, const double* const* fst, const double* const* fstn, const Fluids& fl,
+                 const double* mu, const double* rho, const double* rhon, double* const* E, const double* l1, const double* l2,
                  const double* phi, double dy, double uwall, double* wallc, const RefineBufs& rb) {
   ABOut out{};
   for (int q = 0; q < 3; ++q) {
@@ -1267,8 +1343,8 @@ void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
     out.rf[q] = rb.r[q];
   }
   // A and B in FP32 pairs, the residual in FP64 (k_src_ab_e<true>)
-  src_prep<true>(s, g, make_vp(dxinv, dyinv, dzinv, dt, harmonic), u, v, w, adv, advo, prs, vis, fst, fstn, grvb,
-                 grvp, mu, rho, rhon, E, F3{{rb.e[0], rb.e[1], rb.e[2]}}, out, l1, l2, phi, dy, wallc, true);
+  src_prep<true>(s, g, make_vp(dxinv, dyinv, dzinv, dt, harmonic), u, v, w, adv, advo, phat, vis, fst, fstn, grvb,
+                 grvp, fl, mu, rho, rhon, E, F3{{rb.e[0], rb.e[1], rb.e[2]}}, out, l1, l2, phi, dy, wallc, true);
   k_to_float<<<4 * 152, 256, 0, s>>>(g.n, mu, rb.mu);
   k_gamma_wall<<<wall_grid(g), kB, 0, s>>>(g, uwall, wallc, u, v, w, rb.gw);
   k_gamma_x<<<xh_grid(g), kB, 0, s>>>(g, u, v, w, rb.gx);

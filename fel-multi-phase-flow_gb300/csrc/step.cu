@@ -81,7 +81,7 @@ struct fmf_ctx {
   double *theta0, *zeta, *l1, *l2, *theta;
   // work
   double *phix, *phiy, *phiz, *flx, *fly, *flz, *rho, *rhon, *rmu, *rmun;
-  double *adv[3], *advo[3], *phat, *prs[3], *tau, *vis[3];
+  double *adv[3], *advo[3], *phat, *tau, *vis[3];
   double *rn[4], *rnn[4], *rkap, *rkapn, *fst[3], *fstn[3], *sfst[3], *sfstn[3], *src[3];
   double *edge[3], *ab[6], *wallc, *sorpart;  // fused viscous solve (fused_visc.cu)
   double *dp, *div, *pr, *pi;
@@ -263,7 +263,6 @@ int fmf_ctx_create(const fmf_params* prm, fmf_ctx** out) {
   for (int q = 0; q < 3; ++q) {
     c->adv[q] = alloc(c, n);
     c->advo[q] = alloc(c, n);
-    c->prs[q] = alloc(c, n);
     c->vis[q] = alloc(c, n);
     c->fst[q] = alloc(c, n);
     c->fstn[q] = alloc(c, n);
@@ -559,7 +558,6 @@ static void seg_pre2(fmf_ctx* c) {
     fused::weno5_both(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->uo, c->vo, c->wo, c->adv, c->advo, c->wprec,
                       c->wsplit);
   op::calphat(s, g, c->p, c->po, c->phat);
-  op::cal_grad_prs(s, g, dxinv, dyinv, dzinv, c->phat, c->prs[0], c->prs[1], c->prs[2]);
   fused::explicit_viscous(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->rmu, c->tau, c->vis, nullptr,
                           c->wprec != 0);
   // :545-570 surface tension (sfst carried over from the previous step's sfstn where
@@ -573,7 +571,7 @@ static void seg_pre2(fmf_ctx* c) {
   // :579-603 (cal_av of rho/rhon at :571-573 feeds nothing downstream)
   const double* advp[3] = {c->adv[0], c->adv[1], c->adv[2]};
   const double* advop[3] = {c->advo[0], c->advo[1], c->advo[2]};
-  const double* prsp[3] = {c->prs[0], c->prs[1], c->prs[2]};
+  const fused::Fluids fl{P.rhol, P.rhog, P.rmul, P.rmug};
   const double* visp[3] = {c->vis[0], c->vis[1], c->vis[2]};
   const double* fstp[3] = {c->sfst[0], c->sfst[1], c->sfst[2]};
   const double* fstnp[3] = {c->sfstn[0], c->sfstn[1], c->sfstn[2]};
@@ -583,12 +581,12 @@ static void seg_pre2(fmf_ctx* c) {
     // the FP64 residual at u and the wall/halo constants of the correction solve;
     // un = u (:605-607) holds implicitly through zero corrections
     fused::refine_prep(s, g, dxinv, dyinv, dzinv, dt, P.harmonic, P.grvb, P.grvp, c->u, c->v, c->w, advp, advop,
-                       prsp, visp, fstp, fstnp, c->rmun, c->rho, c->rhon, c->edge, c->l1, c->l2, phi1, P.dy, P.uwall,
+                       c->phat, visp, fstp, fstnp, fl, c->rmun, c->rho, c->rhon, c->edge, c->l1, c->l2, phi1, P.dy, P.uwall,
                        c->wallc, c->rb);
     return;
   }
   fused::src_visc_prep(s, g, dxinv, dyinv, dzinv, dt, P.harmonic, P.grvb, P.grvp, c->u, c->v, c->w, advp, advop,
-                       prsp, visp, fstp, fstnp, c->rmun, c->rho, c->rhon, c->edge, c->ab, c->l1, c->l2, phi1, P.dy,
+                       c->phat, visp, fstp, fstnp, fl, c->rmun, c->rho, c->rhon, c->edge, c->ab, c->l1, c->l2, phi1, P.dy,
                        c->wallc, c->wprec == 2);
   // :605-607
   op::copy(s, n, c->u, c->un);
@@ -940,12 +938,12 @@ int fmf_ctx_check_sor(fmf_ctx* c, double* out) {
     // the FP64 factors of the same system
     const double* advp[3] = {c->adv[0], c->adv[1], c->adv[2]};
     const double* advop[3] = {c->advo[0], c->advo[1], c->advo[2]};
-    const double* prsp[3] = {c->prs[0], c->prs[1], c->prs[2]};
+    const fused::Fluids fl{P.rhol, P.rhog, P.rmul, P.rmug};
     const double* visp[3] = {c->vis[0], c->vis[1], c->vis[2]};
     const double* fstp[3] = {c->sfst[0], c->sfst[1], c->sfst[2]};
     const double* fstnp[3] = {c->sfstn[0], c->sfstn[1], c->sfstn[2]};
     fused::src_visc_prep(s, g, dxinv, dyinv, dzinv, P.dt, P.harmonic, P.grvb, P.grvp, c->u, c->v, c->w, advp, advop,
-                         prsp, visp, fstp, fstnp, c->rmun, c->rho, c->rhon, c->edge, c->ab, c->l1, c->l2,
+                         c->phat, visp, fstp, fstnp, fl, c->rmun, c->rho, c->rhon, c->edge, c->ab, c->l1, c->l2,
                          c->phi + n, P.dy, c->wallc);
   }
   double *q64[3] = {q, q + n, q + 2 * n}, *qx[3] = {q + 3 * n, q + 4 * n, q + 5 * n};
