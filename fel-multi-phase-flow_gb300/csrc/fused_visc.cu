@@ -12,14 +12,17 @@
 // colours that differ in every index parity never read each other, so one launch
 // per pair gives the sequential result.  The wall/halo refresh after every second
 // colour (bndu + bnd_periodic of the swept component, solu_sor4.f:176-180) is one
-// kernel (k_refresh; three ordered plane kernels on grids under 8 cells a side).
+// kernel (k_refresh; three ordered plane kernels on grids under 8 cells a side) after a
+// component's first pair and done by the sweep itself after the others.
 //
 // The mixed-precision step solves the same system by one step of iterative
 // refinement: the residual of the first sweep is formed in FP64 at u, then the
 // sweeps run in FP32 on the correction d = un - u (FP32 storage and arithmetic),
 // and un = u + d is formed in FP64 at the end.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 
 #include "df64.cuh"
 #include "fused.cuh"
@@ -96,8 +99,17 @@ struct ABOut {
   double *a[3], *b[3];
   float *af[3], *rf[3];
 };
+// the grid factors in the arithmetic type of a viscous sum, converted on the host (a
+// conversion in a kernel takes an FP64-pipe slot)
+template <class T>
+struct Fac {
+  T dx2, dy2, dz2, dxy, dxz, dyz;
+  Fac() = default;
+  explicit Fac(const VP& p)
+      : dx2((T)p.dx2), dy2((T)p.dy2), dz2((T)p.dz2), dxy((T)p.dxy), dxz((T)p.dxz), dyz((T)p.dyz) {}
+};
 template <int COMP, class T>
-__device__ __forceinline__ T visn_at(const Grid& g, const VP& p, long c, const T* __restrict__ mu,
+__device__ __forceinline__ T visn_at(const Grid& g, const Fac<T>& p, long c, const T* __restrict__ mu,
                                      const T* __restrict__ exy, const T* __restrict__ exz,
                                      const T* __restrict__ eyz, const T* un, const T* vn, const T* wn);
 // FP64 (the FP64 step).  With s = the sum of the four densities (4 rho00), T's
@@ -176,7 +188,7 @@ struct VPS {
   df::D dtinv, dx2, dy2, dz2, dx2x2, dy2x2, dz2x2, grvb, grvp;
 };
 template <bool REFINE>
-__global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pd, SrcIn in, const double* __restrict__ mu,
+__global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pv, Fac<double> pd, SrcIn in, const double* __restrict__ mu,
                                                   const double* __restrict__ exy, const double* __restrict__ exz,
                                                   const double* __restrict__ eyz, ABOut out) {
   using namespace df;
@@ -216,7 +228,7 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pd, SrcIn in
     ap = add(ap, mul(p.dy2, add(L(exy, -Y), L(exy, 0))));
     ap = add(ap, mul(p.dx2x2, add(mu0, L(mu, X))));
     const double vn = REFINE ? visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
-    store(0, r, ap, rsrc(0, in.u, r, p.grvb, X, pd.dxi), vn, in.u);
+    store(0, r, ap, rsrc(0, in.u, r, p.grvb, X, pv.dxi), vn, in.u);
   }
   if (j <= g.nj - 1) {
     const D r = scale(add(r0n0, add(L(in.rho, Y), L(in.rhon, Y))), 0.25f);
@@ -224,7 +236,7 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pd, SrcIn in
     ap = add(ap, mul(p.dy2x2, add(mu0, L(mu, Y))));
     ap = add(ap, mul(p.dx2, add(L(exy, -X), L(exy, 0))));
     const double vn = REFINE ? visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
-    store(1, r, ap, rsrc(1, in.v, r, p.grvp, Y, pd.dyi), vn, in.v);
+    store(1, r, ap, rsrc(1, in.v, r, p.grvp, Y, pv.dyi), vn, in.v);
   }
   {
     const D r = scale(add(r0n0, add(L(in.rho, Z), L(in.rhon, Z))), 0.25f);
@@ -232,7 +244,7 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pd, SrcIn in
     ap = add(ap, mul(p.dy2, add(L(eyz, -Y), L(eyz, 0))));
     ap = add(ap, mul(p.dx2, add(L(exz, -X), L(exz, 0))));
     const double vn = REFINE ? visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
-    store(2, r, ap, rsrc(2, in.w, r, zero, Z, pd.dzi), vn, in.w);
+    store(2, r, ap, rsrc(2, in.w, r, zero, Z, pv.dzi), vn, in.w);
   }
 }
 
@@ -379,18 +391,13 @@ __global__ void __launch_bounds__(256) k_div_stress_e(Grid g, VPT p, const doubl
                         mul(sub(L(2, Z), L(2, 0)), p.dzi)));
 }
 
-// One colour pair of one component.  Thread (a, b, kk) covers, for the pair whose
-// first colour has parities (pi,pj,pk), the point (pi+2a, pj+2b, pk+2kk) and the
-// point of the second colour (all parities flipped) at (pi'+2a, pj'+2b, pk'+2kk).
-// T is the storage type of the iterates and coefficients and the arithmetic type.
-//
 // visn of component COMP at point c (solu_sor4.f:150-170 without the A/B factors)
 template <int COMP, class T>
-__device__ __forceinline__ T visn_at(const Grid& g, const VP& p, long c, const T* __restrict__ mu,
+__device__ __forceinline__ T visn_at(const Grid& g, const Fac<T>& p, long c, const T* __restrict__ mu,
                                      const T* __restrict__ exy, const T* __restrict__ exz,
                                      const T* __restrict__ eyz, const T* un, const T* vn, const T* wn) {
   const long X = 1, Y = g.sy, Z = g.sz;
-  const T dx2 = (T)p.dx2, dy2 = (T)p.dy2, dz2 = (T)p.dz2, dxy = (T)p.dxy, dxz = (T)p.dxz, dyz = (T)p.dyz;
+  const T dx2 = p.dx2, dy2 = p.dy2, dz2 = p.dz2, dxy = p.dxy, dxz = p.dxz, dyz = p.dyz;
   auto U = [&](long o) { return un[c + o]; };
   auto V = [&](long o) { return vn[c + o]; };
   auto W = [&](long o) { return wn[c + o]; };
@@ -413,41 +420,189 @@ __device__ __forceinline__ T visn_at(const Grid& g, const VP& p, long c, const T
   }
 }
 
+// --- the colour-pair sweeps ----------------------------------------------------------
+// visn of component COMP in the sweeps.  FP64: with S the component's own axis and, per
+// transverse axis T with its edge viscosity e and field F,
+//   e(-T) (q(-T) + r (F(-T) - F(S-T))) + e(0) (q(T) + r (F(S) - F(0))),  r = dSinv/dTinv,
+// times dTinv^2: 17 operations, as visn_at's 19 in another grouping.  FP32: visn_at.
+template <class T>
+struct SweepK;
+template <>
+struct SweepK<double> {
+  double own, t1, t2, r1, r2;  // 2 dSinv^2, dTinv^2 and r of the two transverse axes
+  SweepK(const VP& p, int comp) {
+    const double d[3] = {p.dxi, p.dyi, p.dzi};
+    const double s = d[comp], a = d[comp == 0 ? 1 : 0], b = d[comp == 2 ? 1 : 2];
+    own = 2.0 * s * s;
+    t1 = a * a;
+    t2 = b * b;
+    r1 = s / a;
+    r2 = s / b;
+  }
+};
+template <>
+struct SweepK<float> {
+  Fac<float> f;
+  SweepK(const VP& p, int) : f(p) {}
+};
+template <int COMP>
+__device__ __forceinline__ double visn_sweep(const Grid& g, const SweepK<double>& K, long c, const double* __restrict__ mu,
+                                             const double* __restrict__ exy, const double* __restrict__ exz,
+                                             const double* __restrict__ eyz, const double* un, const double* vn,
+                                             const double* wn) {
+  const long X = 1, Y = g.sy, Z = g.sz;
+  const long S = COMP == 0 ? X : (COMP == 1 ? Y : Z), T1 = COMP == 0 ? Y : X, T2 = COMP == 2 ? Y : Z;
+  const double *q = (COMP == 0 ? un : (COMP == 1 ? vn : wn)) + c, *f1 = (COMP == 0 ? vn : un) + c,
+               *f2 = (COMP == 2 ? vn : wn) + c;
+  const double *e1 = (COMP == 2 ? exz : exy) + c, *e2 = (COMP == 0 ? exz : eyz) + c;
+  const double a = fma(__ldg(e1), fma(K.r1, f1[S] - f1[0], q[T1]),
+                       __ldg(e1 - T1) * fma(K.r1, f1[-T1] - f1[S - T1], q[-T1]));
+  const double b = fma(__ldg(e2), fma(K.r2, f2[S] - f2[0], q[T2]),
+                       __ldg(e2 - T2) * fma(K.r2, f2[-T2] - f2[S - T2], q[-T2]));
+  const double o = fma(__ldg(mu + c + S), q[S], __ldg(mu + c) * q[-S]);
+  return fma(K.own, o, fma(K.t1, a, K.t2 * b));
+}
+template <int COMP>
+__device__ __forceinline__ float visn_sweep(const Grid& g, const SweepK<float>& K, long c, const float* __restrict__ mu,
+                                            const float* __restrict__ exy, const float* __restrict__ exz,
+                                            const float* __restrict__ eyz, const float* un, const float* vn,
+                                            const float* wn) {
+  return visn_at<COMP, float>(g, K.f, c, mu, exy, exz, eyz, un, vn, wn);
+}
+
+// The ghost points that one updated point of the swept component fills (k_refresh and
+// k_refresh_d below, seen from the source): its x and z images (the plain periodic copy)
+// and, next to a wall, the wall rows of its column with their images.  ni, nj, nk >= 8.
+struct Ghosts64 {
+  double uwall;
+  const double* wc;
+};
+template <int COMP>
+__device__ __noinline__ void fill_ghosts(const Grid& g, const Ghosts64& G, double* q, int i, int j, int k, double v) {
+  const int NI = g.ni, NJ = g.nj, NK = g.nk;
+  const int ix = i <= 3 ? i + NI : (i >= NI - 2 ? i - NI : i), kx = k <= 3 ? k + NK : (k >= NK - 2 ? k - NK : k);
+  auto put = [&](int jj, double x, bool base) {
+    if (base) q[g.at(i, jj, k)] = x;
+    if (ix != i) q[g.at(ix, jj, k)] = x;
+    if (kx != k) {
+      q[g.at(i, jj, kx)] = x;
+      if (ix != i) q[g.at(ix, jj, kx)] = x;
+    }
+  };
+  put(j, v, false);
+  if (COMP == 1) {  // v(-m) = -v(m), m = 1, 2; v(nj+m) = -v(nj-m), m = 1..3
+    if (j <= 2) put(-j, -v, true);
+    if (j >= NJ - 3) put(2 * NJ - j, -v, true);
+  } else if (j == 1 || j == NJ) {
+    const int side = j == 1 ? 0 : 1, t = side ? 1 : -1;
+    const double* wc = G.wc + (((long)side * (NK + 6) + (k + 2)) * (NI + 6) + (i + 2)) * 2;
+    const double c2 = wc[1];
+    const double x1 = COMP == 0 ? fma(c2, v, wc[0] * (side ? G.uwall : -G.uwall)) : c2 * v;
+    const double x2 = 2.0 * x1 - v;
+    put(j + t, x1, true);
+    put(j + 2 * t, x2, true);
+    put(j + 3 * t, 2.0 * x2 - x1, true);
+  }
+}
+// the same on the mixed step's corrections, each with its constant (k_refresh_d)
+struct Ghosts32 {
+  const float *gw, *gx, *gz;
+};
+constexpr int kGW = 12, kGH = 24;
+__device__ __forceinline__ long wall_slot(const Grid& g, int side, int k, int i) {
+  return (((long)side * (g.nk + 6) + (k + 2)) * (g.ni + 6) + (i + 2));
+}
+__device__ __forceinline__ int gslot(int d, int N, int sh) { return d <= 0 ? d + 2 : d - N + 2 - sh; }
+template <int COMP>
+__device__ __noinline__ void fill_ghosts(const Grid& g, const Ghosts32& G, float* q, int i, int j, int k, float v) {
+  const int NI = g.ni, NJ = g.nj, NK = g.nk;
+  constexpr int xb = COMP == 0 ? 0 : 6 * COMP + 6, zb = 6 * COMP;
+  const int ix = i <= 3 ? i + NI : (i >= NI - 2 ? i - NI : i), kx = k <= 3 ? k + NK : (k >= NK - 2 ? k - NK : k);
+  auto gz = [&](int ii, int jj) {
+    return __ldg(G.gz + ((long)(jj + 2) * (NI + 6) + (ii + 2)) * kGH + zb + gslot(kx, NK, 0));
+  };
+  auto put = [&](int jj, float x, bool base) {
+    if (base) q[g.at(i, jj, k)] = x;
+    if (kx != k) q[g.at(i, jj, kx)] = x + gz(i, jj);
+    if (ix != i) {
+      const float y = x + __ldg(G.gx + ((long)(k + 2) * (NJ + 6) + (jj + 2)) * kGH + xb + gslot(ix, NI, 0));
+      q[g.at(ix, jj, k)] = y;
+      if (kx != k) q[g.at(ix, jj, kx)] = y + gz(ix, jj);
+    }
+  };
+  put(j, v, false);
+  if (COMP == 1) {
+    const float* c0 = G.gw + wall_slot(g, 0, k, i) * kGW + 4;
+    const float* c1 = G.gw + wall_slot(g, 1, k, i) * kGW + 4;
+    if (j <= 2) put(-j, -v + __ldg(c0 + j), true);
+    if (j >= NJ - 3 && j < NJ) put(2 * NJ - j, -v + __ldg(c1 + NJ - j), true);
+  } else if (j == 1 || j == NJ) {
+    const int side = j == 1 ? 0 : 1, t = side ? 1 : -1;
+    const float* c = G.gw + wall_slot(g, side, k, i) * kGW;
+    const float* h = c + (COMP == 0 ? 1 : 8);
+    const float x1 = __ldg(c) * v + __ldg(h), x2 = 2.f * x1 - v + __ldg(h + 1), x3 = 2.f * x2 - x1 + __ldg(h + 2);
+    put(j + t, x1, true);
+    put(j + 2 * t, x2, true);
+    put(j + 3 * t, x3, true);
+  }
+}
+
+// One colour pair of one component, whose first colour has parities (pi, pj, pk); the
+// second has all three flipped.  Thread (a, b) of a colour's (i, j) plane takes kz points
+// of its column, of both colours (BOTH) or of the one blockIdx.z says.
 // T = double: the FP64 step, q_new = A*visn(q) + B on the velocity itself.
 // T = float: the mixed-precision step, d_new = A*visn(d) + R on the correction
 // d = un - u (R is the FP64 first-sweep residual; see refine_prep).
-// part[block] = the block's sum of (q_new - q)^2.
-template <int COMP, class T>
-__global__ void __launch_bounds__(256) k_pair(Grid g, VP p, int pi, int pj, int pk, const T* __restrict__ mu,
-                                              const T* __restrict__ exy, const T* __restrict__ exz,
-                                              const T* __restrict__ eyz, const T* __restrict__ A,
-                                              const T* __restrict__ B, T* un, T* vn, T* wn,
-                                              double* __restrict__ part) {
-  __shared__ T sh[8];
+// GHOSTS: the ghost points of the swept component are refreshed by the points they come
+// from.  The other points of the pair do not read them: an image has its source's
+// colour, and a wall row is read by its own column's point alone, before that writes it.
+// part[block] = (first) or += the block's sum of (q_new - q)^2.
+// The FP64 sweep is bound by the FP64 pipe (20 operations per point and 0.4 for its sum;
+// visn_at's grouping and a shuffle tree per warp took 25): 431 -> 340 us per pair with its
+// refresh at 512x256x256, 12.9 -> 7.6 at 32x32x16.
+template <int COMP, class T, class G, bool GHOSTS, bool BOTH>
+__global__ void __launch_bounds__(128) k_pair(Grid g, SweepK<T> K, int pi, int pj, int pk, int kz,
+                                              const T* __restrict__ mu, const T* __restrict__ exy,
+                                              const T* __restrict__ exz, const T* __restrict__ eyz,
+                                              const T* __restrict__ A, const T* __restrict__ B, T* un, T* vn, T* wn,
+                                              G gh, double* __restrict__ part, int first) {
+  __shared__ T sh[128];
   const int jmax = COMP == 1 ? g.nj - 1 : g.nj;
   T* q = COMP == 0 ? un : (COMP == 1 ? vn : wn);
   T e = 0;
+  const int a = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const int rows = (g.nj / 2 + (int)blockDim.y - 1) / (int)blockDim.y;
+  const int b = (int)(blockIdx.y % rows) * blockDim.y + threadIdx.y;
+  const int k0 = (int)(blockIdx.y / rows) * kz, k1 = min(g.nk / 2, k0 + kz);
+  const int t = (int)(threadIdx.y * blockDim.x + threadIdx.x);
+  double* o = part + ((long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  const double before = t == 0 && !first ? *o : 0.0;  // in flight while the points are
+#pragma unroll 1
+  for (int kk = k0; kk < k1; ++kk) {
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int i = (h ? 3 - pi : pi) + 2 * (int)(blockIdx.x * 32 + threadIdx.x);
-    const int j = (h ? 3 - pj : pj) + 2 * (int)(blockIdx.y * 8 + threadIdx.y);
-    const int k = (h ? 3 - pk : pk) + 2 * (int)blockIdx.z;
-    if (i > g.ni || j > jmax || k > g.nk) continue;
-    const long c = g.at(i, j, k);
-    const T visn = visn_at<COMP, T>(g, p, c, mu, exy, exz, eyz, un, vn, wn);
-    const T qn = __ldg(A + c) * visn + __ldg(B + c);
-    const T d = qn - q[c];
-    q[c] = qn;
-    e += d * d;
+    for (int hh = 0; hh < (BOTH ? 2 : 1); ++hh) {
+      const bool h = BOTH ? hh != 0 : blockIdx.z != 0;
+      const int i = (h ? 3 - pi : pi) + 2 * a, j = (h ? 3 - pj : pj) + 2 * b, k = (h ? 3 - pk : pk) + 2 * kk;
+      if (i > g.ni || j > jmax) continue;
+      const long c = g.at(i, j, k);
+      const T visn = visn_sweep<COMP>(g, K, c, mu, exy, exz, eyz, un, vn, wn);
+      const T qn = __ldg(A + c) * visn + __ldg(B + c);
+      const T d = qn - q[c];
+      q[c] = qn;
+      if (GHOSTS && (i <= 3 || i >= g.ni - 2 || j <= 3 || j >= g.nj - 3 || k <= 3 || k >= g.nk - 2))
+        fill_ghosts<COMP>(g, gh, q, i, j, k, qn);
+      e += d * d;
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
-  if (threadIdx.x == 0) sh[threadIdx.y] = e;
+  // the block's sum: one warp adds the others' values before the tree, which costs 8 FP64
+  // operations per block and not 5 per warp
+  const int nt = (int)(blockDim.x * blockDim.y);
+  sh[t] = e;
   __syncthreads();
-  if (threadIdx.y == 0 && threadIdx.x == 0) {
-    T t = 0;
-    for (int w = 0; w < 8; ++w) t += sh[w];
-    part[((long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x] = (double)t;
-  }
+  if (t >= 32) return;
+  for (int w = 32; w < nt; w += 32) e += sh[w + t];
+  for (int o = 16; o > 0; o >>= 1) e += __shfl_down_sync(0xffffffffu, e, o);
+  if (t == 0) *o = before + (double)e;
 }
 
 // --- wall/halo refresh: bndu(un,vn,wn) then bnd_periodic(swept component) ----------
@@ -739,15 +894,9 @@ __global__ void __launch_bounds__(256) k_refresh(Grid g, int normal, double uwal
 // gamma_dst = f(u_src) - u_dst, formed once per step in FP64 from u.
 //
 // Wall constants per (side, k, i), 12 floats: c2, gamma_u[3], gamma_v[4], gamma_w[3], pad.
-constexpr int kGW = 12;
 // x-halo constants per (j, k) and z-halo constants per (i, j), 24 floats: the six
 // destinations of the plain copy of u, v, w and the five of bndu's shifted copy
 // (u in x: slots 6..10, v 12..17, w 18..23; z: u 0..5, v 6..11, w 12..17, shifted w 18..22).
-constexpr int kGH = 24;
-
-__device__ __forceinline__ long wall_slot(const Grid& g, int side, int k, int i) {
-  return (((long)side * (g.nk + 6) + (k + 2)) * (g.ni + 6) + (i + 2));
-}
 
 __global__ void __launch_bounds__(256) k_gamma_wall(Grid g, double uwall, const double* __restrict__ wc,
                                                     const double* __restrict__ u, const double* __restrict__ v,
@@ -970,7 +1119,6 @@ __global__ void __launch_bounds__(256) k_halo_z_d(Grid g, int normal, const floa
 // the other rows of the x-ghost columns, one thread per (j, k, component);
 // the rest: the other rows of the z-ghost planes of the columns that are not x
 // destinations, one thread per (i, j, component).
-__device__ __forceinline__ int gslot(int d, int N, int sh) { return d <= 0 ? d + 2 : d - N + 2 - sh; }
 __global__ void __launch_bounds__(256) k_refresh_d(Grid g, int normal, const float* __restrict__ gw,
                                                    const float* __restrict__ gx, const float* __restrict__ gz,
                                                    float* __restrict__ du, float* __restrict__ dv,
@@ -1099,17 +1247,17 @@ __global__ void k_refine_finish(long n, const double* __restrict__ u, const doub
   }
 }
 
-__global__ void k_sum_parts2(const double* part, long n, double* out) {
-  __shared__ double sh[256];
+__global__ void __launch_bounds__(1024) k_sum_parts2(const double* part, long n, double* out) {
+  __shared__ double sh[32];
   double a = 0.0;
-  for (long t = threadIdx.x; t < n; t += 256) a += part[t];
-  sh[threadIdx.x] = a;
+  for (long t = threadIdx.x; t < n; t += 1024) a += part[t];
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = a;
   __syncthreads();
-  for (int st = 128; st > 0; st >>= 1) {
-    if ((int)threadIdx.x < st) sh[threadIdx.x] += sh[threadIdx.x + st];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[0] = sh[0];
+  if (threadIdx.x >= 32) return;
+  a = sh[threadIdx.x];
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+  if (threadIdx.x == 0) out[0] = a;
 }
 
 // The one-pass refresh kernels where the grid allows them, unless FMF_REFRESH_ORDERED
@@ -1139,8 +1287,34 @@ const dim3 kB(32, 8, 1);
 dim3 wall_grid(const Grid& g) { return dim3((g.ni + 6 + 31) / 32, (2 * (g.nk + 6) + 7) / 8); }
 dim3 xh_grid(const Grid& g) { return dim3((g.nj + 6 + 31) / 32, (g.nk + 6 + 7) / 8); }
 dim3 zh_grid(const Grid& g) { return dim3((g.ni + 6 + 31) / 32, (g.nj + 6 + 7) / 8); }
-dim3 pair_grid(const Grid& g) {
-  return dim3((unsigned)((g.ni / 2 + 31) / 32), (unsigned)((g.nj / 2 + 7) / 8), (unsigned)(g.nk / 2));
+struct PairShape {
+  dim3 grid, block;
+  int kz;
+  bool both, ghosts;
+};
+// The split of a colour pair's points, by what bounds the sweep at each size.  Small grids:
+// the launch and one warp's chain, so two-warp blocks and one point per thread, the two
+// colours apart.  FP64 beyond: the FP64 pipe, with both colours in a thread for the rows
+// they share and, on the largest, 4 planes per thread (fewer sums and partials).  FP32:
+// memory, so both colours together once the fields leave L2, and on the sizes between the
+// ghosts refreshed apart (the sweep's own scattered writes cost it more there than the
+// launches).  One outer iteration, us, as
+// (block, both or split, planes): FP64 32x32x16 (64, s, 1) 92, (64, b, 1) 115; 128x64x64
+// (64, s, 1) 162, (64, b, 1) 147, (128, b, 4) 224; 256x128x128 (64, b, 1) 677, (128, b, 4)
+// 655; 512x256x256 4267, 4086.  FP32 32x32x16 (64, s, 1) 97, (64, b, 1) 116; 256x128x128
+// 405, 415, (64, s, 1) with the refresh apart 393; 512x256x256 2598, 2115, (128, b, 1) 2104.
+PairShape pair_shape(const Grid& g, bool fp64) {
+  PairShape p;
+  const long n = g.cells();
+  p.both = n >= (fp64 ? 1L << 18 : 1L << 23);
+  p.kz = fp64 && n >= 1L << 21 ? 4 : 1;
+  p.ghosts = fp64 || n < 1L << 20 || n >= 1L << 23;
+  const int nt = n >= (fp64 ? 1L << 21 : 1L << 23) ? 128 : 64;
+  const int bx = std::min(32, g.ni / 2), by = nt / bx;
+  p.block = dim3((unsigned)bx, (unsigned)by);
+  const int rows = (g.nj / 2 + by - 1) / by, planes = (g.nk / 2 + p.kz - 1) / p.kz;
+  p.grid = dim3((unsigned)((g.ni / 2 + bx - 1) / bx), (unsigned)((long)rows * planes), p.both ? 1 : 2);
+  return p;
 }
 // first colour of each pair (solu_sor4.f:94-120): (1,1,1) (1,1,2) (1,2,1) (2,1,1)
 const int kPi[4] = {1, 1, 1, 2}, kPj[4] = {1, 1, 2, 1}, kPk[4] = {1, 2, 1, 1};
@@ -1183,7 +1357,7 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
     ps.dz2x2 = split_double(2.0 * p.dz2);
     ps.grvb = split_double(grvb);
     ps.grvp = split_double(grvp);
-    k_src_ab_e<REFINE><<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, ps, p, in, mu, E[0], E[1],
+    k_src_ab_e<REFINE><<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, ps, p, Fac<double>(p), in, mu, E[0], E[1],
                                                                                  E[2], out);
   } else {
     SrcK K;
@@ -1216,19 +1390,39 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
   count_launch(3);
 }
 
-// The colour-pair sweeps of one outer iteration: per component 4 pairs, each
-// followed by the wall/halo refresh; then the residual sum into errsum[0].
-template <class T, class PairFn, class HaloFn>
-void sweep_all(cudaStream_t s, const Grid& g, double* part, double* errsum, PairFn pair, HaloFn halo) {
-  const long nb = (long)pair_grid(g).x * pair_grid(g).y * pair_grid(g).z;
+// The colour-pair sweeps of one outer iteration: per component 4 pairs, each followed
+// by the wall/halo refresh; then the residual sum into errsum[0].  The refresh after a
+// component's first pair moves its ghosts from bndu's copies to the plain periodic ones
+// (and the previous component's back), so it runs in full; after the other three only
+// the swept component's ghosts change, and the points write them (GHOSTS) where the grid
+// allows the one-pass refresh.
+template <class T, class G, class HaloFn>
+void sweep_all(cudaStream_t s, const Grid& g, const VP& p, const T* mu, const T* exy, const T* exz, const T* eyz,
+               T* const* A, T* const* B, T* un, T* vn, T* wn, const G& gh, double* part, double* errsum, HaloFn halo) {
+  const PairShape sp = pair_shape(g, sizeof(T) == 8);
+  const bool fill = one_pass_refresh(g) && sp.ghosts;
   for (int comp = 0; comp < 3; ++comp) {
+    const SweepK<T> K(p, comp);
     for (int pr = 0; pr < 4; ++pr) {
-      pair(comp, pr, part + (long)(comp * 4 + pr) * nb);
-      count_launch();
-      halo(1 << comp);
+      auto run = [&](auto fn) {
+        fn<<<sp.grid, sp.block, 0, s>>>(g, K, kPi[pr], kPj[pr], kPk[pr], sp.kz, mu, exy, exz, eyz, A[comp], B[comp],
+                                        un, vn, wn, gh, part, comp == 0 && pr == 0);
+        count_launch();
+      };
+      auto pair = [&](auto ghosts, auto both) {
+        if (comp == 0) run(k_pair<0, T, G, ghosts.value, both.value>);
+        else if (comp == 1) run(k_pair<1, T, G, ghosts.value, both.value>);
+        else run(k_pair<2, T, G, ghosts.value, both.value>);
+      };
+      const bool own = fill && pr > 0;
+      if (own && sp.both) pair(std::true_type(), std::true_type());
+      else if (own) pair(std::true_type(), std::false_type());
+      else if (sp.both) pair(std::false_type(), std::true_type());
+      else pair(std::false_type(), std::false_type());
+      if (!own) halo(1 << comp);
     }
   }
-  k_sum_parts2<<<1, 256, 0, s>>>(part, nb * 12, errsum);
+  k_sum_parts2<<<1, 1024, 0, s>>>(part, (long)sp.grid.x * sp.grid.y * sp.grid.z, errsum);
   count_launch();
 }
 }  // namespace
@@ -1308,19 +1502,11 @@ void wall_halo(cudaStream_t s, const Grid& g, int normal, double uwall, const do
 void sor_iteration(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, int harmonic,
                    const double* mu, double* const* E, double* const* AB, double uwall, const double* wallc,
                    double* un, double* vn, double* wn, double* part, double* errsum) {
-  const VP p = make_vp(dxinv, dyinv, dzinv, 0.0, harmonic);
-  const dim3 grd = pair_grid(g);
-  sweep_all<double>(
-      s, g, part, errsum,
-      [&](int comp, int pr, double* pp) {
-#define FMF_PAIR(C) \
-  k_pair<C, double><<<grd, kB, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], mu, E[0], E[1], E[2], AB[2 * C], AB[2 * C + 1], un, vn, wn, pp)
-        if (comp == 0) FMF_PAIR(0);
-        else if (comp == 1) FMF_PAIR(1);
-        else FMF_PAIR(2);
-#undef FMF_PAIR
-      },
-      [&](int normal) { wall_halo(s, g, normal, uwall, wallc, un, vn, wn); });
+  double* const A[3] = {AB[0], AB[2], AB[4]};
+  double* const B[3] = {AB[1], AB[3], AB[5]};
+  sweep_all<double>(s, g, make_vp(dxinv, dyinv, dzinv, 0.0, harmonic), mu, E[0], E[1], E[2], A, B, un, vn, wn,
+                    Ghosts64{uwall, wallc}, part, errsum,
+                    [&](int normal) { wall_halo(s, g, normal, uwall, wallc, un, vn, wn); });
 }
 
 long refine_floats(const Grid& g, int part) {
@@ -1355,19 +1541,10 @@ void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
 
 void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv,
                           const RefineBufs& rb, double* part, double* errsum) {
-  const VP p = make_vp(dxinv, dyinv, dzinv, 0.0, 0);
-  const dim3 grd = pair_grid(g);
   float *du = rb.d[0], *dv = rb.d[1], *dw = rb.d[2];
   sweep_all<float>(
-      s, g, part, errsum,
-      [&](int comp, int pr, double* pp) {
-#define FMF_PAIR(C) \
-  k_pair<C, float><<<grd, kB, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], rb.mu, rb.e[0], rb.e[1], rb.e[2], rb.a[C], rb.r[C], du, dv, dw, pp)
-        if (comp == 0) FMF_PAIR(0);
-        else if (comp == 1) FMF_PAIR(1);
-        else FMF_PAIR(2);
-#undef FMF_PAIR
-      },
+      s, g, make_vp(dxinv, dyinv, dzinv, 0.0, 0), rb.mu, rb.e[0], rb.e[1], rb.e[2], rb.a, rb.r, du, dv, dw,
+      Ghosts32{rb.gw, rb.gx, rb.gz}, part, errsum,
       [&](int normal) {
         if (one_pass_refresh(g)) {
           const long tw = 2L * (g.ni + 6) * (g.nk + 6), tx = 3L * g.nj * (g.nk + 6), tz = 3L * (g.ni + 1) * g.nj;
@@ -1390,7 +1567,8 @@ void refine_finish(cudaStream_t s, const Grid& g, const double* u, const double*
 }
 
 long sor_parts(const Grid& g) {
-  return (long)((g.ni / 2 + 31) / 32) * ((g.nj / 2 + 7) / 8) * (g.nk / 2) * 12;
+  const dim3 a = pair_shape(g, true).grid, b = pair_shape(g, false).grid;
+  return std::max((long)a.x * a.y * a.z, (long)b.x * b.y * b.z);
 }
 
 }  // namespace fused
