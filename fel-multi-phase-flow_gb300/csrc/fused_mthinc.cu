@@ -107,15 +107,8 @@ __device__ __forceinline__ double avg8(const double* __restrict__ p, long c, lon
          0.125;
 }
 
-__device__ __forceinline__ double ex(double x) { return exp(x); }
 __device__ __forceinline__ float ex(float x) { return expf(fminf(x, 80.0f)); }
 
-// 1/(1+e) for e >= 0: the division-free reciprocal in double (an overflowed e gives
-// exactly 0, as the quotient does; NaN stays NaN), the quotient in float
-__device__ __forceinline__ double inv1p(double e) {
-  const double a = 1.0 + e;
-  return (__double2hiint(a) == 0x7ff00000 && __double2loint(a) == 0) ? 0.0 : recip_h(a);
-}
 __device__ __forceinline__ float inv1p(float e) { return 1.0f / (1.0f + e); }
 
 // The sum over the 8 Gauss points t of w/(1+exp(m2b (a_t + d))) (m2b = -2 bet) and,
@@ -210,12 +203,10 @@ __global__ void __launch_bounds__(256) k_classify(Grid g, MC m, const double* __
   if (k == g.nk + 1 && !t_) fz[c] = 0.0;
 }
 
-// R = double: the FP64 step.  R = float: the mixed-precision step (normal, band
-// test and the fluxes' storage stay double; the Newton solve and the Gauss-point
-// integrals run in float with the exponent argument clamped to the float range
-// and the Newton regularisation 1e-99 raised to 1e-30).
-template <class R>
-__global__ void __launch_bounds__(128) k_band(Grid g, MC m, const double* __restrict__ phi,
+// The mixed-precision step (normal, band test and the fluxes' storage stay double; the
+// Newton solve and the Gauss-point integrals run in float with the exponent argument
+// clamped to the float range and the Newton regularisation 1e-99 raised to 1e-30).
+__global__ void __launch_bounds__(128) k_band_f32(Grid g, MC m, const double* __restrict__ phi,
                                               const double* __restrict__ gx, const double* __restrict__ gy,
                                               const double* __restrict__ gz, const double* __restrict__ u,
                                               const double* __restrict__ v, const double* __restrict__ w,
@@ -223,10 +214,11 @@ __global__ void __launch_bounds__(128) k_band(Grid g, MC m, const double* __rest
                                               double* __restrict__ fz, const int* __restrict__ list,
                                               const int* __restrict__ count, double* __restrict__ newton,
                                               long cap) {
+  using R = float;
   const int n = *count;
   const long X = 1, Y = g.sy, Z = g.sz;
   const R m2b = (R)(-2.0 * m.bet), gp1 = (R)m.gp1, gp2 = (R)m.gp2, bet = (R)m.bet, dtt = (R)m.dt;
-  const R reg = sizeof(R) == 8 ? (R)1.0e-99 : (R)1.0e-30;
+  const R reg = (R)1.0e-30;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const long c = list[e];
     double nx = avg8(gx, c, X, Y, Z), ny = avg8(gy, c, X, Y, Z), nz = avg8(gz, c, X, Y, Z);
@@ -246,15 +238,14 @@ __global__ void __launch_bounds__(128) k_band(Grid g, MC m, const double* __rest
       const R f = sig8f<R>(E, (R)0.125, ex(m2b * ddd), &sd) - ph;
       // df = 0.5 bet sum 0.125/cosh^2 = 0.5 bet * 0.125 * 4 * sum s(1-s)
       const R df = (R)0.25 * bet * sd;
-      step = sizeof(R) == 8 ? (R)((double)(f * df) * recip_h((double)(df * df + reg))) : f * df / (df * df + reg);
+      step = f * df / (df * df + reg);
       const R dn = ddd - step;
       // once d no longer changes, every remaining iteration recomputes the same
-      // f, df and step: stopping here is the ten-step result bit for bit.  In
-      // float the iterate can dither in its last bit instead; there a step below
-      // float precision ends the loop.
+      // f, df and step; the iterate can dither in its last bit instead, so a step
+      // below float precision ends the loop as well.
       if (dn == ddd) break;
       ddd = dn;
-      if (sizeof(R) == 4 && fabs((double)step) <= 1.0e-7 * (1.0 + fabs((double)ddd))) break;
+      if (fabs((double)step) <= 1.0e-7 * (1.0 + fabs((double)ddd))) break;
     }
     if (newton) {
       newton[e] = (double)ddd;
@@ -280,6 +271,128 @@ __global__ void __launch_bounds__(128) k_band(Grid g, MC m, const double* __rest
     if (vn > 0.0) side(vn, m.dyi, 1, false, fy + c);
     if (wb < 0.0) side(wb, m.dzi, 2, true, fz + c - Z);
     if (wt > 0.0) side(wt, m.dzi, 2, false, fz + c);
+  }
+}
+// FP64 band cells, bound by the FP64 pipe: 10 Newton steps per warp in nearly all (a cell
+// with phi near 0 or 1 takes them, at about 1/(2 bet) each, and may not have converged),
+// then the fluxes.
+//  * The centred Gauss points come in pairs of opposite signs, so with E + 1/E = k and
+//    y = exp(m2b d) a pair's sum of sigmoids is (2 + k y)/(1 + k y + y^2) and its sum of
+//    s (1 - s) is y (k + 4 y + k y^2)/(1 + k y + y^2)^2: four reciprocals per step instead
+//    of eight.  On the swept axis the factors F1, F2 take the two other axes' pairs with
+//    F y in the place of y.
+//  * The iteration runs in y, which is all the fluxes need of the offset: a step of d
+//    multiplies y by exp(-m2b step).
+//  * A step below 1e-9 (1 + |d|) is the last: Newton's error squares per step and leaves
+//    the root to rounding, where the ten steps of solphi_mthinc1.f dither.
+//  * The exponentials have small arguments: exp16 below.
+// 1.57 -> 1.06 ms at 512x256x256, 317 -> 190 us at 128x64x64, 63 -> 45 at 32x32x16.
+// Sixteenths: exp(k/16), k = -64 .. 64, formed on the host.
+struct Exp16 {
+  double t[129];
+};
+// exp(z) = exp(k/16) exp(r), k the integer nearest 16 z, |r| <= 1/32, the second factor by
+// its Taylor polynomial (the term after z^7/7! is below 3e-17 of the sum); |z| > 4 and NaN:
+// exp itself
+__device__ __forceinline__ double exp16(const Exp16& T, double z) {
+  if (!(mag(z) <= mag(4.0))) return exp(z);
+  const double s = fma(z, 16.0, 6755399441055744.0);  // 1.5 * 2^52: the sum's low bits are k
+  const int k = __double2loint(s);
+  const double r = fma(s - 6755399441055744.0, -0.0625, z);
+  double p = fma(r, 1.0 / 5040.0, 1.0 / 720.0);
+  p = fma(p, r, 1.0 / 120.0);
+  p = fma(p, r, 1.0 / 24.0);
+  p = fma(p, r, 1.0 / 6.0);
+  p = fma(p, r, 0.5);
+  p = fma(p, r, 1.0);
+  const double e = T.t[k + 64];
+  return fma(p * r, e, e);
+}
+// 1/D for D >= 1 (an overflowed D gives exactly 0; NaN stays NaN)
+__device__ __forceinline__ double recip_ge1(double d) {
+  return (__double2hiint(d) == 0x7ff00000 && __double2loint(d) == 0) ? 0.0 : recip_h(d);
+}
+__global__ void __launch_bounds__(64) k_band(Grid g, MC m, __grid_constant__ const Exp16 T,
+                                             const double* __restrict__ phi, const double* __restrict__ gx,
+                                             const double* __restrict__ gy, const double* __restrict__ gz,
+                                             const double* __restrict__ u, const double* __restrict__ v,
+                                             const double* __restrict__ w, double* __restrict__ fx,
+                                             double* __restrict__ fy, double* __restrict__ fz,
+                                             const int* __restrict__ list, const int* __restrict__ count,
+                                             double* __restrict__ newton, long cap) {
+  const int n = *count;
+  const long X = 1, Y = g.sy, Z = g.sz;
+  const double m2b = -2.0 * m.bet;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const long c = list[e];
+    const double nx = avg8(gx, c, X, Y, Z), ny = avg8(gy, c, X, Y, Z), nz = avg8(gz, c, X, Y, Z);
+    const double coef = m2b * rsqrt_h(fma(nz, nz, fma(ny, ny, nx * nx)));
+    const double b[3] = {nx * coef, ny * coef, nz * coef};  // m2b times the unit normal
+    // per axis exp(b gp) of the two centred Gauss points (gp1 = -gp2)
+    const double X2 = exp16(T, b[0] * m.gp2), Y2 = exp16(T, b[1] * m.gp2), Z2 = exp16(T, b[2] * m.gp2);
+    const double X1 = recip_h(X2), Y1 = recip_h(Y2), Z1 = recip_h(Z2);
+    // k = E + 1/E of the pairs: same and opposite signs on the two axes other than x, y, z
+    const double yz = Y2 * Z2, yzi = Y1 * Z1, yoz = Y2 * Z1, zoy = Y1 * Z2;
+    const double kx0 = yz + yzi, kx1 = yoz + zoy;
+    const double ky0 = fma(X2, Z2, X1 * Z1), ky1 = fma(X2, Z1, X1 * Z2);
+    const double kz0 = fma(X2, Y2, X1 * Y1), kz1 = fma(X2, Y1, X1 * Y2);
+    const double ph = __ldg(phi + c);
+    double y = 1.0, ddd = 0.0, step = 0.0;
+    {
+      const double kk[4] = {fma(X2, yz, X1 * yzi), fma(X1, yz, X2 * yzi), fma(X2, yoz, X1 * zoy), fma(X1, yoz, X2 * zoy)};
+#pragma unroll 1
+      for (int it = 0; it < 10; ++it) {
+        const double y2 = y * y, y4 = 4.0 * y2;
+        double s = 0.0, q = 0.0;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const double ky = kk[t] * y, r = recip_ge1(fma(y, y, 1.0 + ky));
+          s = fma(2.0 + ky, r, s);
+          q = fma(fma(ky, y2 * r, (ky + y4) * r), r, q);  // y^2 r <= 1: no overflow
+        }
+        // df = 0.5 bet sum 0.125/cosh^2 = 0.5 bet * 0.125 * 4 * sum s(1-s)
+        const double f = fma(s, 0.125, -ph), df = 0.25 * m.bet * q;
+        step = f * df * recip_h(fma(df, df, 1.0e-99));
+        ddd -= step;
+        if (mag(step) == 0) break;
+        y *= exp16(T, -m2b * step);
+        if (mag(y) > mag(1.0e150) && !is_nan(y)) y = 1.0e150;  // y^2 stays finite
+        if (mag(step) <= mag(fma(fabs(ddd), 1.0e-9, 1.0e-9))) {
+          step = 0.0;  // converged: the next step is rounding
+          break;
+        }
+      }
+    }
+    if (newton) {
+      newton[e] = ddd;
+      newton[cap + e] = step;
+    }
+    const double uw = __ldg(u + c - X), ue = __ldg(u + c), vs = __ldg(v + c - Y), vn = __ldg(v + c),
+                 wb = __ldg(w + c - Z), wt = __ldg(w + c);
+    // the flux through one face (low: the west, south or bottom one) along an axis with
+    // b, k0, k1: the Gauss points of the swept interval lie vd (1/2 +/- gp) from the face
+    auto side = [&](double vel, double dtd, double bb, double k0, double k1, bool low, double* out) {
+      const double vd = vel * dtd;
+      double s = 0.0;
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const double gp = t ? m.gp2 : m.gp1;
+        const double o = low ? fma(-vd, 0.5 + gp, -0.5) : fma(vd, gp - 0.5, 0.5);
+        const double f = y * exp16(T, bb * o);
+        const double a = k0 * f, d = k1 * f;
+        s = fma(2.0 + a, recip_ge1(fma(f, f, 1.0 + a)), s);
+        s = fma(2.0 + d, recip_ge1(fma(f, f, 1.0 + d)), s);
+      }
+      *out = 0.125 * vd * s;
+    };
+    auto neg = [](double x) { return __double_as_longlong(x) < 0 && mag(x) != 0; };
+    auto pos = [](double x) { return __double_as_longlong(x) > 0; };
+    if (neg(uw)) side(uw, m.dtdx, b[0], kx0, kx1, true, fx + c - X);
+    if (pos(ue)) side(ue, m.dtdx, b[0], kx0, kx1, false, fx + c);
+    if (neg(vs)) side(vs, m.dtdy, b[1], ky0, ky1, true, fy + c - Y);
+    if (pos(vn)) side(vn, m.dtdy, b[1], ky0, ky1, false, fy + c);
+    if (neg(wb)) side(wb, m.dtdz, b[2], kz0, kz1, true, fz + c - Z);
+    if (pos(wt)) side(wt, m.dtdz, b[2], kz0, kz1, false, fz + c);
   }
 }
 // cal_grad_p2a.f:46-60 for the fused step: the vertex gradient at (i+1/2, j+1/2,
@@ -364,6 +477,15 @@ void mthinc_snap(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
   count_launch();
 }
 
+static const Exp16& exp16_table() {
+  static const Exp16 table = [] {
+    Exp16 e;
+    for (int k = -64; k <= 64; ++k) e.t[k + 64] = std::exp(k / 16.0);
+    return e;
+  }();
+  return table;
+}
+
 void mthinc_fluxes(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt, double bet,
                    const double* phi, const double* gx, const double* gy, const double* gz, const double* u,
                    const double* v, const double* w, double* fx, double* fy, double* fz, int* list, int* count,
@@ -375,9 +497,9 @@ void mthinc_fluxes(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
   k_classify<<<gr, b, 0, s>>>(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count);
   const long cap = (long)(g.ni + 2) * (g.nj + 2) * (g.nk + 2);
   if (fp32)
-    k_band<float><<<152 * 8, 128, 0, s>>>(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
+    k_band_f32<<<152 * 8, 128, 0, s>>>(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
   else
-    k_band<double><<<152 * 8, 128, 0, s>>>(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
+    k_band<<<152 * 16, 64, 0, s>>>(g, m, exp16_table(), phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
   count_launch(2);
 }
 
