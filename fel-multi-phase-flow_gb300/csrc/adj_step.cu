@@ -147,6 +147,11 @@ struct fmf_adj {
   // transposes (carry_in).
   double* lcarry = nullptr;
   bool carry_in = false;
+  // small grids: the forward viscous solve in one launch with its stop rule
+  // (fused::solve_small; FMF_DEVICE_LOOP=0 at creation: the host applies the rule)
+  bool small = false;
+  fused::SorLoop* loop = nullptr;  // device
+  int* sorlog = nullptr;           // device, one entry
   double* host_norm = nullptr;  // pinned
   double* tdma = nullptr;       // the pressure solve's Thomas factors (fused::tdma_coef)
   fmf_adj* worker = nullptr;    // recomputes the next segment while this handle reverses one
@@ -549,33 +554,47 @@ int record_step(fmf_adj* a, bool graphs) {
       fused::sor_iteration(s, g, dxi, dyi, dzi, P.harmonic, a->rmun, a->E, a->AB, P.uwall, a->wallc, a->un[0],
                            a->un[1], a->un[2], a->sorpart, a->red + 4);
   };
-  long long per_launch = 0;
-  const cudaGraphExec_t exec =
-      adj::cached_graph(s, &a->fgraphs,
-                        {a->rmun, a->E[0], a->E[1], a->E[2], a->AB[0], a->AB[1], a->AB[2], a->AB[3], a->AB[4],
-                         a->AB[5], a->wallc, a->un[0], a->un[1], a->un[2], a->sorpart, a->red},
-                        iteration, &per_launch);
-  double err0 = 0.0;
-  int lp;
-  for (lp = 0; lp < a->sor_max; ++lp) {
-    if (exec) {
-      FMF_CUDA(cudaGraphLaunch(exec, s));
-      count_launch((int)per_launch);
-    } else {
-      iteration();
-    }
-    double e = 0.0;
-    FMF_CUDA(cudaMemcpyAsync(&e, a->red + 4, sizeof(double), cudaMemcpyDeviceToHost, s));
+  if (a->small) {
+    fused::sor_rule(s, a->loop, a->sor_tol, a->sor_max, (double)g.cells());
+    if (a->mixed)
+      fused::solve_small_refine(s, g, dxi, dyi, dzi, a->rb, a->loop, a->sorlog);
+    else
+      fused::solve_small(s, g, dxi, dyi, dzi, a->rmun, a->E, a->AB, P.uwall, a->wallc, a->un[0], a->un[1], a->un[2],
+                         a->loop, a->sorlog);
+    int entry = 0;
+    FMF_CUDA(cudaMemcpyAsync(&entry, a->sorlog, sizeof(int), cudaMemcpyDeviceToHost, s));
     FMF_CUDA(cudaStreamSynchronize(s));
-    if (!std::isfinite(e)) {
-      set_status(FMF_ERR_NONFINITE);
-      break;
+    if (entry & fused::kSorNonfinite) set_status(FMF_ERR_NONFINITE);
+    a->sor_total += (entry & (fused::kSorCapped - 1)) + (entry & fused::kSorCapped ? 1 : 0);
+  } else {
+    long long per_launch = 0;
+    const cudaGraphExec_t exec =
+        adj::cached_graph(s, &a->fgraphs,
+                          {a->rmun, a->E[0], a->E[1], a->E[2], a->AB[0], a->AB[1], a->AB[2], a->AB[3], a->AB[4],
+                           a->AB[5], a->wallc, a->un[0], a->un[1], a->un[2], a->sorpart, a->red},
+                          iteration, &per_launch);
+    double err0 = 0.0;
+    int lp;
+    for (lp = 0; lp < a->sor_max; ++lp) {
+      if (exec) {
+        FMF_CUDA(cudaGraphLaunch(exec, s));
+        count_launch((int)per_launch);
+      } else {
+        iteration();
+      }
+      double e = 0.0;
+      FMF_CUDA(cudaMemcpyAsync(&e, a->red + 4, sizeof(double), cudaMemcpyDeviceToHost, s));
+      FMF_CUDA(cudaStreamSynchronize(s));
+      if (!std::isfinite(e)) {
+        set_status(FMF_ERR_NONFINITE);
+        break;
+      }
+      const double err = std::sqrt(e / (double)g.cells()) + 1.0e-99;
+      if (lp == 0) err0 = err;
+      if (err / err0 <= a->sor_tol) break;
     }
-    const double err = std::sqrt(e / (double)g.cells()) + 1.0e-99;
-    if (lp == 0) err0 = err;
-    if (err / err0 <= a->sor_tol) break;
+    a->sor_total += lp + 1;
   }
-  a->sor_total += lp + 1;
   // the step after the viscous solve
   auto post = [&]() {
     if (a->mixed) fused::refine_finish(s, g, S[SU], S[SV], S[SW], a->rb, a->un[0], a->un[1], a->un[2]);
@@ -994,6 +1013,10 @@ int fmf_adj_create(const fmf_params* prm, fmf_adj** out) {
   a->ib_wallc = dalloc(a, nwc);
   a->snaps = dalloc(a, 39 * n);
   a->sorpart = dalloc(a, fused::sor_parts(a->g));
+  const char* dl = std::getenv("FMF_DEVICE_LOOP");
+  a->small = !(dl && std::atoi(dl) == 0) && fused::solve_small_supported(a->g, !a->mixed);
+  a->loop = (fused::SorLoop*)dalloc(a, (sizeof(fused::SorLoop) + 7) / 8);
+  a->sorlog = (int*)dalloc(a, 1);
   a->csfwork = dalloc(a, 21 * n);
   a->work = dalloc(a, 3 * n + 1024 + 63 * n);  // SOR adjoint, then CSF (42n) or WENO5 (63n) adjoints
   a->fb[0] = dalloc(a, 3 * n);

@@ -111,6 +111,26 @@ void sor_iteration(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
                    double* un, double* vn, double* wn, double* part, double* errsum);
 long sor_parts(const Grid& g);
 
+// The stop rule of the viscous solve on the device (solu_sor4.f:130,291-293): err =
+// sqrt(e / cells) + 1e-99 after each outer iteration, err0 = that of the first, stop at
+// err/err0 <= tol or after maxit iterations (kSorMax at most, whatever this memory
+// holds).  A finished solve's log entry is its iteration count with the two bits.
+struct SorLoop {
+  double tol, cells, err0, pad;
+  int maxit, it, nlog, flags;
+};
+constexpr int kSorLog = 4096, kSorMax = 100000;
+constexpr int kSorCapped = 1 << 20, kSorNonfinite = 1 << 21;
+// sets the rule and empties the log
+void sor_rule(cudaStream_t s, SorLoop* L, double tol, int maxit, double cells);
+// The whole solve of a small grid in one launch, with its stop rule and log entry, where
+// supported: what sor_iteration (sor_iteration_refine) repeated until the rule gives, bit
+// for bit
+bool solve_small_supported(const Grid& g, bool fp64);
+void solve_small(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const double* mu,
+                 double* const* E, double* const* AB, double uwall, const double* wallc, double* un, double* vn,
+                 double* wn, SorLoop* L, int* log);
+
 // The pressure Poisson solve (solp_fft_tdma1-3) on the half spectrum of the real
 // divergence: div -> dp interior.  pr, pi: (ni/2+1) nj nk doubles each (the spectrum
 // after the forward transform and the Thomas solve).
@@ -150,6 +170,8 @@ void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
 // one outer iteration on the corrections; errsum[0] = sum of squared increments
 void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv,
                           const RefineBufs& rb, double* part, double* errsum);
+void solve_small_refine(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const RefineBufs& rb,
+                        SorLoop* L, int* log);
 // un = u + d, vn = v + d_v, wn = w + d_w at every point
 void refine_finish(cudaStream_t s, const Grid& g, const double* u, const double* v, const double* w,
                    const RefineBufs& rb, double* un, double* vn, double* wn);

@@ -19,6 +19,8 @@
 // refinement: the residual of the first sweep is formed in FP64 at u, then the
 // sweeps run in FP32 on the correction d = un - u (FP32 storage and arithmetic),
 // and un = u + d is formed in FP64 at the end.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -470,8 +472,8 @@ __device__ __forceinline__ float visn_sweep(const Grid& g, const SweepK<float>& 
   return visn_at<COMP, float>(g, K.f, c, mu, exy, exz, eyz, un, vn, wn);
 }
 
-// The ghost points that one updated point of the swept component fills (k_refresh and
-// k_refresh_d below, seen from the source): its x and z images (the plain periodic copy)
+// The ghost points that one updated point of the swept component fills (refresh below,
+// seen from the source): its x and z images (the plain periodic copy)
 // and, next to a wall, the wall rows of its column with their images.  ni, nj, nk >= 8.
 struct Ghosts64 {
   double uwall;
@@ -504,7 +506,7 @@ __device__ __noinline__ void fill_ghosts(const Grid& g, const Ghosts64& G, doubl
     put(j + 3 * t, 2.0 * x2 - x1, true);
   }
 }
-// the same on the mixed step's corrections, each with its constant (k_refresh_d)
+// the same on the mixed step's corrections, each with its constant
 struct Ghosts32 {
   const float *gw, *gx, *gz;
 };
@@ -780,15 +782,15 @@ __global__ void __launch_bounds__(256) k_halo_x8(Grid g, int normal, double* __r
 // columns, one thread per (j, k, component) for its six ghost slots; the rest: the
 // other rows of the z-ghost planes over the columns that are not x destinations,
 // one thread per (i, j, component).  A thread reads all its sources before writing.
-__global__ void __launch_bounds__(256) k_refresh(Grid g, int normal, double uwall, const double* __restrict__ wc,
-                                                 double* __restrict__ uk, double* __restrict__ vk,
-                                                 double* __restrict__ wk, int nbW, int nbX) {
+// (refresh: thread t of one of the three regions)
+__device__ __forceinline__ void refresh(const Grid& g, int normal, const Ghosts64& G, double* uk, double* vk, double* wk,
+                                        int region, long t) {
+  const double uwall = G.uwall;
+  const double* __restrict__ wc = G.wc;
   const int shu = !(normal & 1), shw = !(normal & 4);  // bndu's shifted copies: u along x, w along z
   const int NI = g.ni, NJ = g.nj, NK = g.nk;
   const long Y = g.sy;
-  const int b = (int)blockIdx.x;
-  if (b < nbW) {
-    const long t = (long)b * 256 + threadIdx.x;
+  if (region == 0) {
     const int W = NI + 6;
     if (t >= 2L * W * (NK + 6)) return;
     const int i = (int)(t % W) - 2;
@@ -841,8 +843,8 @@ __global__ void __launch_bounds__(256) k_refresh(Grid g, int normal, double uwal
     }
     return;
   }
-  if (b < nbW + nbX) {
-    const long task = (long)(b - nbW) * 256 + threadIdx.x;
+  if (region == 1) {
+    const long task = t;
     if (task >= 3L * NJ * (NK + 6)) return;
     const int cmp = (int)(task / ((long)NJ * (NK + 6)));
     const int rem = (int)(task % ((long)NJ * (NK + 6)));
@@ -864,7 +866,6 @@ __global__ void __launch_bounds__(256) k_refresh(Grid g, int normal, double uwal
     }
     return;
   }
-  const long t = (long)(b - nbW - nbX) * 256 + threadIdx.x;
   const int i = 1 + (int)(t % (NI + 1));
   const long r = t / (NI + 1);
   const int j = 1 + (int)(r % NJ);
@@ -1119,10 +1120,9 @@ __global__ void __launch_bounds__(256) k_halo_z_d(Grid g, int normal, const floa
 // the other rows of the x-ghost columns, one thread per (j, k, component);
 // the rest: the other rows of the z-ghost planes of the columns that are not x
 // destinations, one thread per (i, j, component).
-__global__ void __launch_bounds__(256) k_refresh_d(Grid g, int normal, const float* __restrict__ gw,
-                                                   const float* __restrict__ gx, const float* __restrict__ gz,
-                                                   float* __restrict__ du, float* __restrict__ dv,
-                                                   float* __restrict__ dw, int nbW, int nbX) {
+__device__ __forceinline__ void refresh(const Grid& g, int normal, const Ghosts32& G, float* du, float* dv, float* dw,
+                                        int region, long t) {
+  const float *__restrict__ gw = G.gw, *__restrict__ gx = G.gx, *__restrict__ gz = G.gz;
   const int shu = !(normal & 1), shw = !(normal & 4);
   const int NI = g.ni, NJ = g.nj, NK = g.nk;
   // constant slots: x (per (k, j)): u 0, shifted u 6, v 12, w 18; z (per (j, i)): u 0,
@@ -1131,9 +1131,7 @@ __global__ void __launch_bounds__(256) k_refresh_d(Grid g, int normal, const flo
   auto zb = [&](int cmp) { return cmp == 2 ? (shw ? 18 : 12) : 6 * cmp; };
   auto GX = [&](int j, int k, int slot) { return __ldg(gx + ((long)(k + 2) * (NJ + 6) + (j + 2)) * kGH + slot); };
   auto GZ = [&](int i, int j, int slot) { return __ldg(gz + ((long)(j + 2) * (NI + 6) + (i + 2)) * kGH + slot); };
-  const int b = (int)blockIdx.x;
-  if (b < nbW) {
-    const long t = (long)b * 256 + threadIdx.x;
+  if (region == 0) {
     const int W = NI + 6;
     if (t >= 2L * W * (NK + 6)) return;
     const int i = (int)(t % W) - 2;
@@ -1182,8 +1180,8 @@ __global__ void __launch_bounds__(256) k_refresh_d(Grid g, int normal, const flo
     }
     return;
   }
-  if (b < nbW + nbX) {
-    const long task = (long)(b - nbW) * 256 + threadIdx.x;
+  if (region == 1) {
+    const long task = t;
     if (task >= 3L * NJ * (NK + 6)) return;
     const int cmp = (int)(task / ((long)NJ * (NK + 6)));
     const int rem = (int)(task % ((long)NJ * (NK + 6)));
@@ -1210,7 +1208,6 @@ __global__ void __launch_bounds__(256) k_refresh_d(Grid g, int normal, const flo
     }
     return;
   }
-  const long t = (long)(b - nbW - nbX) * 256 + threadIdx.x;
   const int i = 1 + (int)(t % (NI + 1));
   const long r = t / (NI + 1);
   const int j = 1 + (int)(r % NJ);
@@ -1229,6 +1226,129 @@ __global__ void __launch_bounds__(256) k_refresh_d(Grid g, int normal, const flo
   for (int m = 0; m < 6; ++m) {
     const int d = halo_dest(m, NK, sz);
     if (d != kNoHalo) a[g.at(i, j, d)] = v[m];
+  }
+}
+// threads of the three regions: the wall rows, the x-ghost columns, the z-ghost planes
+__host__ __device__ __forceinline__ long refresh_tasks(const Grid& g, int region) {
+  return region == 0 ? 2L * (g.ni + 6) * (g.nk + 6) : (region == 1 ? 3L * g.nj * (g.nk + 6) : 3L * (g.ni + 1) * g.nj);
+}
+template <class T, class G>
+__global__ void __launch_bounds__(256) k_refresh(Grid g, int normal, G gh, T* uk, T* vk, T* wk, int nbW, int nbX) {
+  const int b = (int)blockIdx.x, region = b < nbW ? 0 : (b < nbW + nbX ? 1 : 2);
+  refresh(g, normal, gh, uk, vk, wk, region, (long)(b - (region > 0 ? nbW : 0) - (region > 1 ? nbX : 0)) * 256 + threadIdx.x);
+}
+
+// The whole viscous solve of a small grid in one launch: a cluster of 16 blocks runs outer
+// iterations (sweeps and refreshes as sweep_all orders them, a cluster barrier between
+// them) until the stop rule of solu_sor4.f:130,291-293 ends it (SorLoop), and logs it.
+// A phase costs about 2.3 us for its barrier, its stores' way to L2 and the next loads'
+// back, and the sweep's arithmetic on 16 SMs; a launch costs 4, and the rule's loop two
+// more and a conditional node per iteration.  A step, us (launches -> cluster): FP64
+// 32x16x16 436 -> 367, 32x32x16 459 -> 407, 64x32x16 482 -> 489 (16 SMs' FP64 pipes are
+// full); mixed 32x32x16 467 -> 413, 64x32x16 484 -> 436, 64x32x32 526 -> 531: hence the two
+// limits.
+constexpr int kClusterBlocks = 16, kClusterThreads = 512;
+constexpr long kClusterCells64 = 1L << 14, kClusterCells32 = 1L << 15;
+template <class T>
+struct SolveK {
+  SweepK<T> k[3];
+  const T *mu, *exy, *exz, *eyz, *A[3], *B[3];
+  T *un, *vn, *wn;
+};
+template <int COMP, bool GHOSTS, class T, class G>
+__device__ __forceinline__ T cluster_pair(const Grid& g, const SolveK<T>& K, const G& gh, int pi, int pj, int pk,
+                                          int me) {
+  const int lw = 31 - __clz(g.ni / 2), lj = 31 - __clz(g.nj / 2), half = (g.ni / 2) * (g.nj / 2) * (g.nk / 2);
+  const int jmax = COMP == 1 ? g.nj - 1 : g.nj;
+  T* q = COMP == 0 ? K.un : (COMP == 1 ? K.vn : K.wn);
+  T e = 0;
+#pragma unroll 1
+  for (int p = me; p < 2 * half; p += kClusterBlocks * kClusterThreads) {
+    const bool h = p >= half;
+    const int r = h ? p - half : p;
+    const int i = (h ? 3 - pi : pi) + 2 * (r & (g.ni / 2 - 1)), j = (h ? 3 - pj : pj) + 2 * ((r >> lw) & (g.nj / 2 - 1)),
+              k = (h ? 3 - pk : pk) + 2 * (r >> (lw + lj));
+    if (j > jmax) continue;
+    const long c = g.at(i, j, k);
+    const T visn = visn_sweep<COMP>(g, K.k[COMP], c, K.mu, K.exy, K.exz, K.eyz, K.un, K.vn, K.wn);
+    const T qn = __ldg(K.A[COMP] + c) * visn + __ldg(K.B[COMP] + c);
+    const T d = qn - q[c];
+    q[c] = qn;
+    if (GHOSTS && (i <= 3 || i >= g.ni - 2 || j <= 3 || j >= g.nj - 3 || k <= 3 || k >= g.nk - 2))
+      fill_ghosts<COMP>(g, gh, q, i, j, k, qn);
+    e += d * d;
+  }
+  return e;
+}
+template <int COMP, class T, class G, class Sync>
+__device__ __forceinline__ T cluster_component(const Grid& g, const SolveK<T>& K, const G& gh, int me, Sync sync) {
+  T e = cluster_pair<COMP, false>(g, K, gh, 1, 1, 1, me);
+  sync();
+  for (int region = 0; region < 3; ++region)
+    for (long t = me; t < refresh_tasks(g, region); t += kClusterBlocks * kClusterThreads)
+      refresh(g, 1 << COMP, gh, K.un, K.vn, K.wn, region, t);
+  sync();
+  e += cluster_pair<COMP, true>(g, K, gh, 1, 1, 2, me);
+  sync();
+  e += cluster_pair<COMP, true>(g, K, gh, 1, 2, 1, me);
+  sync();
+  e += cluster_pair<COMP, true>(g, K, gh, 2, 1, 1, me);
+  sync();
+  return e;
+}
+template <class T, class G>
+__global__ void __launch_bounds__(kClusterThreads) k_solve_cluster(Grid g, SolveK<T> K, G gh, SorLoop* L, int* log) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ double parts[kClusterBlocks], warps[kClusterThreads / 32];
+  __shared__ int verdict;
+  // tasks by warps, a warp of every block in turn: few tasks spread over all 16 SMs
+  const int t = (int)threadIdx.x, me = ((t >> 5) * kClusterBlocks + (int)cl.block_rank()) * 32 + (t & 31);
+  auto sync = [&] { cl.sync(); };
+  const double tol = L->tol, cells = L->cells;
+  const int mx = min(max(L->maxit, 1), kSorMax);
+  double err0 = 0.0;
+  for (int it = 1;; ++it) {
+    T e = cluster_component<0>(g, K, gh, me, sync);
+    e += cluster_component<1>(g, K, gh, me, sync);
+    e += cluster_component<2>(g, K, gh, me, sync);
+    // every block gets every block's sum and applies the rule to the same total
+    double s = (double)e;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((t & 31) == 0) warps[t >> 5] = s;
+    __syncthreads();
+    if (t < 32) {
+      s = t < kClusterThreads / 32 ? warps[t] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (t < kClusterBlocks) *cl.map_shared_rank(&parts[cl.block_rank()], t) = s;
+    }
+    cl.sync();
+    if (t < 32) {
+      s = t < kClusterBlocks ? parts[t] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (t == 0) {
+        int entry = it;
+        bool done = it >= mx;
+        if (!isfinite(s)) {
+          entry |= kSorNonfinite;
+          done = true;
+        } else {
+          const double err = sqrt(s / cells) + 1.0e-99;
+          if (it == 1) err0 = err;
+          if (err / err0 <= tol)
+            done = true;
+          else if (done)
+            entry |= kSorCapped;
+        }
+        verdict = done ? entry : 0;
+      }
+    }
+    __syncthreads();
+    if (verdict) break;
+  }
+  if (me == 0) {
+    if (L->nlog < kSorLog) log[L->nlog] = verdict;
+    L->nlog += 1;
   }
 }
 __global__ void k_to_float(long n, const double* __restrict__ a, float* __restrict__ b) {
@@ -1484,9 +1604,9 @@ void explicit_viscous(cudaStream_t s, const Grid& g, double dxinv, double dyinv,
 void wall_halo(cudaStream_t s, const Grid& g, int normal, double uwall, const double* wallc, double* un, double* vn,
                double* wn) {
   if (one_pass_refresh(g)) {
-    const long tw = 2L * (g.ni + 6) * (g.nk + 6), tx = 3L * g.nj * (g.nk + 6), tz = 3L * (g.ni + 1) * g.nj;
+    const long tw = refresh_tasks(g, 0), tx = refresh_tasks(g, 1), tz = refresh_tasks(g, 2);
     const int nbW = (int)((tw + 255) / 256), nbX = (int)((tx + 255) / 256), nbZ = (int)((tz + 255) / 256);
-    k_refresh<<<nbW + nbX + nbZ, 256, 0, s>>>(g, normal, uwall, wallc, un, vn, wn, nbW, nbX);
+    k_refresh<<<nbW + nbX + nbZ, 256, 0, s>>>(g, normal, Ghosts64{uwall, wallc}, un, vn, wn, nbW, nbX);
     count_launch();
     return;
   }
@@ -1507,6 +1627,75 @@ void sor_iteration(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
   sweep_all<double>(s, g, make_vp(dxinv, dyinv, dzinv, 0.0, harmonic), mu, E[0], E[1], E[2], A, B, un, vn, wn,
                     Ghosts64{uwall, wallc}, part, errsum,
                     [&](int normal) { wall_halo(s, g, normal, uwall, wallc, un, vn, wn); });
+}
+
+__global__ void k_sor_rule(SorLoop* L, double tol, int maxit, double cells) {
+  L->tol = tol;
+  L->maxit = maxit;
+  L->cells = cells;
+  L->nlog = 0;
+}
+void sor_rule(cudaStream_t s, SorLoop* L, double tol, int maxit, double cells) {
+  k_sor_rule<<<1, 1, 0, s>>>(L, tol, maxit, cells);
+  count_launch();
+}
+// whether a cluster of 16 blocks of the kernel fits this device (asked once per device)
+template <class T, class G>
+static bool cluster_fits() {
+  static thread_local int cached_dev = -1;
+  static thread_local bool cached = false;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev == cached_dev) return cached;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = kClusterBlocks;
+  cfg.blockDim = kClusterThreads;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kClusterBlocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  cached = cudaFuncSetAttribute(k_solve_cluster<T, G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+           cudaOccupancyMaxActiveClusters(&n, k_solve_cluster<T, G>, &cfg) == cudaSuccess && n > 0;
+  cudaGetLastError();  // a device without such clusters takes the separate launches
+  cached_dev = dev;
+  return cached;
+}
+template <class T, class G>
+static void solve_cluster(cudaStream_t s, const Grid& g, const SolveK<T>& K, const G& gh, SorLoop* L, int* log) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = kClusterBlocks;
+  cfg.blockDim = kClusterThreads;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kClusterBlocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  FMF_CUDA(cudaLaunchKernelEx(&cfg, k_solve_cluster<T, G>, g, K, gh, L, log));
+  count_launch();
+}
+bool solve_small_supported(const Grid& g, bool fp64) {
+  if (!one_pass_refresh(g) || g.cells() > (fp64 ? kClusterCells64 : kClusterCells32)) return false;
+  return fp64 ? cluster_fits<double, Ghosts64>() : cluster_fits<float, Ghosts32>();
+}
+void solve_small(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const double* mu,
+                 double* const* E, double* const* AB, double uwall, const double* wallc, double* un, double* vn,
+                 double* wn, SorLoop* L, int* log) {
+  const VP p = make_vp(dxinv, dyinv, dzinv, 0.0, 0);
+  const SolveK<double> K{{{p, 0}, {p, 1}, {p, 2}}, mu, E[0], E[1], E[2], {AB[0], AB[2], AB[4]}, {AB[1], AB[3], AB[5]},
+                         un, vn, wn};
+  solve_cluster(s, g, K, Ghosts64{uwall, wallc}, L, log);
+}
+void solve_small_refine(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const RefineBufs& rb,
+                        SorLoop* L, int* log) {
+  const VP p = make_vp(dxinv, dyinv, dzinv, 0.0, 0);
+  const SolveK<float> K{{{p, 0}, {p, 1}, {p, 2}}, rb.mu, rb.e[0], rb.e[1], rb.e[2], {rb.a[0], rb.a[1], rb.a[2]},
+                        {rb.r[0], rb.r[1], rb.r[2]}, rb.d[0], rb.d[1], rb.d[2]};
+  solve_cluster(s, g, K, Ghosts32{rb.gw, rb.gx, rb.gz}, L, log);
 }
 
 long refine_floats(const Grid& g, int part) {
@@ -1547,9 +1736,9 @@ void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dy
       Ghosts32{rb.gw, rb.gx, rb.gz}, part, errsum,
       [&](int normal) {
         if (one_pass_refresh(g)) {
-          const long tw = 2L * (g.ni + 6) * (g.nk + 6), tx = 3L * g.nj * (g.nk + 6), tz = 3L * (g.ni + 1) * g.nj;
+          const long tw = refresh_tasks(g, 0), tx = refresh_tasks(g, 1), tz = refresh_tasks(g, 2);
           const int nbW = (int)((tw + 255) / 256), nbX = (int)((tx + 255) / 256), nbZ = (int)((tz + 255) / 256);
-          k_refresh_d<<<nbW + nbX + nbZ, 256, 0, s>>>(g, normal, rb.gw, rb.gx, rb.gz, du, dv, dw, nbW, nbX);
+          k_refresh<<<nbW + nbX + nbZ, 256, 0, s>>>(g, normal, Ghosts32{rb.gw, rb.gx, rb.gz}, du, dv, dw, nbW, nbX);
           count_launch();
           return;
         }

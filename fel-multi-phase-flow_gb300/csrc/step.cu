@@ -104,21 +104,18 @@ struct fmf_ctx {
   // after the call's steps.  FMF_DEVICE_LOOP=0 at creation: the host applies the
   // rule after every iteration.
   bool dev_loop = true;
-  struct SorLoop* loop = nullptr;  // device
+  bool small = false;              // small grids: the whole solve in one launch (fused::solve_small)
+  fused::SorLoop* loop = nullptr;  // device
   int* sorlog = nullptr;           // device, kSorLog entries
   int pending = 0;                 // solves logged on the device since the last read
   long long per_iter = 0;          // kernels of one outer iteration (the loop body)
 };
 
-// The device side of the stop rule (solu_sor4.f:130,291-293 as step_once applies
-// it on the host): err = sqrt(e / cells) + 1e-99 after each outer iteration,
-// err0 = that of the first, stop at err/err0 <= tol or after maxit iterations.
-struct SorLoop {
-  double tol, cells, err0, pad;
-  int maxit, it, nlog, flags;
-};
-constexpr int kSorLog = 4096;
-constexpr int kLogCapped = 1 << 20, kLogNonfinite = 1 << 21;
+using fused::kSorCapped;
+using fused::kSorLog;
+using fused::kSorMax;
+using fused::kSorNonfinite;
+using fused::SorLoop;
 
 namespace {
 // *same = 0 where any of the nf field pairs a[f], b[f] (n doubles each) differ in a bit
@@ -153,11 +150,6 @@ void verify_upload(cudaStream_t s, long n, int nf, const double* const* src, dou
   count_launch(2);
 }
 
-__global__ void k_sor_rule(SorLoop* L, double tol, int maxit, double cells) {
-  L->tol = tol;
-  L->maxit = maxit;
-  L->cells = cells;
-}
 __global__ void k_sor_log_reset(SorLoop* L) {
   L->nlog = 0;
   L->flags = 0;
@@ -169,13 +161,13 @@ __global__ void k_sor_begin(SorLoop* L) { L->it = 0; }
 // clamped to the 100000 fmf_ctx_set_sor allows, whatever the loop state holds.
 __global__ void k_sor_ctl(cudaGraphConditionalHandle h, const double* esum, SorLoop* L, int* log) {
   const double e = *esum;
-  const int mx = min(max(L->maxit, 1), 100000);
+  const int mx = min(max(L->maxit, 1), kSorMax);
   const int it = L->it + 1;
   L->it = it;
   int entry = it;
   bool done = it >= mx || it < 1;
   if (!isfinite(e)) {
-    entry |= kLogNonfinite;
+    entry |= kSorNonfinite;
     done = true;
   } else {
     const double err = sqrt(e / L->cells) + 1.0e-99;
@@ -183,7 +175,7 @@ __global__ void k_sor_ctl(cudaGraphConditionalHandle h, const double* esum, SorL
     if (err / L->err0 <= L->tol)
       done = true;
     else if (done)
-      entry |= kLogCapped;
+      entry |= kSorCapped;
   }
   if (done) {
     if (L->nlog < kSorLog) log[L->nlog] = entry;
@@ -311,12 +303,11 @@ int fmf_ctx_create(const fmf_params* prm, fmf_ctx** out) {
   }
   FMF_CUDA(cudaMallocHost(&c->host_err, sizeof(double) * 8));
   if (const char* e = std::getenv("FMF_DEVICE_LOOP")) c->dev_loop = std::atoi(e) != 0;
+  c->small = c->dev_loop && fused::solve_small_supported(c->g, !c->mixed);
   c->loop = (SorLoop*)alloc(c, (sizeof(SorLoop) + 7) / 8);
   c->sorlog = (int*)alloc(c, kSorLog / 2);
   if (c->loop) {
-    k_sor_rule<<<1, 1, 0, c->s>>>(c->loop, c->sor_tol, c->sor_max, (double)c->g.cells());
-    k_sor_log_reset<<<1, 1, 0, c->s>>>(c->loop);
-    count_launch(2);
+    fused::sor_rule(c->s, c->loop, c->sor_tol, c->sor_max, (double)c->g.cells());
   }
   if (get_status()) {
     fmf_ctx_destroy(c);
@@ -542,8 +533,10 @@ static void seg_pre2(fmf_ctx* c) {
   const fmf_params& P = c->prm;
   const Grid& g = c->g;
   cudaStream_t s = c->s;
-  k_sor_begin<<<1, 1, 0, s>>>(c->loop);  // the device stop rule's iteration count
-  count_launch();
+  if (!c->small) {
+    k_sor_begin<<<1, 1, 0, s>>>(c->loop);  // the device stop rule's iteration count
+    count_launch();
+  }
   const long n = g.n;
   const double dxinv = 1.0 / P.dx, dyinv = 1.0 / P.dy, dzinv = 1.0 / P.dz, dt = P.dt;
   double* phi1 = c->phi + n;
@@ -701,11 +694,11 @@ static void read_sor_log(fmf_ctx* c) {
   if (h.nlog != c->pending) set_status(FMF_ERR_CUDA);  // a solve that did not finish
   long long its = 0;
   for (int e : lg) {
-    const int n = e & (kLogCapped - 1);
+    const int n = e & (kSorCapped - 1);
     c->sor_iters.push_back(n);
     its += n;
-    if (e & kLogCapped) ++c->capped;
-    if (e & kLogNonfinite) set_status(FMF_ERR_NONFINITE);
+    if (e & kSorCapped) ++c->capped;
+    if (e & kSorNonfinite) set_status(FMF_ERR_NONFINITE);
   }
   count_launch((int)(its * c->per_iter));
   c->pending = 0;
@@ -733,6 +726,27 @@ static void seg_post(fmf_ctx* c) {
   // :695-697 phi(l) = phin(l); phin keeps its values (cpy leaves the source intact),
   // so after the pointer swap below the new phin must equal the new phi
   op::copy(s, 2 * n, c->phin, c->phi);
+}
+
+// a small grid's solve in one launch
+static void seg_small(fmf_ctx* c) {
+  const fmf_params& P = c->prm;
+  const double dxinv = 1.0 / P.dx, dyinv = 1.0 / P.dy, dzinv = 1.0 / P.dz;
+  if (c->mixed)
+    fused::solve_small_refine(c->s, c->g, dxinv, dyinv, dzinv, c->rb, c->loop, c->sorlog);
+  else
+    fused::solve_small(c->s, c->g, dxinv, dyinv, dzinv, c->rmun, c->edge, c->ab, P.uwall, c->wallc, c->un, c->vn,
+                       c->wn, c->loop, c->sorlog);
+}
+// the parts of a step that nothing on the host interrupts, as one segment (one graph)
+static void seg_before(fmf_ctx* c) {
+  seg_pre(c);
+  seg_pre2(c);
+}
+static void seg_all(fmf_ctx* c) {
+  seg_before(c);
+  seg_small(c);
+  seg_post(c);
 }
 
 // Runs one segment: eagerly, or as a CUDA graph captured the first time this
@@ -779,16 +793,25 @@ static int step_once(fmf_ctx* c, const StepHooks* hk = nullptr) {
   auto hook = [&](const std::function<void()> StepHooks::*f) {
     if (hk && hk->*f) (hk->*f)();
   };
-  run_segment(c, 0, seg_pre_a);
-  hook(&StepHooks::before_b);
-  run_segment(c, 5, seg_pre_b);
-  hook(&StepHooks::after_b);
-  hook(&StepHooks::before_c);
-  run_segment(c, 6, seg_pre_c);
-  hook(&StepHooks::before_pre2);
-  run_segment(c, 3, seg_pre2);
-  const cudaGraphExec_t sx = c->graphs && c->dev_loop ? solve_exec(c) : nullptr;
-  if (sx) {
+  if (hk) {
+    run_segment(c, 0, seg_pre_a);
+    hook(&StepHooks::before_b);
+    run_segment(c, 5, seg_pre_b);
+    hook(&StepHooks::after_b);
+    hook(&StepHooks::before_c);
+    run_segment(c, 6, seg_pre_c);
+    hook(&StepHooks::before_pre2);
+    run_segment(c, 3, seg_pre2);
+  } else if (c->small) {
+    run_segment(c, 8, seg_all);
+  } else {
+    run_segment(c, 7, seg_before);
+  }
+  const cudaGraphExec_t sx = c->graphs && c->dev_loop && !c->small ? solve_exec(c) : nullptr;
+  if (c->small) {
+    if (hk) run_segment(c, 9, seg_small);
+    ++c->pending;
+  } else if (sx) {
     // the rule on the device; the counts are read after the call's steps
     FMF_CUDA(cudaGraphLaunch(sx, c->s));
     ++c->pending;
@@ -811,7 +834,7 @@ static int step_once(fmf_ctx* c, const StepHooks* hk = nullptr) {
     c->sor_iters.push_back((lp < c->sor_max ? lp : c->sor_max - 1) + 1);
     if (lp == c->sor_max) ++c->capped;  // reported after the call; the step carries on
   }
-  run_segment(c, 2, seg_post);
+  if (hk || !c->small) run_segment(c, 2, seg_post);
   // :686-697 rotation by pointer
   double* t;
   t = c->uo; c->uo = c->u; c->u = c->un; c->un = t;
@@ -1100,8 +1123,7 @@ int fmf_ctx_set_sor(fmf_ctx* c, double tol, int max_iter) {
   if (!c || !(tol > 0.0) || max_iter < 1 || max_iter > 100000) return FMF_ERR_ARG;
   c->sor_tol = tol;
   c->sor_max = max_iter;
-  k_sor_rule<<<1, 1, 0, c->s>>>(c->loop, tol, max_iter, (double)c->g.cells());
-  count_launch();
+  fused::sor_rule(c->s, c->loop, tol, max_iter, (double)c->g.cells());
   return take_status();
 }
 
