@@ -55,6 +55,16 @@ __host__ __device__ __forceinline__ Pr operator-(Pr a, Pr b) { return df::sub(a.
 __host__ __device__ __forceinline__ Pr operator*(Pr a, Pr b) { return df::mul(a.v, b.v); }
 __host__ __device__ __forceinline__ Pr operator-(Pr a) { return df::neg(a.v); }
 
+// bits: whether a and b differ, whether a vector is 0 (either sign), whether a is finite
+__device__ __forceinline__ bool differ(float a, float b) { return __float_as_uint(a) != __float_as_uint(b); }
+__device__ __forceinline__ bool differ(Pr a, Pr b) { return differ(a.v.h, b.v.h) || differ(a.v.l, b.v.l); }
+__device__ __forceinline__ bool finite(float a) { return (__float_as_uint(a) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ bool finite(Pr a) { return finite(a.v.h) && finite(a.v.l); }
+__device__ __forceinline__ bool nonzero(float a) { return (__float_as_uint(a) << 1) != 0; }
+__device__ __forceinline__ bool nonzero(Pr a) { return nonzero(a.v.h) || nonzero(a.v.l); }
+__device__ __forceinline__ float zero(float) { return 0.0f; }
+__device__ __forceinline__ Pr zero(Pr) { return df::D{0.0f, 0.0f}; }
+
 template <class R>
 struct CsfP {
   R dxi, dyi, dzi, gx, gy, gz, vs2, vs8;  // vs2 = 2 vs, vs8 = 8 vs
@@ -76,7 +86,7 @@ struct Smem {
 // vs scaled by 1/c: N(c w) = w/(|w| + vs/c).
 // FP32: where |v| < 1e-15 the squares would leave the normal range, so numerator
 // and denominator are both scaled by 2^64 first (an exact power-of-two scaling).
-__device__ __forceinline__ void unit(float x, float y, float z, float vs, float* o) {
+__device__ __forceinline__ void unit_of(float x, float y, float z, float vs, float* o) {
   float s = x * x + y * y + z * z;
   if (s < 1.0e-30f) {
     const float c = 18446744073709551616.0f;  // 2^64
@@ -95,7 +105,7 @@ __device__ __forceinline__ void unit(float x, float y, float z, float vs, float*
 // FP32 pairs.  Where |v| is below about 2^-50 the squares approach float's normal
 // range, so v and vs are scaled by 2^64 first (exact; N is unchanged); a sum of
 // squares below 2^-126 after that counts as 0 (|v| + vs = vs).
-__device__ __forceinline__ void unit(Pr x, Pr y, Pr z, Pr vs, Pr* o) {
+__device__ __forceinline__ void unit_of(Pr x, Pr y, Pr z, Pr vs, Pr* o) {
   using namespace df;
   D X = x.v, Y = y.v, Z = z.v, V = vs.v;
   D s = add(add(sqr(X), sqr(Y)), sqr(Z));
@@ -120,6 +130,15 @@ __device__ __forceinline__ void unit(Pr x, Pr y, Pr z, Pr vs, Pr* o) {
   o[2] = mul(Z, inv);
 }
 
+// a warp of zero vectors takes the zeros without the reciprocal
+template <class R>
+__device__ __forceinline__ void unit(R x, R y, R z, R vs, R* o) {
+  if (__any_sync(__activemask(), nonzero(x) || nonzero(y) || nonzero(z)))
+    unit_of(x, y, z, vs, o);
+  else
+    o[0] = o[1] = o[2] = zero(x);
+}
+
 // vertex gradient at (i+1/2, j+1/2, k+1/2) from two staged planes (Qa = plane k, Qb =
 // plane k+1)
 template <class R>
@@ -129,6 +148,13 @@ __device__ void grad_staged(const CsfP<R>& p, const R* Qa, const R* Qb, R (*G)[G
     const int c = b * QX + a;
     const R q000 = Qa[c], qp00 = Qa[c + 1], q0p0 = Qa[c + QX], qpp0 = Qa[c + QX + 1];
     const R q00p = Qb[c], qp0p = Qb[c + 1], q0pp = Qb[c + QX], qppp = Qb[c + QX + 1];
+    // a warp of flat points stores the zeros that the sums would give
+    const bool varies = !finite(q000) || differ(q000, qp00) || differ(q000, q0p0) || differ(q000, qpp0) ||
+                        differ(q000, q00p) || differ(q000, qp0p) || differ(q000, q0pp) || differ(q000, qppp);
+    if (!__any_sync(__activemask(), varies)) {
+      G[0][e] = G[1][e] = G[2][e] = zero(q000);
+      continue;
+    }
     if constexpr (std::is_same<R, Pr>::value) {
       // the FP64 path's sums and differences of the two planes (15 pair additions)
       const R s00 = q000 + q00p, sp0 = qp00 + qp0p, s0p = q0p0 + q0pp, spp = qpp0 + qppp;
@@ -238,18 +264,23 @@ __global__ void __launch_bounds__(256) k_csf(Grid g, CsfP<R> p, int kchunk, cons
       const long c = g.at(i, j, k);
       const int e = ty * NX + tx;            // npp point (i, j)
       const int f = (ty + 1) * NX + tx + 1;  // n12/n13/n23 point (i, j)
-      const R ku = (S.pp[sp][0][e + 1] - S.pp[sp][0][e]) * p.dxi + (S.a12[sp][1][f] - S.a12[sp][1][f - NX]) * p.dyi +
-                   (S.a13[sm ^ 1][1][f] - S.a13[sm][1][f]) * p.dzi;
-      const R kv = (S.a12[sp][0][f] - S.a12[sp][0][f - 1]) * p.dxi + (S.pp[sp][1][e + NX] - S.pp[sp][1][e]) * p.dyi +
-                   (S.a23[sm ^ 1][1][f] - S.a23[sm][1][f]) * p.dzi;
-      const R kw = (S.a13[sm ^ 1][0][f] - S.a13[sm ^ 1][0][f - 1]) * p.dxi +
-                   (S.a23[sm ^ 1][0][f] - S.a23[sm ^ 1][0][f - NX]) * p.dyi + (S.pp[sp ^ 1][2][e] - S.pp[sp][2][e]) * p.dzi;
       const int cq = (ty + 1) * QX + tx + 1;
       const R* Qk = S.Q[k % 3];
       const R ph = Qk[cq], px = Qk[cq + 1], py = Qk[cq + QX], pz = S.Q[(k + 1) % 3][cq];
-      fu[c] = (double)(ku * (px - ph) * p.fx);
-      fv[c] = (double)(kv * (py - ph) * p.fy);
-      fw[c] = (double)(kw * (pz - ph) * p.fz);
+      const bool varies = !finite(ph) || differ(ph, px) || differ(ph, py) || differ(ph, pz);
+      if (__any_sync(__activemask(), varies)) {
+        const R ku = (S.pp[sp][0][e + 1] - S.pp[sp][0][e]) * p.dxi + (S.a12[sp][1][f] - S.a12[sp][1][f - NX]) * p.dyi +
+                     (S.a13[sm ^ 1][1][f] - S.a13[sm][1][f]) * p.dzi;
+        const R kv = (S.a12[sp][0][f] - S.a12[sp][0][f - 1]) * p.dxi + (S.pp[sp][1][e + NX] - S.pp[sp][1][e]) * p.dyi +
+                     (S.a23[sm ^ 1][1][f] - S.a23[sm][1][f]) * p.dzi;
+        const R kw = (S.a13[sm ^ 1][0][f] - S.a13[sm ^ 1][0][f - 1]) * p.dxi +
+                     (S.a23[sm ^ 1][0][f] - S.a23[sm ^ 1][0][f - NX]) * p.dyi + (S.pp[sp ^ 1][2][e] - S.pp[sp][2][e]) * p.dzi;
+        fu[c] = (double)(ku * (px - ph) * p.fx);
+        fv[c] = (double)(kv * (py - ph) * p.fy);
+        fw[c] = (double)(kw * (pz - ph) * p.fz);
+      } else {
+        fu[c] = fv[c] = fw[c] = 0.0;
+      }
     }
     __syncthreads();
     gA ^= 1;

@@ -94,7 +94,7 @@ struct SrcIn {
   const double *u, *v, *w, *rho, *rhon, *adv[3], *advo[3], *phat, *vis[3], *fst[3], *fstn[3];
   double grvb, grvp;
 };
-// Outputs: FP64 A and B per component, or (REFINE) FP32 A and the FP64 first-sweep
+// Outputs: FP64 A and B per component, or (k_src_ab_e) FP32 A and the FP64 first-sweep
 // residual R = A*visn(u) + B - u rounded to FP32 (the right-hand side of the
 // correction sweeps of the mixed-precision solve).
 struct ABOut {
@@ -176,20 +176,18 @@ __global__ void __launch_bounds__(256) k_src_ab(Grid g, SrcK K, SrcIn in, const 
   store(2, in.w, sw, Aw, L(in.phat, Z) - p0, K.pz);
 }
 
-// k_src_ab with A and B in FP32-pair arithmetic (each double read split into a
-// pair, A and B rounded to doubles once).  The FP64-accurate step (FMF_FP64E, REFINE
-// false) stores them.  The mixed-precision step (REFINE true) forms the first-sweep
-// residual R = A visn(u) + B - u from them in FP64: the
-// viscous sum visn reads 20 doubles for about 25 operations, and with it in pairs
-// as well the kernel measured 10.2 ms against 9.7 for an all-FP64 kernel at
-// 512x256x256 (the splits cost more than the FP64 operations they replace); in
-// this form, 6.7 ms.  The momentum-factor denominator is
+// The mixed-precision step's factors: A and B in FP32-pair arithmetic (each double read
+// split into a pair, A and B rounded to doubles once) and from them the first-sweep
+// residual R = A visn(u) + B - u in FP64.  The viscous sum visn reads 20 doubles for about
+// 25 operations; in pairs as well the kernel measured 10.2 ms against 9.7 for an all-FP64
+// kernel at 512x256x256 (the splits cost more than the FP64 operations they replace); in
+// this form, 6.7 ms.  (The FP64-accurate step took A and B alone from here; k_src_ab is
+// faster now: 1.9 ms against 3.6.)  The momentum-factor denominator is
 // grouped as dz2 (e(-Z) + e(0)) + dy2 (e(-Y) + e(0)) + 2 dx2 (mu(0) + mu(X)) (and
 // likewise per component), the same sum.
 struct VPS {
   df::D dtinv, dx2, dy2, dz2, dx2x2, dy2x2, dz2x2, grvb, grvp;
 };
-template <bool REFINE>
 __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pv, Fac<double> pd, SrcIn in, const double* __restrict__ mu,
                                                   const double* __restrict__ exy, const double* __restrict__ exz,
                                                   const double* __restrict__ eyz, ABOut out) {
@@ -211,17 +209,12 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pv, Fac<doub
     t = add(t, grav);
     return add(sub(mul(r, t), prs), scale(L(in.vis[q], 0), 0.5f));
   };
-  // A = T/2, B = rs T; REFINE: A and R = A visn + B - u (FP64) as floats
+  // A = T/2, B = rs T; A and R = A visn + B - u (FP64) as floats
   auto store = [&](int q, D r, D ap, D rs, double vn, const double* vel) {
     const D T = div(D{1.0f, 0.0f}, add(mul(r, p.dtinv), scale(ap, 0.5f)));
     const double A = to_double(scale(T, 0.5f)), B = to_double(mul(rs, T));
-    if (REFINE) {
-      out.af[q][c] = (float)A;
-      out.rf[q][c] = (float)(A * vn + B - __ldg(vel + c));
-    } else {
-      out.a[q][c] = A;
-      out.b[q][c] = B;
-    }
+    out.af[q][c] = (float)A;
+    out.rf[q][c] = (float)(A * vn + B - __ldg(vel + c));
   };
   const D zero{0.0f, 0.0f};
   {
@@ -229,7 +222,7 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pv, Fac<doub
     D ap = mul(p.dz2, add(L(exz, -Z), L(exz, 0)));
     ap = add(ap, mul(p.dy2, add(L(exy, -Y), L(exy, 0))));
     ap = add(ap, mul(p.dx2x2, add(mu0, L(mu, X))));
-    const double vn = REFINE ? visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
+    const double vn = visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
     store(0, r, ap, rsrc(0, in.u, r, p.grvb, X, pv.dxi), vn, in.u);
   }
   if (j <= g.nj - 1) {
@@ -237,7 +230,7 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pv, Fac<doub
     D ap = mul(p.dz2, add(L(eyz, -Z), L(eyz, 0)));
     ap = add(ap, mul(p.dy2x2, add(mu0, L(mu, Y))));
     ap = add(ap, mul(p.dx2, add(L(exy, -X), L(exy, 0))));
-    const double vn = REFINE ? visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
+    const double vn = visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
     store(1, r, ap, rsrc(1, in.v, r, p.grvp, Y, pv.dyi), vn, in.v);
   }
   {
@@ -245,7 +238,7 @@ __global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pv, Fac<doub
     D ap = mul(p.dz2x2, add(mu0, L(mu, Z)));
     ap = add(ap, mul(p.dy2, add(L(eyz, -Y), L(eyz, 0))));
     ap = add(ap, mul(p.dx2, add(L(exz, -X), L(exz, 0))));
-    const double vn = REFINE ? visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w) : 0.0;
+    const double vn = visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
     store(2, r, ap, rsrc(2, in.w, r, zero, Z, pv.dzi), vn, in.w);
   }
 }
@@ -1439,14 +1432,13 @@ PairShape pair_shape(const Grid& g, bool fp64) {
 // first colour of each pair (solu_sor4.f:94-120): (1,1,1) (1,1,2) (1,2,1) (2,1,1)
 const int kPi[4] = {1, 1, 1, 2}, kPj[4] = {1, 1, 2, 1}, kPk[4] = {1, 2, 1, 1};
 
-// k_edges + k_src_ab<REFINE> + k_wall_coef
+// k_edges, k_src_ab or (REFINE) k_src_ab_e, k_wall_coef
 template <bool REFINE>
 void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const double* v, const double* w,
               const double* const* adv, const double* const* advo, const double* phat,
               const double* const* vis, const double* const* fst, const double* const* fstn, double grvb,
               double grvp, const Fluids& fl, const double* mu, const double* rho, const double* rhon, double* const* E,
-              F3 ef, ABOut out, const double* l1, const double* l2, const double* phi, double dy, double* wallc,
-              bool pairs) {
+              F3 ef, ABOut out, const double* l1, const double* l2, const double* phi, double dy, double* wallc) {
   SrcIn in;
   in.u = u;
   in.v = v;
@@ -1465,7 +1457,7 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
   in.grvp = grvp;
   k_edges<<<dim3((unsigned)(((long)(g.ni + 1) * (g.nj + 1) + 127) / 128), (unsigned)(g.nk + 1)), 128, 0, s>>>(
       g, p, mu, E[0], E[1], E[2], ef);
-  if (pairs) {
+  if (REFINE) {
     using df::split_double;
     VPS ps;
     ps.dtinv = split_double(p.dtinv);
@@ -1477,7 +1469,7 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
     ps.dz2x2 = split_double(2.0 * p.dz2);
     ps.grvb = split_double(grvb);
     ps.grvp = split_double(grvp);
-    k_src_ab_e<REFINE><<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, ps, p, Fac<double>(p), in, mu, E[0], E[1],
+    k_src_ab_e<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, ps, p, Fac<double>(p), in, mu, E[0], E[1],
                                                                                  E[2], out);
   } else {
     SrcK K;
@@ -1552,14 +1544,14 @@ void src_visc_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
                    const double* const* adv, const double* const* advo, const double* phat,
                    const double* const* vis, const double* const* fst, const double* const* fstn, const Fluids& fl,
                    const double* mu, const double* rho, const double* rhon, double* const* E, double* const* AB, const double* l1,
-                   const double* l2, const double* phi, double dy, double* wallc, bool pairs) {
+                   const double* l2, const double* phi, double dy, double* wallc) {
   ABOut out{};
   for (int q = 0; q < 3; ++q) {
     out.a[q] = AB[2 * q];
     out.b[q] = AB[2 * q + 1];
   }
   src_prep<false>(s, g, make_vp(dxinv, dyinv, dzinv, dt, harmonic), u, v, w, adv, advo, phat, vis, fst, fstn, grvb,
-                  grvp, fl, mu, rho, rhon, E, F3{{nullptr, nullptr, nullptr}}, out, l1, l2, phi, dy, wallc, pairs);
+                  grvp, fl, mu, rho, rhon, E, F3{{nullptr, nullptr, nullptr}}, out, l1, l2, phi, dy, wallc);
 }
 
 void wall_coef(cudaStream_t s, const Grid& g, double dy, const double* l1, const double* l2, const double* phi,
@@ -1717,9 +1709,9 @@ void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
     out.af[q] = rb.a[q];
     out.rf[q] = rb.r[q];
   }
-  // A and B in FP32 pairs, the residual in FP64 (k_src_ab_e<true>)
+  // A and B in FP32 pairs, the residual in FP64 (k_src_ab_e)
   src_prep<true>(s, g, make_vp(dxinv, dyinv, dzinv, dt, harmonic), u, v, w, adv, advo, phat, vis, fst, fstn, grvb,
-                 grvp, fl, mu, rho, rhon, E, F3{{rb.e[0], rb.e[1], rb.e[2]}}, out, l1, l2, phi, dy, wallc, true);
+                 grvp, fl, mu, rho, rhon, E, F3{{rb.e[0], rb.e[1], rb.e[2]}}, out, l1, l2, phi, dy, wallc);
   k_to_float<<<4 * 152, 256, 0, s>>>(g.n, mu, rb.mu);
   k_gamma_wall<<<wall_grid(g), kB, 0, s>>>(g, uwall, wallc, u, v, w, rb.gw);
   k_gamma_x<<<xh_grid(g), kB, 0, s>>>(g, u, v, w, rb.gx);
