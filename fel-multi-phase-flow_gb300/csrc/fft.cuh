@@ -7,18 +7,21 @@ namespace fmf {
 // In-place decimation-in-time FFT of L complex values (L a power of two) in shared
 // memory (re, im), run by the nthr threads t = 0..nthr-1 of a group; every thread
 // of the block reaches the same __syncthreads.  tw[m] = (cos, sin)(2 pi m / L),
-// m < L/2, computed on the host; sign sgn = -1 forward, +1 inverse.  After the
+// m < L/2, computed on the host; sign SGN = -1 forward, +1 inverse.  After the
 // bit-reversal permutation the radix-2 stages are taken two at a time (radix
 // 2^2): with span h, the four points x0..x3 at a, a+h, a+2h, a+3h (m = a mod h)
 // and w = W_4h^m,
 //   t1 = w^2 x1, t2 = w x2, t3 = w^3 x3,
 //   X0 = x0 + t1 + (t2 + t3),  X2 = x0 + t1 - (t2 + t3),
-//   X1 = x0 - t1 + sgn i (t2 - t3),  X3 = x0 - t1 - sgn i (t2 - t3),
-// which is the two radix-2 stages of spans h and 2h (W_4h^h = sgn i) with three
+//   X1 = x0 - t1 + SGN i (t2 - t3),  X3 = x0 - t1 - SGN i (t2 - t3),
+// which is the two radix-2 stages of spans h and 2h (W_4h^h = SGN i) with three
 // twiddle products instead of four and one pass over shared memory instead of
-// two; a single radix-2 stage first where log2 L is odd.
-__device__ __forceinline__ void group_fft(double* re, double* im, int L, double sgn, int t, int nthr,
+// two; a single radix-2 stage first where log2 L is odd.  Bound by the FP64 pipe: 28
+// operations per four points (the signs are the compiler's and bit flips, not products).
+template <int SGN>
+__device__ __forceinline__ void group_fft(double* re, double* im, int L, int t, int nthr,
                                           const double2* __restrict__ tw) {
+  constexpr double sgn = SGN;
   int lg = 0;
   while ((1 << lg) < L) ++lg;
   for (int a = t; a < L; a += nthr) {
@@ -55,16 +58,12 @@ __device__ __forceinline__ void group_fft(double* re, double* im, int L, double 
       double t1r = x1r, t1i = x1i, t2r = x2r, t2i = x2i, t3r = x3r, t3i = x3i;
       if (m) {
         const double2 w1 = __ldg(tw + m * step), w2 = __ldg(tw + 2 * m * step);
-        const int k3 = 3 * m;
-        double2 w3;
-        double s3 = 1.0;
-        if (k3 < 2 * h) {
-          w3 = __ldg(tw + k3 * step);
-        } else {  // W^k = -W^(k - 2h)
-          w3 = __ldg(tw + (k3 - 2 * h) * step);
-          s3 = -1.0;
-        }
-        const double c1 = w1.x, s1 = sgn * w1.y, c2 = w2.x, s2 = sgn * w2.y, c3 = s3 * w3.x, sn3 = s3 * sgn * w3.y;
+        // W^k = -W^(k - 2h)
+        const int k3 = 3 * m, flip = k3 < 2 * h ? 0 : (int)0x80000000;
+        double2 w3 = __ldg(tw + (flip ? k3 - 2 * h : k3) * step);
+        w3.x = __hiloint2double(__double2hiint(w3.x) ^ flip, __double2loint(w3.x));
+        w3.y = __hiloint2double(__double2hiint(w3.y) ^ flip, __double2loint(w3.y));
+        const double c1 = w1.x, s1 = sgn * w1.y, c2 = w2.x, s2 = sgn * w2.y, c3 = w3.x, sn3 = sgn * w3.y;
         t1r = c2 * x1r - s2 * x1i;  // w^2 x1
         t1i = c2 * x1i + s2 * x1r;
         t2r = c1 * x2r - s1 * x2i;  // w x2

@@ -145,7 +145,8 @@ __device__ __forceinline__ void gexp8(R* E, R X1, R X2, R Y1, R Y2, R Z1, R Z2) 
   E[6] = c * Z2;
   E[7] = d * Z2;
 }
-__global__ void __launch_bounds__(256) k_classify(Grid g, MC m, const double* __restrict__ phi,
+// (five blocks per SM, 199 -> 178 us at 256x128x128)
+__global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double* __restrict__ phi,
                                                   const double* __restrict__ gx, const double* __restrict__ gy,
                                                   const double* __restrict__ gz, const double* __restrict__ u,
                                                   const double* __restrict__ v, const double* __restrict__ w,

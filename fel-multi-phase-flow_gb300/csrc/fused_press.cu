@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256) k_rfft_x_fwd(Grid g, const double* __rest
     im[n] = div[c0 + 2 * n + 1];
   }
   __syncthreads();
-  group_fft(re, im, M, -1.0, t, kRowThreads, twM);
+  group_fft<-1>(re, im, M, t, kRowThreads, twM);
   const long o = ((long)(k - 1) * g.nj + (j - 1)) * H;
   for (int m = t; m < H; m += kRowThreads) {
     const int a = m % M, b = (M - m) % M;
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) k_rfft_x_inv(Grid g, const double* __rest
     yi[m] = ai + cr;
   }
   __syncthreads();
-  group_fft(yr, yi, M, +1.0, t, kRowThreads, twM);
+  group_fft<1>(yr, yi, M, t, kRowThreads, twM);
   const long c0 = g.at(1, j, k);
   for (int n = t; n < M; n += kRowThreads) {
     dp[c0 + 2 * n] = yr[n];
@@ -102,9 +102,10 @@ __global__ void __launch_bounds__(256) k_rfft_x_inv(Grid g, const double* __rest
 
 // z transform of the half spectrum, 16 columns kx per block, one j per grid y;
 // in and out in the spectrum layout (in place allowed), scaled by `scale`
+// (SGN = 1: scale 1)
+template <int SGN>
 __global__ void __launch_bounds__(256) k_fft_z_half(Grid g, const double* tr, const double* ti, double* pr,
-                                                    double* pi, const double2* __restrict__ tw, double sgn,
-                                                    double scale) {
+                                                    double* pi, const double2* __restrict__ tw, double scale) {
   extern __shared__ double sm[];
   const int L = g.nk, H = g.ni / 2 + 1, NJ = g.nj;
   const int j = blockIdx.y;
@@ -117,13 +118,13 @@ __global__ void __launch_bounds__(256) k_fft_z_half(Grid g, const double* tr, co
   }
   __syncthreads();
   const int col = threadIdx.x / 16;
-  group_fft(sm + col * 2 * L, sm + col * 2 * L + L, L, sgn, threadIdx.x % 16, 16, tw);
+  group_fft<SGN>(sm + col * 2 * L, sm + col * 2 * L + L, L, threadIdx.x % 16, 16, tw);
   for (int e = threadIdx.x; e < L * kTileZ; e += blockDim.x) {
     const int cl = e % kTileZ, kz = e / kTileZ, kx = kx0 + cl;
     if (kx >= H) continue;
     const long o = ((long)kz * NJ + j) * H + kx;
-    pr[o] = sm[cl * 2 * L + kz] * scale;
-    pi[o] = sm[cl * 2 * L + L + kz] * scale;
+    pr[o] = SGN > 0 ? sm[cl * 2 * L + kz] : sm[cl * 2 * L + kz] * scale;
+    pi[o] = SGN > 0 ? sm[cl * 2 * L + L + kz] : sm[cl * 2 * L + L + kz] * scale;
   }
 }
 
@@ -300,9 +301,10 @@ void pressure_half(cudaStream_t s, const Grid& g, double rho, double dxinv, doub
   cudaFuncSetAttribute(k_rfft_x_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf);
   cudaFuncSetAttribute(k_rfft_x_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smi);
   k_rfft_x_fwd<<<rows / kRows, 256, smf, s>>>(g, div, tr, ti, twM, twN);
-  cudaFuncSetAttribute(k_fft_z_half, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
+  cudaFuncSetAttribute(k_fft_z_half<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
+  cudaFuncSetAttribute(k_fft_z_half<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
   const dim3 gz((unsigned)((H + kTileZ - 1) / kTileZ), (unsigned)g.nj);
-  k_fft_z_half<<<gz, 256, smz, s>>>(g, tr, ti, pr, pi, twz, -1.0, 1.0 / ((double)g.ni * (double)g.nk));
+  k_fft_z_half<-1><<<gz, 256, smz, s>>>(g, tr, ti, pr, pi, twz, 1.0 / ((double)g.ni * (double)g.nk));
   const double pi_ = 3.141592653589793238462643383279502884;
   const double dx2r = dxinv * dxinv / rho, dz2r = dzinv * dzinv / rho;
   if (coef)
@@ -310,7 +312,7 @@ void pressure_half(cudaStream_t s, const Grid& g, double rho, double dxinv, doub
   else
     k_tdma_half<<<dim3((unsigned)((H + 127) / 128), (unsigned)g.nk), 128, 0, s>>>(
         g, dx2r, dz2r, pi_ * 2.0 / (double)g.ni, pi_ * 2.0 / (double)g.nk, as_f, an_f, ap_f, pr, pi, at);
-  k_fft_z_half<<<gz, 256, smz, s>>>(g, pr, pi, tr, ti, twz, +1.0, 1.0);
+  k_fft_z_half<1><<<gz, 256, smz, s>>>(g, pr, pi, tr, ti, twz, 1.0);
   k_rfft_x_inv<<<rows / kRows, 256, smi, s>>>(g, tr, ti, dp, twM, twN);
   count_launch(5);
 }

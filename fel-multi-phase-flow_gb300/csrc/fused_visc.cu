@@ -188,7 +188,9 @@ __global__ void __launch_bounds__(256) k_src_ab(Grid g, SrcK K, SrcIn in, const 
 struct VPS {
   df::D dtinv, dx2, dy2, dz2, dx2x2, dy2x2, dz2x2, grvb, grvp;
 };
-__global__ void __launch_bounds__(256) k_src_ab_e(Grid g, VPS p, VP pv, Fac<double> pd, SrcIn in, const double* __restrict__ mu,
+// (four blocks per SM: at the 80 registers it would take, the FP64 pipe is 65 % busy and
+// 872 us go by at 256x128x128; at 64, 777)
+__global__ void __launch_bounds__(256, 4) k_src_ab_e(Grid g, VPS p, VP pv, Fac<double> pd, SrcIn in, const double* __restrict__ mu,
                                                   const double* __restrict__ exy, const double* __restrict__ exz,
                                                   const double* __restrict__ eyz, ABOut out) {
   using namespace df;

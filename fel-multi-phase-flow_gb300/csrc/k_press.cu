@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(256) k_fft_x_fwd(Grid g, const double* div, do
     im[a] = 0.0;
   }
   __syncthreads();
-  group_fft(re, im, L, -1.0, threadIdx.x, blockDim.x, tw);
+  group_fft<-1>(re, im, L, threadIdx.x, blockDim.x, tw);
   const long o = ((long)(k - 1) * g.nj + (j - 1)) * L;
   for (int a = threadIdx.x; a < L; a += blockDim.x) {
     tr[o + a] = re[a];
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256) k_fft_x_inv(Grid g, const double* tr, con
     im[a] = ti[o + a];
   }
   __syncthreads();
-  group_fft(re, im, L, +1.0, threadIdx.x, blockDim.x, tw);
+  group_fft<1>(re, im, L, threadIdx.x, blockDim.x, tw);
   const long c0 = g.at(1, j, k);
   for (int a = threadIdx.x; a < L; a += blockDim.x) dp[c0 + a] = re[a];
 }
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) k_fft_z_fwd(Grid g, const double* tr, con
   }
   __syncthreads();
   const int col = threadIdx.x / 16;
-  group_fft(sm + col * 2 * L, sm + col * 2 * L + L, L, -1.0, threadIdx.x % 16, 16, tw);
+  group_fft<-1>(sm + col * 2 * L, sm + col * 2 * L + L, L, threadIdx.x % 16, 16, tw);
   const double scale = (double)((long)NI * g.nk);
   for (int e = threadIdx.x; e < L * kTile; e += blockDim.x) {
     const int cl = e % kTile, kz = e / kTile;
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256) k_fft_z_inv(Grid g, const double* pr, con
   }
   __syncthreads();
   const int col = threadIdx.x / 16;
-  group_fft(sm + col * 2 * L, sm + col * 2 * L + L, L, +1.0, threadIdx.x % 16, 16, tw);
+  group_fft<1>(sm + col * 2 * L, sm + col * 2 * L + L, L, threadIdx.x % 16, 16, tw);
   for (int e = threadIdx.x; e < L * kTile; e += blockDim.x) {
     const int cl = e % kTile, kz = e / kTile;
     const long o = ((long)kz * NJ + (j - 1)) * NI + kx0 + cl;
