@@ -237,10 +237,11 @@ void src_ab_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi,
               double grvp, const SrcArgs& a, const double* const* lAB, const SrcAdj& l);
 void edges_T(cudaStream_t s, const Grid& g, int harmonic, const double* mu, const double* const* lE, double* lmu);
 // the forward states before each of the 12 sweeps of one outer iteration started at
-// ustar: snaps = 39n doubles (12 x 3 fields, then the running state)
-void sor_replay(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, const double* mu,
+// ustar: snaps = 39n doubles (12 x 3 fields, then the running state); part as in
+// fused::sor_iteration
+void sor_replay(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, int harmonic, const double* mu,
                 double* const* E, double* const* AB, double uwall, const double* wallc, const double* const* ustar,
-                double* snaps);
+                double* snaps, double* part);
 // CUDA graphs of one transposed iteration, keyed by the buffers they read and write
 using GraphCache = std::map<std::vector<const void*>, std::pair<cudaGraphExec_t, long long>>;
 // The executable graph of `body` for this set of buffers (key): captured on s the
@@ -250,7 +251,7 @@ cudaGraphExec_t cached_graph(cudaStream_t s, GraphCache* cache, const std::vecto
                              const std::function<void()>& body, long long* per_launch);
 // transposed fixed-point solve and gradient collection; lam: 3 output arrays (the
 // converged adjoint of un*, consumed by the gradient pass); lAB, lmu, lE, lwc
-// accumulate; work: >= 3n + 1026 doubles; host_norm: 2 pinned doubles; cache may
+// accumulate; work: >= 1026 doubles; host_norm: 2 pinned doubles; cache may
 // be null (no graphs).  fb_out (3n) receives the feedback term G^T lam of the
 // solve and *fb_norm its norm.  Where *fb_norm > 0 on entry, fb holds the previous
 // solve's feedback term (and fb_prev, if not null, the one before): the solve

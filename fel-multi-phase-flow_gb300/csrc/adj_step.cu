@@ -747,7 +747,8 @@ void reverse_step(fmf_adj* a, const double* st, bool defer) {
   // :605-623 the viscous solve
   {  // the 12 sweep snapshots of the fixed point, replayed as a CUDA graph per record slot
     auto replay = [&]() {
-      adj::sor_replay(s, g, dxi, dyi, dzi, a->rmun, a->E, a->AB, P.uwall, a->wallc, a->ustar, a->snaps);
+      adj::sor_replay(s, g, dxi, dyi, dzi, P.harmonic, a->rmun, a->E, a->AB, P.uwall, a->wallc, a->ustar,
+                      a->snaps, a->sorpart);
     };
     long long per_launch = 0;
     const cudaGraphExec_t exec =

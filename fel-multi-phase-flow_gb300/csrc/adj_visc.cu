@@ -10,6 +10,9 @@
 // more backward sweep that collects the gradients with respect to A, B, the edge
 // viscosities, mu and the slip coefficients.  The forward states before each sweep
 // of one cycle at the fixed point are replayed from un* (12 snapshots).
+#include <algorithm>
+#include <type_traits>
+
 #include "../../include/fmf_capi.h"
 #include "adj.cuh"
 #include "fused.cuh"
@@ -32,74 +35,6 @@ VPa make_vpa(double dxi, double dyi, double dzi) {
   p.dyz = dyi * dzi;
   return p;
 }
-// The 14 terms of visn for component COMP at c: term t reads array arr[t] (0 u,
-// 1 v, 2 w) at c + off[t] with coefficient mult[t] * coefficient cf[t], where the
-// coefficient is mu (ca[t] = 0) or edge array ca[t]-1 at index ci[t].
-struct Sten {
-  int arr[14], ca[14];
-  long off[14], ci[14];
-  double mult[14];
-};
-template <int COMP>
-__device__ void stencil(const Grid& g, const VPa& p, long c, Sten& S) {
-  const long X = 1, Y = g.sy, Z = g.sz;
-  int t = 0;
-  auto put = [&](int arr, long off, double mult, int ca, long ci) {
-    S.arr[t] = arr;
-    S.off[t] = off;
-    S.mult[t] = mult;
-    S.ca[t] = ca;
-    S.ci[t] = ci;
-    ++t;
-  };
-  // edge arrays: 1 = exy, 2 = exz, 3 = eyz
-  if (COMP == 0) {
-    put(0, -Z, p.dz2, 2, c - Z);
-    put(0, Z, p.dz2, 2, c);
-    put(0, -Y, p.dy2, 1, c - Y);
-    put(0, Y, p.dy2, 1, c);
-    put(0, -X, 2.0 * p.dx2, 0, c);
-    put(0, X, 2.0 * p.dx2, 0, c + X);
-    put(1, -Y, p.dxy, 1, c - Y);
-    put(1, X - Y, -p.dxy, 1, c - Y);
-    put(1, X, p.dxy, 1, c);
-    put(1, 0, -p.dxy, 1, c);
-    put(2, -Z, p.dxz, 2, c - Z);
-    put(2, X - Z, -p.dxz, 2, c - Z);
-    put(2, X, p.dxz, 2, c);
-    put(2, 0, -p.dxz, 2, c);
-  } else if (COMP == 1) {
-    put(1, -Z, p.dz2, 3, c - Z);
-    put(1, Z, p.dz2, 3, c);
-    put(1, -Y, 2.0 * p.dy2, 0, c);
-    put(1, Y, 2.0 * p.dy2, 0, c + Y);
-    put(1, -X, p.dx2, 1, c - X);
-    put(1, X, p.dx2, 1, c);
-    put(0, -X, p.dxy, 1, c - X);
-    put(0, -X + Y, -p.dxy, 1, c - X);
-    put(0, Y, p.dxy, 1, c);
-    put(0, 0, -p.dxy, 1, c);
-    put(2, -Z, p.dyz, 3, c - Z);
-    put(2, Y - Z, -p.dyz, 3, c - Z);
-    put(2, Y, p.dyz, 3, c);
-    put(2, 0, -p.dyz, 3, c);
-  } else {
-    put(2, -Z, 2.0 * p.dz2, 0, c);
-    put(2, Z, 2.0 * p.dz2, 0, c + Z);
-    put(2, -Y, p.dy2, 3, c - Y);
-    put(2, Y, p.dy2, 3, c);
-    put(2, -X, p.dx2, 2, c - X);
-    put(2, X, p.dx2, 2, c);
-    put(0, -X, p.dxz, 2, c - X);
-    put(0, -X + Z, -p.dxz, 2, c - X);
-    put(0, Z, p.dxz, 2, c);
-    put(0, 0, -p.dxz, 2, c);
-    put(1, -Y, p.dyz, 3, c - Y);
-    put(1, -Y + Z, -p.dyz, 3, c - Y);
-    put(1, Z, p.dyz, 3, c);
-    put(1, 0, -p.dyz, 3, c);
-  }
-}
 struct Arr3 {
   double* a[3];
 };
@@ -113,102 +48,142 @@ struct CArr3 {
   const double* a[3];
 };
 
-// transposed sweep of one colour pair: l_C at the swept points is scattered to the
-// 14 neighbours (times A) and cleared
-template <int COMP>
-__global__ void __launch_bounds__(256) k_pair_T(Grid g, VPa p, int pi, int pj, int pk, CArr4 cf,
-                                                const double* __restrict__ A, Arr3 l) {
-  const int jmax = COMP == 1 ? g.nj - 1 : g.nj;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int i = (h ? 3 - pi : pi) + 2 * (int)(blockIdx.x * 32 + threadIdx.x);
-    const int j = (h ? 3 - pj : pj) + 2 * (int)(blockIdx.y * 8 + threadIdx.y);
-    const int k = (h ? 3 - pk : pk) + 2 * (int)blockIdx.z;
-    if (i > g.ni || j > jmax || k > g.nk) continue;
-    const long c = g.at(i, j, k);
-    const double m = l.a[COMP][c];
-    if (m == 0.0) continue;
-    l.a[COMP][c] = 0.0;
-    Sten S;
-    stencil<COMP>(g, p, c, S);
-    const double ma = m * A[c];
-    for (int t = 0; t < 14; ++t) aadd(l.a[S.arr[t]] + c + S.off[t], ma * S.mult[t] * cf.a[S.ca[t]][S.ci[t]]);
-  }
+// The factors of visn of component COMP in the form of the forward sweeps: with S its own
+// axis and, per transverse axis T with edge viscosity e and component F along T,
+//   own (mu(S) q(S) + mu q(-S)) + sum_T k_T (e(-T) b(-T) + e b(T)),
+//   b(T) = q(T) + r_T (F(S) - F(0)),  b(-T) = q(-T) + r_T (F(-T) - F(S-T)).
+struct SwK {
+  double own, k1, k2, r1, r2;
+};
+SwK make_swk(double dxi, double dyi, double dzi, int comp) {
+  const double d[3] = {dxi, dyi, dzi};
+  const double s = d[comp], a = d[comp == 0 ? 1 : 0], b = d[comp == 2 ? 1 : 2];
+  return SwK{2.0 * s * s, a * a, b * b, s / a, s / b};
 }
-// gradient collection of one pair at the fixed point: lB += l, lA += l * visn(q),
-// and the coefficient adjoints (q = the forward state before this sweep)
-template <int COMP>
-__global__ void __launch_bounds__(256) k_pair_grad(Grid g, VPa p, int pi, int pj, int pk, CArr4 cf,
-                                                   const double* __restrict__ A, CArr3 q, Arr3 l, double* lA,
-                                                   double* lB, Arr4 lcf) {
-  const int jmax = COMP == 1 ? g.nj - 1 : g.nj;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int i = (h ? 3 - pi : pi) + 2 * (int)(blockIdx.x * 32 + threadIdx.x);
-    const int j = (h ? 3 - pj : pj) + 2 * (int)(blockIdx.y * 8 + threadIdx.y);
-    const int k = (h ? 3 - pk : pk) + 2 * (int)blockIdx.z;
-    if (i > g.ni || j > jmax || k > g.nk) continue;
-    const long c = g.at(i, j, k);
-    const double m = l.a[COMP][c];
-    if (m == 0.0) continue;
-    Sten S;
-    stencil<COMP>(g, p, c, S);
-    double visn = 0.0;
-    for (int t = 0; t < 14; ++t) {
-      const double qv = q.a[S.arr[t]][c + S.off[t]];
-      visn += S.mult[t] * cf.a[S.ca[t]][S.ci[t]] * qv;
-      aadd(lcf.a[S.ca[t]] + S.ci[t], m * A[c] * S.mult[t] * qv);
+struct GradIn {
+  const double *q0, *q1, *q2;  // the forward state before this sweep: own, T1's, T2's
+  double *lA, *lB, *lmu, *le1, *le2;
+};
+
+// Transposed sweep of one colour pair: l at the swept points (OWN: with the adjoints of
+// their x and z images, cleared; the wall rows of their columns hold none yet: within the
+// component only the points of the wall row themselves scatter into those, after this, and
+// before it the full transposed refresh cleared them) is scattered to their 14 neighbours
+// (times A) and cleared.  blockIdx.z takes the planes of the first colour, then of the
+// second.  Of the pair's points one at most reads a given point of another component
+// (their four offsets have four parities in the two axes and one in the third, and the
+// second colour has all three flipped), a given edge or a given mu: those adjoints are
+// read, added to and stored; only the swept component's own neighbours are read by two and
+// take atomics.
+// GRAD: the gradients at the fixed point too: lB += l, lA += l visn(q), and those of mu and
+// the edge viscosities.
+// Bound by the latency of its one round of loads at these sizes and by the atomics: with
+// all 14 as atomics, each point a thread for both colours and the full transposed refresh
+// (8 us) before every pair, a pair took 13.7 + 8 us at 128x64x64; now 9.4, with the images
+// 11; gradients in a kernel of their own 23 + 13.7, together 19.
+template <int COMP, bool OWN, bool GRAD>
+__global__ void __launch_bounds__(64, GRAD ? 10 : 16) k_pair_T(Grid g, SwK K, int pi, int pj, int pk, CArr4 cf,
+                                                const double* __restrict__ A, Arr3 la, GradIn G) {
+  const bool h = (int)blockIdx.z >= g.nk / 2;
+  const int i = (h ? 3 - pi : pi) + 2 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const int j = (h ? 3 - pj : pj) + 2 * (int)(blockIdx.y * blockDim.y + threadIdx.y);
+  const int k = (h ? 3 - pk : pk) + 2 * (int)(h ? blockIdx.z - g.nk / 2 : blockIdx.z);
+  if (i > g.ni || j > (COMP == 1 ? g.nj - 1 : g.nj)) return;
+  const long c = g.at(i, j, k), X = 1, Y = g.sy, Z = g.sz;
+  const long S = COMP == 0 ? X : (COMP == 1 ? Y : Z), T1 = COMP == 0 ? Y : X, T2 = COMP == 2 ? Y : Z;
+  double* l = la.a[COMP];
+  double* f1 = la.a[COMP == 0 ? 1 : 0] + c;
+  double* f2 = la.a[COMP == 2 ? 1 : 2] + c;
+  const double* e1 = cf.a[COMP == 2 ? 2 : 1] + c;
+  const double* e2 = cf.a[COMP == 0 ? 2 : 3] + c;
+  double m = l[c];
+  const double Ac = __ldg(A + c), m0 = __ldg(cf.a[0] + c), m1 = __ldg(cf.a[0] + c + S), e1n = __ldg(e1 - T1),
+               e1p = __ldg(e1), e2n = __ldg(e2 - T2), e2p = __ldg(e2);
+  const double a0 = f1[0], a1 = f1[S], a2 = f1[-T1], a3 = f1[S - T1];
+  const double b0 = f2[0], b1 = f2[S], b2 = f2[-T2], b3 = f2[S - T2];
+  if (OWN) {
+    const bool hx = i <= 3 || i >= g.ni - 2, hz = k <= 3 || k >= g.nk - 2;
+    const int ix = i <= 3 ? i + g.ni : i - g.ni, kx = k <= 3 ? k + g.nk : k - g.nk;
+    if (hx || hz) {
+      double *px = l + g.at(ix, j, k), *pz = l + g.at(i, j, kx), *pxz = l + g.at(ix, j, kx);
+      const double vx = hx ? *px : 0.0, vz = hz ? *pz : 0.0, vxz = hx && hz ? *pxz : 0.0;
+      m += (vx + vz) + vxz;
+      if (hx) *px = 0.0;
+      if (hz) *pz = 0.0;
+      if (hx && hz) *pxz = 0.0;
     }
-    lB[c] += m;
-    lA[c] += m * visn;
   }
-}
-// the forward sweep (same arithmetic role as fused k_pair<.., double>, without the residual)
-template <int COMP>
-__global__ void __launch_bounds__(256) k_pair_fwd(Grid g, VPa p, int pi, int pj, int pk, CArr4 cf,
-                                                  const double* __restrict__ A, const double* __restrict__ B,
-                                                  Arr3 q) {
-  const int jmax = COMP == 1 ? g.nj - 1 : g.nj;
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int i = (h ? 3 - pi : pi) + 2 * (int)(blockIdx.x * 32 + threadIdx.x);
-    const int j = (h ? 3 - pj : pj) + 2 * (int)(blockIdx.y * 8 + threadIdx.y);
-    const int k = (h ? 3 - pk : pk) + 2 * (int)blockIdx.z;
-    if (i > g.ni || j > jmax || k > g.nk) continue;
-    const long c = g.at(i, j, k);
-    Sten S;
-    stencil<COMP>(g, p, c, S);
-    double visn = 0.0;
-    for (int t = 0; t < 14; ++t) visn += S.mult[t] * cf.a[S.ca[t]][S.ci[t]] * q.a[S.arr[t]][c + S.off[t]];
-    q.a[COMP][c] = A[c] * visn + B[c];
+  if (m == 0.0) return;
+  l[c] = 0.0;
+  const double ma = m * Ac, x1 = ma * K.k1, x2 = ma * K.k2;
+  if (GRAD) {
+    const double *q = G.q0 + c, *p1 = G.q1 + c, *p2 = G.q2 + c;
+    const double qn = K.own * q[-S], qp = K.own * q[S];
+    const double d1n = q[-T1] + K.r1 * (p1[-T1] - p1[S - T1]), d1p = q[T1] + K.r1 * (p1[S] - p1[0]);
+    const double d2n = q[-T2] + K.r2 * (p2[-T2] - p2[S - T2]), d2p = q[T2] + K.r2 * (p2[S] - p2[0]);
+    G.lB[c] += m;
+    G.lA[c] += m * (m0 * qn + m1 * qp + K.k1 * (e1n * d1n + e1p * d1p) + K.k2 * (e2n * d2n + e2p * d2p));
+    G.lmu[c] += ma * qn;
+    G.lmu[c + S] += ma * qp;
+    G.le1[c - T1] += x1 * d1n;
+    G.le1[c] += x1 * d1p;
+    G.le2[c - T2] += x2 * d2n;
+    G.le2[c] += x2 * d2p;
   }
+  const double xo = ma * K.own, n1 = x1 * e1n, w1 = x1 * e1p, n2 = x2 * e2n, w2 = x2 * e2p;
+  aadd(l + c - S, xo * m0);
+  aadd(l + c + S, xo * m1);
+  aadd(l + c - T1, n1);
+  aadd(l + c + T1, w1);
+  aadd(l + c - T2, n2);
+  aadd(l + c + T2, w2);
+  f1[0] = a0 - K.r1 * w1;
+  f1[S] = a1 + K.r1 * w1;
+  f1[-T1] = a2 + K.r1 * n1;
+  f1[S - T1] = a3 - K.r1 * n1;
+  f2[0] = b0 - K.r2 * w2;
+  f2[S] = b1 + K.r2 * w2;
+  f2[-T2] = b2 + K.r2 * n2;
+  f2[S - T2] = b3 - K.r2 * n2;
 }
 const int kPi[4] = {1, 1, 1, 2}, kPj[4] = {1, 1, 2, 1}, kPk[4] = {1, 2, 1, 1};
-dim3 pgrid(const Grid& g) {
-  return dim3((unsigned)((g.ni / 2 + 31) / 32), (unsigned)((g.nj / 2 + 7) / 8), (unsigned)(g.nk / 2));
-}
-__global__ void k_copy3(long n, Arr3 a, double* __restrict__ b) {
+__global__ void k_copy3(long n, CArr3 a, double* __restrict__ b) {
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
     b[t] = a.a[0][t];
     b[t + n] = a.a[1][t];
     b[t + 2 * n] = a.a[2][t];
   }
 }
-// l holds G^T l_old: fb = l (the feedback term), l += lout; part[block] = sum of
-// (l - prev)^2, part[512 + block] = sum of fb^2 (gridDim.x <= 512)
-__global__ void k_add_diff3(long n, Arr3 l, CArr3 o, const double* __restrict__ prev, double* part,
-                            double* __restrict__ fb) {
+// l holds G^T l_old, fb the feedback term l_old - lout: part[block] = sum of
+// (l - fb)^2 = |l_new - l_old|^2, part[kParts + block] = sum of l^2, fb = l, l += lout
+constexpr int kParts = 512;
+__global__ void __launch_bounds__(256) k_add_diff3(long n, Arr3 l, CArr3 o, double* part, double* fb) {
   __shared__ double sh[2][256];
   double acc = 0.0, acf = 0.0;
-  for (long t = blockIdx.x * 256L + threadIdx.x; t < n; t += (long)gridDim.x * 256) {
-    for (int c = 0; c < 3; ++c) {
-      const double f = l.a[c][t];
-      fb[t + c * n] = f;
-      acf += f * f;
-      const double v = f + o.a[c][t];
-      l.a[c][t] = v;
-      const double d = v - prev[t + c * n];
-      acc += d * d;
+  const long step = kParts * 256L;
+  for (int c = 0; c < 3; ++c) {
+    double *lc = l.a[c], *fc = fb + c * n;
+    const double* oc = o.a[c];
+    for (long t0 = blockIdx.x * 256L + threadIdx.x; t0 < n; t0 += 4 * step) {
+      double f[4], p[4], q[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const long t = t0 + u * step;
+        const bool on = t < n;
+        f[u] = on ? lc[t] : 0.0;
+        p[u] = on ? fc[t] : 0.0;
+        q[u] = on ? oc[t] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const long t = t0 + u * step;
+        if (t >= n) break;
+        fc[t] = f[u];
+        lc[t] = f[u] + q[u];
+        const double d = f[u] - p[u];
+        acf += f[u] * f[u];
+        acc += d * d;
+      }
     }
   }
   sh[0][threadIdx.x] = acc;
@@ -223,25 +198,30 @@ __global__ void k_add_diff3(long n, Arr3 l, CArr3 o, const double* __restrict__ 
   }
   if (threadIdx.x == 0) {
     part[blockIdx.x] = sh[0][0];
-    part[512 + blockIdx.x] = sh[1][0];
+    part[kParts + blockIdx.x] = sh[1][0];
   }
 }
-// l = lout + fb (the warm start), or lout + 2 fb - fb2 (fb2 the feedback term one
-// solve earlier: linear extrapolation in time)
-__global__ void k_warm3(long n, Arr3 l, CArr3 o, const double* __restrict__ fb, const double* __restrict__ fb2) {
+// The start: fbo = 0 (no fb), fb (the warm start) or 2 fb - fb2 (fb2 the feedback term one
+// solve earlier: linear extrapolation in time; may be fbo itself), l = lout + fbo
+__global__ void k_start3(long n, Arr3 l, CArr3 o, const double* fb, const double* fb2, double* fbo) {
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
     for (int c = 0; c < 3; ++c) {
-      const double f = fb[t + c * n];
-      l.a[c][t] = o.a[c][t] + (fb2 ? f + (f - fb2[t + c * n]) : f);
+      double f = 0.0;
+      if (fb) {
+        f = fb[t + c * n];
+        if (fb2) f += f - fb2[t + c * n];
+      }
+      fbo[t + c * n] = f;
+      l.a[c][t] = o.a[c][t] + f;
     }
 }
-// out[0] = sum of part[0..n), out[1] = sum of part[512..512+n)
+// out[0] = sum of part[0..n), out[1] = sum of part[kParts..kParts+n)
 __global__ void k_sum_small(const double* part, int n, double* out) {
   __shared__ double sh[2][256];
   double acc = 0.0, acf = 0.0;
   for (int t = threadIdx.x; t < n; t += 256) {
     acc += part[t];
-    acf += part[512 + t];
+    acf += part[kParts + t];
   }
   sh[0][threadIdx.x] = acc;
   sh[1][threadIdx.x] = acf;
@@ -346,27 +326,36 @@ void edges_T(cudaStream_t s, const Grid& g, int harmonic, const double* mu, cons
   });
 }
 
-void sor_replay(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, const double* mu,
+// After a component's first pair the forward cycle changes that component alone, so the
+// later pairs' states share the other two arrays (where the grid allows the one-pass
+// refresh): 24 array copies, not 36.
+namespace {
+CArr3 replay_state(const Grid& g, const double* snaps, int comp, int pr) {
+  const bool share = pr > 1 && fused::one_pass_refresh(g);
+  CArr3 q;
+  for (int c = 0; c < 3; ++c) q.a[c] = snaps + (3L * (4 * comp + (share && c != comp ? 1 : pr)) + c) * g.n;
+  return q;
+}
+}  // namespace
+void sor_replay(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, int harmonic, const double* mu,
                 double* const* E, double* const* AB, double uwall, const double* wallc, const double* const* ustar,
-                double* snaps) {
-  const VPa p = make_vpa(dxi, dyi, dzi);
+                double* snaps, double* part) {
   const long n = g.n;
-  const CArr4 cf{{mu, E[0], E[1], E[2]}};
   double* q[3] = {snaps + 36 * n, snaps + 37 * n, snaps + 38 * n};  // running state
-  for (int c = 0; c < 3; ++c) FMF_CUDA(cudaMemcpyAsync(q[c], ustar[c], sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  const dim3 grd = pgrid(g), blk(32, 8);
-  for (int comp = 0; comp < 3; ++comp)
-    for (int pr = 0; pr < 4; ++pr) {
-      const int idx = comp * 4 + pr;
-      for (int c = 0; c < 3; ++c)
-        FMF_CUDA(cudaMemcpyAsync(snaps + (3 * idx + c) * n, q[c], sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-      const Arr3 Q{{q[0], q[1], q[2]}};
-      if (comp == 0) k_pair_fwd<0><<<grd, blk, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], cf, AB[0], AB[1], Q);
-      else if (comp == 1) k_pair_fwd<1><<<grd, blk, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], cf, AB[2], AB[3], Q);
-      else k_pair_fwd<2><<<grd, blk, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], cf, AB[4], AB[5], Q);
-      count_launch();
-      fused::wall_halo(s, g, 1 << comp, uwall, wallc, q[0], q[1], q[2]);
-    }
+  const CArr3 run{{q[0], q[1], q[2]}};
+  k_copy3<<<608, 256, 0, s>>>(n, CArr3{{ustar[0], ustar[1], ustar[2]}}, q[0]);
+  count_launch();
+  fused::sor_iteration(s, g, dxi, dyi, dzi, harmonic, mu, E, AB, uwall, wallc, q[0], q[1], q[2], part, nullptr,
+                       [&](int comp, int pr) {
+                         const CArr3 st = replay_state(g, snaps, comp, pr);
+                         double* own = snaps + (3L * (4 * comp + pr) + comp) * n;
+                         if (st.a[(comp + 1) % 3] == snaps + (3L * (4 * comp + pr) + (comp + 1) % 3) * n) {
+                           k_copy3<<<608, 256, 0, s>>>(n, run, snaps + 3L * (4 * comp + pr) * n);
+                           count_launch();
+                         } else {
+                           FMF_CUDA(cudaMemcpyAsync(own, q[comp], sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
+                         }
+                       });
 }
 
 cudaGraphExec_t cached_graph(cudaStream_t s, GraphCache* cache, const std::vector<const void*>& key,
@@ -400,55 +389,56 @@ int sor_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, con
           const double* const* lout, double* const* lam, double* const* lAB, double* lmu, double* const* lE,
           double* lwc, double tol, int maxit, double* work, double* host_norm, GraphCache* cache, double* fb,
           double* fb_norm, const double* fb_prev, double* fb_out) {
-  const VPa p = make_vpa(dxi, dyi, dzi);
   const long n = g.n;
   const CArr4 cf{{mu, E[0], E[1], E[2]}};
-  const dim3 grd = pgrid(g), blk(32, 8);
-  double* prev = work;               // 3n
-  double* part = work + 3 * n;       // 1024
-  double* nrm = work + 3 * n + 1024; // 2 doubles
+  double* part = work;             // 2 kParts
+  double* nrm = work + 2 * kParts; // 2 doubles
   const Arr3 L3{{lam[0], lam[1], lam[2]}};
   const CArr3 O3{{lout[0], lout[1], lout[2]}};
   // l = lout, or lout plus the previous solve's feedback term
   const bool warm = *fb_norm > 0.0;
-  if (warm) {
-    k_warm3<<<608, 256, 0, s>>>(n, L3, O3, fb, fb_prev);
-    count_launch();
-  } else {
-    for (int c = 0; c < 3; ++c)
-      FMF_CUDA(cudaMemcpyAsync(lam[c], lout[c], sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  }
-  auto backward_cycle = [&](bool grad) {
-    const Arr3 L{{lam[0], lam[1], lam[2]}};
-    for (int comp = 2; comp >= 0; --comp)
+  k_start3<<<608, 256, 0, s>>>(n, L3, O3, warm ? fb : nullptr, fb_prev, fb_out);
+  count_launch();
+  // The 12 sweeps backwards, the refresh after each transposed before it.  The forward
+  // cycle after a component's second to fourth pair changes that component's ghosts
+  // alone, which the swept points gather (OWN); the full refresh is after the first.
+  // lout holds nothing in the wall rows (a transposed refresh has gone over it).
+  const bool one_pass = fused::one_pass_refresh(g);
+  const int bx = std::min(32, g.ni / 2), by = 64 / bx;
+  const dim3 blk(bx, by), grd((g.ni / 2 + bx - 1) / bx, (g.nj / 2 + by - 1) / by, g.nk);
+  auto backward_cycle = [&](auto grad) {
+    constexpr bool GR = decltype(grad)::value;
+    for (int comp = 2; comp >= 0; --comp) {
+      const SwK K = make_swk(dxi, dyi, dzi, comp);
       for (int pr = 3; pr >= 0; --pr) {
-        const int idx = comp * 4 + pr;
-        // transposed refresh; the slip-coefficient adjoint only in the gradient pass
-        wall_halo_T(s, g, 1 << comp, uwall, wallc, ustar[0], ustar[2], lam[0], lam[1], lam[2],
-                    grad ? lwc : nullptr);
-        if (grad) {
-          const CArr3 dq{{snaps + (3 * idx) * n, snaps + (3 * idx + 1) * n, snaps + (3 * idx + 2) * n}};
-          const Arr4 lcf{{lmu, lE[0], lE[1], lE[2]}};
-          if (comp == 0) k_pair_grad<0><<<grd, blk, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], cf, AB[0], dq, L, lAB[0], lAB[1], lcf);
-          else if (comp == 1) k_pair_grad<1><<<grd, blk, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], cf, AB[2], dq, L, lAB[2], lAB[3], lcf);
-          else k_pair_grad<2><<<grd, blk, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], cf, AB[4], dq, L, lAB[4], lAB[5], lcf);
-          count_launch();
+        GradIn G{};
+        if (GR) {
+          const CArr3 q = replay_state(g, snaps, comp, pr);
+          const int t1 = comp == 0 ? 1 : 0, t2 = comp == 2 ? 1 : 2;
+          G = GradIn{q.a[comp],         q.a[t1], q.a[t2],                lAB[2 * comp],
+                     lAB[2 * comp + 1], lmu,     lE[comp == 2 ? 1 : 0], lE[comp == 0 ? 1 : 2]};
         }
-        if (comp == 0) k_pair_T<0><<<grd, blk, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], cf, AB[0], L);
-        else if (comp == 1) k_pair_T<1><<<grd, blk, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], cf, AB[2], L);
-        else k_pair_T<2><<<grd, blk, 0, s>>>(g, p, kPi[pr], kPj[pr], kPk[pr], cf, AB[4], L);
-        count_launch();
+        const bool own = one_pass && pr > 0;
+        // the slip-coefficient adjoint only in the gradient pass
+        if (!own) wall_halo_T(s, g, 1 << comp, uwall, wallc, ustar[0], ustar[2], lam[0], lam[1], lam[2], GR ? lwc : nullptr);
+        auto run = [&](auto fn) {
+          fn<<<grd, blk, 0, s>>>(g, K, kPi[pr], kPj[pr], kPk[pr], cf, AB[2 * comp], L3, G);
+          count_launch();
+        };
+        if (comp == 0) own ? run(k_pair_T<0, true, GR>) : run(k_pair_T<0, false, GR>);
+        else if (comp == 1) own ? run(k_pair_T<1, true, GR>) : run(k_pair_T<1, false, GR>);
+        else own ? run(k_pair_T<2, true, GR>) : run(k_pair_T<2, false, GR>);
       }
+    }
   };
   // one iteration l <- lout + G^T l, |l_new - l_old|^2 and |G^T l|^2 into nrm and
-  // the feedback term G^T l into fb: 51 kernels, replayed as a CUDA graph (one per
+  // the feedback term G^T l into fb: 17 kernels, replayed as a CUDA graph (one per
   // set of buffers)
   auto iteration = [&]() {
-    k_copy3<<<608, 256, 0, s>>>(n, L3, prev);
-    backward_cycle(false);
-    k_add_diff3<<<512, 256, 0, s>>>(n, L3, O3, prev, part, fb_out);
-    k_sum_small<<<1, 256, 0, s>>>(part, 512, nrm);
-    count_launch(3);
+    backward_cycle(std::false_type());
+    k_add_diff3<<<kParts, 256, 0, s>>>(n, L3, O3, part, fb_out);
+    k_sum_small<<<1, 256, 0, s>>>(part, kParts, nrm);
+    count_launch(2);
   };
   long long per_launch = 0;
   cudaGraphExec_t exec =
@@ -481,7 +471,7 @@ int sor_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, con
     if (!(d > tol * (n0 + 1e-300))) break;
   }
   // gradient pass at the converged adjoint
-  backward_cycle(true);
+  backward_cycle(std::true_type());
   return it + 1;
 }
 

@@ -3,6 +3,8 @@
 // subroutines, skip work whose result the step never reads, and let nvcc
 // contract multiply-adds; they are checked against the oracle at 1e-10.
 #pragma once
+#include <functional>
+
 #include "fmf_common.cuh"
 
 namespace fmf {
@@ -100,15 +102,18 @@ void src_visc_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
 void wall_coef(cudaStream_t s, const Grid& g, double dy, const double* l1, const double* l2, const double* phi,
                double* wallc);
 // bndu followed by bnd_periodic of the components whose bit is set in `normal`.
+bool one_pass_refresh(const Grid& g);
 void wall_halo(cudaStream_t s, const Grid& g, int normal, double uwall, const double* wallc, double* un, double* vn,
                double* wn);
 // one outer iteration (u, v, w sweeps of 4 colour pairs each); errsum[0] = sum du^2;
-// part: sor_parts(g) doubles of scratch.  FP64 in the FP64-accurate step as well (a
+// part: sor_parts(g) doubles of scratch.  before(comp, pair) is called ahead of each pair;
+// a null errsum leaves the sum out (the adjoint's replay).  FP64 in the FP64-accurate step as well (a
 // point update reads 23 doubles for about 30 operations; measured in FP32 pairs the
 // splits cost more than the arithmetic saves)
 void sor_iteration(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, int harmonic,
                    const double* mu, double* const* E, double* const* AB, double uwall, const double* wallc,
-                   double* un, double* vn, double* wn, double* part, double* errsum);
+                   double* un, double* vn, double* wn, double* part, double* errsum,
+                   const std::function<void(int, int)>& before = nullptr);
 long sor_parts(const Grid& g);
 
 // The stop rule of the viscous solve on the device (solu_sor4.f:130,291-293): err =

@@ -1375,6 +1375,8 @@ __global__ void __launch_bounds__(1024) k_sum_parts2(const double* part, long n,
   if (threadIdx.x == 0) out[0] = a;
 }
 
+}  // namespace
+
 // The one-pass refresh kernels where the grid allows them, unless FMF_REFRESH_ORDERED
 // is set in the environment (then the ordered plane kernels, which give the same
 // values: the tests compare the two).
@@ -1383,6 +1385,7 @@ bool one_pass_refresh(const Grid& g) {
   return !ordered && refresh_one_pass(g.ni, g.nj, g.nk);
 }
 
+namespace {
 VP make_vp(double dxinv, double dyinv, double dzinv, double dt, int harmonic) {
   VP p;
   p.dxi = dxinv;
@@ -1512,12 +1515,14 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
 // allows the one-pass refresh.
 template <class T, class G, class HaloFn>
 void sweep_all(cudaStream_t s, const Grid& g, const VP& p, const T* mu, const T* exy, const T* exz, const T* eyz,
-               T* const* A, T* const* B, T* un, T* vn, T* wn, const G& gh, double* part, double* errsum, HaloFn halo) {
+               T* const* A, T* const* B, T* un, T* vn, T* wn, const G& gh, double* part, double* errsum, HaloFn halo,
+               const std::function<void(int, int)>& before = nullptr) {
   const PairShape sp = pair_shape(g, sizeof(T) == 8);
   const bool fill = one_pass_refresh(g) && sp.ghosts;
   for (int comp = 0; comp < 3; ++comp) {
     const SweepK<T> K(p, comp);
     for (int pr = 0; pr < 4; ++pr) {
+      if (before) before(comp, pr);
       auto run = [&](auto fn) {
         fn<<<sp.grid, sp.block, 0, s>>>(g, K, kPi[pr], kPj[pr], kPk[pr], sp.kz, mu, exy, exz, eyz, A[comp], B[comp],
                                         un, vn, wn, gh, part, comp == 0 && pr == 0);
@@ -1536,6 +1541,7 @@ void sweep_all(cudaStream_t s, const Grid& g, const VP& p, const T* mu, const T*
       if (!own) halo(1 << comp);
     }
   }
+  if (!errsum) return;
   k_sum_parts2<<<1, 1024, 0, s>>>(part, (long)sp.grid.x * sp.grid.y * sp.grid.z, errsum);
   count_launch();
 }
@@ -1615,12 +1621,13 @@ void wall_halo(cudaStream_t s, const Grid& g, int normal, double uwall, const do
 
 void sor_iteration(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, int harmonic,
                    const double* mu, double* const* E, double* const* AB, double uwall, const double* wallc,
-                   double* un, double* vn, double* wn, double* part, double* errsum) {
+                   double* un, double* vn, double* wn, double* part, double* errsum,
+                   const std::function<void(int, int)>& before) {
   double* const A[3] = {AB[0], AB[2], AB[4]};
   double* const B[3] = {AB[1], AB[3], AB[5]};
   sweep_all<double>(s, g, make_vp(dxinv, dyinv, dzinv, 0.0, harmonic), mu, E[0], E[1], E[2], A, B, un, vn, wn,
                     Ghosts64{uwall, wallc}, part, errsum,
-                    [&](int normal) { wall_halo(s, g, normal, uwall, wallc, un, vn, wn); });
+                    [&](int normal) { wall_halo(s, g, normal, uwall, wallc, un, vn, wn); }, before);
 }
 
 __global__ void k_sor_rule(SorLoop* L, double tol, int maxit, double cells) {
