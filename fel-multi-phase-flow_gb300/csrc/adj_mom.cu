@@ -1,7 +1,10 @@
 // adj_mom.cu -- adjoints of the WENO5 advection (cal_advu_weno5 + weno5.h) and of
 // the CSF surface-tension force (cal_grad_p2a, calrn x4, calrkap, cal_grad_p2uvw,
 // calfst).
+#include <cstring>
+
 #include "adj.cuh"
+#include "bits.cuh"
 #include "fused.cuh"
 #include "ops.cuh"
 #include "recip.cuh"
@@ -418,6 +421,33 @@ void weno_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, c
 }
 
 // ---- CSF --------------------------------------------------------------------------
+namespace {
+// the vertex gradients at the eight vertices behind c (bit t of the corner: axis t behind);
+// false if none of this warp's has a component of magnitude bits `half` or more
+__device__ __forceinline__ bool resolved_vertices(const double* Gv, long n, long c, long X, long Y, long Z,
+                                                  unsigned long long half, double p[3][8]) {
+  bool any = false;
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      p[q][t] = Gv[q * n + c - (t & 1 ? X : 0) - (t & 2 ? Y : 0) - (t & 4 ? Z : 0)];
+      any |= mag(p[q][t]) >= half;
+    }
+  return __any_sync(__activemask(), any);
+}
+// family 0: the sum of the eight vertices; families 1 to 3: of the two along z, y, x (each
+// four times in calrn's eight)
+__device__ __forceinline__ void family_sum(int f, const double p[3][8], double r[3]) {
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    r[q] = f == 0 ? ((p[q][7] + p[q][6]) + (p[q][5] + p[q][4])) + ((p[q][3] + p[q][2]) + (p[q][1] + p[q][0]))
+                  : p[q][f == 1 ? 4 : (f == 2 ? 2 : 1)] + p[q][0];
+}
+__device__ __forceinline__ double inv_length(double s2) {
+  return (mag(s2) >> 53) >= 23 ? rsqrt_h(s2) : rsqrt(s2);  // 2^-1000 and above
+}
+}  // namespace
 void csf_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, double rhol, double rhog,
            double sigma, const double* phi, const double* const* lf, double* lphi, double* work) {
   const Grid G = g;
@@ -443,40 +473,45 @@ void csf_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, do
   // others (equal to the step's wherever the normals are resolved), and those
   // normals pass no adjoint to the vertex gradients.
   const double tau = 1.0e-6 * std::sqrt(dxi * dxi + dyi * dyi + dzi * dzi);
-  const double vs = std::sqrt(dxi * dxi + dyi * dyi + dzi * dzi) * 1.0e-30;
+  // The normals are formed from the sums of the eight (family 0) or two vertex gradients,
+  // |v| + vs is |v| (vs is below 1e-24 |v| above the floor), and a warp whose vertices are
+  // all below half the floor has zeros.  Bound by the FP64 pipe: at 128x64x64 the normals
+  // took 145 us and the two gathers 212 and 52 with the means, Newton reciprocals and no
+  // such test, now 89, 144 and 50.
+  auto bits = [](double x) {
+    unsigned long long b;
+    std::memcpy(&b, &x, sizeof b);
+    return b << 1;
+  };
+  const unsigned long long floor8 = bits(64.0 * tau * tau), floor2 = bits(4.0 * tau * tau), half = bits(0.5 * tau);
   // forward recompute: vertex gradients, normals (calrn.f:45-87 with the floor),
   // curvature (calrkap.f) and face gradients
   fused::vertex_gradient(s, g, dxi, dyi, dzi, phi, Gv, Gv + n, Gv + 2 * n);
   range3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int i, int j, int k) {
-    const long X = 1, Y = G.sy, Z = G.sz;
     const long c = G.at(i, j, k);
+    const long X = i > -2 ? 1 : 0, Y = j > -2 ? G.sy : 0, Z = k > -2 ? G.sz : 0;
+    double p[3][8];
+    if (!resolved_vertices(Gv, n, c, X, Y, Z, half, p)) {
+#pragma unroll
+      for (int t = 0; t < 12; ++t) rn[t * n + c] = 0.0;
+      return;
+    }
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
       const int ip = f == 0 || f == 3, jp = f == 0 || f == 2, kp = f == 0 || f == 1;
       double* out = rn + 3 * n * f + c;
-      if (i < -2 + ip || j < -2 + jp || k < -2 + kp) {  // calrn does not write o
-        out[0] = out[n] = out[2 * n] = 0.0;
-        continue;
-      }
-      const long Xf = ip ? X : 0, Yf = jp ? Y : 0, Zf = kp ? Z : 0;
-      const long b = c - Xf - Yf - Zf;
       double r[3];
-#pragma unroll
-      for (int q3 = 0; q3 < 3; ++q3) {
-        const double* p = Gv + q3 * n + b;
-        r[q3] = f == 0 ? (p[0] + p[Xf] + p[Yf] + p[Xf + Yf] + p[Zf] + p[Xf + Zf] + p[Yf + Zf] + p[Xf + Yf + Zf]) * 0.125
-                       : (p[0] + p[Xf + Yf + Zf]) * 0.5;
-      }
+      family_sum(f, p, r);
       const double s2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
-      if (s2 <= tau * tau) {
+      // calrn does not write the first points; below the noise floor
+      if (i < -2 + ip || j < -2 + jp || k < -2 + kp || mag(s2) <= (f == 0 ? floor8 : floor2)) {
         out[0] = out[n] = out[2 * n] = 0.0;
         continue;
       }
-      // v/(|v| + vs) by Newton-Raphson reciprocals (s2 is a normal number here)
-      const double ia = recip_nr(s2 * rsqrt_nr(s2) + vs);
-      out[0] = r[0] * ia;
-      out[n] = r[1] * ia;
-      out[2 * n] = r[2] * ia;
+      const double im = inv_length(s2);
+      out[0] = r[0] * im;
+      out[n] = r[1] * im;
+      out[2 * n] = r[2] * im;
     }
   });
   op::calrkap(s, g, dxi, dyi, dzi, rn, rn + 3 * n, rn + 6 * n, rn + 9 * n, kap);
@@ -519,6 +554,13 @@ void csf_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, do
     // kap_u = dxi (pp_x[+X] - pp_x) + dyi (r12_y - r12_y[-Y]) + dzi (r13_z - r13_z[-Z]),
     // kap_v = dxi (r12_x - r12_x[-X]) + dyi (pp_y[+Y] - pp_y) + dzi (r23_z - r23_z[-Z]),
     // kap_w = dxi (r13_x - r13_x[-X]) + dyi (r23_y - r23_y[-Y]) + dzi (pp_z[+Z] - pp_z)
+    const long Xb = i > -2 ? X : 0, Yb = j > -2 ? Y : 0, Zb = k > -2 ? Z : 0;
+    double p[3][8];
+    if (!resolved_vertices(Gv, n, c, Xb, Yb, Zb, half, p)) {
+#pragma unroll
+      for (int t = 0; t < 12; ++t) lv[t * n + c] = 0.0;
+      return;
+    }
     double L[4][3];
     L[0][0] = dxi * (ku(i - 1, j, k, c - X) - ku(i, j, k, c));
     L[0][1] = dyi * (kv(i, j - 1, k, c - Y) - kv(i, j, k, c));
@@ -535,83 +577,52 @@ void csf_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, do
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
       const int ip = f == 0 || f == 3, jp = f == 0 || f == 2, kp = f == 0 || f == 1;
-      if (i < -2 + ip || j < -2 + jp || k < -2 + kp) continue;  // calrn does not write o
       double* out = lv + 3 * n * f + c;
       const double lx = L[f][0], ly = L[f][1], lz = L[f][2];
-      if (lx == 0.0 && ly == 0.0 && lz == 0.0) {
-        out[0] = out[n] = out[2 * n] = 0.0;
-        continue;
-      }
-      const long Xf = ip ? X : 0, Yf = jp ? Y : 0, Zf = kp ? Z : 0;
-      const long b = c - Xf - Yf - Zf;
       double r[3];
-#pragma unroll
-      for (int q3 = 0; q3 < 3; ++q3) {
-        const double* p = Gv + q3 * n + b;
-        // family 0 averages 8 vertex gradients; families 1-3 (one offset only) the
-        // two along that offset, each four times in the 8-term mean
-        r[q3] = f == 0 ? (p[0] + p[Xf] + p[Yf] + p[Xf + Yf] + p[Zf] + p[Xf + Zf] + p[Yf + Zf] + p[Xf + Yf + Zf]) * 0.125
-                       : (p[0] + p[Xf + Yf + Zf]) * 0.5;
-      }
-      // dN/dv = I/a - v v^T/(a^2 m) with m = |v|, a = m + vs:
-      // lv = (l - v (v.l)/(m a)) / a, the factor formed as ((v.l)/m)/a, which stays
-      // finite for any m > 0
-      // (division-free reciprocals where s2 is a normal number; subnormal and zero
-      // s2 take the library functions)
+      family_sum(f, p, r);
       const double s2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
-      if (s2 <= tau * tau) {  // below the noise floor: a constant normal
+      if (i < -2 + ip || j < -2 + jp || k < -2 + kp || (mag(lx) | mag(ly) | mag(lz)) == 0 ||
+          mag(s2) <= (f == 0 ? floor8 : floor2)) {  // below the noise floor: a constant normal
         out[0] = out[n] = out[2 * n] = 0.0;
         continue;
       }
-      double ia, t = 0.0;
-      if (s2 >= 0x1p-1000) {
-        const double im = rsqrt_nr(s2);
-        ia = recip_nr(s2 * im + vs);
-        t = ((r[0] * lx + r[1] * ly + r[2] * lz) * im) * ia;
-      } else if (s2 > 0.0) {
-        const double im = rsqrt(s2);
-        ia = 1.0 / (s2 * im + vs);
-        t = ((r[0] * lx + r[1] * ly + r[2] * lz) * im) * ia;
-      } else {
-        ia = 1.0 / vs;
-      }
-      out[0] = (lx - r[0] * t) * ia;
-      out[n] = (ly - r[1] * t) * ia;
-      out[2 * n] = (lz - r[2] * t) * ia;
+      // dN/dr = (I - r r^T/|r|^2)/|r| of the sum r, each of whose vertices it hands this to
+      const double im = inv_length(s2);
+      const double t = (r[0] * lx + r[1] * ly + r[2] * lz) * (im * im);
+      out[0] = (lx - r[0] * t) * im;
+      out[n] = (ly - r[1] * t) * im;
+      out[2 * n] = (lz - r[2] * t) * im;
     }
   });
-  // pass 2, per vertex p: 0.125 lv over the (family, corner) pairs whose mean reads
-  // p, i.e. o = p + {0,X_f} + {0,Y_f} + {0,Z_f} (families 1-3 read two points, four
-  // times each)
+  // pass 2, per vertex p: lv over the (family, corner) pairs whose sum reads p, i.e.
+  // o = p + {0,X_f} + {0,Y_f} + {0,Z_f} (families 1-3 read two points)
   range3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int i, int j, int k) {
-    const long X = 1, Y = G.sy, Z = G.sz;
     const long c = G.at(i, j, k);
-    auto ok = [&](int f, int a, int b, int e) {
-      const int ip = f == 0 || f == 3, jp = f == 0 || f == 2, kp = f == 0 || f == 1;
-      return a >= -2 + ip && a <= G.ni + 3 && b >= -2 + jp && b <= G.nj + 3 && e >= -2 + kp && e <= G.nk + 3;
-    };
-    const bool a1 = ok(1, i, j, k), b1 = ok(1, i, j, k + 1), a2 = ok(2, i, j, k), b2 = ok(2, i, j + 1, k),
-               a3 = ok(3, i, j, k), b3 = ok(3, i + 1, j, k);
+    // lv is zero where calrn does not write: only the upper end is out of range
+    const long X = i <= G.ni + 2 ? 1 : 0, Y = j <= G.nj + 2 ? G.sy : 0, Z = k <= G.nk + 2 ? G.sz : 0;
+    double p[3][14];
+    unsigned long long any = 0;
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const double* L0 = lv + q * n + c;
-      double acc = 0.0;
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const int di = t & 1, dj = (t >> 1) & 1, dk = t >> 2;
-        if (ok(0, i + di, j + dj, k + dk)) acc += L0[di * X + dj * Y + dk * Z];
+      for (int t = 0; t < 14; ++t) {
+        const int f = t < 8 ? 0 : 1 + (t - 8) / 2;
+        const int d = t < 8 ? t : ((t - 8) % 2 == 0 ? 0 : (f == 1 ? 4 : (f == 2 ? 2 : 1)));
+        const bool on = (!(d & 1) || X) && (!(d & 2) || Y) && (!(d & 4) || Z);
+        p[q][t] = on ? lv[(3 * f + q) * n + c + (d & 1 ? X : 0) + (d & 2 ? Y : 0) + (d & 4 ? Z : 0)] : 0.0;
+        any |= (unsigned long long)__double_as_longlong(p[q][t]) << 1;
       }
-      const double* L1 = L0 + 3 * n;
-      const double* L2 = L0 + 6 * n;
-      const double* L3 = L0 + 9 * n;
-      double acc4 = 0.0;
-      if (a1) acc4 += L1[0];
-      if (b1) acc4 += L1[Z];
-      if (a2) acc4 += L2[0];
-      if (b2) acc4 += L2[Y];
-      if (a3) acc4 += L3[0];
-      if (b3) acc4 += L3[X];
-      lG[q * n + c] = 0.125 * (acc + 4.0 * acc4);
+    }
+    if (!__any_sync(__activemask(), any != 0)) {
+      lG[c] = lG[n + c] = lG[2 * n + c] = 0.0;
+      return;
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const double* t = p[q];
+      lG[q * n + c] = (((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]))) +
+                      (((t[8] + t[9]) + (t[10] + t[11])) + (t[12] + t[13]));
     }
   });
   grad_p2a_T(s, g, dxi, dyi, dzi, lG, lG + n, lG + 2 * n, lphi);
