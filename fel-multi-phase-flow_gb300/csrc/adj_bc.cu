@@ -539,7 +539,7 @@ void wall_coef_T(cudaStream_t s, const Grid& g, double dy, const double* l1, con
 void grad_p2a_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, const double* lqx,
                 const double* lqy, const double* lqz, double* lq) {
   const Grid G = g;
-  range3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int x, int y, int z) {
+  tiles3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int x, int y, int z) {
     const long o = G.at(x, y, z);
     if (x > -2 && y > -2 && z > -2 && x < G.ni + 3 && y < G.nj + 3 && z < G.nk + 3) {
       const double* L[3] = {lqx + o, lqy + o, lqz + o};

@@ -4,7 +4,6 @@
 #include <cstring>
 
 #include "adj.cuh"
-#include "bits.cuh"
 #include "fused.cuh"
 #include "ops.cuh"
 #include "recip.cuh"
@@ -487,7 +486,7 @@ void csf_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, do
   // forward recompute: vertex gradients, normals (calrn.f:45-87 with the floor),
   // curvature (calrkap.f) and face gradients
   fused::vertex_gradient(s, g, dxi, dyi, dzi, phi, Gv, Gv + n, Gv + 2 * n);
-  range3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int i, int j, int k) {
+  tiles3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int i, int j, int k) {
     const long c = G.at(i, j, k);
     const long X = i > -2 ? 1 : 0, Y = j > -2 ? G.sy : 0, Z = k > -2 ? G.sz : 0;
     double p[3][8];
@@ -536,7 +535,7 @@ void csf_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, do
   // k >= -1, j <= nj+2, i >= -1, the w one where k <= nk+2, j >= -1, i >= -1.
   // pass 1, per normal point o and family: the normal's adjoint gathered from the
   // curvatures that read it, then lv = (dN/dv)^T lrn
-  range3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int i, int j, int k) {
+  tiles3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int i, int j, int k) {
     const long X = 1, Y = G.sy, Z = G.sz;
     const long c = G.at(i, j, k);
     auto in = [&](int a, int b, int e) {
@@ -597,7 +596,7 @@ void csf_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, do
   });
   // pass 2, per vertex p: lv over the (family, corner) pairs whose sum reads p, i.e.
   // o = p + {0,X_f} + {0,Y_f} + {0,Z_f} (families 1-3 read two points)
-  range3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int i, int j, int k) {
+  tiles3(s, -2, g.ni + 3, -2, g.nj + 3, -2, g.nk + 3, [=] __device__(int i, int j, int k) {
     const long c = G.at(i, j, k);
     // lv is zero where calrn does not write: only the upper end is out of range
     const long X = i <= G.ni + 2 ? 1 : 0, Y = j <= G.nj + 2 ? G.sy : 0, Z = k <= G.nk + 2 ? G.sz : 0;

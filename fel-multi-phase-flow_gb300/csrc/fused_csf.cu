@@ -378,12 +378,10 @@ __device__ __forceinline__ double inv_norm(double s, double vs, double big) {
 __global__ void __launch_bounds__(128) k_csf_grad(Grid g, CsfD p, const double* __restrict__ phi,
                                                   double* __restrict__ G, const int* __restrict__ skip) {
   if (skip && *skip) return;
-  const int W = g.ni + 3;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= W * (g.nj + 3)) return;
-  const int b = t / W, a = t - b * W;
+  const Tile T = warp_tile(g.ni + 3);
+  if (T.x >= g.ni + 3 || T.y >= g.nj + 3) return;
   const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
-  const long c = g.at(a - 1, b - 1, (int)blockIdx.y - 1);
+  const long c = g.at(T.x - 1, T.y - 1, (int)blockIdx.z - 1);
   const double q000 = __ldg(phi + c), qp00 = __ldg(phi + c + X), q0p0 = __ldg(phi + c + Y),
                qpp0 = __ldg(phi + c + X + Y), q00p = __ldg(phi + c + Z), qp0p = __ldg(phi + c + X + Z),
                q0pp = __ldg(phi + c + Y + Z), qppp = __ldg(phi + c + X + Y + Z);
@@ -417,12 +415,11 @@ __global__ void __launch_bounds__(128) k_csf_normals(Grid g, CsfD p, int m, cons
                                                      double* __restrict__ pp, double* __restrict__ n12,
                                                      double* __restrict__ nside, const int* __restrict__ skip) {
   if (skip && *skip) return;
-  const int W = g.ni + 2;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= W * (g.nj + 2)) return;
-  const int b = t / W, a = t - b * W;
+  const Tile T = warp_tile(g.ni + 2);
+  const int a = T.x, b = T.y;
+  if (a >= g.ni + 2 || b >= g.nj + 2) return;
   const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
-  const int k0 = (int)blockIdx.y * m, k1 = min(g.nk + 2, k0 + m);
+  const int k0 = (int)blockIdx.z * m, k1 = min(g.nk + 2, k0 + m);
   long c = g.at(a, b, k0 - 1);  // the plane below the first
   double g0[3], P0[3];
   unsigned long long any0 = 0;
@@ -508,8 +505,8 @@ __global__ void __launch_bounds__(256) k_csf_force(Grid g, CsfD p, const double*
                                                    double* __restrict__ fv, double* __restrict__ fw,
                                                    const int* __restrict__ skip) {
   if (skip && *skip) return;
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
+  const Tile T = warp_tile(g.ni);
+  const int i = 1 + T.x, j = 1 + T.y;
   if (i > g.ni || j > g.nj) return;
   const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
   const long c = g.at(i, j, 1 + (int)blockIdx.z);
@@ -555,17 +552,15 @@ void csf_fp64(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double 
   p.fy = -st * dyinv;
   p.fz = -st * dzinv;
   double *G = work[0], *pp = work[1], *n12 = work[2], *nside = work[3];
-  k_csf_grad<<<dim3((unsigned)(((long)(g.ni + 3) * (g.nj + 3) + 127) / 128), (unsigned)(g.nk + 3)), 128, 0, s>>>(
-      g, p, phi, G, skip);
+  k_csf_grad<<<tile_grid(g.ni + 3, g.nj + 3, g.nk + 3, 128), 128, 0, s>>>(g, p, phi, G, skip);
   // planes per walk: the first costs 9 additions more; as many as leave a warp for each
   // of the 608 quarter SMs, 8 at most
   const long cols = (long)(g.ni + 2) * (g.nj + 2);
   int m = 1;
   while (m < 8 && cols * (g.nk + 2) >= 2L * m * 768 * 32) m *= 2;
-  k_csf_normals<<<dim3((unsigned)((cols + 127) / 128), (unsigned)((g.nk + 2 + m - 1) / m)), 128, 0, s>>>(
-      g, p, m, G, pp, n12, nside, skip);
-  k_csf_force<<<dim3((unsigned)(g.ni / TX), (unsigned)(g.nj / TY), (unsigned)g.nk), dim3(TX, TY), 0, s>>>(
-      g, p, phi, pp, n12, nside, fu, fv, fw, skip);
+  k_csf_normals<<<tile_grid(g.ni + 2, g.nj + 2, (g.nk + 2 + m - 1) / m, 128), 128, 0, s>>>(g, p, m, G, pp, n12, nside,
+                                                                                           skip);
+  k_csf_force<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, p, phi, pp, n12, nside, fu, fv, fw, skip);
   count_launch(3);
 }
 }  // namespace

@@ -145,7 +145,8 @@ __device__ __forceinline__ void gexp8(R* E, R X1, R X2, R Y1, R Y2, R Z1, R Z2) 
   E[6] = c * Z2;
   E[7] = d * Z2;
 }
-// (five blocks per SM, 199 -> 178 us at 256x128x128)
+// (at 256x128x128: 199 us, 178 with five blocks per SM, 151 with warps of 8 x 4 and the
+// fluxes and sign tests below)
 __global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double* __restrict__ phi,
                                                   const double* __restrict__ gx, const double* __restrict__ gy,
                                                   const double* __restrict__ gz, const double* __restrict__ u,
@@ -153,9 +154,8 @@ __global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double*
                                                   double* __restrict__ fx, double* __restrict__ fy,
                                                   double* __restrict__ fz, int* __restrict__ list,
                                                   int* __restrict__ count) {
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int k = (int)blockIdx.z;
+  const Tile T = warp_tile(g.ni + 2);
+  const int i = T.x, j = T.y, k = (int)blockIdx.z;
   if (i > g.ni + 1 || j > g.nj + 1) return;
   const long X = 1, Y = g.sy, Z = g.sz;
   const long c = g.at(i, j, k);
@@ -174,9 +174,13 @@ __global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double*
   // the flux is zero), west/south/bottom when < 0; band cells leave the donated
   // faces to k_band but still zero the owned faces they do not donate through.
   // Fluxes are v phi dt/dx with phi dt/dx formed first.
+  // One product per axis, of the velocity that donates, and a second where a lane donates
+  // both ways, formed by the whole warp (stores under their lanes' signs alone: products
+  // under them were issued per set of lanes, 15 slots of the FP64 pipe for 3 products).
   const long long pb = __double_as_longlong(phi00);
   double pdx = 0.0, pdy = 0.0, pdz = 0.0;
-  if (__any_sync(warp, pb != 0)) {
+  const bool filled = __any_sync(warp, pb != 0);
+  if (filled) {
     if (__any_sync(warp, pb != 0 && pb != kOneBits)) {
       pdx = phi00 * m.dtdx;
       pdy = phi00 * m.dtdy;
@@ -188,13 +192,22 @@ __global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double*
     }
   }
   const bool e_ = nonneg(ue), w_ = nonneg(uw), n_ = nonneg(vn), s_ = nonneg(vs), t_ = nonneg(wt), b_ = nonneg(wb);
-  auto flux = [&](double vel, double pd) { return __any_sync(__activemask(), pb != 0) ? vel * pd : 0.0; };
-  if (e_) fx[c] = flux(ue, pdx);
-  if (!w_) fx[c - X] = flux(uw, pdx);
-  if (n_) fy[c] = flux(vn, pdy);
-  if (!s_) fy[c - Y] = flux(vs, pdy);
-  if (t_) fz[c] = flux(wt, pdz);
-  if (!b_) fz[c - Z] = flux(wb, pdz);
+  const bool two_x = __any_sync(warp, e_ && !w_), two_y = __any_sync(warp, n_ && !s_), two_z = __any_sync(warp, t_ && !b_);
+  double xe = 0.0, xw = 0.0, yn = 0.0, ys = 0.0, zt = 0.0, zb = 0.0;
+  if (filled) {
+    xe = xw = (e_ ? ue : uw) * pdx;
+    yn = ys = (n_ ? vn : vs) * pdy;
+    zt = zb = (t_ ? wt : wb) * pdz;
+    if (two_x) xw = uw * pdx;
+    if (two_y) ys = vs * pdy;
+    if (two_z) zb = wb * pdz;
+  }
+  if (e_) fx[c] = xe;
+  if (!w_) fx[c - X] = xw;
+  if (n_) fy[c] = yn;
+  if (!s_) fy[c - Y] = ys;
+  if (t_) fz[c] = zt;
+  if (!b_) fz[c - Z] = zb;
   // west/south/bottom faces of the first cells with no in-range donor stay zero
   if (i == 0 && w_) fx[c - X] = 0.0;
   if (j == 0 && s_) fy[c - Y] = 0.0;
@@ -397,8 +410,7 @@ __global__ void __launch_bounds__(64) k_band(Grid g, MC m, __grid_constant__ con
   }
 }
 // cal_grad_p2a.f:46-60 for the fused step: the vertex gradient at (i+1/2, j+1/2,
-// k+1/2), i, j, k in -2..n+2, from the 8 surrounding points (threads over the flattened
-// (i, j) plane, so that every warp is full).  Per (i, j) corner the sum s and difference
+// k+1/2), i, j, k in -2..n+2, from the 8 surrounding points.  Per (i, j) corner the sum s and difference
 // d of the two k planes; with ta = s(+,+) - s(0,0) and tb = s(+,0) - s(0,+) the x sum is
 // ta + tb, the y sum ta - tb and the z sum the four differences: 18 FP64 operations per
 // point instead of the reference's 27, none in a warp whose points are all flat.
@@ -410,12 +422,10 @@ template <bool NEAR1>
 __global__ void __launch_bounds__(128) k_vertex_grad(Grid g, double cx, double cy, double cz,
                                                      const double* __restrict__ q, double* __restrict__ qx,
                                                      double* __restrict__ qy, double* __restrict__ qz) {
-  const int W = g.ni + 5;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= W * (g.nj + 5)) return;
-  const int b = t / W, a = t - b * W;
+  const Tile T = warp_tile(g.ni + 5);
+  if (T.x >= g.ni + 5 || T.y >= g.nj + 5) return;
   const long X = 1, Y = g.sy, Z = g.sz;
-  const long c = g.at(a - 2, b - 2, (int)blockIdx.y - 2);
+  const long c = g.at(T.x - 2, T.y - 2, (int)blockIdx.z - 2);
   const double q000 = __ldg(q + c), qp00 = __ldg(q + c + X), q0p0 = __ldg(q + c + Y), qpp0 = __ldg(q + c + X + Y),
                q00p = __ldg(q + c + Z), qp0p = __ldg(q + c + X + Z), q0pp = __ldg(q + c + Y + Z),
                qppp = __ldg(q + c + X + Y + Z);
@@ -446,10 +456,9 @@ __global__ void __launch_bounds__(128) k_vertex_grad(Grid g, double cx, double c
 __global__ void __launch_bounds__(256) k_snap(Grid g, MC m, const double* __restrict__ gx,
                                               const double* __restrict__ gy, const double* __restrict__ gz,
                                               double* __restrict__ phin) {
-  const int W = g.ni + 2;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= W * (g.nj + 2)) return;
-  const int j = t / W, i = t - j * W, k = (int)blockIdx.y;
+  const Tile T = warp_tile(g.ni + 2);
+  const int i = T.x, j = T.y, k = (int)blockIdx.z;
+  if (i > g.ni + 1 || j > g.nj + 1) return;
   const long X = 1, Y = g.sy, Z = g.sz;
   const long c = g.at(i, j, k);
   G8 ax, ay, az;
@@ -463,7 +472,7 @@ __global__ void __launch_bounds__(256) k_snap(Grid g, MC m, const double* __rest
 
 void vertex_gradient(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const double* q,
                      double* qx, double* qy, double* qz, bool near1) {
-  const dim3 gr((unsigned)(((long)(g.ni + 5) * (g.nj + 5) + 127) / 128), (unsigned)(g.nk + 5));
+  const dim3 gr = tile_grid(g.ni + 5, g.nj + 5, g.nk + 5, 128);
   if (near1)
     k_vertex_grad<true><<<gr, 128, 0, s>>>(g, 0.25 * dxinv, 0.25 * dyinv, 0.25 * dzinv, q, qx, qy, qz);
   else
@@ -473,7 +482,7 @@ void vertex_gradient(cudaStream_t s, const Grid& g, double dxinv, double dyinv, 
 
 void mthinc_snap(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double bet,
                  const double* gx, const double* gy, const double* gz, double* phin) {
-  const dim3 gr((unsigned)(((long)(g.ni + 2) * (g.nj + 2) + 255) / 256), (unsigned)(g.nk + 2));
+  const dim3 gr = tile_grid(g.ni + 2, g.nj + 2, g.nk + 2, 256);
   k_snap<<<gr, 256, 0, s>>>(g, make_mc(dxinv, dyinv, dzinv, 0.0, bet), gx, gy, gz, phin);
   count_launch();
 }
@@ -493,9 +502,7 @@ void mthinc_fluxes(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
                    bool fp32, double* newton) {
   const MC m = make_mc(dxinv, dyinv, dzinv, dt, bet);
   FMF_CUDA(cudaMemsetAsync(count, 0, sizeof(int), s));
-  dim3 b(32, 8, 1);
-  dim3 gr((unsigned)((g.ni + 2 + 31) / 32), (unsigned)((g.nj + 2 + 7) / 8), (unsigned)(g.nk + 2));
-  k_classify<<<gr, b, 0, s>>>(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count);
+  k_classify<<<tile_grid(g.ni + 2, g.nj + 2, g.nk + 2, 256), 256, 0, s>>>(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count);
   const long cap = (long)(g.ni + 2) * (g.nj + 2) * (g.nk + 2);
   if (fp32)
     k_band_f32<<<152 * 8, 128, 0, s>>>(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);

@@ -26,6 +26,7 @@
 #include <cstring>
 #include <type_traits>
 
+#include "bits.cuh"
 #include "df64.cuh"
 #include "fused.cuh"
 #include "recip.cuh"
@@ -61,10 +62,9 @@ struct F3 {
 // such points takes it without the arithmetic.  Threads over the flattened (i, j) plane.
 __global__ void __launch_bounds__(128) k_edges(Grid g, VP p, const double* __restrict__ mu, double* __restrict__ exy,
                                                double* __restrict__ exz, double* __restrict__ eyz, F3 f) {
-  const int W = g.ni + 1;
-  const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  if (t >= W * (g.nj + 1)) return;
-  const int j = t / W, i = t - j * W, k = (int)blockIdx.y;
+  const Tile T = warp_tile(g.ni + 1);
+  const int i = T.x, j = T.y, k = (int)blockIdx.z;
+  if (i > g.ni || j > g.nj) return;
   const long X = 1, Y = g.sy, Z = g.sz;
   const long c = g.at(i, j, k);
   const double m0 = __ldg(mu + c), mx = __ldg(mu + c + X), my = __ldg(mu + c + Y), mz = __ldg(mu + c + Z),
@@ -132,9 +132,8 @@ struct SrcK {
 __global__ void __launch_bounds__(256) k_src_ab(Grid g, SrcK K, SrcIn in, const double* __restrict__ mu,
                                                 const double* __restrict__ exy, const double* __restrict__ exz,
                                                 const double* __restrict__ eyz, ABOut out) {
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int k = 1 + (int)blockIdx.z;
+  const Tile T = warp_tile(g.ni);
+  const int i = 1 + T.x, j = 1 + T.y, k = 1 + (int)blockIdx.z;
   if (i > g.ni || j > g.nj) return;
   const long X = 1, Y = g.sy, Z = g.sz;
   const long c = g.at(i, j, k);
@@ -1460,7 +1459,7 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
   in.phat = phat;
   in.grvb = grvb;
   in.grvp = grvp;
-  k_edges<<<dim3((unsigned)(((long)(g.ni + 1) * (g.nj + 1) + 127) / 128), (unsigned)(g.nk + 1)), 128, 0, s>>>(
+  k_edges<<<tile_grid(g.ni + 1, g.nj + 1, g.nk + 1, 128), 128, 0, s>>>(
       g, p, mu, E[0], E[1], E[2], ef);
   if (REFINE) {
     using df::split_double;
@@ -1501,7 +1500,7 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
       K.a[q][1] = 1.0 / (2.0 * rf[q] * p.dtinv + xx + 2.0 * yy + zz);
       K.a[q][2] = 1.0 / (2.0 * rf[q] * p.dtinv + xx + yy + 2.0 * zz);
     }
-    k_src_ab<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, K, in, mu, E[0], E[1], E[2], out);
+    k_src_ab<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, K, in, mu, E[0], E[1], E[2], out);
   }
   k_wall_coef<<<wall_grid(g), kB, 0, s>>>(g, dy, l1, l2, phi, wallc);
   count_launch(3);

@@ -24,8 +24,8 @@ __global__ void __launch_bounds__(256) k_advance(Grid g, double dxi, double dyi,
                                                  const double* __restrict__ fx, const double* __restrict__ fy,
                                                  const double* __restrict__ fz, const double* __restrict__ phi,
                                                  double* __restrict__ phin) {
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
+  const Tile T = warp_tile(g.ni);
+  const int i = 1 + T.x, j = 1 + T.y;
   if (i > g.ni || j > g.nj) return;
   const long X = 1, Y = g.sy, Z = g.sz;
   const long c = g.at(i, j, 1 + (int)blockIdx.z);
@@ -48,8 +48,8 @@ __global__ void __launch_bounds__(256) k_advance(Grid g, double dxi, double dyi,
 __global__ void __launch_bounds__(256) k_offset(Grid g, const double* __restrict__ sums, double* __restrict__ phin,
                                                 double* __restrict__ phin0) {
   __shared__ double off;
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
+  const Tile T = warp_tile(g.ni);
+  const int i = 1 + T.x, j = 1 + T.y;
   const int k = 1 + (int)blockIdx.z;
   const bool in = i <= g.ni && j <= g.nj;
   const long c = in ? g.at(i, j, k) : 0;
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(256) k_offset(Grid g, const double* __restrict
   const long long pb = __double_as_longlong(p);
   const bool between = pb != 0 && pb != kOneBits;
   if (__syncthreads_or(between)) {
-    if (threadIdx.x == 0 && threadIdx.y == 0) off = (sums[0] - sums[1]) * recip_nr(sums[2] + 1.0e-99);
+    if (threadIdx.x == 0) off = (sums[0] - sums[1]) * recip_nr(sums[2] + 1.0e-99);
     __syncthreads();
     if (between) p = clip01(p + off * (p * p) * (1.0 - p));
   }
@@ -140,8 +140,6 @@ void halos(cudaStream_t s, const Grid& g, double* q) {
   k_halos<WALLS><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, nx, nz, q);
   count_launch();
 }
-const dim3 kCell(32, 8, 1);
-dim3 cell_grid(const Grid& g) { return dim3((unsigned)((g.ni + 31) / 32), (unsigned)((g.nj + 7) / 8), (unsigned)g.nk); }
 }  // namespace
 
 void halo_periodic(cudaStream_t s, const Grid& g, double* q) { halos<false>(s, g, q); }
@@ -150,7 +148,7 @@ void halo_neumann_periodic(cudaStream_t s, const Grid& g, double* q) { halos<tru
 void mthinc_advance(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt,
                     const double* u, const double* v, const double* w, const double* fx, const double* fy,
                     const double* fz, const double* phi, double* phin) {
-  k_advance<<<cell_grid(g), kCell, 0, s>>>(g, dxinv, dyinv, dzinv, dt, u, v, w, fx, fy, fz, phi, phin);
+  k_advance<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, dxinv, dyinv, dzinv, dt, u, v, w, fx, fy, fz, phi, phin);
   count_launch();
 }
 
@@ -170,7 +168,7 @@ void mthinc_volume_fix(cudaStream_t s, const Grid& g, double dxinv, double dyinv
         r[2] = b == 0 || b == kOneBits ? 0.0 : p * p * (1.0 - p);
       },
       sums);
-  k_offset<<<cell_grid(g), kCell, 0, s>>>(g, sums, phin, phin0);
+  k_offset<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, sums, phin, phin0);
   count_launch();
 }
 
