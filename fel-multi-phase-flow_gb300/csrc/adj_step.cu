@@ -99,6 +99,7 @@ struct fmf_adj {
   double *gx1[3], *fl[3], *pa, *gxn[3], *pb, *pass, *sums, *pc, *theta, *phn1f;
   double *rho, *rhon, *rmu, *rmun, *adv[3], *advo[3], *phat, *prs[3], *sk, *tau, *vis[3];
   double *sfst[3], *sfstn[3], *E[3], *AB[6], *wallc, *ustar[3], *un2[3], *snaps, *sorpart;
+  fused::FlatFluid flat;  // as the product step's
   double *un[3], *pn, *dp, *div, *pr, *pi, *as_f, *an_f, *ap_f, *red;
   double* csfwork;  // forward CSF chain (drop-in): G(3n) rn(12n) kap(3n) g(3n) f(3n)
   int* band;        // MTHINC band-cell list and its length
@@ -534,7 +535,7 @@ int record_step(fmf_adj* a, bool graphs) {
     // the FP64 factors A, B the reverse differentiates (the viscous solve's fixed
     // point is un* = A visn(un*) + B in either precision)
     fused::src_visc_prep(s, g, dxi, dyi, dzi, dt, P.harmonic, P.grvb, P.grvp, S[SU], S[SV], S[SW], advp, advop,
-                         a->phat, visp, fstp, fstnp, fl, a->rmun, a->rho, a->rhon, a->E, a->AB, a->l1, a->l2, phi1, P.dy, a->wallc);
+                         a->phat, visp, fstp, fstnp, fl, a->rmun, a->rho, a->rhon, a->E, a->AB, a->l1, a->l2, phi1, P.dy, a->wallc, a->flat);
     if (a->mixed)
       // the mixed solve's FP64 first-sweep residual, FP32 factors and wall/halo
       // constants; un = u through zero corrections
@@ -552,7 +553,7 @@ int record_step(fmf_adj* a, bool graphs) {
       fused::sor_iteration_refine(s, g, dxi, dyi, dzi, a->rb, a->sorpart, a->red + 4);
     else
       fused::sor_iteration(s, g, dxi, dyi, dzi, P.harmonic, a->rmun, a->E, a->AB, P.uwall, a->wallc, a->un[0],
-                           a->un[1], a->un[2], a->sorpart, a->red + 4);
+                           a->un[1], a->un[2], a->sorpart, a->red + 4, a->flat);
   };
   if (a->small) {
     fused::sor_rule(s, a->loop, a->sor_tol, a->sor_max, (double)g.cells());
@@ -1014,6 +1015,10 @@ int fmf_adj_create(const fmf_params* prm, fmf_adj** out) {
   a->ib_wallc = dalloc(a, nwc);
   a->snaps = dalloc(a, 39 * n);
   a->sorpart = dalloc(a, fused::sor_parts(a->g));
+  if (!a->mixed && fused::flat_sweeps(a->g))
+    a->flat = fused::make_flat(a->g, 1.0 / prm->dx, 1.0 / prm->dy, 1.0 / prm->dz, prm->dt,
+                               fused::Fluids{prm->rhol, prm->rhog, prm->rmul, prm->rmug},
+                               (unsigned char*)dalloc(a, (fused::flat_bytes(a->g) + 7) / 8));
   const char* dl = std::getenv("FMF_DEVICE_LOOP");
   a->small = !(dl && std::atoi(dl) == 0) && fused::solve_small_supported(a->g, !a->mixed);
   a->loop = (fused::SorLoop*)dalloc(a, (sizeof(fused::SorLoop) + 7) / 8);

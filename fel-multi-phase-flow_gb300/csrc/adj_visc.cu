@@ -346,6 +346,7 @@ void sor_replay(cudaStream_t s, const Grid& g, double dxi, double dyi, double dz
   k_copy3<<<608, 256, 0, s>>>(n, CArr3{{ustar[0], ustar[1], ustar[2]}}, q[0]);
   count_launch();
   fused::sor_iteration(s, g, dxi, dyi, dzi, harmonic, mu, E, AB, uwall, wallc, q[0], q[1], q[2], part, nullptr,
+                       fused::FlatFluid(),
                        [&](int comp, int pr) {
                          const CArr3 st = replay_state(g, snaps, comp, pr);
                          double* own = snaps + (3L * (4 * comp + pr) + comp) * n;

@@ -87,6 +87,21 @@ void explicit_viscous(cudaStream_t s, const Grid& g, double dxinv, double dyinv,
 struct Fluids {
   double rhol, rhog, rmul, rmug;
 };
+// Per cell (n bytes) whether everything the momentum factors of its three points read is
+// one fluid's own (0 or 1; 2: not), as src_visc_prep writes it, with that fluid's A per
+// component and viscosity: the sweeps take these without reading the fields where `enough`
+// of the cells (count) are such (fluid null: never).  make_flat: for grids of a size whose
+// sweeps use it, with flat_bytes(g) of memory.
+struct FlatFluid {
+  unsigned char* fluid = nullptr;
+  int* count = nullptr;
+  int enough = 0;
+  double a[2][3] = {}, mu[2] = {};
+};
+bool flat_sweeps(const Grid& g);
+inline long flat_bytes(const Grid& g) { return g.n + 8; }
+FlatFluid make_flat(const Grid& g, double dxinv, double dyinv, double dzinv, double dt, const Fluids& fl,
+                    unsigned char* bytes);
 // Viscous solve.  src_visc_prep: edge viscosities E[0..2] (xy, xz, yz edges, i,j,k in
 // 0..n), per-component A/B (AB[0..5] = Au Bu Av Bv Aw Bw) with the momentum
 // right-hand side of cal_srcu formed in registers (its pressure gradient from phat =
@@ -97,7 +112,7 @@ void src_visc_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
                    const double* const* adv, const double* const* advo, const double* phat,
                    const double* const* vis, const double* const* fst, const double* const* fstn, const Fluids& fl,
                    const double* mu, const double* rho, const double* rhon, double* const* E, double* const* AB, const double* l1,
-                   const double* l2, const double* phi, double dy, double* wallc);
+                   const double* l2, const double* phi, double dy, double* wallc, const FlatFluid& flat = FlatFluid());
 // the Navier-slip coefficients wallc alone (as src_visc_prep computes them)
 void wall_coef(cudaStream_t s, const Grid& g, double dy, const double* l1, const double* l2, const double* phi,
                double* wallc);
@@ -113,6 +128,7 @@ void wall_halo(cudaStream_t s, const Grid& g, int normal, double uwall, const do
 void sor_iteration(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, int harmonic,
                    const double* mu, double* const* E, double* const* AB, double uwall, const double* wallc,
                    double* un, double* vn, double* wn, double* part, double* errsum,
+                   const FlatFluid& flat = FlatFluid(),
                    const std::function<void(int, int)>& before = nullptr);
 long sor_parts(const Grid& g);
 

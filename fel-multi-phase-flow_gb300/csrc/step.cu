@@ -84,6 +84,7 @@ struct fmf_ctx {
   double *adv[3], *advo[3], *phat, *tau, *vis[3];
   double *rn[4], *rnn[4], *rkap, *rkapn, *fst[3], *fstn[3], *sfst[3], *sfstn[3], *src[3];
   double *edge[3], *ab[6], *wallc, *sorpart;  // fused viscous solve (fused_visc.cu)
+  fused::FlatFluid flat;                      // FP64 sweeps: the cells of one fluid alone
   double *dp, *div, *pr, *pi;
   double *as_f, *an_f, *ap_f;
   double* red;  // small reduction outputs
@@ -272,6 +273,10 @@ int fmf_ctx_create(const fmf_params* prm, fmf_ctx** out) {
   for (int q = 0; q < 3; ++q) c->edge[q] = alloc(c, n);
   for (int q = 0; q < 6; ++q) c->ab[q] = alloc(c, n);
   c->wallc = alloc(c, 4L * (prm->nk + 6) * (prm->ni + 6));
+  if (!c->mixed && fused::flat_sweeps(c->g))
+    c->flat = fused::make_flat(c->g, 1.0 / prm->dx, 1.0 / prm->dy, 1.0 / prm->dz, prm->dt,
+                               fused::Fluids{prm->rhol, prm->rhog, prm->rmul, prm->rmug},
+                               (unsigned char*)alloc(c, (fused::flat_bytes(c->g) + 7) / 8));
   c->sorpart = alloc(c, fused::sor_parts(c->g));
   c->pr = alloc(c, nm);
   c->pi = alloc(c, nm);
@@ -580,7 +585,7 @@ static void seg_pre2(fmf_ctx* c) {
   }
   fused::src_visc_prep(s, g, dxinv, dyinv, dzinv, dt, P.harmonic, P.grvb, P.grvp, c->u, c->v, c->w, advp, advop,
                        c->phat, visp, fstp, fstnp, fl, c->rmun, c->rho, c->rhon, c->edge, c->ab, c->l1, c->l2, phi1, P.dy,
-                       c->wallc);
+                       c->wallc, c->flat);
   // :605-607
   op::copy(s, n, c->u, c->un);
   op::copy(s, n, c->v, c->vn);
@@ -620,7 +625,7 @@ static void iter_kernels(fmf_ctx* c) {
     fused::sor_iteration_refine(c->s, c->g, dxinv, dyinv, dzinv, c->rb, c->sorpart, c->red + 8);
   else
     fused::sor_iteration(c->s, c->g, dxinv, dyinv, dzinv, P.harmonic, c->rmun, c->edge, c->ab, P.uwall, c->wallc,
-                         c->un, c->vn, c->wn, c->sorpart, c->red + 8);
+                         c->un, c->vn, c->wn, c->sorpart, c->red + 8, c->flat);
 }
 // the same, with the residual sum copied to the host (the host applies the rule)
 static void seg_iter(fmf_ctx* c) {
@@ -879,7 +884,7 @@ int fmf_ctx_time_stage(fmf_ctx* c, int stage, int reps, float* ms) {
           fused::sor_iteration_refine(s, g, dxinv, dyinv, dzinv, c->rb, c->sorpart, c->red + 8);
         else
           fused::sor_iteration(s, g, dxinv, dyinv, dzinv, P.harmonic, c->rmun, c->edge, c->ab, P.uwall, c->wallc,
-                               c->un, c->vn, c->wn, c->sorpart, c->red + 8);
+                               c->un, c->vn, c->wn, c->sorpart, c->red + 8, c->flat);
         break;
       case 2:
         fused::pressure_half(s, g, P.rhog, dxinv, dzinv, c->as_f, c->an_f, c->ap_f, c->div, c->pr, c->pi, c->dp,
@@ -967,7 +972,7 @@ int fmf_ctx_check_sor(fmf_ctx* c, double* out) {
     const double* fstnp[3] = {c->sfstn[0], c->sfstn[1], c->sfstn[2]};
     fused::src_visc_prep(s, g, dxinv, dyinv, dzinv, P.dt, P.harmonic, P.grvb, P.grvp, c->u, c->v, c->w, advp, advop,
                          c->phat, visp, fstp, fstnp, fl, c->rmun, c->rho, c->rhon, c->edge, c->ab, c->l1, c->l2,
-                         c->phi + n, P.dy, c->wallc);
+                         c->phi + n, P.dy, c->wallc, c->flat);
   }
   double *q64[3] = {q, q + n, q + 2 * n}, *qx[3] = {q + 3 * n, q + 4 * n, q + 5 * n};
   double* acc = q + 10 * n;
@@ -975,7 +980,7 @@ int fmf_ctx_check_sor(fmf_ctx* c, double* out) {
   const double* unp[3] = {c->un, c->vn, c->wn};
   auto iter64 = [&](double* const* v) {
     fused::sor_iteration(s, g, dxinv, dyinv, dzinv, P.harmonic, c->rmun, c->edge, c->ab, P.uwall, c->wallc, v[0],
-                         v[1], v[2], c->sorpart, c->red + 8);
+                         v[1], v[2], c->sorpart, c->red + 8, c->flat);
     FMF_CUDA(cudaMemcpyAsync(c->host_err, c->red + 8, sizeof(double), cudaMemcpyDeviceToHost, s));
     return read_err();
   };
