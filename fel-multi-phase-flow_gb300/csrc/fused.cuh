@@ -77,11 +77,11 @@ void csf_force(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double
 // The explicit viscous term (calsij, cal_arith_tau, cal_div_tensor) at the interior
 // u, v, w points into vis[0..2]; tau: 6 n doubles of workspace; sk (optional, 6 n):
 // the strain components at the points 0..n+1 the interior divergence reads
-// (pairs: the stresses and their divergence in FP32-pair arithmetic, the strain
+// (uvw, the split pairs of u, v, w: in FP32-pair arithmetic from these, the strain
 // still FP64; the FP64-accurate and the mixed-precision steps)
 void explicit_viscous(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const double* u,
                       const double* v, const double* w, const double* mu, double* tau, double* const* vis,
-                      double* sk = nullptr, bool pairs = false);
+                      double* sk = nullptr, const float2* uvw = nullptr);
 
 // the densities and viscosities of the two fluids (phi = 0 and phi = 1)
 struct Fluids {

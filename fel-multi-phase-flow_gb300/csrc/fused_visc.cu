@@ -334,36 +334,55 @@ __global__ void __launch_bounds__(256) k_div_stress(Grid g, StressK K, const dou
 
 // The FP64-accurate and mixed-precision steps: the stresses themselves and their
 // divergence in FP32-pair arithmetic (each double read split into a pair, each output
-// rounded to a double once).
+// rounded to a double once).  Bound by the integer and FP32 pipes, the conversions
+// (df::split_double, to_double) in front: at 256x128x128 207 + 129 us with every double
+// read split where it is read, 129 + 67 as below.
 // With sk (the adjoint's record of a mixed-precision step) the strain components
 // are written as well, in FP64 as k_stress forms them.
 struct VPT {
   df::D dxi2, dyi2, dzi2, hx, hy, hz, dxi, dyi, dzi;  // 2 dxi, ..., dxi/4, ..., dxi, ...
   double dxd, dyd, dzd;                               // dxi, dyi, dzi (the strain in FP64)
 };
-__global__ void __launch_bounds__(256) k_stress_e(Grid g, VPT p, const double* __restrict__ u,
-                                                  const double* __restrict__ v, const double* __restrict__ w,
-                                                  const double* __restrict__ mu, double* __restrict__ tau,
-                                                  double* __restrict__ sk) {
+// uvw: the split pairs of u, v, w (those of the WENO5 stage), field f at uvw[f n ..]; tau is
+// stored as the split pairs of the doubles the stresses round to, which is what
+// k_div_stress_e reads: 15 + 12 fewer conversions per cell.
+__global__ void __launch_bounds__(256) k_stress_e(Grid g, VPT p, const float2* __restrict__ uvw,
+                                                  const double* __restrict__ u, const double* __restrict__ v,
+                                                  const double* __restrict__ w, const double* __restrict__ mu,
+                                                  float2* __restrict__ tau, double* __restrict__ sk) {
   using namespace df;
-  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int k = (int)blockIdx.z;
+  const Tile T = warp_tile(g.ni + 2);
+  const int i = T.x, j = T.y, k = (int)blockIdx.z;
   if (i > g.ni + 1 || j > g.nj + 1) return;
   const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
   const long c = g.at(i, j, k);
-  auto L = [&](const double* a, long o) { return split_double(__ldg(a + c + o)); };
-  const D m0 = L(mu, 0), mx = L(mu, X), my = L(mu, Y), mz = L(mu, Z);
-  const D u0 = L(u, 0), v0 = L(v, 0), w0 = L(w, 0);
-  tau[c] = to_double(mul(mul(sub(u0, L(u, -X)), m0), p.dxi2));
-  tau[c + n] = to_double(mul(mul(sub(v0, L(v, -Y)), m0), p.dyi2));
-  tau[c + 2 * n] = to_double(mul(mul(sub(w0, L(w, -Z)), m0), p.dzi2));
-  tau[c + 3 * n] = to_double(mul(add(mul(sub(L(u, Y), u0), p.hy), mul(sub(L(v, X), v0), p.hx)),
-                                 add(add(m0, mx), add(my, L(mu, X + Y)))));
-  tau[c + 4 * n] = to_double(mul(add(mul(sub(L(u, Z), u0), p.hz), mul(sub(L(w, X), w0), p.hx)),
-                                 add(add(m0, mx), add(mz, L(mu, X + Z)))));
-  tau[c + 5 * n] = to_double(mul(add(mul(sub(L(v, Z), v0), p.hz), mul(sub(L(w, Y), w0), p.hy)),
-                                 add(add(m0, my), add(mz, L(mu, Y + Z)))));
+  const double d0 = __ldg(mu + c), dx = __ldg(mu + c + X), dy = __ldg(mu + c + Y), dz = __ldg(mu + c + Z),
+               dxy = __ldg(mu + c + X + Y), dxz = __ldg(mu + c + X + Z), dyz = __ldg(mu + c + Y + Z);
+  auto L = [&](int f, long o) {
+    const float2 q = __ldg(uvw + f * n + c + o);
+    return D{q.x, q.y};
+  };
+  auto put = [&](int q, D t) {
+    const D r = split_double(to_double(t));
+    tau[q * n + c] = make_float2(r.h, r.l);
+  };
+  const D m0 = split_double(d0), u0 = L(0, 0), v0 = L(1, 0), w0 = L(2, 0);
+  D sxy, sxz, syz;  // the sums of four viscosities
+  if (__any_sync(__activemask(), !(same_bits(d0, dx, dy, dz, dxy) && same_bits(d0, dxz, dyz, d0, d0)))) {
+    const D mx = split_double(dx), my = split_double(dy), mz = split_double(dz);
+    sxy = add(add(m0, mx), add(my, split_double(dxy)));
+    sxz = add(add(m0, mx), add(mz, split_double(dxz)));
+    syz = add(add(m0, my), add(mz, split_double(dyz)));
+  } else {
+    const D two = add(m0, m0);
+    sxy = sxz = syz = add(two, two);
+  }
+  put(0, mul(mul(sub(u0, L(0, -X)), m0), p.dxi2));
+  put(1, mul(mul(sub(v0, L(1, -Y)), m0), p.dyi2));
+  put(2, mul(mul(sub(w0, L(2, -Z)), m0), p.dzi2));
+  put(3, mul(add(mul(sub(L(0, Y), u0), p.hy), mul(sub(L(1, X), v0), p.hx)), sxy));
+  put(4, mul(add(mul(sub(L(0, Z), u0), p.hz), mul(sub(L(2, X), w0), p.hx)), sxz));
+  put(5, mul(add(mul(sub(L(1, Z), v0), p.hz), mul(sub(L(2, Y), w0), p.hy)), syz));
   if (sk) {
     const double dxi = p.dxd, dyi = p.dyd, dzi = p.dzd;
     const double ud = __ldg(u + c), vd = __ldg(v + c), wd = __ldg(w + c);
@@ -375,7 +394,7 @@ __global__ void __launch_bounds__(256) k_stress_e(Grid g, VPT p, const double* _
     sk[c + 5 * n] = ((__ldg(v + c + Z) - vd) * dzi + (__ldg(w + c + Y) - wd) * dyi) * 0.5;
   }
 }
-__global__ void __launch_bounds__(256) k_div_stress_e(Grid g, VPT p, const double* __restrict__ t,
+__global__ void __launch_bounds__(256) k_div_stress_e(Grid g, VPT p, const float2* __restrict__ t,
                                                       double* __restrict__ vu, double* __restrict__ vv,
                                                       double* __restrict__ vw) {
   using namespace df;
@@ -385,7 +404,10 @@ __global__ void __launch_bounds__(256) k_div_stress_e(Grid g, VPT p, const doubl
   if (i > g.ni || j > g.nj) return;
   const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
   const long c = g.at(i, j, k);
-  auto L = [&](int q, long o) { return split_double(__ldg(t + q * n + c + o)); };
+  auto L = [&](int q, long o) {
+    const float2 r = __ldg(t + q * n + c + o);
+    return D{r.x, r.y};
+  };
   const D a4 = L(3, 0), a5 = L(4, 0), a6 = L(5, 0);
   vu[c] = to_double(add(add(mul(sub(L(0, X), L(0, 0)), p.dxi), mul(sub(a4, L(3, -Y)), p.dyi)),
                         mul(sub(a5, L(4, -Z)), p.dzi)));
@@ -1690,8 +1712,8 @@ void wall_coef(cudaStream_t s, const Grid& g, double dy, const double* l1, const
 
 void explicit_viscous(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const double* u,
                       const double* v, const double* w, const double* mu, double* tau, double* const* vis,
-                      double* sk, bool pairs) {
-  if (pairs) {
+                      double* sk, const float2* uvw) {
+  if (uvw) {
     using df::split_double;
     VPT p;
     p.dxd = dxinv;
@@ -1706,9 +1728,9 @@ void explicit_viscous(cudaStream_t s, const Grid& g, double dxinv, double dyinv,
     p.dxi = split_double(dxinv);
     p.dyi = split_double(dyinv);
     p.dzi = split_double(dzinv);
-    k_stress_e<<<dim3((g.ni + 2 + 31) / 32, (g.nj + 2 + 7) / 8, g.nk + 2), kB, 0, s>>>(g, p, u, v, w, mu, tau,
-                                                                                                 sk);
-    k_div_stress_e<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, p, tau, vis[0], vis[1], vis[2]);
+    float2* tp = (float2*)tau;
+    k_stress_e<<<tile_grid(g.ni + 2, g.nj + 2, g.nk + 2, 256), 256, 0, s>>>(g, p, uvw, u, v, w, mu, tp, sk);
+    k_div_stress_e<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, p, tp, vis[0], vis[1], vis[2]);
     count_launch(2);
     return;
   }

@@ -557,7 +557,7 @@ static void seg_pre2(fmf_ctx* c) {
                       c->wsplit);
   op::calphat(s, g, c->p, c->po, c->phat);
   fused::explicit_viscous(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->rmu, c->tau, c->vis, nullptr,
-                          c->wprec != 0);
+                          c->wprec ? c->wsplit : nullptr);
   // :545-570 surface tension (sfst carried over from the previous step's sfstn where
   // the state continues)
   if (c->verify && fused::csf_supported(g))
