@@ -536,13 +536,13 @@ int record_step(fmf_adj* a, bool graphs) {
     // the FP64 factors A, B the reverse differentiates (the viscous solve's fixed
     // point is un* = A visn(un*) + B in either precision)
     fused::src_visc_prep(s, g, dxi, dyi, dzi, dt, P.harmonic, P.grvb, P.grvp, S[SU], S[SV], S[SW], advp, advop,
-                         a->phat, visp, fstp, fstnp, fl, a->rmun, a->rho, a->rhon, a->E, a->AB, a->l1, a->l2, phi1, P.dy, a->wallc, a->flat);
+                         a->phat, visp, fstp, fstnp, fl, a->rmun, a->rho, a->rhon, a->E, a->AB, a->l1, a->l2, phi1, P.dy, a->wallc, a->mixed ? fused::FlatFluid() : a->flat);
     if (a->mixed)
       // the mixed solve's FP64 first-sweep residual, FP32 factors and wall/halo
       // constants; un = u through zero corrections
       fused::refine_prep(s, g, dxi, dyi, dzi, dt, P.harmonic, P.grvb, P.grvp, S[SU], S[SV], S[SW], advp, advop,
                          a->phat, visp, fstp, fstnp, fl, a->rmun, a->rho, a->rhon, a->E, a->l1, a->l2, phi1, P.dy, P.uwall,
-                         a->wallc, a->rb);
+                         a->wallc, a->rb, a->flat);
     else
       for (int q = 0; q < 3; ++q) dcopy(a, S[SU + q], a->un[q], n);
   };
@@ -551,7 +551,7 @@ int record_step(fmf_adj* a, bool graphs) {
   // CUDA graph per record slot
   auto iteration = [&]() {
     if (a->mixed)
-      fused::sor_iteration_refine(s, g, dxi, dyi, dzi, a->rb, a->sorpart, a->red + 4);
+      fused::sor_iteration_refine(s, g, dxi, dyi, dzi, a->rb, a->sorpart, a->red + 4, a->flat);
     else
       fused::sor_iteration(s, g, dxi, dyi, dzi, P.harmonic, a->rmun, a->E, a->AB, P.uwall, a->wallc, a->un[0],
                            a->un[1], a->un[2], a->sorpart, a->red + 4, a->flat);
@@ -1016,10 +1016,10 @@ int fmf_adj_create(const fmf_params* prm, fmf_adj** out) {
   a->ib_wallc = dalloc(a, nwc);
   a->snaps = dalloc(a, 39 * n);
   a->sorpart = dalloc(a, fused::sor_parts(a->g));
-  if (!a->mixed && fused::flat_sweeps(a->g))
-    a->flat = fused::make_flat(a->g, 1.0 / prm->dx, 1.0 / prm->dy, 1.0 / prm->dz, prm->dt,
+  if (a->mixed || fused::flat_sweeps(a->g))
+    a->flat = fused::make_flat(a->s, a->g, 1.0 / prm->dx, 1.0 / prm->dy, 1.0 / prm->dz, prm->dt,
                                fused::Fluids{prm->rhol, prm->rhog, prm->rmul, prm->rmug},
-                               (unsigned char*)dalloc(a, (fused::flat_bytes(a->g) + 7) / 8));
+                               (unsigned char*)dalloc(a, (fused::flat_bytes(a->g) + 7) / 8), a->mixed);
   const char* dl = std::getenv("FMF_DEVICE_LOOP");
   a->small = !(dl && std::atoi(dl) == 0) && fused::solve_small_supported(a->g, !a->mixed);
   a->loop = (fused::SorLoop*)dalloc(a, (sizeof(fused::SorLoop) + 7) / 8);

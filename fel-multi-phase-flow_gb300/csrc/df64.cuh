@@ -214,6 +214,30 @@ DF_FN D split_double(double q) {
   return {hi, sg ? -lo : lo};
 }
 
+// A double rounded to the nearest float (ties to even) from its bits, as a conversion
+// rounds it (which takes an FP64-pipe instruction).
+DF_FN float d2f(double x) {
+  uint64_t b;
+#if defined(__CUDA_ARCH__)
+  b = (uint64_t)__double_as_longlong(x);
+#else
+  std::memcpy(&b, &x, 8);
+#endif
+  const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b, e = (hi >> 20) & 0x7ffu, sg = hi & 0x80000000u;
+  uint32_t m, rest, half = 0x10000000u;  // the float's bits, cut; what was cut; half a unit
+  if (e >= 897u) {
+    if (e > 1150u) return bitsf(sg | (e == 2047u && ((hi & 0xfffffu) | lo) ? 0x7fc00000u : 0x7f800000u));
+    m = ((e - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+    rest = lo & 0x1fffffffu;
+  } else {  // below 2^-126: units of 2^-149; the last bit of rest: whether more was cut
+    if (e < 873u) return bitsf(sg);
+    const uint32_t top = 0x800000u | ((hi & 0xfffffu) << 3) | (lo >> 29), sh = 897u - e;  // 1..24
+    m = top >> sh;
+    rest = ((top << (32u - sh)) >> 3) | ((lo & 0x1fffffffu) ? 1u : 0u);
+  }
+  return bitsf(sg | (m + ((rest > half || (rest == half && (m & 1u))) ? 1u : 0u)));
+}
+
 // A pair from a double, on the host (constants): h = (float)v, l = (float)(v - h)
 DF_FN D from_double_host(double v) {
   const float h = (float)v;

@@ -88,20 +88,21 @@ struct Fluids {
   double rhol, rhog, rmul, rmug;
 };
 // Per cell (n bytes) whether everything the momentum factors of its three points read is
-// one fluid's own (0 or 1; 2: not), as src_visc_prep writes it, with that fluid's A per
+// one fluid's own (0 or 1; 2: not), as src_visc_prep (refine_prep) writes it, with that fluid's A per
 // component and viscosity: the sweeps take these without reading the fields where `enough`
-// of the cells (count) are such (fluid null: never).  make_flat: for grids of a size whose
-// sweeps use it, with flat_bytes(g) of memory.
+// of the cells (count) are such (fluid null: never; small grids).  make_flat: with
+// flat_bytes(g) of memory.
 struct FlatFluid {
   unsigned char* fluid = nullptr;
   int* count = nullptr;
   int enough = 0;
   double a[2][3] = {}, mu[2] = {};
+  const float2* pairs = nullptr;  // mixed precision: per fluid rho00 and T of each component
 };
 bool flat_sweeps(const Grid& g);
-inline long flat_bytes(const Grid& g) { return g.n + 8; }
-FlatFluid make_flat(const Grid& g, double dxinv, double dyinv, double dzinv, double dt, const Fluids& fl,
-                    unsigned char* bytes);
+inline long flat_bytes(const Grid& g) { return g.n + 8 + 8 * (long)sizeof(float2); }
+FlatFluid make_flat(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt,
+                    const Fluids& fl, unsigned char* bytes, bool mixed);
 // Viscous solve.  src_visc_prep: edge viscosities E[0..2] (xy, xz, yz edges, i,j,k in
 // 0..n), per-component A/B (AB[0..5] = Au Bu Av Bv Aw Bw) with the momentum
 // right-hand side of cal_srcu formed in registers (its pressure gradient from phat =
@@ -187,10 +188,11 @@ void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
                  const double* const* adv, const double* const* advo, const double* phat,
                  const double* const* vis, const double* const* fst, const double* const* fstn, const Fluids& fl,
                  const double* mu, const double* rho, const double* rhon, double* const* E, const double* l1, const double* l2,
-                 const double* phi, double dy, double uwall, double* wallc, const RefineBufs& rb);
+                 const double* phi, double dy, double uwall, double* wallc, const RefineBufs& rb, const FlatFluid& flat);
 // one outer iteration on the corrections; errsum[0] = sum of squared increments
 void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv,
-                          const RefineBufs& rb, double* part, double* errsum);
+                          const RefineBufs& rb, double* part, double* errsum,
+                          const FlatFluid& flat = FlatFluid());
 void solve_small_refine(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const RefineBufs& rb,
                         SorLoop* L, int* log);
 // un = u + d, vn = v + d_v, wn = w + d_w at every point

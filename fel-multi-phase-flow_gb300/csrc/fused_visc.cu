@@ -81,9 +81,9 @@ __global__ void __launch_bounds__(128) k_edges(Grid g, VP p, const double* __res
   exz[c] = b;
   eyz[c] = d;
   if (f.f[0]) {
-    f.f[0][c] = (float)a;
-    f.f[1][c] = (float)b;
-    f.f[2][c] = (float)d;
+    f.f[0][c] = df::d2f(a);
+    f.f[1][c] = df::d2f(b);
+    f.f[2][c] = df::d2f(d);
   }
 }
 
@@ -195,20 +195,65 @@ __global__ void __launch_bounds__(256) k_src_ab(Grid g, SrcK K, SrcIn in, const 
 struct VPS {
   df::D dtinv, dx2, dy2, dz2, dx2x2, dy2x2, dz2x2, grvb, grvp;
 };
-// (four blocks per SM: at the 80 registers it would take, the FP64 pipe is 65 % busy and
-// 872 us go by at 256x128x128; at 64, 777)
-__global__ void __launch_bounds__(256, 4) k_src_ab_e(Grid g, VPS p, VP pv, Fac<double> pd, SrcIn in, const double* __restrict__ mu,
+struct FlatE {
+  const float2* pairs;
+  unsigned char* fluid;
+  int* count;
+  long long rb[2], mb[2];
+};
+// T = 1/(rho00/dt + a_p/2), a_p = ka (sum of two) + kb (..) + kc (..)
+__device__ __forceinline__ df::D diag_e(const VPS& p, df::D r, df::D ka, df::D a, df::D kb, df::D b, df::D kc, df::D c) {
+  using namespace df;
+  const D ap = add(add(mul(ka, a), mul(kb, b)), mul(kc, c));
+  return div(D{1.0f, 0.0f}, add(mul(r, p.dtinv), scale(ap, 0.5f)));
+}
+// FlatFluid's pairs: what the general branch below forms where every density and viscosity
+// it reads is fluid f's
+__global__ void k_flat_pairs(VPS p, Fluids fl, float2* __restrict__ out) {
+  using namespace df;
+  const int f = (int)threadIdx.x;
+  if (f > 1) return;
+  const D R = split_double(f ? fl.rhog : fl.rhol), M = split_double(f ? fl.rmug : fl.rmul);
+  const D R2 = add(R, R), M2 = add(M, M), r = scale(add(R2, R2), 0.25f);
+  const D T[3] = {diag_e(p, r, p.dz2, M2, p.dy2, M2, p.dx2x2, M2), diag_e(p, r, p.dz2, M2, p.dy2x2, M2, p.dx2, M2),
+                  diag_e(p, r, p.dz2x2, M2, p.dy2, M2, p.dx2, M2)};
+  out[4 * f] = make_float2(r.h, r.l);
+  for (int q = 0; q < 3; ++q) out[4 * f + 1 + q] = make_float2(T[q].h, T[q].l);
+}
+// FE.pairs: a warp whose points are each in one fluid takes rho00 and T from there.  Bound
+// by the FP64 pipe (78 operations per cell).  At 256x128x128 872 us with the 80 registers
+// it would take and the FP64 pipe 65 % busy, 777 with 64 (four blocks per SM), 734 with
+// the floats rounded by integer operations (df::d2f) and the pairs of the pure fluids.
+__global__ void __launch_bounds__(256, 4) k_src_ab_e(Grid g, VPS p, VP pv, Fac<double> pd, SrcIn in, FlatE FE,
+                                                  const double* __restrict__ mu,
                                                   const double* __restrict__ exy, const double* __restrict__ exz,
                                                   const double* __restrict__ eyz, ABOut out) {
   using namespace df;
-  const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-  const int k = 1 + (int)blockIdx.z;
+  const Tile tile = warp_tile(g.ni);
+  const int i = 1 + tile.x, j = 1 + tile.y, k = 1 + (int)blockIdx.z;
   if (i > g.ni || j > g.nj) return;
   const long X = 1, Y = g.sy, Z = g.sz;
   const long c = g.at(i, j, k);
+  int f = 2;
+  {
+    auto V = [&](const double* a, long o) { return __ldg(a + c + o); };
+    const double r0 = V(in.rho, 0), m0 = V(mu, 0);
+    const long long rb = __double_as_longlong(r0), mb = __double_as_longlong(m0);
+    const bool flat =
+        same_bits(r0, V(in.rho, X), V(in.rho, Y), V(in.rho, Z), V(in.rhon, 0)) &&
+        same_bits(r0, V(in.rhon, X), V(in.rhon, Y), V(in.rhon, Z), r0) &&
+        same_bits(m0, V(mu, X), V(mu, Y), V(mu, Z), V(exy, 0)) &&
+        same_bits(m0, V(exy, -X), V(exy, -Y), V(exz, 0), V(exz, -X)) &&
+        same_bits(m0, V(exz, -Z), V(eyz, 0), V(eyz, -Y), V(eyz, -Z));
+    if (flat && rb == FE.rb[1] && mb == FE.mb[1]) f = 1;
+    if (flat && rb == FE.rb[0] && mb == FE.mb[0]) f = 0;
+  }
+  if (FE.fluid) {
+    FE.fluid[c] = (unsigned char)f;
+    const int flats = __syncthreads_count(f != 2);
+    if (threadIdx.x == 0 && flats) atomicAdd(FE.count, flats);
+  }
   auto L = [&](const double* a, long o) { return split_double(__ldg(a + c + o)); };
-  const D r0n0 = add(L(in.rho, 0), L(in.rhon, 0)), mu0 = L(mu, 0);
   // rho00 * src; the pressure gradient as cal_grad_prs rounds it
   const double p0 = __ldg(in.phat + c);
   auto rsrc = [&](int q, const double* vel, D r, D grav, long S, double di) {
@@ -218,37 +263,50 @@ __global__ void __launch_bounds__(256, 4) k_src_ab_e(Grid g, VPS p, VP pv, Fac<d
     t = add(t, grav);
     return add(sub(mul(r, t), prs), scale(L(in.vis[q], 0), 0.5f));
   };
-  // A = T/2, B = rs T; A and R = A visn + B - u (FP64) as floats
-  auto store = [&](int q, D r, D ap, D rs, double vn, const double* vel) {
-    const D T = div(D{1.0f, 0.0f}, add(mul(r, p.dtinv), scale(ap, 0.5f)));
+  // A = T/2, B = rs T; A and R = A visn + B - u (FP64) as floats (T.h is the nearest float
+  // of the pair T)
+  auto store = [&](int q, D T, D rs, double vn, const double* vel) {
     const double A = to_double(scale(T, 0.5f)), B = to_double(mul(rs, T));
-    out.af[q][c] = (float)A;
-    out.rf[q][c] = (float)(A * vn + B - __ldg(vel + c));
+    out.af[q][c] = 0.5f * T.h;
+    out.rf[q][c] = d2f(A * vn + B - __ldg(vel + c));
   };
   const D zero{0.0f, 0.0f};
-  {
-    const D r = scale(add(r0n0, add(L(in.rho, X), L(in.rhon, X))), 0.25f);
-    D ap = mul(p.dz2, add(L(exz, -Z), L(exz, 0)));
-    ap = add(ap, mul(p.dy2, add(L(exy, -Y), L(exy, 0))));
-    ap = add(ap, mul(p.dx2x2, add(mu0, L(mu, X))));
-    const double vn = visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
-    store(0, r, ap, rsrc(0, in.u, r, p.grvb, X, pv.dxi), vn, in.u);
-  }
-  if (j <= g.nj - 1) {
-    const D r = scale(add(r0n0, add(L(in.rho, Y), L(in.rhon, Y))), 0.25f);
-    D ap = mul(p.dz2, add(L(eyz, -Z), L(eyz, 0)));
-    ap = add(ap, mul(p.dy2x2, add(mu0, L(mu, Y))));
-    ap = add(ap, mul(p.dx2, add(L(exy, -X), L(exy, 0))));
-    const double vn = visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
-    store(1, r, ap, rsrc(1, in.v, r, p.grvp, Y, pv.dyi), vn, in.v);
-  }
-  {
-    const D r = scale(add(r0n0, add(L(in.rho, Z), L(in.rhon, Z))), 0.25f);
-    D ap = mul(p.dz2x2, add(mu0, L(mu, Z)));
-    ap = add(ap, mul(p.dy2, add(L(eyz, -Y), L(eyz, 0))));
-    ap = add(ap, mul(p.dx2, add(L(exz, -X), L(exz, 0))));
-    const double vn = visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
-    store(2, r, ap, rsrc(2, in.w, r, zero, Z, pv.dzi), vn, in.w);
+  if (__any_sync(__activemask(), f == 2)) {
+    const D r0n0 = add(L(in.rho, 0), L(in.rhon, 0)), mu0 = L(mu, 0);
+    {
+      const D r = scale(add(r0n0, add(L(in.rho, X), L(in.rhon, X))), 0.25f);
+      const D T = diag_e(p, r, p.dz2, add(L(exz, -Z), L(exz, 0)), p.dy2, add(L(exy, -Y), L(exy, 0)), p.dx2x2,
+                         add(mu0, L(mu, X)));
+      const double vn = visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
+      store(0, T, rsrc(0, in.u, r, p.grvb, X, pv.dxi), vn, in.u);
+    }
+    if (j <= g.nj - 1) {
+      const D r = scale(add(r0n0, add(L(in.rho, Y), L(in.rhon, Y))), 0.25f);
+      const D T = diag_e(p, r, p.dz2, add(L(eyz, -Z), L(eyz, 0)), p.dy2x2, add(mu0, L(mu, Y)), p.dx2,
+                         add(L(exy, -X), L(exy, 0)));
+      const double vn = visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
+      store(1, T, rsrc(1, in.v, r, p.grvp, Y, pv.dyi), vn, in.v);
+    }
+    {
+      const D r = scale(add(r0n0, add(L(in.rho, Z), L(in.rhon, Z))), 0.25f);
+      const D T = diag_e(p, r, p.dz2x2, add(mu0, L(mu, Z)), p.dy2, add(L(eyz, -Y), L(eyz, 0)), p.dx2,
+                         add(L(exz, -X), L(exz, 0)));
+      const double vn = visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
+      store(2, T, rsrc(2, in.w, r, zero, Z, pv.dzi), vn, in.w);
+    }
+  } else {
+    auto P = [&](int q) {
+      const float2 t = __ldg(FE.pairs + 4 * f + q);
+      return D{t.x, t.y};
+    };
+    const D r = P(0);
+    store(0, P(1), rsrc(0, in.u, r, p.grvb, X, pv.dxi),
+          visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w), in.u);
+    if (j <= g.nj - 1)
+      store(1, P(2), rsrc(1, in.v, r, p.grvp, Y, pv.dyi),
+            visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w), in.v);
+    store(2, P(3), rsrc(2, in.w, r, zero, Z, pv.dzi),
+          visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w), in.w);
   }
 }
 
@@ -418,32 +476,38 @@ __global__ void __launch_bounds__(256) k_div_stress_e(Grid g, VPT p, const float
 }
 
 // visn of component COMP at point c (solu_sor4.f:150-170 without the A/B factors)
-template <int COMP, class T>
-__device__ __forceinline__ T visn_at(const Grid& g, const Fac<T>& p, long c, const T* __restrict__ mu,
-                                     const T* __restrict__ exy, const T* __restrict__ exz,
-                                     const T* __restrict__ eyz, const T* un, const T* vn, const T* wn) {
+template <int COMP, class T, class M>
+__device__ __forceinline__ T visn_of(const Grid& g, const Fac<T>& p, long c, M coef, const T* un, const T* vn,
+                                     const T* wn) {
   const long X = 1, Y = g.sy, Z = g.sz;
   const T dx2 = p.dx2, dy2 = p.dy2, dz2 = p.dz2, dxy = p.dxy, dxz = p.dxz, dyz = p.dyz;
   auto U = [&](long o) { return un[c + o]; };
   auto V = [&](long o) { return vn[c + o]; };
   auto W = [&](long o) { return wn[c + o]; };
-  auto M = [&](const T* a, long o) { return __ldg(a + c + o); };
+  constexpr int mu = 0, exy = 1, exz = 2, eyz = 3;
   if (COMP == 0) {
-    const T ym = M(exy, -Y), yp = M(exy, 0), zm = M(exz, -Z), zp = M(exz, 0);
+    const T ym = coef(exy, -Y), yp = coef(exy, 0), zm = coef(exz, -Z), zp = coef(exz, 0);
     return dz2 * (zm * U(-Z) + zp * U(Z)) + dy2 * (ym * U(-Y) + yp * U(Y)) +
-           (T)2 * dx2 * (M(mu, 0) * U(-X) + M(mu, X) * U(X)) + dxy * (ym * (V(-Y) - V(X - Y)) + yp * (V(X) - V(0))) +
+           (T)2 * dx2 * (coef(mu, 0) * U(-X) + coef(mu, X) * U(X)) + dxy * (ym * (V(-Y) - V(X - Y)) + yp * (V(X) - V(0))) +
            dxz * (zm * (W(-Z) - W(X - Z)) + zp * (W(X) - W(0)));
   } else if (COMP == 1) {
-    const T xm = M(exy, -X), xp = M(exy, 0), zm = M(eyz, -Z), zp = M(eyz, 0);
-    return dz2 * (zm * V(-Z) + zp * V(Z)) + (T)2 * dy2 * (M(mu, 0) * V(-Y) + M(mu, Y) * V(Y)) +
+    const T xm = coef(exy, -X), xp = coef(exy, 0), zm = coef(eyz, -Z), zp = coef(eyz, 0);
+    return dz2 * (zm * V(-Z) + zp * V(Z)) + (T)2 * dy2 * (coef(mu, 0) * V(-Y) + coef(mu, Y) * V(Y)) +
            dx2 * (xm * V(-X) + xp * V(X)) + dxy * (xm * (U(-X) - U(-X + Y)) + xp * (U(Y) - U(0))) +
            dyz * (zm * (W(-Z) - W(Y - Z)) + zp * (W(Y) - W(0)));
   } else {
-    const T xm = M(exz, -X), xp = M(exz, 0), ym = M(eyz, -Y), yp = M(eyz, 0);
-    return (T)2 * dz2 * (M(mu, 0) * W(-Z) + M(mu, Z) * W(Z)) + dy2 * (ym * W(-Y) + yp * W(Y)) +
+    const T xm = coef(exz, -X), xp = coef(exz, 0), ym = coef(eyz, -Y), yp = coef(eyz, 0);
+    return (T)2 * dz2 * (coef(mu, 0) * W(-Z) + coef(mu, Z) * W(Z)) + dy2 * (ym * W(-Y) + yp * W(Y)) +
            dx2 * (xm * W(-X) + xp * W(X)) + dxz * (xm * (U(-X) - U(-X + Z)) + xp * (U(Z) - U(0))) +
            dyz * (ym * (V(-Y) - V(-Y + Z)) + yp * (V(Z) - V(0)));
   }
+}
+template <int COMP, class T>
+__device__ __forceinline__ T visn_at(const Grid& g, const Fac<T>& p, long c, const T* __restrict__ mu,
+                                     const T* __restrict__ exy, const T* __restrict__ exz,
+                                     const T* __restrict__ eyz, const T* un, const T* vn, const T* wn) {
+  auto coef = [&](int a, long o) { return __ldg((a == 0 ? mu : (a == 1 ? exy : (a == 2 ? exz : eyz))) + c + o); };
+  return visn_of<COMP, T>(g, p, c, coef, un, vn, wn);
 }
 
 // --- the colour-pair sweeps ----------------------------------------------------------
@@ -481,12 +545,27 @@ struct SweepK<double> {
 template <>
 struct SweepK<float> {
   Fac<float> f;
-  SweepK(const VP& p, int, const FlatFluid& = FlatFluid()) : f(p) {}
+  const unsigned char* fluid;
+  const int* count;
+  int enough;
+  float mu[2];
+  SweepK(const VP& p, int, const FlatFluid& flat = FlatFluid())
+      : f(p), fluid(flat.fluid), count(flat.count), enough(flat.enough), mu{(float)flat.mu[0], (float)flat.mu[1]} {}
 };
+// A visn + B of a point in fluid f alone, in FP32: the same operations, the viscosities
+// not read
+template <int COMP>
+__device__ __forceinline__ float flat_sweep(std::true_type, const Grid& g, const SweepK<float>& K, long c, bool f,
+                                            const float* A, float B, const float* un, const float* vn,
+                                            const float* wn) {
+  const float m = f ? K.mu[1] : K.mu[0];
+  const float visn = visn_of<COMP, float>(g, K.f, c, [&](int, long) { return m; }, un, vn, wn);
+  return __ldg(A + c) * visn + B;
+}
 // A visn + B of a point in fluid f alone (A, mu and the edge viscosities constant): 16
 // operations and 16 values read, not 20 and 23
 template <int COMP>
-__device__ __forceinline__ double flat_sweep(std::true_type, const Grid& g, const SweepK<double>& K, long c, bool f, double B,
+__device__ __forceinline__ double flat_sweep(std::true_type, const Grid& g, const SweepK<double>& K, long c, bool f, const double*, double B,
                                              const double* un, const double* vn, const double* wn) {
   const long X = 1, Y = g.sy, Z = g.sz;
   const long S = COMP == 0 ? X : (COMP == 1 ? Y : Z), T1 = COMP == 0 ? Y : X, T2 = COMP == 2 ? Y : Z;
@@ -673,7 +752,7 @@ __global__ void __launch_bounds__(128) k_pair(Grid g, SweepK<T> K, int pi, int p
         const long c = g.at(i, j, k);
         T qn;
         if constexpr (flat.value) {
-          qn = flat_sweep<COMP>(flat, g, K, c, second[hh], __ldg(B + c), un, vn, wn);
+          qn = flat_sweep<COMP>(flat, g, K, c, second[hh], A, __ldg(B + c), un, vn, wn);
         } else {
           const T visn = visn_sweep<COMP>(g, K, c, mu, exy, exz, eyz, un, vn, wn);
           qn = __ldg(A + c) * visn + __ldg(B + c);
@@ -1217,7 +1296,7 @@ __global__ void __launch_bounds__(256) k_halo_z_d(Grid g, int normal, const floa
 // the rest: the other rows of the z-ghost planes of the columns that are not x
 // destinations, one thread per (i, j, component).
 __device__ __forceinline__ void refresh(const Grid& g, int normal, const Ghosts32& G, float* du, float* dv, float* dw,
-                                        int region, long t) {
+                                        int region, long t, int only = -1) {
   const float *__restrict__ gw = G.gw, *__restrict__ gx = G.gx, *__restrict__ gz = G.gz;
   const int shu = !(normal & 1), shw = !(normal & 4);
   const int NI = g.ni, NJ = g.nj, NK = g.nk;
@@ -1244,6 +1323,7 @@ __device__ __forceinline__ void refresh(const Grid& g, int normal, const Ghosts3
     // u and w: q(g1) = c2 q1 + G1, q(g2) = 2 q(g1) - q1 + G2, q(g3) = 2 q(g2) - q(g1) + G3
 #pragma unroll
     for (int cmp = 0; cmp < 3; cmp += 2) {
+      if (only >= 0 && cmp != only) continue;
       const int is = halo_src(i, NI, cmp == 0 ? shu : 0), ks = halo_src(k, NK, cmp == 2 ? shw : 0);
       const float4* G4 = reinterpret_cast<const float4*>(gw + wall_slot(g, side, ks, is) * kGW);
       const float4 a = __ldg(G4), e = __ldg(G4 + 2);
@@ -1256,7 +1336,7 @@ __device__ __forceinline__ void refresh(const Grid& g, int normal, const Ghosts3
       q[g.at(i, jw + 2 * tj, k)] = compose(g2, cmp, is, ks, jw + 2 * tj);
       q[g.at(i, jw + 3 * tj, k)] = compose(g3, cmp, is, ks, jw + 3 * tj);
     }
-    {
+    if (only < 0 || only == 1) {
       const int is = halo_src(i, NI, 0), ks = halo_src(k, NK, 0);
       const float4 bb = __ldg(reinterpret_cast<const float4*>(gw + wall_slot(g, side, ks, is) * kGW) + 1);
       const long c = g.at(is, jw, ks);
@@ -1278,8 +1358,8 @@ __device__ __forceinline__ void refresh(const Grid& g, int normal, const Ghosts3
   }
   if (region == 1) {
     const long task = t;
-    if (task >= 3L * NJ * (NK + 6)) return;
-    const int cmp = (int)(task / ((long)NJ * (NK + 6)));
+    if (task >= (only >= 0 ? 1L : 3L) * NJ * (NK + 6)) return;
+    const int cmp = only >= 0 ? only : (int)(task / ((long)NJ * (NK + 6)));
     const int rem = (int)(task % ((long)NJ * (NK + 6)));
     const int j = 1 + rem % NJ, k = -2 + rem / NJ;
     if (cmp == 1 && j == NJ) return;  // a wall row of v
@@ -1307,7 +1387,8 @@ __device__ __forceinline__ void refresh(const Grid& g, int normal, const Ghosts3
   const int i = 1 + (int)(t % (NI + 1));
   const long r = t / (NI + 1);
   const int j = 1 + (int)(r % NJ);
-  const int cmp = (int)(r / NJ);
+  const int cmp = only >= 0 ? only : (int)(r / NJ);
+  if (only >= 0 && r >= NJ) return;
   if (cmp >= 3 || (cmp == 1 && j == NJ)) return;
   const int sx = cmp == 0 ? shu : 0, sz = cmp == 2 ? shw : 0;
   if (halo_src(i, NI, sx) != i) return;  // an x-ghost column: done above
@@ -1327,6 +1408,13 @@ __device__ __forceinline__ void refresh(const Grid& g, int normal, const Ghosts3
 // threads of the three regions: the wall rows, the x-ghost columns, the z-ghost planes
 __host__ __device__ __forceinline__ long refresh_tasks(const Grid& g, int region) {
   return region == 0 ? 2L * (g.ni + 6) * (g.nk + 6) : (region == 1 ? 3L * g.nj * (g.nk + 6) : 3L * (g.ni + 1) * g.nj);
+}
+// (the FP32 corrections' refresh of one component only)
+__global__ void __launch_bounds__(256) k_refresh_one(Grid g, int comp, Ghosts32 gh, float* du, float* dv, float* dw,
+                                                     int nbW, int nbX) {
+  const int b = (int)blockIdx.x, region = b < nbW ? 0 : (b < nbW + nbX ? 1 : 2);
+  refresh(g, 1 << comp, gh, du, dv, dw, region,
+          (long)(b - (region > 0 ? nbW : 0) - (region > 1 ? nbX : 0)) * 256 + threadIdx.x, comp);
 }
 template <class T, class G>
 __global__ void __launch_bounds__(256) k_refresh(Grid g, int normal, G gh, T* uk, T* vk, T* wk, int nbW, int nbX) {
@@ -1515,21 +1603,23 @@ struct PairShape {
 // the launch and one warp's chain, so two-warp blocks and one point per thread, the two
 // colours apart.  FP64 beyond: the FP64 pipe, with both colours in a thread for the rows
 // they share and, on the largest, 4 planes per thread (fewer sums and partials).  FP32:
-// memory, so both colours together once the fields leave L2, and on the sizes between the
-// ghosts refreshed apart (the sweep's own scattered writes cost it more there than the
-// launches).  One outer iteration, us, as
+// memory, so both colours together once the fields leave L2, and beyond the ghosts
+// refreshed apart, the swept component's alone (the sweep's own scattered writes cost it
+// more there than the launches).  One outer iteration, us, as
 // (block, both or split, planes): FP64 32x32x16 (64, s, 1) 92, (64, b, 1) 115; 128x64x64
 // (64, s, 1) 162, (64, b, 1) 147, (128, b, 4) 224; 256x128x128 (64, b, 1) 677, (128, b, 4)
-// 655; 512x256x256 4267, 4086.  FP32 32x32x16 (64, s, 1) 97, (64, b, 1) 116; 256x128x128
-// 405, 415, (64, s, 1) with the refresh apart 393; 512x256x256 2598, 2115, (128, b, 1) 2104.
+// 655; 512x256x256 4267, 4086.  FP32, g: with the ghosts: 128x64x64 (64, s, 1) g 122,
+// (64, b, 1) g 131, (64, b, 1) 154; 256x64x64 g 152, (128, b, 1) g 145, (64, b, 1) 159;
+// 256x128x64 (FLAT, a drop) g 224, (64, b, 1) 205; 256x128x128 (64, s, 1) 342, (64, b, 1)
+// 311, (128, b, 2) 319, g 358; 512x256x256 1779, 1661, 1606, g 1696.
 PairShape pair_shape(const Grid& g, bool fp64) {
   PairShape p;
   const long n = g.cells();
-  p.both = n >= (fp64 ? 1L << 18 : 1L << 23);
-  p.kz = fp64 && n >= 1L << 21 ? 4 : 1;
-  p.ghosts = fp64 || n < 1L << 20 || n >= 1L << 23;
-  const int nt = n >= (fp64 ? 1L << 21 : 1L << 23) ? 128 : 64;
-  p.flat = fp64 && flat_sweeps(g);
+  p.both = n >= (fp64 ? 1L << 18 : 1L << 20);
+  p.kz = fp64 && n >= 1L << 21 ? 4 : (!fp64 && n >= 1L << 23 ? 2 : 1);
+  p.ghosts = fp64 || n < 1L << 21;
+  const int nt = n >= (fp64 ? 1L << 21 : 1L << 23) || (!fp64 && p.both && p.ghosts) ? 128 : 64;
+  p.flat = flat_sweeps(g);
   const int bx = std::min(32, g.ni / 2), by = nt / bx;
   p.block = dim3((unsigned)bx, (unsigned)by);
   const int rows = (g.nj / 2 + by - 1) / by, planes = (g.nk / 2 + p.kz - 1) / p.kz;
@@ -1538,6 +1628,21 @@ PairShape pair_shape(const Grid& g, bool fp64) {
 }
 // first colour of each pair (solu_sor4.f:94-120): (1,1,1) (1,1,2) (1,2,1) (2,1,1)
 const int kPi[4] = {1, 1, 1, 2}, kPj[4] = {1, 1, 2, 1}, kPk[4] = {1, 2, 1, 1};
+
+VPS make_vps(const VP& p, double grvb, double grvp) {
+  using df::split_double;
+  VPS ps;
+  ps.dtinv = split_double(p.dtinv);
+  ps.dx2 = split_double(p.dx2);
+  ps.dy2 = split_double(p.dy2);
+  ps.dz2 = split_double(p.dz2);
+  ps.dx2x2 = split_double(2.0 * p.dx2);
+  ps.dy2x2 = split_double(2.0 * p.dy2);
+  ps.dz2x2 = split_double(2.0 * p.dz2);
+  ps.grvb = split_double(grvb);
+  ps.grvp = split_double(grvp);
+  return ps;
+}
 
 // A of component t in a fluid of density r and viscosity m
 double fluid_a(const VP& p, double r, double m, int t) {
@@ -1572,19 +1677,17 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
   k_edges<<<tile_grid(g.ni + 1, g.nj + 1, g.nk + 1, 128), 128, 0, s>>>(
       g, p, mu, E[0], E[1], E[2], ef, flat.count);
   if (REFINE) {
-    using df::split_double;
-    VPS ps;
-    ps.dtinv = split_double(p.dtinv);
-    ps.dx2 = split_double(p.dx2);
-    ps.dy2 = split_double(p.dy2);
-    ps.dz2 = split_double(p.dz2);
-    ps.dx2x2 = split_double(2.0 * p.dx2);
-    ps.dy2x2 = split_double(2.0 * p.dy2);
-    ps.dz2x2 = split_double(2.0 * p.dz2);
-    ps.grvb = split_double(grvb);
-    ps.grvp = split_double(grvp);
-    k_src_ab_e<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, ps, p, Fac<double>(p), in, mu, E[0], E[1],
-                                                                                 E[2], out);
+    FlatE FE;
+    FE.pairs = flat.pairs;
+    FE.fluid = flat.fluid;
+    FE.count = flat.count;
+    const double rf[2] = {fl.rhol, fl.rhog}, mf[2] = {fl.rmul, fl.rmug};
+    for (int q = 0; q < 2; ++q) {
+      std::memcpy(&FE.rb[q], &rf[q], sizeof(double));
+      std::memcpy(&FE.mb[q], &mf[q], sizeof(double));
+    }
+    k_src_ab_e<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, make_vps(p, grvb, grvp), p, Fac<double>(p), in, FE,
+                                                                mu, E[0], E[1], E[2], out);
   } else {
     SrcK K;
     K.hdt = 0.5 * p.dtinv;
@@ -1644,24 +1747,13 @@ void sweep_all(cudaStream_t s, const Grid& g, const VP& p, const T* mu, const T*
       };
       constexpr std::true_type yes;
       constexpr std::false_type no;
-      bool done = false;
-      if constexpr (sizeof(T) == 8) {
-        if (sp.flat && flat.fluid) {  // (with both colours in a thread: sizes, pair_shape)
-          own ? pair(yes, yes, yes) : pair(no, yes, yes);
-          done = true;
-        }
-      }
-      if (done) {
-      } else if (own && sp.both) {
-        pair(yes, yes, no);
-      } else if (own) {
-        pair(yes, no, no);
-      } else if (sp.both) {
-        pair(no, yes, no);
-      } else {
-        pair(no, no, no);
-      }
-      if (!own) halo(1 << comp);
+      auto kinds = [&](auto fl) {  // (FLAT's sizes have both colours in a thread)
+        if (own && sp.both) pair(yes, yes, fl);
+        else if (sp.both) pair(no, yes, fl);
+        else if constexpr (!fl.value) own ? pair(yes, no, fl) : pair(no, no, fl);
+      };
+      sp.flat && flat.fluid ? kinds(yes) : kinds(no);
+      if (!own) halo(1 << comp, pr == 0);
     }
   }
   if (!errsum) return;
@@ -1687,11 +1779,18 @@ void src_visc_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
 
 // (below, a plane's loads no longer hide the bytes': 64x64x64 119 us without, 124 with)
 bool flat_sweeps(const Grid& g) { return g.cells() >= 1L << 21; }
-FlatFluid make_flat(const Grid& g, double dxinv, double dyinv, double dzinv, double dt, const Fluids& fl,
-                    unsigned char* bytes) {
+FlatFluid make_flat(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt,
+                    const Fluids& fl, unsigned char* bytes, bool mixed) {
   FlatFluid f;
-  if (!bytes || !flat_sweeps(g)) return f;
+  if (!bytes) return f;
   const VP p = make_vp(dxinv, dyinv, dzinv, dt, 0);
+  if (mixed) {
+    float2* pairs = (float2*)(bytes + g.n + 8);  // (g.n is a multiple of 8)
+    k_flat_pairs<<<1, 32, 0, s>>>(make_vps(p, 0.0, 0.0), fl, pairs);
+    count_launch();
+    f.pairs = pairs;
+  }
+  if (!flat_sweeps(g)) return f;
   f.fluid = bytes;
   f.count = (int*)(bytes + g.n);
   f.enough = (int)(g.cells() - g.cells() / 10);
@@ -1769,7 +1868,7 @@ void sor_iteration(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
   double* const B[3] = {AB[1], AB[3], AB[5]};
   sweep_all<double>(s, g, make_vp(dxinv, dyinv, dzinv, 0.0, harmonic), mu, E[0], E[1], E[2], A, B, un, vn, wn,
                     Ghosts64{uwall, wallc}, part, errsum,
-                    [&](int normal) { wall_halo(s, g, normal, uwall, wallc, un, vn, wn); }, flat, before);
+                    [&](int normal, bool) { wall_halo(s, g, normal, uwall, wallc, un, vn, wn); }, flat, before);
 }
 
 __global__ void k_sor_rule(SorLoop* L, double tol, int maxit, double cells) {
@@ -1854,7 +1953,8 @@ void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
                  const double* const* adv, const double* const* advo, const double* phat,
                  const double* const* vis, const double* const* fst, const double* const* fstn, const Fluids& fl,
                  const double* mu, const double* rho, const double* rhon, double* const* E, const double* l1, const double* l2,
-                 const double* phi, double dy, double uwall, double* wallc, const RefineBufs& rb) {
+                 const double* phi, double dy, double uwall, double* wallc, const RefineBufs& rb,
+                 const FlatFluid& flat) {
   ABOut out{};
   for (int q = 0; q < 3; ++q) {
     out.af[q] = rb.a[q];
@@ -1862,7 +1962,7 @@ void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
   }
   // A and B in FP32 pairs, the residual in FP64 (k_src_ab_e)
   src_prep<true>(s, g, make_vp(dxinv, dyinv, dzinv, dt, harmonic), u, v, w, adv, advo, phat, vis, fst, fstn, grvb,
-                 grvp, fl, mu, rho, rhon, E, F3{{rb.e[0], rb.e[1], rb.e[2]}}, out, l1, l2, phi, dy, wallc);
+                 grvp, fl, mu, rho, rhon, E, F3{{rb.e[0], rb.e[1], rb.e[2]}}, out, l1, l2, phi, dy, wallc, flat);
   k_to_float<<<4 * 152, 256, 0, s>>>(g.n, mu, rb.mu);
   k_gamma_wall<<<wall_grid(g), kB, 0, s>>>(g, uwall, wallc, u, v, w, rb.gw);
   k_gamma_x<<<xh_grid(g), kB, 0, s>>>(g, u, v, w, rb.gx);
@@ -1872,12 +1972,20 @@ void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
 }
 
 void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv,
-                          const RefineBufs& rb, double* part, double* errsum) {
+                          const RefineBufs& rb, double* part, double* errsum, const FlatFluid& flat) {
   float *du = rb.d[0], *dv = rb.d[1], *dw = rb.d[2];
   sweep_all<float>(
       s, g, make_vp(dxinv, dyinv, dzinv, 0.0, 0), rb.mu, rb.e[0], rb.e[1], rb.e[2], rb.a, rb.r, du, dv, dw,
       Ghosts32{rb.gw, rb.gx, rb.gz}, part, errsum,
-      [&](int normal) {
+      [&](int normal, bool first) {
+        if (one_pass_refresh(g) && !first) {  // the swept component's ghosts alone change
+          const int nbW = (int)((refresh_tasks(g, 0) + 255) / 256), nbX = (int)((refresh_tasks(g, 1) / 3 + 255) / 256),
+                    nbZ = (int)((refresh_tasks(g, 2) / 3 + 255) / 256);
+          k_refresh_one<<<nbW + nbX + nbZ, 256, 0, s>>>(g, normal >> 1, Ghosts32{rb.gw, rb.gx, rb.gz}, du, dv, dw, nbW,
+                                                        nbX);
+          count_launch();
+          return;
+        }
         if (one_pass_refresh(g)) {
           const long tw = refresh_tasks(g, 0), tx = refresh_tasks(g, 1), tz = refresh_tasks(g, 2);
           const int nbW = (int)((tw + 255) / 256), nbX = (int)((tx + 255) / 256), nbZ = (int)((tz + 255) / 256);
@@ -1889,7 +1997,8 @@ void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dy
         k_halo_x_d<<<xh_grid(g), kB, 0, s>>>(g, normal, rb.gx, du, dv, dw);
         k_halo_z_d<<<zh_grid(g), kB, 0, s>>>(g, normal, rb.gz, du, dv, dw);
         count_launch(3);
-      });
+      },
+      flat);
 }
 
 void refine_finish(cudaStream_t s, const Grid& g, const double* u, const double* v, const double* w,

@@ -273,10 +273,6 @@ int fmf_ctx_create(const fmf_params* prm, fmf_ctx** out) {
   for (int q = 0; q < 3; ++q) c->edge[q] = alloc(c, n);
   for (int q = 0; q < 6; ++q) c->ab[q] = alloc(c, n);
   c->wallc = alloc(c, 4L * (prm->nk + 6) * (prm->ni + 6));
-  if (!c->mixed && fused::flat_sweeps(c->g))
-    c->flat = fused::make_flat(c->g, 1.0 / prm->dx, 1.0 / prm->dy, 1.0 / prm->dz, prm->dt,
-                               fused::Fluids{prm->rhol, prm->rhog, prm->rmul, prm->rmug},
-                               (unsigned char*)alloc(c, (fused::flat_bytes(c->g) + 7) / 8));
   c->sorpart = alloc(c, fused::sor_parts(c->g));
   c->pr = alloc(c, nm);
   c->pi = alloc(c, nm);
@@ -300,6 +296,10 @@ int fmf_ctx_create(const fmf_params* prm, fmf_ctx** out) {
     rb.gz = allocf(c, fused::refine_floats(c->g, 2));
     c->wsplit = (float2*)alloc(c, 6 * n);
   }
+  if (c->mixed || fused::flat_sweeps(c->g))
+    c->flat = fused::make_flat(c->s, c->g, 1.0 / prm->dx, 1.0 / prm->dy, 1.0 / prm->dz, prm->dt,
+                               fused::Fluids{prm->rhol, prm->rhog, prm->rmul, prm->rmug},
+                               (unsigned char*)alloc(c, (fused::flat_bytes(c->g) + 7) / 8), c->mixed);
   c->wprec = c->mixed ? 1 : prm->precision == FMF_FP64E ? 2 : 0;
   if (c->wprec == 2) c->wsplit = (float2*)alloc(c, 6 * n);
   {
@@ -580,7 +580,7 @@ static void seg_pre2(fmf_ctx* c) {
     // un = u (:605-607) holds implicitly through zero corrections
     fused::refine_prep(s, g, dxinv, dyinv, dzinv, dt, P.harmonic, P.grvb, P.grvp, c->u, c->v, c->w, advp, advop,
                        c->phat, visp, fstp, fstnp, fl, c->rmun, c->rho, c->rhon, c->edge, c->l1, c->l2, phi1, P.dy, P.uwall,
-                       c->wallc, c->rb);
+                       c->wallc, c->rb, c->flat);
     return;
   }
   fused::src_visc_prep(s, g, dxinv, dyinv, dzinv, dt, P.harmonic, P.grvb, P.grvp, c->u, c->v, c->w, advp, advop,
@@ -622,7 +622,7 @@ static void iter_kernels(fmf_ctx* c) {
   const fmf_params& P = c->prm;
   const double dxinv = 1.0 / P.dx, dyinv = 1.0 / P.dy, dzinv = 1.0 / P.dz;
   if (c->mixed)
-    fused::sor_iteration_refine(c->s, c->g, dxinv, dyinv, dzinv, c->rb, c->sorpart, c->red + 8);
+    fused::sor_iteration_refine(c->s, c->g, dxinv, dyinv, dzinv, c->rb, c->sorpart, c->red + 8, c->flat);
   else
     fused::sor_iteration(c->s, c->g, dxinv, dyinv, dzinv, P.harmonic, c->rmun, c->edge, c->ab, P.uwall, c->wallc,
                          c->un, c->vn, c->wn, c->sorpart, c->red + 8, c->flat);
@@ -881,7 +881,7 @@ int fmf_ctx_time_stage(fmf_ctx* c, int stage, int reps, float* ms) {
         break;
       case 1:
         if (mixed)
-          fused::sor_iteration_refine(s, g, dxinv, dyinv, dzinv, c->rb, c->sorpart, c->red + 8);
+          fused::sor_iteration_refine(s, g, dxinv, dyinv, dzinv, c->rb, c->sorpart, c->red + 8, c->flat);
         else
           fused::sor_iteration(s, g, dxinv, dyinv, dzinv, P.harmonic, c->rmun, c->edge, c->ab, P.uwall, c->wallc,
                                c->un, c->vn, c->wn, c->sorpart, c->red + 8, c->flat);

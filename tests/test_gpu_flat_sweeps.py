@@ -1,5 +1,6 @@
-"""The FP64 colour-pair sweeps of warps in one fluid (2^21 cells and more, nine tenths of
-them away from the interface) against the oracle: a drop in a box of 256x128x64."""
+"""The colour-pair sweeps and momentum factors of warps in one fluid (2^21 cells and more,
+nine tenths of them away from the interface) against the oracle: a drop in a box of
+256x128x64."""
 import numpy as np
 import pytest
 
@@ -29,3 +30,18 @@ def test_flat_sweeps(orc, fmf_lib, precision):
     for f, name in enumerate(C.STATE_FIELDS):
         err = np.abs(got[f] - st[f]).max() / max(np.abs(st[f]).max(), 1e-30)
         assert err <= 1e-10, (name, err)
+
+
+def test_flat_sweeps_mixed(orc, fmf_lib):
+    """The mixed-precision step on the same box: within its 1e-5 of the oracle."""
+    cfg = C.get("droplet256", ni=256, nj=128, nk=64)
+    s, st = _start(orc, cfg, 5)
+    g = capi.Stepper(cfg, capi.FMF_MIXED)
+    g.upload(st)
+    g.step(2)
+    got = g.get_state()
+    g.close()
+    s.step(st, 2)
+    for f, name in enumerate(C.STATE_FIELDS):
+        err = np.abs(got[f] - st[f]).max() / max(np.abs(st[f]).max(), 1e-30)
+        assert err <= 1e-5, (name, err)
