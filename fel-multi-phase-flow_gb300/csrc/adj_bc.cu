@@ -550,7 +550,7 @@ void grad_p2a_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dz
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
           p[q][t] = L[q][-(t & 1 ? 1 : 0) - (t & 2 ? G.sy : 0) - (t & 4 ? G.sz : 0)];
-          any |= (unsigned long long)__double_as_longlong(p[q][t]) << 1;
+          any |= (unsigned long long)raw(p[q][t]) << 1;
         }
       if (!__any_sync(__activemask(), any != 0)) return;  // away from the interface
       const double sx = ((p[0][1] - p[0][0]) + (p[0][3] - p[0][2])) + ((p[0][5] - p[0][4]) + (p[0][7] - p[0][6]));

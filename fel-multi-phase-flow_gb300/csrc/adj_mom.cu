@@ -78,8 +78,8 @@ __device__ double wline_T(const double* __restrict__ q, long c, long S, double v
   for (int m = 0; m < 6; ++m) lD[m] = 0.0;
   const double lr = lout * di;
   // zero and sign tested on the bits (no FP64-pipe comparison)
-  if ((__double_as_longlong(lr) << 1) == 0) return 0.0;
-  const long long vb = __double_as_longlong(vel);
+  if ((raw(lr) << 1) == 0) return 0.0;
+  const long long vb = raw(vel);
   Walk A;
   if ((vb << 1) == 0) {
     // both sides enter d(out)/d(vel) of weno5.h, (R_minus + R_plus)/12, where the
@@ -234,8 +234,8 @@ __device__ double wline_T_df(const double* __restrict__ q, long c, long S, doubl
                              double* lD) {
   for (int m = 0; m < 6; ++m) lD[m] = 0.0;
   const double lr = lout * di;
-  if ((__double_as_longlong(lr) << 1) == 0) return 0.0;
-  const long long vb = __double_as_longlong(vel);
+  if ((raw(lr) << 1) == 0) return 0.0;
+  const long long vb = raw(vel);
   WalkP A;
   if ((vb << 1) == 0) {
     WalkP B;
@@ -610,7 +610,7 @@ void csf_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, do
         const int d = t < 8 ? t : ((t - 8) % 2 == 0 ? 0 : (f == 1 ? 4 : (f == 2 ? 2 : 1)));
         const bool on = (!(d & 1) || X) && (!(d & 2) || Y) && (!(d & 4) || Z);
         p[q][t] = on ? lv[(3 * f + q) * n + c + (d & 1 ? X : 0) + (d & 2 ? Y : 0) + (d & 4 ? Z : 0)] : 0.0;
-        any |= (unsigned long long)__double_as_longlong(p[q][t]) << 1;
+        any |= (unsigned long long)raw(p[q][t]) << 1;
       }
     }
     if (!__any_sync(__activemask(), any != 0)) {

@@ -369,7 +369,7 @@ struct CsfD {
 // patterns: all are non-negative); s = 0 gives 0 (the components it multiplies are 0 or
 // their squares underflowed), other small s the exact expression.
 __device__ __forceinline__ double inv_norm(double s, double vs, double big) {
-  if (__double_as_longlong(s) > __double_as_longlong(big)) return rsqrt_h(s);
+  if (raw(s) > raw(big)) return rsqrt_h(s);
   return mag(s) == 0 ? 0.0 : 1.0 / (sqrt(s) + vs);
 }
 
@@ -386,8 +386,8 @@ __global__ void __launch_bounds__(128) k_csf_grad(Grid g, CsfD p, const double* 
                qpp0 = __ldg(phi + c + X + Y), q00p = __ldg(phi + c + Z), qp0p = __ldg(phi + c + X + Z),
                q0pp = __ldg(phi + c + Y + Z), qppp = __ldg(phi + c + X + Y + Z);
   // all eight equal in every bit and finite: the gradient is 0
-  const long long r = __double_as_longlong(q000);
-  auto df = [&](double x) { return (unsigned long long)(__double_as_longlong(x) ^ r); };
+  const long long r = raw(q000);
+  auto df = [&](double x) { return (unsigned long long)(raw(x) ^ r); };
   const bool varies = (df(qp00) | df(q0p0) | df(qpp0) | df(q00p) | df(qp0p) | df(q0pp) | df(qppp)) != 0 ||
                       !finite_bits(r);
   if (!__any_sync(__activemask(), varies)) {
@@ -511,9 +511,9 @@ __global__ void __launch_bounds__(256) k_csf_force(Grid g, CsfD p, const double*
   const long X = 1, Y = g.sy, Z = g.sz, n = g.n;
   const long c = g.at(i, j, 1 + (int)blockIdx.z);
   const double ph = __ldg(phi + c), px = __ldg(phi + c + X), py = __ldg(phi + c + Y), pz = __ldg(phi + c + Z);
-  const long long r = __double_as_longlong(ph);
-  const bool varies = ((__double_as_longlong(px) ^ r) | (__double_as_longlong(py) ^ r) |
-                       (__double_as_longlong(pz) ^ r)) != 0 || !finite_bits(r);
+  const long long r = raw(ph);
+  const bool varies = ((raw(px) ^ r) | (raw(py) ^ r) |
+                       (raw(pz) ^ r)) != 0 || !finite_bits(r);
   if (!__any_sync(__activemask(), varies)) {
     fu[c] = 0.0;
     fv[c] = 0.0;

@@ -96,9 +96,9 @@ struct G8 {
 __device__ __forceinline__ bool outside_band(const G8& gx, const G8& gy, const G8& gz, const MC& m) {
   const double x = gx.mean(), y = gy.mean(), z = gz.mean();
   const double q2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
-  const long long qb = __double_as_longlong(q2);
-  return qb < __double_as_longlong(m.lim2lo) ? true
-                                             : (qb > __double_as_longlong(m.lim2hi) ? false : sqrt(q2) <= m.lim);
+  const long long qb = raw(q2);
+  return qb < raw(m.lim2lo) ? true
+                                             : (qb > raw(m.lim2hi) ? false : sqrt(q2) <= m.lim);
 }
 
 __device__ __forceinline__ double avg8(const double* __restrict__ p, long c, long X, long Y, long Z) {
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double*
   // One product per axis, of the velocity that donates, and a second where a lane donates
   // both ways, formed by the whole warp (stores under their lanes' signs alone: products
   // under them were issued per set of lanes, 15 slots of the FP64 pipe for 3 products).
-  const long long pb = __double_as_longlong(phi00);
+  const long long pb = raw(phi00);
   double pdx = 0.0, pdy = 0.0, pdz = 0.0;
   const bool filled = __any_sync(warp, pb != 0);
   if (filled) {
@@ -300,7 +300,9 @@ __global__ void __launch_bounds__(128) k_band_f32(Grid g, MC m, const double* __
 //  * A step below 1e-9 (1 + |d|) is the last: Newton's error squares per step and leaves
 //    the root to rounding, where the ten steps of solphi_mthinc1.f dither.
 //  * The exponentials have small arguments: exp16 below.
-// 1.57 -> 1.06 ms at 512x256x256, 317 -> 190 us at 128x64x64, 63 -> 45 at 32x32x16.
+//  * One pass per axis for the faces of both sides: lanes of unlike velocity share it.
+// 1.57 -> 0.96 ms at 512x256x256, 317 -> 182 us at 128x64x64, 63 -> 45 at 32x32x16 (the last
+// of these 616 -> 543 us of the couette 256x128x128).
 // Sixteenths: exp(k/16), k = -64 .. 64, formed on the host.
 struct Exp16 {
   double t[129];
@@ -383,30 +385,35 @@ __global__ void __launch_bounds__(64) k_band(Grid g, MC m, __grid_constant__ con
     }
     const double uw = __ldg(u + c - X), ue = __ldg(u + c), vs = __ldg(v + c - Y), vn = __ldg(v + c),
                  wb = __ldg(w + c - Z), wt = __ldg(w + c);
-    // the flux through one face (low: the west, south or bottom one) along an axis with
-    // b, k0, k1: the Gauss points of the swept interval lie vd (1/2 +/- gp) from the face
-    auto side = [&](double vel, double dtd, double bb, double k0, double k1, bool low, double* out) {
-      const double vd = vel * dtd;
-      double s = 0.0;
+    // the fluxes along an axis with b, k0, k1 through the low face (west, south, bottom) where
+    // its velocity is negative and the high one where its is positive: the Gauss points of the
+    // swept interval lie |vd| (1/2 + gp) inside the face, the high face's mirrored (-b).  One
+    // pass for the lanes that donate, through either, and another where one does through both.
+    auto axis = [&](double lo, double hi, double dtd, double bb, double k0, double k1, double* flo, double* fhi) {
+      const bool dl = raw(lo) < 0 && mag(lo) != 0, dh = raw(hi) > 0;
+      bool high = dh, on = dl || dh;
+#pragma unroll 1
+      for (int pass = 0; pass < 2; ++pass) {
+        if (on) {
+          const double vd = (high ? hi : lo) * dtd, bs = high ? -bb : bb, av = fabs(vd);
+          double s = 0.0;
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const double gp = t ? m.gp2 : m.gp1;
-        const double o = low ? fma(-vd, 0.5 + gp, -0.5) : fma(vd, gp - 0.5, 0.5);
-        const double f = y * exp16(T, bb * o);
-        const double a = k0 * f, d = k1 * f;
-        s = fma(2.0 + a, recip_ge1(fma(f, f, 1.0 + a)), s);
-        s = fma(2.0 + d, recip_ge1(fma(f, f, 1.0 + d)), s);
+          for (int t = 0; t < 2; ++t) {
+            const double f = y * exp16(T, bs * fma(av, 0.5 + (t ? m.gp2 : m.gp1), -0.5));
+            const double a = k0 * f, d = k1 * f;
+            s = fma(2.0 + a, recip_ge1(fma(f, f, 1.0 + a)), s);
+            s = fma(2.0 + d, recip_ge1(fma(f, f, 1.0 + d)), s);
+          }
+          *(high ? fhi : flo) = 0.125 * vd * s;
+        }
+        on = dl && dh;
+        high = false;
+        if (!__any_sync(__activemask(), on)) break;
       }
-      *out = 0.125 * vd * s;
     };
-    auto neg = [](double x) { return __double_as_longlong(x) < 0 && mag(x) != 0; };
-    auto pos = [](double x) { return __double_as_longlong(x) > 0; };
-    if (neg(uw)) side(uw, m.dtdx, b[0], kx0, kx1, true, fx + c - X);
-    if (pos(ue)) side(ue, m.dtdx, b[0], kx0, kx1, false, fx + c);
-    if (neg(vs)) side(vs, m.dtdy, b[1], ky0, ky1, true, fy + c - Y);
-    if (pos(vn)) side(vn, m.dtdy, b[1], ky0, ky1, false, fy + c);
-    if (neg(wb)) side(wb, m.dtdz, b[2], kz0, kz1, true, fz + c - Z);
-    if (pos(wt)) side(wt, m.dtdz, b[2], kz0, kz1, false, fz + c);
+    axis(uw, ue, m.dtdx, b[0], kx0, kx1, fx + c - X, fx + c);
+    axis(vs, vn, m.dtdy, b[1], ky0, ky1, fy + c - Y, fy + c);
+    axis(wb, wt, m.dtdz, b[2], kz0, kz1, fz + c - Z, fz + c);
   }
 }
 // cal_grad_p2a.f:46-60 for the fused step: the vertex gradient at (i+1/2, j+1/2,
@@ -429,11 +436,11 @@ __global__ void __launch_bounds__(128) k_vertex_grad(Grid g, double cx, double c
   const double q000 = __ldg(q + c), qp00 = __ldg(q + c + X), q0p0 = __ldg(q + c + Y), qpp0 = __ldg(q + c + X + Y),
                q00p = __ldg(q + c + Z), qp0p = __ldg(q + c + X + Z), q0pp = __ldg(q + c + Y + Z),
                qppp = __ldg(q + c + X + Y + Z);
-  const long long r = __double_as_longlong(q000);
-  auto df = [&](double x) { return (unsigned long long)(__double_as_longlong(x) ^ r); };
+  const long long r = raw(q000);
+  auto df = [&](double x) { return (unsigned long long)(raw(x) ^ r); };
   bool flat = (df(qp00) | df(q0p0) | df(qpp0) | df(q00p) | df(qp0p) | df(q0pp) | df(qppp)) == 0 && finite_bits(r);
   if (NEAR1) {
-    auto below = [&](double x) { return (unsigned long long)(kOneBits - __double_as_longlong(x)); };
+    auto below = [&](double x) { return (unsigned long long)(kOneBits - raw(x)); };
     flat = flat || (below(q000) | below(qp00) | below(q0p0) | below(qpp0) | below(q00p) | below(qp0p) | below(q0pp) |
                     below(qppp)) < 64;
   }

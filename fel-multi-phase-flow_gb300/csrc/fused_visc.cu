@@ -43,9 +43,9 @@ struct VP {
 
 // whether five doubles have the same bits
 __device__ __forceinline__ bool same_bits(double a, double b, double c, double d, double e) {
-  const long long r = __double_as_longlong(a);
-  return ((__double_as_longlong(b) ^ r) | (__double_as_longlong(c) ^ r) | (__double_as_longlong(d) ^ r) |
-          (__double_as_longlong(e) ^ r)) == 0;
+  const long long r = raw(a);
+  return ((raw(b) ^ r) | (raw(c) ^ r) | (raw(d) ^ r) |
+          (raw(e) ^ r)) == 0;
 }
 __device__ __forceinline__ double mean4(double a, double b, double c, double d, int harm) {
   if (!harm) return 0.25 * (a + b + c + d);
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256) k_src_ab(Grid g, SrcK K, SrcIn in, const 
   const double m0 = L(mu, 0), mx = L(mu, X), my = L(mu, Y), mz = L(mu, Z);
   const double xy0 = L(exy, 0), xyx = L(exy, -X), xyy = L(exy, -Y), xz0 = L(exz, 0), xzx = L(exz, -X),
                xzz = L(exz, -Z), yz0 = L(eyz, 0), yzy = L(eyz, -Y), yzz = L(eyz, -Z);
-  const long long rb = __double_as_longlong(r0), mb = __double_as_longlong(m0);
+  const long long rb = raw(r0), mb = raw(m0);
   const bool flat = same_bits(r0, rx, ry, rz, n0) && same_bits(r0, nx, ny, nz, r0) && same_bits(m0, mx, my, mz, xy0) &&
                     same_bits(m0, xyx, xyy, xz0, xzx) && same_bits(m0, xzz, yz0, yzy, yzz);
   const int f = flat && rb == K.rb[0] && mb == K.mb[0] ? 0 : (flat && rb == K.rb[1] && mb == K.mb[1] ? 1 : -1);
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(256, 4) k_src_ab_e(Grid g, VPS p, VP pv, Fac<d
   {
     auto V = [&](const double* a, long o) { return __ldg(a + c + o); };
     const double r0 = V(in.rho, 0), m0 = V(mu, 0);
-    const long long rb = __double_as_longlong(r0), mb = __double_as_longlong(m0);
+    const long long rb = raw(r0), mb = raw(m0);
     const bool flat =
         same_bits(r0, V(in.rho, X), V(in.rho, Y), V(in.rho, Z), V(in.rhon, 0)) &&
         same_bits(r0, V(in.rhon, X), V(in.rhon, Y), V(in.rhon, Z), r0) &&

@@ -12,6 +12,7 @@
 #include <cstring>
 
 #include "../../include/fmf_capi.h"
+#include "bits.cuh"
 #include "fused.cuh"
 #include "recip.cuh"
 #include "weno5_df.cuh"
@@ -246,7 +247,8 @@ __global__ void __launch_bounds__(128) k_weno2_df(Grid g, int nlev, const int* _
 // whose lanes lie along j, the second and third pass over adv) hides behind it.  32
 // FP64 operations per derivative, 288 per cell, against 484 with one thread per cell
 // and its nine stencils: 30.85 -> 19.3 ms at 512x256x256, 3.86 -> 2.51 at 256x128x128,
-// 0.488 -> 0.344 at 128x64x64, the pipe 86 % busy either way.
+// 0.488 -> 0.344 at 128x64x64, the pipe 86 % busy either way.  (The zero test of vsum as the
+// compiler's comparison took one more: 2.51 -> 2.44 since.)
 template <int DIR>
 __global__ void __launch_bounds__(32) k_weno_line(Grid g, int m, const int* __restrict__ keep, double kd,
                                                    const double* __restrict__ u, const double* __restrict__ v,
@@ -302,7 +304,7 @@ __global__ void __launch_bounds__(32) k_weno_line(Grid g, int m, const int* __re
       as = __ldg(a + c + S + Sq);
     }
     // sign and zero of vsum from its bits (a double comparison takes an FP64-pipe slot)
-    const long long vb = __double_as_longlong(vsum);
+    const long long vb = raw(vsum);
     const bool pos = vb >= 0;
     const double E1 = pos ? e0 : e4, E2 = pos ? e1 : e3, E4 = pos ? e3 : e1, U1 = pos ? u0 : u2;
     const double a1 = pos ? dm : -dp;
@@ -431,7 +433,7 @@ __global__ void k_check_split(long n, unsigned long long* worst) {
     const double q = __longlong_as_double((long long)(sg | (e << 52) | (long long)(h & 0xFFFFFFFFFFFFFull)));
     const float2 p = split_pair(q);
     const double rel = fabs(((double)p.x + (double)p.y) - q) / fabs(q);
-    const unsigned long long b = (unsigned long long)__double_as_longlong(rel);
+    const unsigned long long b = (unsigned long long)raw(rel);
     m = b > m ? b : m;
   }
   atomicMax(worst, m);

@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256) k_offset(Grid g, const double* __restrict
   const bool in = i <= g.ni && j <= g.nj;
   const long c = in ? g.at(i, j, k) : 0;
   double p = in ? phin[c] : 0.0;  // in flight while the offset is formed
-  const long long pb = __double_as_longlong(p);
+  const long long pb = raw(p);
   const bool between = pb != 0 && pb != kOneBits;
   if (__syncthreads_or(between)) {
     if (threadIdx.x == 0) off = (sums[0] - sums[1]) * recip_nr(sums[2] + 1.0e-99);
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) k_offset(Grid g, const double* __restrict
 struct Mix {
   double rl, rg, ml, mg;
   __device__ __forceinline__ void operator()(double a, double* rho, double* mu) const {
-    const long long b = __double_as_longlong(a);
+    const long long b = raw(a);
     if (b == 0 || b == kOneBits) {
       *rho = b ? rg : rl;
       *mu = b ? mg : ml;
@@ -162,7 +162,7 @@ void mthinc_volume_fix(cudaStream_t s, const Grid& g, double dxinv, double dyinv
       [=] __device__(int i, int j, int k, double* r) {
         const long c = G.at(i, j, k);
         const double p = phin[c];
-        const long long b = __double_as_longlong(p);
+        const long long b = raw(p);
         r[0] = phi[c];
         r[1] = p;
         r[2] = b == 0 || b == kOneBits ? 0.0 : p * p * (1.0 - p);
