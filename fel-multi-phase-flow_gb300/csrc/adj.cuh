@@ -32,12 +32,13 @@ namespace adj {
 // range3 with warps of 8 x 4 points (bits.cuh: fn skips work where a whole warp is flat)
 template <class Fn>
 __global__ void __launch_bounds__(256) k_tiles3(int i0, int i1, int j0, int j1, int k0, Fn fn) {
+  after_previous();
   const Tile T = warp_tile(i1 - i0 + 1);
   if (i0 + T.x <= i1 && j0 + T.y <= j1) fn(i0 + T.x, j0 + T.y, k0 + (int)blockIdx.z);
 }
 template <class Fn>
 inline void tiles3(cudaStream_t s, int i0, int i1, int j0, int j1, int k0, int k1, Fn fn) {
-  k_tiles3<<<tile_grid(i1 - i0 + 1, j1 - j0 + 1, k1 - k0 + 1, 256), 256, 0, s>>>(i0, i1, j0, j1, k0, fn);
+  chain(s, tile_grid(i1 - i0 + 1, j1 - j0 + 1, k1 - k0 + 1, 256), 256, k_tiles3<Fn>)(i0, i1, j0, j1, k0, fn);
   count_launch();
 }
 

@@ -9,6 +9,7 @@ namespace adj {
 namespace {
 // out[0] = sum of a[0..n-1] (two-stage tree; partials in scratch slot 11)
 __global__ void k_sum_stage(const double* a, long n, double* part) {
+  after_previous();
   __shared__ double sh[256];
   double acc = 0.0;
   for (long t = blockIdx.x * 256L + threadIdx.x; t < n; t += (long)gridDim.x * 256) acc += a[t];
@@ -23,8 +24,8 @@ __global__ void k_sum_stage(const double* a, long n, double* part) {
 void sum_all(cudaStream_t s, long n, const double* a, double* out) {
   const int nb = 152 * 4;
   double* part = (double*)scratch(sizeof(double) * nb, 11);
-  k_sum_stage<<<nb, 256, 0, s>>>(a, n, part);
-  k_sum_stage<<<1, 256, 0, s>>>(part, nb, out);
+  chain(s, nb, 256, k_sum_stage)(a, n, part);
+  chain(s, 1, 256, k_sum_stage)(part, nb, out);
   count_launch(2);
 }
 }  // namespace
@@ -72,6 +73,7 @@ __device__ __forceinline__ void line_T(double* __restrict__ a, long r, long S, i
 // x lines (one thread per (j,k)), normal: bit c set = plain copy of component c
 __global__ void __launch_bounds__(256) k_halo_x_T(Grid g, int normal, double* __restrict__ lu,
                                                   double* __restrict__ lv, double* __restrict__ lw) {
+  after_previous();
   const int j = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int k = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (j > g.nj + 3 || k > g.nk + 3) return;
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(256) k_halo_x_T(Grid g, int normal, double* __
 // z lines (one thread per (i,j)); w is the shifted component
 __global__ void __launch_bounds__(256) k_halo_z_T(Grid g, int normal, double* __restrict__ lu,
                                                   double* __restrict__ lv, double* __restrict__ lw) {
+  after_previous();
   const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > g.ni + 3 || j > g.nj + 3) return;
@@ -100,6 +103,7 @@ __global__ void __launch_bounds__(256) k_halo_z_T(Grid g, int normal, double* __
 // no lane's destination is another lane's source, so the lanes are independent.
 __global__ void __launch_bounds__(256) k_halo_x_T8(Grid g, int normal, double* __restrict__ lu,
                                                    double* __restrict__ lv, double* __restrict__ lw) {
+  after_previous();
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const int m = (int)(t & 7);
   const long task = t >> 3;
@@ -128,15 +132,15 @@ dim3 xh_grid(const Grid& g) { return dim3((g.nj + 6 + 31) / 32, (g.nk + 6 + 7) /
 dim3 zh_grid(const Grid& g) { return dim3((g.ni + 6 + 31) / 32, (g.nj + 6 + 7) / 8); }
 void launch_halo_x_T(cudaStream_t s, const Grid& g, int normal, double* lu, double* lv, double* lw) {
   if (g.ni >= 8)
-    k_halo_x_T8<<<(unsigned)((24L * (g.nj + 6) * (g.nk + 6) + 255) / 256), 256, 0, s>>>(g, normal, lu, lv, lw);
+    chain(s, (unsigned)((24L * (g.nj + 6) * (g.nk + 6) + 255) / 256), 256, k_halo_x_T8)(g, normal, lu, lv, lw);
   else
-    k_halo_x_T<<<xh_grid(g), dim3(32, 8), 0, s>>>(g, normal, lu, lv, lw);
+    chain(s, xh_grid(g), dim3(32, 8), k_halo_x_T)(g, normal, lu, lv, lw);
 }
 
 // bnd_periodic: x copies over every (j,k) then z copies over every (i,j); the adjoint
 // runs z first.
 void periodic_T(cudaStream_t s, const Grid& g, double* lq) {
-  k_halo_z_T<<<zh_grid(g), dim3(32, 8), 0, s>>>(g, 4, nullptr, nullptr, lq);
+  chain(s, zh_grid(g), dim3(32, 8), k_halo_z_T)(g, 4, nullptr, nullptr, lq);
   launch_halo_x_T(s, g, 1, lq, nullptr, nullptr);
   count_launch(2);
 }
@@ -269,6 +273,7 @@ __global__ void __launch_bounds__(256) k_wall_T(Grid G, double uwall, const doub
                                                 const double* __restrict__ uk, const double* __restrict__ wk,
                                                 double* __restrict__ lu, double* __restrict__ lv,
                                                 double* __restrict__ lw, double* __restrict__ lwc) {
+  after_previous();
   const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int kk = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > G.ni + 3 || kk > 2 * (G.nk + 6) - 3) return;
@@ -383,6 +388,7 @@ __global__ void __launch_bounds__(256) k_refresh_T(Grid G, int normal, double uw
                                                    double* __restrict__ lu, double* __restrict__ lv,
                                                    double* __restrict__ lw, double* __restrict__ lwc, int nbW,
                                                    int nb1) {
+  after_previous();
   const int shu = !(normal & 1), shw = !(normal & 4);
   const int NI = G.ni, NJ = G.nj, NK = G.nk;
   const int b = (int)blockIdx.x;
@@ -478,7 +484,7 @@ __global__ void __launch_bounds__(256) k_refresh_T(Grid G, int normal, double uw
 }
 void wall_T(cudaStream_t s, const Grid& g, double uwall, const double* wc, const double* uk, const double* wk,
             double* lu, double* lv, double* lw, double* lwc) {
-  k_wall_T<<<dim3((g.ni + 6 + 31) / 32, (2 * (g.nk + 6) + 7) / 8), dim3(32, 8), 0, s>>>(g, uwall, wc, uk, wk, lu, lv,
+  chain(s, dim3((g.ni + 6 + 31) / 32, (2 * (g.nk + 6) + 7) / 8), dim3(32, 8), k_wall_T)(g, uwall, wc, uk, wk, lu, lv,
                                                                                        lw, lwc);
   count_launch();
 }
@@ -489,7 +495,7 @@ void halo_x_T(cudaStream_t s, const Grid& g, int normal, double* lu, double* lv,
 }
 
 void halo_z_T(cudaStream_t s, const Grid& g, int normal, double* lu, double* lv, double* lw) {
-  k_halo_z_T<<<zh_grid(g), dim3(32, 8), 0, s>>>(g, normal, lu, lv, lw);
+  chain(s, zh_grid(g), dim3(32, 8), k_halo_z_T)(g, normal, lu, lv, lw);
   count_launch();
 }
 
@@ -499,7 +505,7 @@ void wall_halo_T(cudaStream_t s, const Grid& g, int normal, double uwall, const 
     const long tw = 6L * (g.ni + 6) * (g.nk + 6), t1 = 3L * (g.nj - 6) * (g.nk + 6),
                t2 = 3L * (g.ni + 1) * (g.nj - 6);
     const int nbW = (int)((tw + 255) / 256), nb1 = (int)((t1 + 255) / 256), nb2 = (int)((t2 + 255) / 256);
-    k_refresh_T<<<nbW + nb1 + nb2, 256, 0, s>>>(g, normal, uwall, wc, u, w, lu, lv, lw, lwc, nbW, nb1);
+    chain(s, nbW + nb1 + nb2, 256, k_refresh_T)(g, normal, uwall, wc, u, w, lu, lv, lw, lwc, nbW, nb1);
     count_launch();
     return;
   }

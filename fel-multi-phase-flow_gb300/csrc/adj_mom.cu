@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(256) k_weno_T1(Grid g, double dxi, double dyi,
                                                  const double* __restrict__ w, const double* __restrict__ la0,
                                                  const double* __restrict__ la1, const double* __restrict__ la2,
                                                  double* __restrict__ D, double* __restrict__ V) {
+  after_previous();
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   const int line = (int)blockIdx.z % 9, k = 1 + (int)blockIdx.z / 9;
@@ -306,6 +307,7 @@ __global__ void __launch_bounds__(256) k_weno_T1_f32(Grid g, float dxi, float dy
                                                      const float2* __restrict__ sp, const double* __restrict__ la0,
                                                      const double* __restrict__ la1, const double* __restrict__ la2,
                                                      double* __restrict__ D, double* __restrict__ V) {
+  after_previous();
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   const int line = (int)blockIdx.z % 9, k = 1 + (int)blockIdx.z / 9;
@@ -333,6 +335,7 @@ __global__ void __launch_bounds__(256) k_weno_T1_df(Grid g, double dxi, double d
                                                     const double* __restrict__ la0, const double* __restrict__ la1,
                                                     const double* __restrict__ la2, double* __restrict__ D,
                                                     double* __restrict__ V) {
+  after_previous();
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   const int line = (int)blockIdx.z % 9, k = 1 + (int)blockIdx.z / 9;
@@ -359,6 +362,7 @@ __global__ void __launch_bounds__(256) k_weno_T1_df(Grid g, double dxi, double d
 __global__ void __launch_bounds__(256) k_weno_T2(Grid g, const double* __restrict__ D,
                                                  const double* __restrict__ V, double* __restrict__ lu,
                                                  double* __restrict__ lv, double* __restrict__ lw) {
+  after_previous();
   const int x = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int y = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   const int z = -2 + (int)blockIdx.z;
@@ -408,14 +412,14 @@ void weno_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, c
   double* V = work + 54 * g.n;
   const dim3 grd((g.ni + 31) / 32, (g.nj + 7) / 8, 9 * g.nk), blk(32, 8);
   if (pairs) {
-    k_weno_T1_df<<<grd, blk, 0, s>>>(g, dxi, dyi, dzi, u, v, w, ladv[0], ladv[1], ladv[2], D, V);
+    chain(s, grd, blk, k_weno_T1_df)(g, dxi, dyi, dzi, u, v, w, ladv[0], ladv[1], ladv[2], D, V);
   } else if (split) {
     fused::split3(s, g, u, v, w, split);
-    k_weno_T1_f32<<<grd, blk, 0, s>>>(g, (float)dxi, (float)dyi, (float)dzi, split, ladv[0], ladv[1], ladv[2], D, V);
+    chain(s, grd, blk, k_weno_T1_f32)(g, (float)dxi, (float)dyi, (float)dzi, split, ladv[0], ladv[1], ladv[2], D, V);
   } else {
-    k_weno_T1<<<grd, blk, 0, s>>>(g, dxi, dyi, dzi, u, v, w, ladv[0], ladv[1], ladv[2], D, V);
+    chain(s, grd, blk, k_weno_T1)(g, dxi, dyi, dzi, u, v, w, ladv[0], ladv[1], ladv[2], D, V);
   }
-  k_weno_T2<<<dim3((g.ni + 6 + 31) / 32, (g.nj + 6 + 7) / 8, g.nk + 6), dim3(32, 8), 0, s>>>(g, D, V, lu, lv, lw);
+  chain(s, dim3((g.ni + 6 + 31) / 32, (g.nj + 6 + 7) / 8, g.nk + 6), dim3(32, 8), k_weno_T2)(g, D, V, lu, lv, lw);
   count_launch(2);
 }
 

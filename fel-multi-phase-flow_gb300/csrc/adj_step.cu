@@ -311,6 +311,7 @@ void dcopy(fmf_adj* a, const double* src, double* dst, long n) {
 // crossing phi(i,1,k) > 0.5 > phi(i+1,1,k); out[0] = J; lphi (zeroed by the caller)
 // receives dJ/dphi at the two crossing points
 __global__ void k_interface(Grid g, const double* phi, double dx, double xl, double* xk, double* lphi) {
+  after_previous();
   const int k = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (k > g.nk) return;
   double x = 0.0;
@@ -330,6 +331,7 @@ __global__ void k_interface(Grid g, const double* phi, double dx, double xl, dou
   xk[k - 1] = x;
 }
 __global__ void k_mean_neg(const double* xk, int nk, double* out) {
+  after_previous();
   if (threadIdx.x != 0) return;
   double s = 0.0;
   for (int k = 0; k < nk; ++k) s = s + xk[k];
@@ -337,6 +339,7 @@ __global__ void k_mean_neg(const double* xk, int nk, double* out) {
 }
 
 __global__ void k_nonfinite(const double* p, long n, int* flag) {
+  after_previous();
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
     if (!isfinite(p[t])) {
       *flag = 1;
@@ -362,7 +365,7 @@ void check_stage(fmf_adj* a, const char* stage) {
       {"ltheta", a->ltheta},   {"lfl0", a->lfl[0]},   {"gtheta0", a->gtheta0}, {"gzeta", a->gzeta},
       {"gl1", a->gl1}};
   for (auto& e : arrs) {
-    k_nonfinite<<<256, 256, 0, a->s>>>(e.second, n, flag);
+    chain(a->s, 256, 256, k_nonfinite)(e.second, n, flag);
     int h = 0;
     FMF_CUDA(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, a->s));
     FMF_CUDA(cudaStreamSynchronize(a->s));
@@ -378,8 +381,8 @@ double objective(fmf_adj* a, const double* phi0, double* lphi) {
   const Grid& g = a->g;
   const double xl = a->prm.dx * a->prm.ni;
   if (lphi) zero(a, lphi, g.n);
-  k_interface<<<(g.nk + 127) / 128, 128, 0, a->s>>>(g, phi0, a->prm.dx, xl, a->red + 16, lphi);
-  k_mean_neg<<<1, 32, 0, a->s>>>(a->red + 16, g.nk, a->red + 8);
+  chain(a->s, (g.nk + 127) / 128, 128, k_interface)(g, phi0, a->prm.dx, xl, a->red + 16, lphi);
+  chain(a->s, 1, 32, k_mean_neg)(a->red + 16, g.nk, a->red + 8);
   count_launch(2);
   double J = 0.0;
   FMF_CUDA(cudaMemcpyAsync(&J, a->red + 8, sizeof(double), cudaMemcpyDeviceToHost, a->s));

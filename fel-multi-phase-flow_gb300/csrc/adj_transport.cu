@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(128) k_band_T(Grid g, MC M, double sx, double 
                                                 double* lw, const int* __restrict__ list,
                                                 const int* __restrict__ count, const double* __restrict__ newton,
                                                 long cap) {
+  after_previous();
   const int nb = *count;
   const long n = g.n;
   const long X = 1, Y = g.sy, Z = g.sz;
@@ -223,6 +224,7 @@ __global__ void __launch_bounds__(128) k_band_T(Grid g, MC M, double sx, double 
   }
 }
 __global__ void k_mark(const int* __restrict__ list, const int* __restrict__ count, double* __restrict__ flag) {
+  after_previous();
   const int nb = *count;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nb; e += gridDim.x * blockDim.x) flag[list[e]] = 1.0;
 }
@@ -239,7 +241,7 @@ void mthinc1_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi
   // lrn[3n + c] = 1 marks the band cells of the forward pass (its classification,
   // not a recomputed one)
   FMF_CUDA(cudaMemsetAsync(lrn, 0, sizeof(double) * 4 * n, s));
-  k_mark<<<152 * 4, 256, 0, s>>>(list, count, lrn + 3 * n);
+  chain(s, 152 * 4, 256, k_mark)(list, count, lrn + 3 * n);
   count_launch();
   range3(s, 0, g.ni + 1, 0, g.nj + 1, 0, g.nk + 1, [=] __device__(int i, int j, int k) {
     const long X = 1, Y = G.sy, Z = G.sz;
@@ -282,7 +284,7 @@ void mthinc1_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi
     }
     // band cells: k_band_T over the forward pass's band list
   });
-  k_band_T<<<152 * 8, 128, 0, s>>>(g, M, dt * dxi, dt * dyi, dt * dzi, bet, phi, gx, gy, gz, u, v, w, lfx, lfy, lfz,
+  chain(s, 152 * 8, 128, k_band_T)(g, M, dt * dxi, dt * dyi, dt * dzi, bet, phi, gx, gy, gz, u, v, w, lfx, lfy, lfz,
                                    lphi, lrn, lu, lv, lw, list, count, newton,
                                    (long)(g.ni + 2) * (g.nj + 2) * (g.nk + 2));
   count_launch();

@@ -84,6 +84,7 @@ struct GradIn {
 template <int COMP, bool OWN, bool GRAD>
 __global__ void __launch_bounds__(64, GRAD ? 10 : 16) k_pair_T(Grid g, SwK K, int pi, int pj, int pk, CArr4 cf,
                                                 const double* __restrict__ A, Arr3 la, GradIn G) {
+  after_previous();
   const bool h = (int)blockIdx.z >= g.nk / 2;
   const int i = (h ? 3 - pi : pi) + 2 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = (h ? 3 - pj : pj) + 2 * (int)(blockIdx.y * blockDim.y + threadIdx.y);
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(64, GRAD ? 10 : 16) k_pair_T(Grid g, SwK K, in
 }
 const int kPi[4] = {1, 1, 1, 2}, kPj[4] = {1, 1, 2, 1}, kPk[4] = {1, 2, 1, 1};
 __global__ void k_copy3(long n, CArr3 a, double* __restrict__ b) {
+  after_previous();
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
     b[t] = a.a[0][t];
     b[t + n] = a.a[1][t];
@@ -158,6 +160,7 @@ __global__ void k_copy3(long n, CArr3 a, double* __restrict__ b) {
 // (l - fb)^2 = |l_new - l_old|^2, part[kParts + block] = sum of l^2, fb = l, l += lout
 constexpr int kParts = 512;
 __global__ void __launch_bounds__(256) k_add_diff3(long n, Arr3 l, CArr3 o, double* part, double* fb) {
+  after_previous();
   __shared__ double sh[2][256];
   double acc = 0.0, acf = 0.0;
   const long step = kParts * 256L;
@@ -204,6 +207,7 @@ __global__ void __launch_bounds__(256) k_add_diff3(long n, Arr3 l, CArr3 o, doub
 // The start: fbo = 0 (no fb), fb (the warm start) or 2 fb - fb2 (fb2 the feedback term one
 // solve earlier: linear extrapolation in time; may be fbo itself), l = lout + fbo
 __global__ void k_start3(long n, Arr3 l, CArr3 o, const double* fb, const double* fb2, double* fbo) {
+  after_previous();
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
     for (int c = 0; c < 3; ++c) {
       double f = 0.0;
@@ -217,6 +221,7 @@ __global__ void k_start3(long n, Arr3 l, CArr3 o, const double* fb, const double
 }
 // out[0] = sum of part[0..n), out[1] = sum of part[kParts..kParts+n)
 __global__ void k_sum_small(const double* part, int n, double* out) {
+  after_previous();
   __shared__ double sh[2][256];
   double acc = 0.0, acf = 0.0;
   for (int t = threadIdx.x; t < n; t += 256) {
@@ -343,7 +348,7 @@ void sor_replay(cudaStream_t s, const Grid& g, double dxi, double dyi, double dz
   const long n = g.n;
   double* q[3] = {snaps + 36 * n, snaps + 37 * n, snaps + 38 * n};  // running state
   const CArr3 run{{q[0], q[1], q[2]}};
-  k_copy3<<<608, 256, 0, s>>>(n, CArr3{{ustar[0], ustar[1], ustar[2]}}, q[0]);
+  chain(s, 608, 256, k_copy3)(n, CArr3{{ustar[0], ustar[1], ustar[2]}}, q[0]);
   count_launch();
   fused::sor_iteration(s, g, dxi, dyi, dzi, harmonic, mu, E, AB, uwall, wallc, q[0], q[1], q[2], part, nullptr,
                        fused::FlatFluid(),
@@ -351,7 +356,7 @@ void sor_replay(cudaStream_t s, const Grid& g, double dxi, double dyi, double dz
                          const CArr3 st = replay_state(g, snaps, comp, pr);
                          double* own = snaps + (3L * (4 * comp + pr) + comp) * n;
                          if (st.a[(comp + 1) % 3] == snaps + (3L * (4 * comp + pr) + (comp + 1) % 3) * n) {
-                           k_copy3<<<608, 256, 0, s>>>(n, run, snaps + 3L * (4 * comp + pr) * n);
+                           chain(s, 608, 256, k_copy3)(n, run, snaps + 3L * (4 * comp + pr) * n);
                            count_launch();
                          } else {
                            FMF_CUDA(cudaMemcpyAsync(own, q[comp], sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
@@ -398,7 +403,7 @@ int sor_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, con
   const CArr3 O3{{lout[0], lout[1], lout[2]}};
   // l = lout, or lout plus the previous solve's feedback term
   const bool warm = *fb_norm > 0.0;
-  k_start3<<<608, 256, 0, s>>>(n, L3, O3, warm ? fb : nullptr, fb_prev, fb_out);
+  chain(s, 608, 256, k_start3)(n, L3, O3, warm ? fb : nullptr, fb_prev, fb_out);
   count_launch();
   // The 12 sweeps backwards, the refresh after each transposed before it.  The forward
   // cycle after a component's second to fourth pair changes that component's ghosts
@@ -423,7 +428,7 @@ int sor_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, con
         // the slip-coefficient adjoint only in the gradient pass
         if (!own) wall_halo_T(s, g, 1 << comp, uwall, wallc, ustar[0], ustar[2], lam[0], lam[1], lam[2], GR ? lwc : nullptr);
         auto run = [&](auto fn) {
-          fn<<<grd, blk, 0, s>>>(g, K, kPi[pr], kPj[pr], kPk[pr], cf, AB[2 * comp], L3, G);
+          chain(s, grd, blk, fn)(g, K, kPi[pr], kPj[pr], kPk[pr], cf, AB[2 * comp], L3, G);
           count_launch();
         };
         if (comp == 0) own ? run(k_pair_T<0, true, GR>) : run(k_pair_T<0, false, GR>);
@@ -437,8 +442,8 @@ int sor_T(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi, con
   // set of buffers)
   auto iteration = [&]() {
     backward_cycle(std::false_type());
-    k_add_diff3<<<kParts, 256, 0, s>>>(n, L3, O3, part, fb_out);
-    k_sum_small<<<1, 256, 0, s>>>(part, kParts, nrm);
+    chain(s, kParts, 256, k_add_diff3)(n, L3, O3, part, fb_out);
+    chain(s, 1, 256, k_sum_small)(part, kParts, nrm);
     count_launch(2);
   };
   long long per_launch = 0;

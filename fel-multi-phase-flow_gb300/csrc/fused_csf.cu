@@ -232,6 +232,7 @@ template <class R>
 __global__ void __launch_bounds__(256) k_csf(Grid g, CsfP<R> p, int kchunk, const double* __restrict__ phi,
                                              double* __restrict__ fu, double* __restrict__ fv,
                                              double* __restrict__ fw, const int* __restrict__ skip) {
+  after_previous();
   if (skip && *skip) return;  // the whole block leaves before any barrier
   extern __shared__ double smraw[];
   Smem<R>& S = *reinterpret_cast<Smem<R>*>(smraw);
@@ -344,7 +345,7 @@ void launch_csf(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doubl
   cudaFuncSetAttribute(k_csf<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const int kchunk = csf_chunk(g, (const void*)k_csf<R>, smem);
   dim3 gr((unsigned)(g.ni / TX), (unsigned)(g.nj / TY), (unsigned)((g.nk + kchunk - 1) / kchunk));
-  k_csf<R><<<gr, 256, smem, s>>>(g, p, kchunk, phi, fu, fv, fw, skip);
+  chain(s, gr, 256, k_csf<R>, smem)(g, p, kchunk, phi, fu, fv, fw, skip);
   count_launch();
 }
 
@@ -377,6 +378,7 @@ __device__ __forceinline__ double inv_norm(double s, double vs, double big) {
 // over the flattened (i, j) plane so that every warp is full
 __global__ void __launch_bounds__(128) k_csf_grad(Grid g, CsfD p, const double* __restrict__ phi,
                                                   double* __restrict__ G, const int* __restrict__ skip) {
+  after_previous();
   if (skip && *skip) return;
   const Tile T = warp_tile(g.ni + 3);
   if (T.x >= g.ni + 3 || T.y >= g.nj + 3) return;
@@ -414,6 +416,7 @@ __global__ void __launch_bounds__(128) k_csf_grad(Grid g, CsfD p, const double* 
 __global__ void __launch_bounds__(128) k_csf_normals(Grid g, CsfD p, int m, const double* __restrict__ G,
                                                      double* __restrict__ pp, double* __restrict__ n12,
                                                      double* __restrict__ nside, const int* __restrict__ skip) {
+  after_previous();
   if (skip && *skip) return;
   const Tile T = warp_tile(g.ni + 2);
   const int a = T.x, b = T.y;
@@ -504,6 +507,7 @@ __global__ void __launch_bounds__(256) k_csf_force(Grid g, CsfD p, const double*
                                                    const double* __restrict__ nside, double* __restrict__ fu,
                                                    double* __restrict__ fv, double* __restrict__ fw,
                                                    const int* __restrict__ skip) {
+  after_previous();
   if (skip && *skip) return;
   const Tile T = warp_tile(g.ni);
   const int i = 1 + T.x, j = 1 + T.y;
@@ -552,15 +556,15 @@ void csf_fp64(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double 
   p.fy = -st * dyinv;
   p.fz = -st * dzinv;
   double *G = work[0], *pp = work[1], *n12 = work[2], *nside = work[3];
-  k_csf_grad<<<tile_grid(g.ni + 3, g.nj + 3, g.nk + 3, 128), 128, 0, s>>>(g, p, phi, G, skip);
+  chain(s, tile_grid(g.ni + 3, g.nj + 3, g.nk + 3, 128), 128, k_csf_grad)(g, p, phi, G, skip);
   // planes per walk: the first costs 9 additions more; as many as leave a warp for each
   // of the 608 quarter SMs, 8 at most
   const long cols = (long)(g.ni + 2) * (g.nj + 2);
   int m = 1;
   while (m < 8 && cols * (g.nk + 2) >= 2L * m * 768 * 32) m *= 2;
-  k_csf_normals<<<tile_grid(g.ni + 2, g.nj + 2, (g.nk + 2 + m - 1) / m, 128), 128, 0, s>>>(g, p, m, G, pp, n12, nside,
+  chain(s, tile_grid(g.ni + 2, g.nj + 2, (g.nk + 2 + m - 1) / m, 128), 128, k_csf_normals)(g, p, m, G, pp, n12, nside,
                                                                                            skip);
-  k_csf_force<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, p, phi, pp, n12, nside, fu, fv, fw, skip);
+  chain(s, tile_grid(g.ni, g.nj, g.nk, 256), 256, k_csf_force)(g, p, phi, pp, n12, nside, fu, fv, fw, skip);
   count_launch(3);
 }
 }  // namespace

@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double*
                                                   double* __restrict__ fx, double* __restrict__ fy,
                                                   double* __restrict__ fz, int* __restrict__ list,
                                                   int* __restrict__ count) {
+  after_previous();
   const Tile T = warp_tile(g.ni + 2);
   const int i = T.x, j = T.y, k = (int)blockIdx.z;
   if (i > g.ni + 1 || j > g.nj + 1) return;
@@ -228,6 +229,7 @@ __global__ void __launch_bounds__(128) k_band_f32(Grid g, MC m, const double* __
                                               double* __restrict__ fz, const int* __restrict__ list,
                                               const int* __restrict__ count, double* __restrict__ newton,
                                               long cap) {
+  after_previous();
   using R = float;
   const int n = *count;
   const long X = 1, Y = g.sy, Z = g.sz;
@@ -336,6 +338,7 @@ __global__ void __launch_bounds__(64) k_band(Grid g, MC m, __grid_constant__ con
                                              double* __restrict__ fy, double* __restrict__ fz,
                                              const int* __restrict__ list, const int* __restrict__ count,
                                              double* __restrict__ newton, long cap) {
+  after_previous();
   const int n = *count;
   const long X = 1, Y = g.sy, Z = g.sz;
   const double m2b = -2.0 * m.bet;
@@ -429,6 +432,7 @@ template <bool NEAR1>
 __global__ void __launch_bounds__(128) k_vertex_grad(Grid g, double cx, double cy, double cz,
                                                      const double* __restrict__ q, double* __restrict__ qx,
                                                      double* __restrict__ qy, double* __restrict__ qz) {
+  after_previous();
   const Tile T = warp_tile(g.ni + 5);
   if (T.x >= g.ni + 5 || T.y >= g.nj + 5) return;
   const long X = 1, Y = g.sy, Z = g.sz;
@@ -463,6 +467,7 @@ __global__ void __launch_bounds__(128) k_vertex_grad(Grid g, double cx, double c
 __global__ void __launch_bounds__(256) k_snap(Grid g, MC m, const double* __restrict__ gx,
                                               const double* __restrict__ gy, const double* __restrict__ gz,
                                               double* __restrict__ phin) {
+  after_previous();
   const Tile T = warp_tile(g.ni + 2);
   const int i = T.x, j = T.y, k = (int)blockIdx.z;
   if (i > g.ni + 1 || j > g.nj + 1) return;
@@ -481,16 +486,16 @@ void vertex_gradient(cudaStream_t s, const Grid& g, double dxinv, double dyinv, 
                      double* qx, double* qy, double* qz, bool near1) {
   const dim3 gr = tile_grid(g.ni + 5, g.nj + 5, g.nk + 5, 128);
   if (near1)
-    k_vertex_grad<true><<<gr, 128, 0, s>>>(g, 0.25 * dxinv, 0.25 * dyinv, 0.25 * dzinv, q, qx, qy, qz);
+    chain(s, gr, 128, k_vertex_grad<true>)(g, 0.25 * dxinv, 0.25 * dyinv, 0.25 * dzinv, q, qx, qy, qz);
   else
-    k_vertex_grad<false><<<gr, 128, 0, s>>>(g, 0.25 * dxinv, 0.25 * dyinv, 0.25 * dzinv, q, qx, qy, qz);
+    chain(s, gr, 128, k_vertex_grad<false>)(g, 0.25 * dxinv, 0.25 * dyinv, 0.25 * dzinv, q, qx, qy, qz);
   count_launch();
 }
 
 void mthinc_snap(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double bet,
                  const double* gx, const double* gy, const double* gz, double* phin) {
   const dim3 gr = tile_grid(g.ni + 2, g.nj + 2, g.nk + 2, 256);
-  k_snap<<<gr, 256, 0, s>>>(g, make_mc(dxinv, dyinv, dzinv, 0.0, bet), gx, gy, gz, phin);
+  chain(s, gr, 256, k_snap)(g, make_mc(dxinv, dyinv, dzinv, 0.0, bet), gx, gy, gz, phin);
   count_launch();
 }
 
@@ -509,12 +514,12 @@ void mthinc_fluxes(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
                    bool fp32, double* newton) {
   const MC m = make_mc(dxinv, dyinv, dzinv, dt, bet);
   FMF_CUDA(cudaMemsetAsync(count, 0, sizeof(int), s));
-  k_classify<<<tile_grid(g.ni + 2, g.nj + 2, g.nk + 2, 256), 256, 0, s>>>(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count);
+  chain(s, tile_grid(g.ni + 2, g.nj + 2, g.nk + 2, 256), 256, k_classify)(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count);
   const long cap = (long)(g.ni + 2) * (g.nj + 2) * (g.nk + 2);
   if (fp32)
-    k_band_f32<<<152 * 8, 128, 0, s>>>(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
+    chain(s, 152 * 8, 128, k_band_f32)(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
   else
-    k_band<<<152 * 16, 64, 0, s>>>(g, m, exp16_table(), phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
+    chain(s, 152 * 16, 64, k_band)(g, m, exp16_table(), phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
   count_launch(2);
 }
 

@@ -34,6 +34,7 @@ constexpr int kTileZ = 16;                  // z transforms: 16 columns of 16 th
 __global__ void __launch_bounds__(256) k_rfft_x_fwd(Grid g, const double* __restrict__ div, double* __restrict__ tr,
                                                     double* __restrict__ ti, const double2* __restrict__ twM,
                                                     const double2* __restrict__ twN) {
+  after_previous();
   extern __shared__ double sm[];
   const int M = g.ni / 2, H = M + 1;
   const int rl = threadIdx.x / kRowThreads, t = threadIdx.x % kRowThreads;
@@ -68,6 +69,7 @@ __global__ void __launch_bounds__(256) k_rfft_x_fwd(Grid g, const double* __rest
 __global__ void __launch_bounds__(256) k_rfft_x_inv(Grid g, const double* __restrict__ tr,
                                                     const double* __restrict__ ti, double* __restrict__ dp,
                                                     const double2* __restrict__ twM, const double2* __restrict__ twN) {
+  after_previous();
   extern __shared__ double sm[];
   const int M = g.ni / 2, H = M + 1;
   const int rl = threadIdx.x / kRowThreads, t = threadIdx.x % kRowThreads;
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(256) k_rfft_x_inv(Grid g, const double* __rest
 template <int SGN>
 __global__ void __launch_bounds__(256) k_fft_z_half(Grid g, const double* tr, const double* ti, double* pr,
                                                     double* pi, const double2* __restrict__ tw, double scale) {
+  after_previous();
   extern __shared__ double sm[];
   const int L = g.nk, H = g.ni / 2 + 1, NJ = g.nj;
   const int j = blockIdx.y;
@@ -134,6 +137,7 @@ __global__ void __launch_bounds__(128) k_tdma_half(Grid g, double dx2r, double d
                                                    const double* __restrict__ as_f, const double* __restrict__ an_f,
                                                    const double* __restrict__ ap_f, double* pr, double* pi,
                                                    double* __restrict__ at) {
+  after_previous();
   const int H = g.ni / 2 + 1, NJ = g.nj;
   const int kx = blockIdx.x * blockDim.x + threadIdx.x;
   const int kz = blockIdx.y;
@@ -175,6 +179,7 @@ __global__ void __launch_bounds__(128) k_tdma_half(Grid g, double dx2r, double d
 __global__ void __launch_bounds__(128) k_tdma_coef(Grid g, double dx2r, double dz2r, double pi2_ni, double pi2_nk,
                                                    const double* __restrict__ as_f, const double* __restrict__ an_f,
                                                    const double* __restrict__ ap_f, double* __restrict__ coef) {
+  after_previous();
   const int H = g.ni / 2 + 1, NJ = g.nj;
   const int kx = blockIdx.x * blockDim.x + threadIdx.x;
   const int kz = blockIdx.y;
@@ -201,6 +206,7 @@ __global__ void __launch_bounds__(128) k_tdma_coef(Grid g, double dx2r, double d
 constexpr int kRowsAhead = 8;
 __global__ void __launch_bounds__(64) k_tdma_pre(Grid g, const double* __restrict__ as_f,
                                                  const double* __restrict__ coef, double* pr, double* pi) {
+  after_previous();
   const int H = g.ni / 2 + 1, NJ = g.nj;
   const long mode = blockIdx.x * (long)blockDim.x + threadIdx.x, nmode = (long)H * g.nk;
   if (mode >= nmode) return;
@@ -256,6 +262,7 @@ __global__ void __launch_bounds__(256) k_project(Grid g, double cx, double cy, d
                                                  const double* __restrict__ dp, const double* __restrict__ phat,
                                                  double* __restrict__ un, double* __restrict__ vn,
                                                  double* __restrict__ wn, double* __restrict__ pn) {
+  after_previous();
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   const int k = 1 + (int)blockIdx.z;
@@ -275,7 +282,7 @@ void tdma_coef(cudaStream_t s, const Grid& g, double rho, double dxinv, double d
                const double* an_f, const double* ap_f, double* coef) {
   const int H = g.ni / 2 + 1;
   const double pi_ = 3.141592653589793238462643383279502884;
-  k_tdma_coef<<<dim3((unsigned)((H + 127) / 128), (unsigned)g.nk), 128, 0, s>>>(
+  chain(s, dim3((unsigned)((H + 127) / 128), (unsigned)g.nk), 128, k_tdma_coef)(
       g, dxinv * dxinv / rho, dzinv * dzinv / rho, pi_ * 2.0 / (double)g.ni, pi_ * 2.0 / (double)g.nk, as_f, an_f,
       ap_f, coef);
   count_launch();
@@ -300,26 +307,26 @@ void pressure_half(cudaStream_t s, const Grid& g, double rho, double dxinv, doub
   }
   cudaFuncSetAttribute(k_rfft_x_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf);
   cudaFuncSetAttribute(k_rfft_x_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smi);
-  k_rfft_x_fwd<<<rows / kRows, 256, smf, s>>>(g, div, tr, ti, twM, twN);
+  chain(s, rows / kRows, 256, k_rfft_x_fwd, smf)(g, div, tr, ti, twM, twN);
   cudaFuncSetAttribute(k_fft_z_half<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
   cudaFuncSetAttribute(k_fft_z_half<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
   const dim3 gz((unsigned)((H + kTileZ - 1) / kTileZ), (unsigned)g.nj);
-  k_fft_z_half<-1><<<gz, 256, smz, s>>>(g, tr, ti, pr, pi, twz, 1.0 / ((double)g.ni * (double)g.nk));
+  chain(s, gz, 256, k_fft_z_half<-1>, smz)(g, tr, ti, pr, pi, twz, 1.0 / ((double)g.ni * (double)g.nk));
   const double pi_ = 3.141592653589793238462643383279502884;
   const double dx2r = dxinv * dxinv / rho, dz2r = dzinv * dzinv / rho;
   if (coef)
-    k_tdma_pre<<<dim3((unsigned)(((long)H * g.nk + 63) / 64), 1, 2), 64, 0, s>>>(g, as_f, coef, pr, pi);
+    chain(s, dim3((unsigned)(((long)H * g.nk + 63) / 64), 1, 2), 64, k_tdma_pre)(g, as_f, coef, pr, pi);
   else
-    k_tdma_half<<<dim3((unsigned)((H + 127) / 128), (unsigned)g.nk), 128, 0, s>>>(
+    chain(s, dim3((unsigned)((H + 127) / 128), (unsigned)g.nk), 128, k_tdma_half)(
         g, dx2r, dz2r, pi_ * 2.0 / (double)g.ni, pi_ * 2.0 / (double)g.nk, as_f, an_f, ap_f, pr, pi, at);
-  k_fft_z_half<1><<<gz, 256, smz, s>>>(g, pr, pi, tr, ti, twz, 1.0);
-  k_rfft_x_inv<<<rows / kRows, 256, smi, s>>>(g, tr, ti, dp, twM, twN);
+  chain(s, gz, 256, k_fft_z_half<1>, smz)(g, pr, pi, tr, ti, twz, 1.0);
+  chain(s, rows / kRows, 256, k_rfft_x_inv, smi)(g, tr, ti, dp, twM, twN);
   count_launch(5);
 }
 
 void project(cudaStream_t s, const Grid& g, double rho, double dxinv, double dyinv, double dzinv, double dt,
              const double* dp, const double* phat, double* un, double* vn, double* wn, double* pn) {
-  k_project<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), dim3(32, 8), 0, s>>>(
+  chain(s, dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), dim3(32, 8), k_project)(
       g, dt * dxinv / rho, dt * dyinv / rho, dt * dzinv / rho, dp, phat, un, vn, wn, pn);
   count_launch();
 }

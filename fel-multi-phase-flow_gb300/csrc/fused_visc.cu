@@ -62,6 +62,7 @@ struct F3 {
 // such points takes it without the arithmetic.  Threads over the flattened (i, j) plane.
 __global__ void __launch_bounds__(128) k_edges(Grid g, VP p, const double* __restrict__ mu, double* __restrict__ exy,
                                                double* __restrict__ exz, double* __restrict__ eyz, F3 f, int* count) {
+  after_previous();
   if (count && (blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) *count = 0;  // k_src_ab adds to it
   const Tile T = warp_tile(g.ni + 1);
   const int i = T.x, j = T.y, k = (int)blockIdx.z;
@@ -135,6 +136,7 @@ struct SrcK {
 __global__ void __launch_bounds__(256) k_src_ab(Grid g, SrcK K, SrcIn in, const double* __restrict__ mu,
                                                 const double* __restrict__ exy, const double* __restrict__ exz,
                                                 const double* __restrict__ eyz, ABOut out) {
+  after_previous();
   const Tile T = warp_tile(g.ni);
   const int i = 1 + T.x, j = 1 + T.y, k = 1 + (int)blockIdx.z;
   if (i > g.ni || j > g.nj) return;
@@ -210,6 +212,7 @@ __device__ __forceinline__ df::D diag_e(const VPS& p, df::D r, df::D ka, df::D a
 // FlatFluid's pairs: what the general branch below forms where every density and viscosity
 // it reads is fluid f's
 __global__ void k_flat_pairs(VPS p, Fluids fl, float2* __restrict__ out) {
+  after_previous();
   using namespace df;
   const int f = (int)threadIdx.x;
   if (f > 1) return;
@@ -228,6 +231,7 @@ __global__ void __launch_bounds__(256, 4) k_src_ab_e(Grid g, VPS p, VP pv, Fac<d
                                                   const double* __restrict__ mu,
                                                   const double* __restrict__ exy, const double* __restrict__ exz,
                                                   const double* __restrict__ eyz, ABOut out) {
+  after_previous();
   using namespace df;
   const Tile tile = warp_tile(g.ni);
   const int i = 1 + tile.x, j = 1 + tile.y, k = 1 + (int)blockIdx.z;
@@ -332,6 +336,7 @@ __global__ void __launch_bounds__(128) k_stress(Grid g, StressK K, const double*
                                                 const double* __restrict__ v, const double* __restrict__ w,
                                                 const double* __restrict__ mu, double* __restrict__ tau,
                                                 double* __restrict__ sk) {
+  after_previous();
   const int W = g.ni + 2;
   const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (t >= W * (g.nj + 2)) return;
@@ -372,6 +377,7 @@ __global__ void __launch_bounds__(128) k_stress(Grid g, StressK K, const double*
 __global__ void __launch_bounds__(256) k_div_stress(Grid g, StressK K, const double* __restrict__ t,
                                                     double* __restrict__ vu, double* __restrict__ vv,
                                                     double* __restrict__ vw) {
+  after_previous();
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   const int k = 1 + (int)blockIdx.z;
@@ -408,6 +414,7 @@ __global__ void __launch_bounds__(256) k_stress_e(Grid g, VPT p, const float2* _
                                                   const double* __restrict__ u, const double* __restrict__ v,
                                                   const double* __restrict__ w, const double* __restrict__ mu,
                                                   float2* __restrict__ tau, double* __restrict__ sk) {
+  after_previous();
   using namespace df;
   const Tile T = warp_tile(g.ni + 2);
   const int i = T.x, j = T.y, k = (int)blockIdx.z;
@@ -455,6 +462,7 @@ __global__ void __launch_bounds__(256) k_stress_e(Grid g, VPT p, const float2* _
 __global__ void __launch_bounds__(256) k_div_stress_e(Grid g, VPT p, const float2* __restrict__ t,
                                                       double* __restrict__ vu, double* __restrict__ vv,
                                                       double* __restrict__ vw) {
+  after_previous();
   using namespace df;
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
@@ -703,6 +711,7 @@ __global__ void __launch_bounds__(128) k_pair(Grid g, SweepK<T> K, int pi, int p
                                               const T* __restrict__ exz, const T* __restrict__ eyz,
                                               const T* __restrict__ A, const T* __restrict__ B, T* un, T* vn, T* wn,
                                               G gh, double* __restrict__ part, int first) {
+  after_previous();
   __shared__ T sh[128];
   const int jmax = COMP == 1 ? g.nj - 1 : g.nj;
   T* q = COMP == 0 ? un : (COMP == 1 ? vn : wn);
@@ -788,6 +797,7 @@ __global__ void __launch_bounds__(128) k_pair(Grid g, SweepK<T> K, int pi, int p
 __global__ void __launch_bounds__(256) k_wall_coef(Grid g, double dy, const double* __restrict__ l1,
                                                    const double* __restrict__ l2, const double* __restrict__ phi,
                                                    double* __restrict__ wc) {
+  after_previous();
   const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int kk = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > g.ni + 3 || kk > 2 * (g.nk + 6) - 3) return;
@@ -808,6 +818,7 @@ __global__ void __launch_bounds__(256) k_wall_coef(Grid g, double dy, const doub
 __global__ void __launch_bounds__(256) k_wall(Grid g, double uwall, const double* __restrict__ wc,
                                               double* __restrict__ uk, double* __restrict__ vk,
                                               double* __restrict__ wk) {
+  after_previous();
   const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int kk = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > g.ni + 3 || kk > 2 * (g.nk + 6) - 3) return;
@@ -858,6 +869,7 @@ __global__ void __launch_bounds__(256) k_wall(Grid g, double uwall, const double
 // clear: bndu's copy, which for u is shifted by one (bndu.f:107-109).
 __global__ void __launch_bounds__(256) k_halo_x(Grid g, int normal, double* __restrict__ uk,
                                                 double* __restrict__ vk, double* __restrict__ wk) {
+  after_previous();
   const int j = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int k = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (j > g.nj + 3 || k > g.nk + 3) return;
@@ -893,6 +905,7 @@ __global__ void __launch_bounds__(256) k_halo_x(Grid g, int normal, double* __re
 // z halos; for w bndu's copy is shifted by one (bndu.f:144-146).
 __global__ void __launch_bounds__(256) k_halo_z(Grid g, int normal, double* __restrict__ uk,
                                                 double* __restrict__ vk, double* __restrict__ wk) {
+  after_previous();
   const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > g.ni + 3 || j > g.nj + 3) return;
@@ -931,6 +944,7 @@ __global__ void __launch_bounds__(256) k_halo_z(Grid g, int normal, double* __re
 // runs instead of 32 rows, and the work spreads over every SM.
 __global__ void __launch_bounds__(256) k_halo_x8(Grid g, int normal, double* __restrict__ uk,
                                                  double* __restrict__ vk, double* __restrict__ wk) {
+  after_previous();
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const int m = (int)(t & 7);
   const long task = t >> 3;
@@ -1077,6 +1091,7 @@ __device__ __forceinline__ void refresh(const Grid& g, int normal, const Ghosts6
 __global__ void __launch_bounds__(256) k_gamma_wall(Grid g, double uwall, const double* __restrict__ wc,
                                                     const double* __restrict__ u, const double* __restrict__ v,
                                                     const double* __restrict__ w, float* __restrict__ gw) {
+  after_previous();
   const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int kk = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > g.ni + 3 || kk > 2 * (g.nk + 6) - 3) return;
@@ -1113,6 +1128,7 @@ __global__ void __launch_bounds__(256) k_gamma_wall(Grid g, double uwall, const 
 }
 __global__ void __launch_bounds__(256) k_gamma_x(Grid g, const double* __restrict__ u, const double* __restrict__ v,
                                                  const double* __restrict__ w, float* __restrict__ gx) {
+  after_previous();
   const int j = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int k = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (j > g.nj + 3 || k > g.nk + 3) return;
@@ -1133,6 +1149,7 @@ __global__ void __launch_bounds__(256) k_gamma_x(Grid g, const double* __restric
 }
 __global__ void __launch_bounds__(256) k_gamma_z(Grid g, const double* __restrict__ u, const double* __restrict__ v,
                                                  const double* __restrict__ w, float* __restrict__ gz) {
+  after_previous();
   const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > g.ni + 3 || j > g.nj + 3) return;
@@ -1154,6 +1171,7 @@ __global__ void __launch_bounds__(256) k_gamma_z(Grid g, const double* __restric
 // k_wall on the corrections
 __global__ void __launch_bounds__(256) k_wall_d(Grid g, const float* __restrict__ gw, float* __restrict__ du,
                                                 float* __restrict__ dv, float* __restrict__ dw) {
+  after_previous();
   const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int kk = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > g.ni + 3 || kk > 2 * (g.nk + 6) - 3) return;
@@ -1199,6 +1217,7 @@ __global__ void __launch_bounds__(256) k_wall_d(Grid g, const float* __restrict_
 __global__ void __launch_bounds__(256) k_halo_x_d(Grid g, int normal, const float* __restrict__ gx,
                                                   float* __restrict__ du, float* __restrict__ dv,
                                                   float* __restrict__ dw) {
+  after_previous();
   const int j = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int k = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (j > g.nj + 3 || k > g.nk + 3) return;
@@ -1244,6 +1263,7 @@ __global__ void __launch_bounds__(256) k_halo_x_d(Grid g, int normal, const floa
 __global__ void __launch_bounds__(256) k_halo_z_d(Grid g, int normal, const float* __restrict__ gz,
                                                   float* __restrict__ du, float* __restrict__ dv,
                                                   float* __restrict__ dw) {
+  after_previous();
   const int i = -2 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = -2 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   if (i > g.ni + 3 || j > g.nj + 3) return;
@@ -1412,12 +1432,14 @@ __host__ __device__ __forceinline__ long refresh_tasks(const Grid& g, int region
 // (the FP32 corrections' refresh of one component only)
 __global__ void __launch_bounds__(256) k_refresh_one(Grid g, int comp, Ghosts32 gh, float* du, float* dv, float* dw,
                                                      int nbW, int nbX) {
+  after_previous();
   const int b = (int)blockIdx.x, region = b < nbW ? 0 : (b < nbW + nbX ? 1 : 2);
   refresh(g, 1 << comp, gh, du, dv, dw, region,
           (long)(b - (region > 0 ? nbW : 0) - (region > 1 ? nbX : 0)) * 256 + threadIdx.x, comp);
 }
 template <class T, class G>
 __global__ void __launch_bounds__(256) k_refresh(Grid g, int normal, G gh, T* uk, T* vk, T* wk, int nbW, int nbX) {
+  after_previous();
   const int b = (int)blockIdx.x, region = b < nbW ? 0 : (b < nbW + nbX ? 1 : 2);
   refresh(g, normal, gh, uk, vk, wk, region, (long)(b - (region > 0 ? nbW : 0) - (region > 1 ? nbX : 0)) * 256 + threadIdx.x);
 }
@@ -1482,6 +1504,7 @@ __device__ __forceinline__ T cluster_component(const Grid& g, const SolveK<T>& K
 }
 template <class T, class G>
 __global__ void __launch_bounds__(kClusterThreads) k_solve_cluster(Grid g, SolveK<T> K, G gh, SorLoop* L, int* log) {
+  after_previous();
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   __shared__ double parts[kClusterBlocks], warps[kClusterThreads / 32];
@@ -1536,6 +1559,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_solve_cluster(Grid g, Solve
   }
 }
 __global__ void k_to_float(long n, const double* __restrict__ a, float* __restrict__ b) {
+  after_previous();
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
     b[t] = (float)a[t];
 }
@@ -1544,6 +1568,7 @@ __global__ void k_refine_finish(long n, const double* __restrict__ u, const doub
                                 const double* __restrict__ w, const float* __restrict__ du,
                                 const float* __restrict__ dv, const float* __restrict__ dw, double* __restrict__ un,
                                 double* __restrict__ vn, double* __restrict__ wn) {
+  after_previous();
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
     un[t] = u[t] + (double)du[t];
     vn[t] = v[t] + (double)dv[t];
@@ -1552,6 +1577,7 @@ __global__ void k_refine_finish(long n, const double* __restrict__ u, const doub
 }
 
 __global__ void __launch_bounds__(1024) k_sum_parts2(const double* part, long n, double* out) {
+  after_previous();
   __shared__ double sh[32];
   double a = 0.0;
   for (long t = threadIdx.x; t < n; t += 1024) a += part[t];
@@ -1674,7 +1700,7 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
   in.phat = phat;
   in.grvb = grvb;
   in.grvp = grvp;
-  k_edges<<<tile_grid(g.ni + 1, g.nj + 1, g.nk + 1, 128), 128, 0, s>>>(
+  chain(s, tile_grid(g.ni + 1, g.nj + 1, g.nk + 1, 128), 128, k_edges)(
       g, p, mu, E[0], E[1], E[2], ef, flat.count);
   if (REFINE) {
     FlatE FE;
@@ -1686,7 +1712,7 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
       std::memcpy(&FE.rb[q], &rf[q], sizeof(double));
       std::memcpy(&FE.mb[q], &mf[q], sizeof(double));
     }
-    k_src_ab_e<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, make_vps(p, grvb, grvp), p, Fac<double>(p), in, FE,
+    chain(s, tile_grid(g.ni, g.nj, g.nk, 256), 256, k_src_ab_e)(g, make_vps(p, grvb, grvp), p, Fac<double>(p), in, FE,
                                                                 mu, E[0], E[1], E[2], out);
   } else {
     SrcK K;
@@ -1712,9 +1738,9 @@ void src_prep(cudaStream_t s, const Grid& g, const VP& p, const double* u, const
     }
     K.fluid = flat.fluid;
     K.count = flat.count;
-    k_src_ab<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, K, in, mu, E[0], E[1], E[2], out);
+    chain(s, tile_grid(g.ni, g.nj, g.nk, 256), 256, k_src_ab)(g, K, in, mu, E[0], E[1], E[2], out);
   }
-  k_wall_coef<<<wall_grid(g), kB, 0, s>>>(g, dy, l1, l2, phi, wallc);
+  chain(s, wall_grid(g), kB, k_wall_coef)(g, dy, l1, l2, phi, wallc);
   count_launch(3);
 }
 
@@ -1735,8 +1761,8 @@ void sweep_all(cudaStream_t s, const Grid& g, const VP& p, const T* mu, const T*
     for (int pr = 0; pr < 4; ++pr) {
       if (before) before(comp, pr);
       auto run = [&](auto fn) {
-        fn<<<sp.grid, sp.block, 0, s>>>(g, K, kPi[pr], kPj[pr], kPk[pr], sp.kz, mu, exy, exz, eyz, A[comp], B[comp],
-                                        un, vn, wn, gh, part, comp == 0 && pr == 0);
+        chain(s, sp.grid, sp.block, fn)(g, K, kPi[pr], kPj[pr], kPk[pr], sp.kz, mu, exy, exz, eyz, A[comp], B[comp], un,
+                                        vn, wn, gh, part, comp == 0 && pr == 0);
         count_launch();
       };
       const bool own = fill && pr > 0;
@@ -1757,7 +1783,7 @@ void sweep_all(cudaStream_t s, const Grid& g, const VP& p, const T* mu, const T*
     }
   }
   if (!errsum) return;
-  k_sum_parts2<<<1, 1024, 0, s>>>(part, (long)sp.grid.x * sp.grid.y * sp.grid.z, errsum);
+  chain(s, 1, 1024, k_sum_parts2)(part, (long)sp.grid.x * sp.grid.y * sp.grid.z, errsum);
   count_launch();
 }
 }  // namespace
@@ -1786,7 +1812,7 @@ FlatFluid make_flat(cudaStream_t s, const Grid& g, double dxinv, double dyinv, d
   const VP p = make_vp(dxinv, dyinv, dzinv, dt, 0);
   if (mixed) {
     float2* pairs = (float2*)(bytes + g.n + 8);  // (g.n is a multiple of 8)
-    k_flat_pairs<<<1, 32, 0, s>>>(make_vps(p, 0.0, 0.0), fl, pairs);
+    chain(s, 1, 32, k_flat_pairs)(make_vps(p, 0.0, 0.0), fl, pairs);
     count_launch();
     f.pairs = pairs;
   }
@@ -1805,7 +1831,7 @@ FlatFluid make_flat(cudaStream_t s, const Grid& g, double dxinv, double dyinv, d
 
 void wall_coef(cudaStream_t s, const Grid& g, double dy, const double* l1, const double* l2, const double* phi,
                double* wallc) {
-  k_wall_coef<<<wall_grid(g), kB, 0, s>>>(g, dy, l1, l2, phi, wallc);
+  chain(s, wall_grid(g), kB, k_wall_coef)(g, dy, l1, l2, phi, wallc);
   count_launch();
 }
 
@@ -1828,17 +1854,17 @@ void explicit_viscous(cudaStream_t s, const Grid& g, double dxinv, double dyinv,
     p.dyi = split_double(dyinv);
     p.dzi = split_double(dzinv);
     float2* tp = (float2*)tau;
-    k_stress_e<<<tile_grid(g.ni + 2, g.nj + 2, g.nk + 2, 256), 256, 0, s>>>(g, p, uvw, u, v, w, mu, tp, sk);
-    k_div_stress_e<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, p, tp, vis[0], vis[1], vis[2]);
+    chain(s, tile_grid(g.ni + 2, g.nj + 2, g.nk + 2, 256), 256, k_stress_e)(g, p, uvw, u, v, w, mu, tp, sk);
+    chain(s, dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, k_div_stress_e)(g, p, tp, vis[0], vis[1], vis[2]);
     count_launch(2);
     return;
   }
   const StressK K{dxinv, dyinv, dzinv, dxinv / dyinv, dxinv / dzinv, dyinv / dzinv, 2.0 * dxinv * dxinv,
                   2.0 * dyinv * dyinv, 2.0 * dzinv * dzinv, 0.25 * dyinv * dyinv, 0.25 * dzinv * dzinv,
                   0.25 * dxinv * dyinv, 0.25 * dxinv * dzinv, 0.25 * dyinv * dzinv};
-  k_stress<<<dim3((unsigned)(((long)(g.ni + 2) * (g.nj + 2) + 127) / 128), (unsigned)(g.nk + 2)), 128, 0, s>>>(
+  chain(s, dim3((unsigned)(((long)(g.ni + 2) * (g.nj + 2) + 127) / 128), (unsigned)(g.nk + 2)), 128, k_stress)(
       g, K, u, v, w, mu, tau, sk);
-  k_div_stress<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, 0, s>>>(g, K, tau, vis[0], vis[1], vis[2]);
+  chain(s, dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), kB, k_div_stress)(g, K, tau, vis[0], vis[1], vis[2]);
   count_launch(2);
 }
 
@@ -1847,16 +1873,16 @@ void wall_halo(cudaStream_t s, const Grid& g, int normal, double uwall, const do
   if (one_pass_refresh(g)) {
     const long tw = refresh_tasks(g, 0), tx = refresh_tasks(g, 1), tz = refresh_tasks(g, 2);
     const int nbW = (int)((tw + 255) / 256), nbX = (int)((tx + 255) / 256), nbZ = (int)((tz + 255) / 256);
-    k_refresh<<<nbW + nbX + nbZ, 256, 0, s>>>(g, normal, Ghosts64{uwall, wallc}, un, vn, wn, nbW, nbX);
+    chain(s, nbW + nbX + nbZ, 256, k_refresh<double, Ghosts64>)(g, normal, Ghosts64{uwall, wallc}, un, vn, wn, nbW, nbX);
     count_launch();
     return;
   }
-  k_wall<<<wall_grid(g), kB, 0, s>>>(g, uwall, wallc, un, vn, wn);
+  chain(s, wall_grid(g), kB, k_wall)(g, uwall, wallc, un, vn, wn);
   if (g.ni >= 8)
-    k_halo_x8<<<(unsigned)((24L * (g.nj + 6) * (g.nk + 6) + 255) / 256), 256, 0, s>>>(g, normal, un, vn, wn);
+    chain(s, (unsigned)((24L * (g.nj + 6) * (g.nk + 6) + 255) / 256), 256, k_halo_x8)(g, normal, un, vn, wn);
   else
-    k_halo_x<<<xh_grid(g), kB, 0, s>>>(g, normal, un, vn, wn);
-  k_halo_z<<<zh_grid(g), kB, 0, s>>>(g, normal, un, vn, wn);
+    chain(s, xh_grid(g), kB, k_halo_x)(g, normal, un, vn, wn);
+  chain(s, zh_grid(g), kB, k_halo_z)(g, normal, un, vn, wn);
   count_launch(3);
 }
 
@@ -1872,13 +1898,14 @@ void sor_iteration(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
 }
 
 __global__ void k_sor_rule(SorLoop* L, double tol, int maxit, double cells) {
+  after_previous();
   L->tol = tol;
   L->maxit = maxit;
   L->cells = cells;
   L->nlog = 0;
 }
 void sor_rule(cudaStream_t s, SorLoop* L, double tol, int maxit, double cells) {
-  k_sor_rule<<<1, 1, 0, s>>>(L, tol, maxit, cells);
+  chain(s, 1, 1, k_sor_rule)(L, tol, maxit, cells);
   count_launch();
 }
 // whether a cluster of 16 blocks of the kernel fits this device (asked once per device)
@@ -1911,12 +1938,14 @@ static void solve_cluster(cudaStream_t s, const Grid& g, const SolveK<T>& K, con
   cfg.gridDim = kClusterBlocks;
   cfg.blockDim = kClusterThreads;
   cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = kClusterBlocks;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kClusterBlocks;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as chain
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
   FMF_CUDA(cudaLaunchKernelEx(&cfg, k_solve_cluster<T, G>, g, K, gh, L, log));
   count_launch();
 }
@@ -1963,10 +1992,10 @@ void refine_prep(cudaStream_t s, const Grid& g, double dxinv, double dyinv, doub
   // A and B in FP32 pairs, the residual in FP64 (k_src_ab_e)
   src_prep<true>(s, g, make_vp(dxinv, dyinv, dzinv, dt, harmonic), u, v, w, adv, advo, phat, vis, fst, fstn, grvb,
                  grvp, fl, mu, rho, rhon, E, F3{{rb.e[0], rb.e[1], rb.e[2]}}, out, l1, l2, phi, dy, wallc, flat);
-  k_to_float<<<4 * 152, 256, 0, s>>>(g.n, mu, rb.mu);
-  k_gamma_wall<<<wall_grid(g), kB, 0, s>>>(g, uwall, wallc, u, v, w, rb.gw);
-  k_gamma_x<<<xh_grid(g), kB, 0, s>>>(g, u, v, w, rb.gx);
-  k_gamma_z<<<zh_grid(g), kB, 0, s>>>(g, u, v, w, rb.gz);
+  chain(s, 4 * 152, 256, k_to_float)(g.n, mu, rb.mu);
+  chain(s, wall_grid(g), kB, k_gamma_wall)(g, uwall, wallc, u, v, w, rb.gw);
+  chain(s, xh_grid(g), kB, k_gamma_x)(g, u, v, w, rb.gx);
+  chain(s, zh_grid(g), kB, k_gamma_z)(g, u, v, w, rb.gz);
   count_launch(4);
   for (int q = 0; q < 3; ++q) FMF_CUDA(cudaMemsetAsync(rb.d[q], 0, sizeof(float) * g.n, s));
 }
@@ -1981,7 +2010,7 @@ void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dy
         if (one_pass_refresh(g) && !first) {  // the swept component's ghosts alone change
           const int nbW = (int)((refresh_tasks(g, 0) + 255) / 256), nbX = (int)((refresh_tasks(g, 1) / 3 + 255) / 256),
                     nbZ = (int)((refresh_tasks(g, 2) / 3 + 255) / 256);
-          k_refresh_one<<<nbW + nbX + nbZ, 256, 0, s>>>(g, normal >> 1, Ghosts32{rb.gw, rb.gx, rb.gz}, du, dv, dw, nbW,
+          chain(s, nbW + nbX + nbZ, 256, k_refresh_one)(g, normal >> 1, Ghosts32{rb.gw, rb.gx, rb.gz}, du, dv, dw, nbW,
                                                         nbX);
           count_launch();
           return;
@@ -1989,13 +2018,14 @@ void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dy
         if (one_pass_refresh(g)) {
           const long tw = refresh_tasks(g, 0), tx = refresh_tasks(g, 1), tz = refresh_tasks(g, 2);
           const int nbW = (int)((tw + 255) / 256), nbX = (int)((tx + 255) / 256), nbZ = (int)((tz + 255) / 256);
-          k_refresh<<<nbW + nbX + nbZ, 256, 0, s>>>(g, normal, Ghosts32{rb.gw, rb.gx, rb.gz}, du, dv, dw, nbW, nbX);
+          chain(s, nbW + nbX + nbZ, 256, k_refresh<float, Ghosts32>)(g, normal, Ghosts32{rb.gw, rb.gx, rb.gz}, du, dv, dw,
+                                                                     nbW, nbX);
           count_launch();
           return;
         }
-        k_wall_d<<<wall_grid(g), kB, 0, s>>>(g, rb.gw, du, dv, dw);
-        k_halo_x_d<<<xh_grid(g), kB, 0, s>>>(g, normal, rb.gx, du, dv, dw);
-        k_halo_z_d<<<zh_grid(g), kB, 0, s>>>(g, normal, rb.gz, du, dv, dw);
+        chain(s, wall_grid(g), kB, k_wall_d)(g, rb.gw, du, dv, dw);
+        chain(s, xh_grid(g), kB, k_halo_x_d)(g, normal, rb.gx, du, dv, dw);
+        chain(s, zh_grid(g), kB, k_halo_z_d)(g, normal, rb.gz, du, dv, dw);
         count_launch(3);
       },
       flat);
@@ -2003,7 +2033,7 @@ void sor_iteration_refine(cudaStream_t s, const Grid& g, double dxinv, double dy
 
 void refine_finish(cudaStream_t s, const Grid& g, const double* u, const double* v, const double* w,
                    const RefineBufs& rb, double* un, double* vn, double* wn) {
-  k_refine_finish<<<4 * 152, 256, 0, s>>>(g.n, u, v, w, rb.d[0], rb.d[1], rb.d[2], un, vn, wn);
+  chain(s, 4 * 152, 256, k_refine_finish)(g.n, u, v, w, rb.d[0], rb.d[1], rb.d[2], un, vn, wn);
   count_launch();
 }
 

@@ -70,6 +70,7 @@ struct SplitSrc {
 // six are skipped where *keep != 0 (their level's advection is carried over)
 template <int NF>
 __global__ void k_split(long n, SplitSrc src, float2* __restrict__ out, const int* __restrict__ keep) {
+  after_previous();
   const int nf = (NF == 6 && keep && *keep) ? 3 : NF;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
 #pragma unroll
@@ -133,6 +134,7 @@ __global__ void __launch_bounds__(128) k_weno2_f32(Grid g, int nlev, const int* 
                                                    double* __restrict__ av, double* __restrict__ aw,
                                                    double* __restrict__ auo, double* __restrict__ avo,
                                                    double* __restrict__ awo) {
+  after_previous();
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   const int k = 1 + (int)blockIdx.z;
@@ -193,6 +195,7 @@ __global__ void __launch_bounds__(128) k_weno2_df(Grid g, int nlev, const int* _
                                                   double* __restrict__ au, double* __restrict__ av,
                                                   double* __restrict__ aw, double* __restrict__ auo,
                                                   double* __restrict__ avo, double* __restrict__ awo) {
+  after_previous();
   using df::add;
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
@@ -254,6 +257,7 @@ __global__ void __launch_bounds__(32) k_weno_line(Grid g, int m, const int* __re
                                                    const double* __restrict__ u, const double* __restrict__ v,
                                                    const double* __restrict__ w, double* __restrict__ au,
                                                    double* __restrict__ av, double* __restrict__ aw) {
+  after_previous();
   if (keep && *keep) return;
   const int nl = DIR == 0 ? g.nj : g.ni, nr = DIR == 2 ? g.nj : g.nk;
   const int nm = DIR == 0 ? g.ni : (DIR == 1 ? g.nj : g.nk);
@@ -357,14 +361,14 @@ static void weno5_levels(cudaStream_t s, const Grid& g, int nlev, double dxi, do
     }
     const SplitSrc src{{u, v, w, uo, vo, wo}};
     if (nlev == 2)
-      k_split<6><<<152 * 8, 256, 0, s>>>(g.n, src, split, keep);
+      chain(s, 152 * 8, 256, k_split<6>)(g.n, src, split, keep);
     else
-      k_split<3><<<152 * 8, 256, 0, s>>>(g.n, src, split, nullptr);
+      chain(s, 152 * 8, 256, k_split<3>)(g.n, src, split, nullptr);
     if (prec == 1)
-      k_weno2_f32<<<gr, b, 0, s>>>(g, nlev, keep, (float)(dxi / 24.0), (float)(dyi / 24.0), (float)(dzi / 24.0),
+      chain(s, gr, b, k_weno2_f32)(g, nlev, keep, (float)(dxi / 24.0), (float)(dyi / 24.0), (float)(dzi / 24.0),
                                    split, adv[0], adv[1], adv[2], ao[0], ao[1], ao[2]);
     else
-      k_weno2_df<<<gr, b, 0, s>>>(g, nlev, keep, df::from_double_host(dxi / 24.0), df::from_double_host(dyi / 24.0),
+      chain(s, gr, b, k_weno2_df)(g, nlev, keep, df::from_double_host(dxi / 24.0), df::from_double_host(dyi / 24.0),
                                   df::from_double_host(dzi / 24.0), split, adv[0], adv[1], adv[2], ao[0], ao[1],
                                   ao[2]);
     count_launch(2);
@@ -389,9 +393,9 @@ static void weno5_levels(cudaStream_t s, const Grid& g, int nlev, double dxi, do
     const double *U = lev ? uo : u, *V = lev ? vo : v, *W = lev ? wo : w;
     double* const* o = lev ? ao : adv;
     const int* kp = lev ? keep : nullptr;
-    k_weno_line<0><<<grid(g.nj, g.nk, g.ni), 32, 0, s>>>(g, m, kp, dxi * (1.0 / 24.0), U, V, W, o[0], o[1], o[2]);
-    k_weno_line<1><<<grid(g.ni, g.nk, g.nj), 32, 0, s>>>(g, m, kp, dyi * (1.0 / 24.0), U, V, W, o[0], o[1], o[2]);
-    k_weno_line<2><<<grid(g.ni, g.nj, g.nk), 32, 0, s>>>(g, m, kp, dzi * (1.0 / 24.0), U, V, W, o[0], o[1], o[2]);
+    chain(s, grid(g.nj, g.nk, g.ni), 32, k_weno_line<0>)(g, m, kp, dxi * (1.0 / 24.0), U, V, W, o[0], o[1], o[2]);
+    chain(s, grid(g.ni, g.nk, g.nj), 32, k_weno_line<1>)(g, m, kp, dyi * (1.0 / 24.0), U, V, W, o[0], o[1], o[2]);
+    chain(s, grid(g.ni, g.nj, g.nk), 32, k_weno_line<2>)(g, m, kp, dzi * (1.0 / 24.0), U, V, W, o[0], o[1], o[2]);
     count_launch(3);
   }
 }
@@ -408,7 +412,7 @@ void weno5_one(cudaStream_t s, const Grid& g, double dxi, double dyi, double dzi
 }
 void split3(cudaStream_t s, const Grid& g, const double* a, const double* b, const double* c, float2* out) {
   const SplitSrc src{{a, b, c, nullptr, nullptr, nullptr}};
-  k_split<3><<<152 * 8, 256, 0, s>>>(g.n, src, out, nullptr);
+  chain(s, 152 * 8, 256, k_split<3>)(g.n, src, out, nullptr);
   count_launch();
 }
 

@@ -198,6 +198,7 @@ namespace {
 // formed once per block
 __global__ void __launch_bounds__(256) k_mthinc3_offset(Grid g, const double* __restrict__ sums,
                                                         double* __restrict__ phin) {
+  after_previous();
   __shared__ double off;
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
@@ -253,7 +254,7 @@ void solphi_mthinc3(cudaStream_t s, const Grid& g, double dxinv, double dyinv, d
         r[2] = p * p * (1.0 - p);
       },
       sums);
-  k_mthinc3_offset<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), dim3(32, 8), 0, s>>>(g, sums, phin);
+  chain(s, dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), dim3(32, 8), k_mthinc3_offset)(g, sums, phin);
   count_launch();
 }
 

@@ -38,6 +38,7 @@ namespace {
 // x-lines: one block per (j,k) row.  Forward: real div -> complex T(kx, j, k).
 __global__ void __launch_bounds__(256) k_fft_x_fwd(Grid g, const double* div, double* tr, double* ti,
                                                    const double2* tw) {
+  after_previous();
   extern __shared__ double sm[];
   const int L = g.ni;
   double* re = sm;
@@ -59,6 +60,7 @@ __global__ void __launch_bounds__(256) k_fft_x_fwd(Grid g, const double* div, do
 // Inverse x: complex T(kx, j, k) -> real part into dp(1..ni, j, k).
 __global__ void __launch_bounds__(256) k_fft_x_inv(Grid g, const double* tr, const double* ti, double* dp,
                                                    const double2* tw) {
+  after_previous();
   extern __shared__ double sm[];
   const int L = g.ni;
   double* re = sm;
@@ -80,6 +82,7 @@ constexpr int kTile = 16;  // x-wavenumbers per z-line block (16 threads per col
 // z-lines forward: T(kx, j, k) for kx in a tile -> phir(ix, j, iz) / (ni*nk), centred.
 __global__ void __launch_bounds__(256) k_fft_z_fwd(Grid g, const double* tr, const double* ti, double* pr,
                                                    double* pi, const double2* tw) {
+  after_previous();
   extern __shared__ double sm[];
   const int L = g.nk, NI = g.ni, NJ = g.nj;
   const int j = 1 + blockIdx.y;
@@ -106,6 +109,7 @@ __global__ void __launch_bounds__(256) k_fft_z_fwd(Grid g, const double* tr, con
 // z-lines inverse: phir(ix, j, iz) -> T(kx, j, k)
 __global__ void __launch_bounds__(256) k_fft_z_inv(Grid g, const double* pr, const double* pi, double* tr,
                                                    double* ti, const double2* tw) {
+  after_previous();
   extern __shared__ double sm[];
   const int L = g.nk, NI = g.ni, NJ = g.nj;
   const int j = 1 + blockIdx.y;
@@ -154,10 +158,10 @@ void fft_forward_planes(cudaStream_t s, const Grid& g, const double* div, double
   const long nm = g.cells();
   double* t = (double*)scratch(sizeof(double) * 2 * nm, 5);
   const double2 *twx = fft_twiddles(g.ni), *twz = fft_twiddles(g.nk);
-  k_fft_x_fwd<<<dim3(g.nj, g.nk), 256, sizeof(double) * 2 * g.ni, s>>>(g, div, t, t + nm, twx);
+  chain(s, dim3(g.nj, g.nk), 256, k_fft_x_fwd, sizeof(double) * 2 * g.ni)(g, div, t, t + nm, twx);
   const size_t smz = sizeof(double) * 2 * g.nk * kTile;
   cudaFuncSetAttribute(k_fft_z_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
-  k_fft_z_fwd<<<dim3(g.ni / kTile, g.nj), 256, smz, s>>>(g, t, t + nm, pr, pi, twz);
+  chain(s, dim3(g.ni / kTile, g.nj), 256, k_fft_z_fwd, smz)(g, t, t + nm, pr, pi, twz);
   count_launch(2);
 }
 // solp_fft_tdma3.f:20-45
@@ -167,8 +171,8 @@ void fft_inverse_planes(cudaStream_t s, const Grid& g, const double* pr, const d
   const double2 *twx = fft_twiddles(g.ni), *twz = fft_twiddles(g.nk);
   const size_t smz = sizeof(double) * 2 * g.nk * kTile;
   cudaFuncSetAttribute(k_fft_z_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz);
-  k_fft_z_inv<<<dim3(g.ni / kTile, g.nj), 256, smz, s>>>(g, pr, pi, t, t + nm, twz);
-  k_fft_x_inv<<<dim3(g.nj, g.nk), 256, sizeof(double) * 2 * g.ni, s>>>(g, t, t + nm, dp, twx);
+  chain(s, dim3(g.ni / kTile, g.nj), 256, k_fft_z_inv, smz)(g, pr, pi, t, t + nm, twz);
+  chain(s, dim3(g.nj, g.nk), 256, k_fft_x_inv, sizeof(double) * 2 * g.ni)(g, t, t + nm, dp, twx);
   count_launch(2);
 }
 
@@ -181,6 +185,7 @@ constexpr int kRowsAhead = 8;
 __global__ void __launch_bounds__(64) k_tdma(Grid g, double dx2r, double dz2r, double pi2_ni, double pi2_nk,
                                              const double* as_f, const double* an_f, const double* ap_f,
                                              double* pr, double* pi, double* at) {
+  after_previous();
   const int NI = g.ni, NJ = g.nj, NK = g.nk;
   const long mode = blockIdx.x * (long)blockDim.x + threadIdx.x, nmode = (long)NI * NK;
   if (mode >= nmode) return;
@@ -242,7 +247,7 @@ void tdma_modes(cudaStream_t s, const Grid& g, double rho, double dxinv, double 
   const double dx2r = dxinv * dxinv / rho, dz2r = dzinv * dzinv / rho;
   const double pi2_ni = pi_ * 2.0 / (double)g.ni, pi2_nk = pi_ * 2.0 / (double)g.nk;
   double* at = (double*)scratch(sizeof(double) * g.cells(), 4);
-  k_tdma<<<(unsigned)(((long)g.ni * g.nk + 63) / 64), 64, 0, s>>>(g, dx2r, dz2r, pi2_ni, pi2_nk, as_f, an_f, ap_f, pr, pi, at);
+  chain(s, (unsigned)(((long)g.ni * g.nk + 63) / 64), 64, k_tdma)(g, dx2r, dz2r, pi2_ni, pi2_nk, as_f, an_f, ap_f, pr, pi, at);
   count_launch();
 }
 

@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(256) k_advance(Grid g, double dxi, double dyi,
                                                  const double* __restrict__ fx, const double* __restrict__ fy,
                                                  const double* __restrict__ fz, const double* __restrict__ phi,
                                                  double* __restrict__ phin) {
+  after_previous();
   const Tile T = warp_tile(g.ni);
   const int i = 1 + T.x, j = 1 + T.y;
   if (i > g.ni || j > g.nj) return;
@@ -47,6 +48,7 @@ __global__ void __launch_bounds__(256) k_advance(Grid g, double dxi, double dyi,
 // (summation.f:222-264), takes the same values.
 __global__ void __launch_bounds__(256) k_offset(Grid g, const double* __restrict__ sums, double* __restrict__ phin,
                                                 double* __restrict__ phin0) {
+  after_previous();
   __shared__ double off;
   const Tile T = warp_tile(g.ni);
   const int i = 1 + T.x, j = 1 + T.y;
@@ -87,6 +89,7 @@ struct Mix {
 __global__ void __launch_bounds__(256) k_means4(long n, const double* __restrict__ p0, const double* __restrict__ p1,
                                                 Mix mix, double* __restrict__ rho, double* __restrict__ rhon,
                                                 double* __restrict__ rmu, double* __restrict__ rmun) {
+  after_previous();
   const long stride = (long)gridDim.x * blockDim.x;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += 2 * stride) {
     const long t2 = t + stride;
@@ -107,6 +110,7 @@ __global__ void __launch_bounds__(256) k_means4(long n, const double* __restrict
 // interior point (of one point of its row, without WALLS), which no thread writes.
 template <bool WALLS>
 __global__ void __launch_bounds__(256) k_halos(Grid g, long nx, long nz, double* __restrict__ q) {
+  after_previous();
   const int NI = g.ni, NJ = g.nj, NK = g.nk;
   auto wrap = [](int i, int n) { return i < 1 ? i + n : (i > n ? i - n : i); };
   auto row = [&](int j) { return !WALLS ? j : (j < 1 ? 1 - j : (j > NJ ? 2 * NJ + 1 - j : j)); };
@@ -137,7 +141,7 @@ template <bool WALLS>
 void halos(cudaStream_t s, const Grid& g, double* q) {
   const long nx = 6L * (g.nj + 6) * (g.nk + 6), nz = 6L * g.ni * (g.nj + 6);
   const long n = nx + nz + (WALLS ? 6L * g.ni * g.nk : 0);
-  k_halos<WALLS><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, nx, nz, q);
+  chain(s, (unsigned)((n + 255) / 256), 256, k_halos<WALLS>)(g, nx, nz, q);
   count_launch();
 }
 }  // namespace
@@ -148,7 +152,7 @@ void halo_neumann_periodic(cudaStream_t s, const Grid& g, double* q) { halos<tru
 void mthinc_advance(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt,
                     const double* u, const double* v, const double* w, const double* fx, const double* fy,
                     const double* fz, const double* phi, double* phin) {
-  k_advance<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, dxinv, dyinv, dzinv, dt, u, v, w, fx, fy, fz, phi, phin);
+  chain(s, tile_grid(g.ni, g.nj, g.nk, 256), 256, k_advance)(g, dxinv, dyinv, dzinv, dt, u, v, w, fx, fy, fz, phi, phin);
   count_launch();
 }
 
@@ -168,13 +172,13 @@ void mthinc_volume_fix(cudaStream_t s, const Grid& g, double dxinv, double dyinv
         r[2] = b == 0 || b == kOneBits ? 0.0 : p * p * (1.0 - p);
       },
       sums);
-  k_offset<<<tile_grid(g.ni, g.nj, g.nk, 256), 256, 0, s>>>(g, sums, phin, phin0);
+  chain(s, tile_grid(g.ni, g.nj, g.nk, 256), 256, k_offset)(g, sums, phin, phin0);
   count_launch();
 }
 
 void mixture_means(cudaStream_t s, const Grid& g, const double* phi0, const double* phin0, double rhol, double rhog,
                    double rmul, double rmug, double* rho, double* rhon, double* rmu, double* rmun) {
-  k_means4<<<152 * 8, 256, 0, s>>>(g.n, phi0, phin0, Mix{rhol, rhog, rmul, rmug}, rho, rhon, rmu, rmun);
+  chain(s, 152 * 8, 256, k_means4)(g.n, phi0, phin0, Mix{rhol, rhog, rmul, rmug}, rho, rhon, rmu, rmun);
   count_launch();
 }
 

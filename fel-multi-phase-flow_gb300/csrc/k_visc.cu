@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(256) k_sor_colour(Grid g, int is, int js, int 
                                                     const double* __restrict__ rhon, Coef15 cf,
                                                     const double* __restrict__ src, double* un, double* vn,
                                                     double* wn, double* part) {
+  after_previous();
   __shared__ double sh[256];
   const int tid = threadIdx.y * 32 + threadIdx.x;
   const int i = is + 2 * (int)(blockIdx.x * 32 + threadIdx.x);
@@ -129,6 +130,7 @@ __global__ void __launch_bounds__(256) k_sor_colour(Grid g, int is, int js, int 
 }
 
 __global__ void k_sum_parts(const double* part, long n, double* out) {
+  after_previous();
   __shared__ double sh[256];
   double a = 0.0;
   for (long t = threadIdx.x; t < n; t += 256) a += part[t];
@@ -162,11 +164,11 @@ void sor_iteration(cudaStream_t s, const Grid& g, double dt, const double* rho, 
     for (int col = 0; col < 8; ++col) {
       double* pp = part + (long)(comp * 8 + col) * nb;
       if (comp == 0)
-        k_sor_colour<0><<<grd, blk, 0, s>>>(g, isor[col], jsor[col], ksor[col], jmax, dtinv, rho, rhon, cf, src[0], un, vn, wn, pp);
+        chain(s, grd, blk, k_sor_colour<0>)(g, isor[col], jsor[col], ksor[col], jmax, dtinv, rho, rhon, cf, src[0], un, vn, wn, pp);
       else if (comp == 1)
-        k_sor_colour<1><<<grd, blk, 0, s>>>(g, isor[col], jsor[col], ksor[col], jmax, dtinv, rho, rhon, cf, src[1], un, vn, wn, pp);
+        chain(s, grd, blk, k_sor_colour<1>)(g, isor[col], jsor[col], ksor[col], jmax, dtinv, rho, rhon, cf, src[1], un, vn, wn, pp);
       else
-        k_sor_colour<2><<<grd, blk, 0, s>>>(g, isor[col], jsor[col], ksor[col], jmax, dtinv, rho, rhon, cf, src[2], un, vn, wn, pp);
+        chain(s, grd, blk, k_sor_colour<2>)(g, isor[col], jsor[col], ksor[col], jmax, dtinv, rho, rhon, cf, src[2], un, vn, wn, pp);
       count_launch();
       if (col % 2 == 1) {
         bndu(s, g, un, vn, wn, uwall, dy, l1, l2, phi);
@@ -174,7 +176,7 @@ void sor_iteration(cudaStream_t s, const Grid& g, double dt, const double* rho, 
       }
     }
   }
-  k_sum_parts<<<1, 256, 0, s>>>(part, nb * 24, errsum);
+  chain(s, 1, 256, k_sum_parts)(part, nb * 24, errsum);
   count_launch();
 }
 

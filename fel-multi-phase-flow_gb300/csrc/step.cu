@@ -125,6 +125,7 @@ struct Pairs3 {
   const double* b[3];
 };
 __global__ void k_same(long n, int nf, Pairs3 p, int* same) {
+  after_previous();
   bool eq = true;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
     for (int f = 0; f < nf; ++f)
@@ -133,6 +134,7 @@ __global__ void k_same(long n, int nf, Pairs3 p, int* same) {
 }
 // b[f] = a[f] unless *same (then they are equal already)
 __global__ void k_copy_unless(long n, int nf, Pairs3 p, const int* same) {
+  after_previous();
   if (*same) return;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
     for (int f = 0; f < nf; ++f) const_cast<double*>(p.b[f])[t] = p.a[f][t];
@@ -146,21 +148,26 @@ void verify_upload(cudaStream_t s, long n, int nf, const double* const* src, dou
     p.b[f] = dst[f];
   }
   FMF_CUDA(cudaMemsetAsync(same, 0xff, sizeof(int), s));
-  k_same<<<152 * 8, 256, 0, s>>>(n, nf, p, same);
-  k_copy_unless<<<152 * 8, 256, 0, s>>>(n, nf, p, same);
+  chain(s, 152 * 8, 256, k_same)(n, nf, p, same);
+  chain(s, 152 * 8, 256, k_copy_unless)(n, nf, p, same);
   count_launch(2);
 }
 
 __global__ void k_sor_log_reset(SorLoop* L) {
+  after_previous();
   L->nlog = 0;
   L->flags = 0;
 }
-__global__ void k_sor_begin(SorLoop* L) { L->it = 0; }
+__global__ void k_sor_begin(SorLoop* L) {
+  after_previous();
+  L->it = 0;
+}
 // After one outer iteration (its residual sum at *esum): the rule, the log entry of
 // a finished solve (iterations, capped and non-finite bits), and the condition of
 // the WHILE node (0 ends the loop).  The iteration count is bounded by maxit, itself
 // clamped to the 100000 fmf_ctx_set_sor allows, whatever the loop state holds.
 __global__ void k_sor_ctl(cudaGraphConditionalHandle h, const double* esum, SorLoop* L, int* log) {
+  after_previous();
   const double e = *esum;
   const int mx = min(max(L->maxit, 1), kSorMax);
   const int it = L->it + 1;
@@ -191,6 +198,7 @@ struct Vel3 {
   const double* q[3];
 };
 __global__ void __launch_bounds__(256) k_diff2(Grid g, Vel3 a, Vel3 b, Vel3 c, double* acc) {
+  after_previous();
   const int i = 1 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int j = 1 + (int)(blockIdx.y * blockDim.y + threadIdx.y);
   const int k = 1 + (int)blockIdx.z;
@@ -539,7 +547,7 @@ static void seg_pre2(fmf_ctx* c) {
   const Grid& g = c->g;
   cudaStream_t s = c->s;
   if (!c->small) {
-    k_sor_begin<<<1, 1, 0, s>>>(c->loop);  // the device stop rule's iteration count
+    chain(s, 1, 1, k_sor_begin)(c->loop);  // the device stop rule's iteration count
     count_launch();
   }
   const long n = g.n;
@@ -663,7 +671,7 @@ static cudaGraphExec_t solve_exec(fmf_ctx* c) {
          cudaSuccess;
     if (ok) {
       iter_kernels(c);
-      k_sor_ctl<<<1, 1, 0, c->s>>>(h, c->red + 8, c->loop, c->sorlog);
+      chain(c->s, 1, 1, k_sor_ctl)(h, c->red + 8, c->loop, c->sorlog);
       count_launch();
       cudaGraph_t captured = nullptr;
       ok = cudaStreamEndCapture(c->s, &captured) == cudaSuccess;
@@ -693,7 +701,7 @@ static void read_sor_log(fmf_ctx* c) {
   std::vector<int> lg((size_t)std::min(c->pending, kSorLog));
   FMF_CUDA(cudaMemcpyAsync(&h, c->loop, sizeof(SorLoop), cudaMemcpyDeviceToHost, c->s));
   FMF_CUDA(cudaMemcpyAsync(lg.data(), c->sorlog, sizeof(int) * lg.size(), cudaMemcpyDeviceToHost, c->s));
-  k_sor_log_reset<<<1, 1, 0, c->s>>>(c->loop);
+  chain(c->s, 1, 1, k_sor_log_reset)(c->loop);
   count_launch();
   FMF_CUDA(cudaStreamSynchronize(c->s));
   if (h.nlog != c->pending) set_status(FMF_ERR_CUDA);  // a solve that did not finish
@@ -1001,7 +1009,7 @@ int fmf_ctx_check_sor(fmf_ctx* c, double* out) {
   copy3(q64, qx);
   out[3] = iter64(qx) / e0;
   FMF_CUDA(cudaMemsetAsync(acc, 0, 2 * sizeof(double), s));
-  k_diff2<<<dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), dim3(32, 8), 0, s>>>(
+  chain(s, dim3((g.ni + 31) / 32, (g.nj + 7) / 8, g.nk), dim3(32, 8), k_diff2)(
       g, Vel3{{c->un, c->vn, c->wn}}, Vel3{{q64[0], q64[1], q64[2]}}, Vel3{{c->u, c->v, c->w}}, acc);
   count_launch();
   double h[2] = {0.0, 0.0};
