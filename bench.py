@@ -291,9 +291,9 @@ def fp64e_case(cfg, st0, steps, warmup, stream, fp64_ms):
     out["steps_compared"] = warmup + steps
     out["max_rel_err_vs_fp64"] = {k: _rel(states["fp64e"][f], states["fp64"][f], cfg) for k, f in FIELDS.items()}
     out["same_viscous_iterations"] = iters["fp64e"] == iters["fp64"]
-    out["precision"] = ("the FP64 step with its WENO5 advection, CSF force, viscous momentum factors and explicit "
+    out["precision"] = ("the FP64 step with its WENO5 advection and explicit "
                         "viscous term in FP32-pair arithmetic (two floats per value, about 48 significant bits) on "
-                        "the FP32 pipe; state, viscous sweeps, pressure solve, projection and volume sums FP64; "
+                        "the FP32 pipe; state, viscous solve, pressure solve, projection and volume sums FP64; "
                         "parity with the oracle at the FP64 step's 1e-10 (tests/test_gpu_fp64e.py)")
     return out
 

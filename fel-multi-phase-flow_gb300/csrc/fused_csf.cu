@@ -11,12 +11,13 @@
 //   n23 at (i,j+1/2,k+1/2) = N(mean over i-1/2, i+1/2),
 // N(v) = v/(|v| + 1e-30*|dxinv|) and vertex gradients from cal_grad_p2a.f:46-60.
 //
-// FP64 (the FP64 step): three kernels over the whole grid, k_csf_grad (the vertex
+// FP64 (the FP64 and the FP64-accurate step): three kernels over the whole grid, k_csf_grad (the vertex
 // gradients G), k_csf_normals (the four families) and k_csf_force, with G and the nine
 // normal components used in device memory (12 n doubles of workspace).
 //
-// FP32 (R = float, the mixed-precision step) and FP32 pairs (R = Pr, the FP64-accurate
-// step FMF_FP64E): one kernel, k_csf.  A block owns a 32 x 8 tile of (i,j) columns and
+// FP32 (R = float, the mixed-precision step) and FP32 pairs (R = Pr: fmf_dev_csf_fused in
+// FMF_FP64E, which needs no workspace; in the step the three kernels are faster, 203
+// against 245 us for a drop at 256x128x128): one kernel, k_csf.  A block owns a 32 x 8 tile of (i,j) columns and
 // marches over a chunk of k planes; each phi plane is converted once into a
 // shared-memory ring of three planes.  Vertex gradients G of planes k, k+1 and the
 // normals of planes k-1..k+1 live in shared memory; H(k+1) = G(k)+G(k+1) gives both

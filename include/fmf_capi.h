@@ -344,8 +344,9 @@ void fmf_dev_cal_advu_weno5(int ni, int nj, int nk, double dxinv, double dyinv, 
 int fmf_dev_weno5_fused(int precision, int ni, int nj, int nk, double dxinv, double dyinv,
                         double dzinv, const double* u, const double* v, const double* w,
                         double* adv_u, double* adv_v, double* adv_w);
-/* the fused step's CSF force of one phi field in a context precision, interior u, v,
- * w points (ni % 32 == 0, nj % 8 == 0); returns a status */
+/* the CSF force of one phi field, FMF_FP64 and FMF_MIXED as the fused step of that
+ * precision forms it, FMF_FP64E in FP32 pairs; interior u, v, w points (ni % 32 == 0,
+ * nj % 8 == 0); returns a status */
 int fmf_dev_csf_fused(int precision, int ni, int nj, int nk, double dx, double dy, double dz,
                       double rhol, double rhog, double sigma, const double* phi, double* fu,
                       double* fv, double* fw);
@@ -381,13 +382,13 @@ typedef struct {
   int precision;                  /* FMF_FP64, FMF_MIXED or FMF_FP64E */
 } fmf_params;
 /* FMF_FP64: every operation in FP64.  FMF_MIXED: FP32 WENO5, MTHINC, CSF and viscous
- * corrections (errors about 1e-6).  FMF_FP64E: the FP64 step with four of its
+ * corrections (errors about 1e-6).  FMF_FP64E: the FP64 step with two of its
  * FP64-pipe-bound stages in FP32-pair arithmetic (a value is the sum of two
- * floats, about 48 significant bits) on the FP32 pipe: the WENO5 advection, the
- * CSF force, the viscous solve's momentum factors (A, B) and the explicit viscous
- * term; each stage reads doubles, splits them into pairs with integer operations
- * and rounds its outputs to doubles once.  The state, the viscous sweeps, the
- * pressure solve, the projection and the volume sums stay FP64, and the step
+ * floats, about 48 significant bits) on the FP32 pipe: the WENO5 advection and the
+ * explicit viscous term; each stage splits the doubles it reads into pairs with
+ * integer operations and rounds its outputs to doubles once.  The state, the CSF
+ * force, the viscous solve (factors and sweeps), the pressure solve, the
+ * projection and the volume sums stay FP64, and the step
  * agrees with the oracle within the FP64 step's 1e-10 with the same viscous
  * iteration counts.  The WENO5 term agrees with FP64's to about 4e-13 of |vel|
  * dxi times the stencil's largest value (its differences are taken between split
