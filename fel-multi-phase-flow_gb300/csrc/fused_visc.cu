@@ -224,10 +224,11 @@ __global__ void k_flat_pairs(VPS p, Fluids fl, float2* __restrict__ out) {
   for (int q = 0; q < 3; ++q) out[4 * f + 1 + q] = make_float2(T[q].h, T[q].l);
 }
 // FE.pairs: a warp whose points are each in one fluid takes rho00 and T from there.  Bound
-// by the FP64 pipe (78 operations per cell).  At 256x128x128 872 us with the 80 registers
-// it would take and the FP64 pipe 65 % busy, 777 with 64 (four blocks per SM), 734 with
-// the floats rounded by integer operations (df::d2f) and the pairs of the pure fluids.
-__global__ void __launch_bounds__(256, 4) k_src_ab_e(Grid g, VPS p, VP pv, Fac<double> pd, SrcIn in, FlatE FE,
+// by the FP64 pipe (78 operations per cell, 80 % busy).  At 256x128x128 872 us with the 80
+// registers it would take, 777 with 64 (four blocks per SM), 734 with the floats rounded by
+// integer operations (df::d2f) and the pairs of the pure fluids, 651 with one copy of the
+// sums after both branches and six blocks per SM (five 685, seven 718).
+__global__ void __launch_bounds__(256, 6) k_src_ab_e(Grid g, VPS p, VP pv, Fac<double> pd, SrcIn in, FlatE FE,
                                                   const double* __restrict__ mu,
                                                   const double* __restrict__ exy, const double* __restrict__ exz,
                                                   const double* __restrict__ eyz, ABOut out) {
@@ -275,43 +276,32 @@ __global__ void __launch_bounds__(256, 4) k_src_ab_e(Grid g, VPS p, VP pv, Fac<d
     out.rf[q][c] = d2f(A * vn + B - __ldg(vel + c));
   };
   const D zero{0.0f, 0.0f};
+  D ru, rv, rw, Tu, Tv, Tw;  // rho00 and T of the components
   if (__any_sync(__activemask(), f == 2)) {
     const D r0n0 = add(L(in.rho, 0), L(in.rhon, 0)), mu0 = L(mu, 0);
-    {
-      const D r = scale(add(r0n0, add(L(in.rho, X), L(in.rhon, X))), 0.25f);
-      const D T = diag_e(p, r, p.dz2, add(L(exz, -Z), L(exz, 0)), p.dy2, add(L(exy, -Y), L(exy, 0)), p.dx2x2,
-                         add(mu0, L(mu, X)));
-      const double vn = visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
-      store(0, T, rsrc(0, in.u, r, p.grvb, X, pv.dxi), vn, in.u);
-    }
-    if (j <= g.nj - 1) {
-      const D r = scale(add(r0n0, add(L(in.rho, Y), L(in.rhon, Y))), 0.25f);
-      const D T = diag_e(p, r, p.dz2, add(L(eyz, -Z), L(eyz, 0)), p.dy2x2, add(mu0, L(mu, Y)), p.dx2,
-                         add(L(exy, -X), L(exy, 0)));
-      const double vn = visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
-      store(1, T, rsrc(1, in.v, r, p.grvp, Y, pv.dyi), vn, in.v);
-    }
-    {
-      const D r = scale(add(r0n0, add(L(in.rho, Z), L(in.rhon, Z))), 0.25f);
-      const D T = diag_e(p, r, p.dz2x2, add(mu0, L(mu, Z)), p.dy2, add(L(eyz, -Y), L(eyz, 0)), p.dx2,
-                         add(L(exz, -X), L(exz, 0)));
-      const double vn = visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w);
-      store(2, T, rsrc(2, in.w, r, zero, Z, pv.dzi), vn, in.w);
-    }
+    ru = scale(add(r0n0, add(L(in.rho, X), L(in.rhon, X))), 0.25f);
+    rv = scale(add(r0n0, add(L(in.rho, Y), L(in.rhon, Y))), 0.25f);
+    rw = scale(add(r0n0, add(L(in.rho, Z), L(in.rhon, Z))), 0.25f);
+    Tu = diag_e(p, ru, p.dz2, add(L(exz, -Z), L(exz, 0)), p.dy2, add(L(exy, -Y), L(exy, 0)), p.dx2x2, add(mu0, L(mu, X)));
+    Tv = diag_e(p, rv, p.dz2, add(L(eyz, -Z), L(eyz, 0)), p.dy2x2, add(mu0, L(mu, Y)), p.dx2, add(L(exy, -X), L(exy, 0)));
+    Tw = diag_e(p, rw, p.dz2x2, add(mu0, L(mu, Z)), p.dy2, add(L(eyz, -Y), L(eyz, 0)), p.dx2, add(L(exz, -X), L(exz, 0)));
   } else {
     auto P = [&](int q) {
       const float2 t = __ldg(FE.pairs + 4 * f + q);
       return D{t.x, t.y};
     };
-    const D r = P(0);
-    store(0, P(1), rsrc(0, in.u, r, p.grvb, X, pv.dxi),
-          visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w), in.u);
-    if (j <= g.nj - 1)
-      store(1, P(2), rsrc(1, in.v, r, p.grvp, Y, pv.dyi),
-            visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w), in.v);
-    store(2, P(3), rsrc(2, in.w, r, zero, Z, pv.dzi),
-          visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w), in.w);
+    ru = rv = rw = P(0);
+    Tu = P(1);
+    Tv = P(2);
+    Tw = P(3);
   }
+  store(0, Tu, rsrc(0, in.u, ru, p.grvb, X, pv.dxi),
+        visn_at<0, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w), in.u);
+  if (j <= g.nj - 1)
+    store(1, Tv, rsrc(1, in.v, rv, p.grvp, Y, pv.dyi),
+          visn_at<1, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w), in.v);
+  store(2, Tw, rsrc(2, in.w, rw, zero, Z, pv.dzi),
+        visn_at<2, double>(g, pd, c, mu, exy, exz, eyz, in.u, in.v, in.w), in.w);
 }
 
 // The explicit viscous term 2 div(mu S) of main.f90:538-541 (calsij, cal_arith_tau,
