@@ -69,6 +69,9 @@ struct fmf_ctx {
   cudaStream_t s = nullptr;
   bool own_stream = false;
   cudaStream_t cs = nullptr;                        // copies overlapping the step (fmf_ctx_step_host)
+  cudaStream_t br[2] = {};                          // branches of a captured step (seg_before)
+  cudaEvent_t ev_br[2] = {};
+  bool forks = false;                               // a step with branches is being captured
   // inputs up (u, v, w; phi(0); the rest); first part of the step done
   cudaEvent_t ev_in = nullptr, ev_in_phi0 = nullptr, ev_in2 = nullptr, ev_pre = nullptr;
   std::vector<void*> allocs;
@@ -357,6 +360,10 @@ int fmf_ctx_destroy(fmf_ctx* c) {
     cudaStreamSynchronize(c->cs);
     cudaStreamDestroy(c->cs);
   }
+  for (int b = 0; b < 2; ++b) {
+    if (c->br[b]) cudaStreamDestroy(c->br[b]);
+    if (c->ev_br[b]) cudaEventDestroy(c->ev_br[b]);
+  }
   if (c->ev_in) cudaEventDestroy(c->ev_in);
   if (c->ev_in_phi0) cudaEventDestroy(c->ev_in_phi0);
   if (c->ev_in2) cudaEventDestroy(c->ev_in2);
@@ -488,7 +495,7 @@ int fmf_ctx_init_bc(fmf_ctx* c) {
 // seg_post: main.f90:625-697 (pressure solve, projection, boundary conditions, rotation
 // of phin into phi).  The pointer rotation of u/uo/un, p/po/pn and phi/phin is done
 // on the host between steps.
-static void csf_one(fmf_ctx* c, const double* phi, double* const* f);
+static void csf_one(fmf_ctx* c, cudaStream_t s, const double* phi, double* const* f);
 
 // The first part in three pieces, so that the host-buffer step can start it while
 // inputs are still on their way: (a) reads phi(1) only, (b) u, v, w as well, (c)
@@ -499,7 +506,7 @@ static void seg_pre_a(fmf_ctx* c) {
   // :491 (the vertex gradients of phi(1))
   fused::vertex_gradient(c->s, c->g, dxinv, dyinv, dzinv, c->phi + c->g.n, c->phix, c->phiy, c->phiz);
 }
-static void seg_pre_b(fmf_ctx* c) {
+static void transport(fmf_ctx* c) {
   const fmf_params& P = c->prm;
   const Grid& g = c->g;
   cudaStream_t s = c->s;
@@ -519,20 +526,37 @@ static void seg_pre_b(fmf_ctx* c) {
   // with the interior of phin(0) (summation, :509)
   fused::mthinc_volume_fix(s, g, dxinv, dyinv, dzinv, P.bet_mthinc, c->phix, c->phiy, c->phiz, phi1, phin1, phin0,
                            c->red);
-  op::gnbc(s, g, c->u, c->w, P.uwall, c->theta0, P.sigma, c->zeta, c->theta);
-  op::bnd_contact_angle(s, g, phin1, c->theta, P.dx, P.dy, P.dz);
-  fused::halo_periodic(s, g, phin1);
+}
+// :498, and the contact-angle passes that read its theta
+static void wall_angles(fmf_ctx* c, cudaStream_t s) {
+  const fmf_params& P = c->prm;
+  op::gnbc(s, c->g, c->u, c->w, P.uwall, c->theta0, P.sigma, c->zeta, c->theta);
+}
+static void phin_ghosts(fmf_ctx* c) {
+  const fmf_params& P = c->prm;
+  op::bnd_contact_angle(c->s, c->g, c->phin + c->g.n, c->theta, P.dx, P.dy, P.dz);
+  fused::halo_periodic(c->s, c->g, c->phin + c->g.n);
   // :510-517 on phin (the contact-angle pass on phi(0) of :515, independent of
   // these, follows in part c)
-  fused::halo_neumann_periodic(s, g, phin0);
+  fused::halo_neumann_periodic(c->s, c->g, c->phin);
+}
+static void seg_pre_b(fmf_ctx* c) {
+  transport(c);
+  wall_angles(c, c->s);
+  phin_ghosts(c);
+}
+static void phi0_ghosts(fmf_ctx* c, cudaStream_t s) {
+  const fmf_params& P = c->prm;
+  op::bnd_contact_angle(s, c->g, c->phi, c->theta, P.dx, P.dy, P.dz);  // gnbc result unchanged since :498
+}
+static void means(fmf_ctx* c) {
+  const fmf_params& P = c->prm;
+  // :526-529
+  fused::mixture_means(c->s, c->g, c->phi, c->phin, P.rhol, P.rhog, P.rmul, P.rmug, c->rho, c->rhon, c->rmu, c->rmun);
 }
 static void seg_pre_c(fmf_ctx* c) {
-  const fmf_params& P = c->prm;
-  const Grid& g = c->g;
-  double* phi0 = c->phi;
-  op::bnd_contact_angle(c->s, g, phi0, c->theta, P.dx, P.dy, P.dz);  // gnbc result unchanged since :498
-  // :526-529
-  fused::mixture_means(c->s, g, phi0, c->phin, P.rhol, P.rhog, P.rmul, P.rmug, c->rho, c->rhon, c->rmu, c->rmun);
+  phi0_ghosts(c, c->s);
+  means(c);
 }
 static void seg_pre(fmf_ctx* c) {
   seg_pre_a(c);
@@ -540,6 +564,44 @@ static void seg_pre(fmf_ctx* c) {
   seg_pre_c(c);
 }
 
+// A captured step's branches: work that reads nothing the step's stream writes meanwhile.
+static void branch(fmf_ctx* c, int b, const std::function<void(cudaStream_t)>& work) {
+  FMF_CUDA(cudaEventRecord(c->ev_br[b], c->s));
+  FMF_CUDA(cudaStreamWaitEvent(c->br[b], c->ev_br[b]));
+  work(c->br[b]);
+  FMF_CUDA(cudaEventRecord(c->ev_br[b], c->br[b]));
+}
+static void join(fmf_ctx* c, int b) { FMF_CUDA(cudaStreamWaitEvent(c->s, c->ev_br[b])); }
+// the parts of the right-hand side that read u, v, w, uo, vo, wo, p and po alone
+static void advection(fmf_ctx* c, cudaStream_t s) {
+  const fmf_params& P = c->prm;
+  const Grid& g = c->g;
+  const double dxinv = 1.0 / P.dx, dyinv = 1.0 / P.dy, dzinv = 1.0 / P.dz;
+  // :532-541 (advo carried over from the previous step where the state continues)
+  if (c->verify)
+    fused::weno5_keep(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->uo, c->vo, c->wo, c->adv, c->advo, c->same,
+                      c->wprec, c->wsplit);
+  else if (c->cont)
+    fused::weno5_one(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->adv, c->wprec, c->wsplit);
+  else
+    fused::weno5_both(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->uo, c->vo, c->wo, c->adv, c->advo, c->wprec,
+                      c->wsplit);
+  op::calphat(s, g, c->p, c->po, c->phat);
+}
+// :545-570 surface tension (sfst carried over from the previous step's sfstn where the
+// state continues)
+static void surface_tension(fmf_ctx* c, cudaStream_t s) {
+  const fmf_params& P = c->prm;
+  const Grid& g = c->g;
+  const double dxinv = 1.0 / P.dx, dyinv = 1.0 / P.dy, dzinv = 1.0 / P.dz;
+  double *phi1 = c->phi + g.n, *phin1 = c->phin + g.n;
+  if (c->verify && fused::csf_supported(g))
+    fused::csf_force(s, g, dxinv, dyinv, dzinv, P.rhol, P.rhog, P.sigma, phi1, c->sfst[0], c->sfst[1], c->sfst[2],
+                     c->mixed, c->rn, c->same + 1);
+  else if (!c->cont || c->verify)
+    csf_one(c, s, phi1, c->sfst);
+  csf_one(c, s, phin1, c->sfstn);
+}
 // The rest of the step before the viscous solve: reads uo, vo, wo, p, po (the
 // first part reads u, v, w and phi only).
 static void seg_pre2(fmf_ctx* c) {
@@ -554,26 +616,13 @@ static void seg_pre2(fmf_ctx* c) {
   const double dxinv = 1.0 / P.dx, dyinv = 1.0 / P.dy, dzinv = 1.0 / P.dz, dt = P.dt;
   double* phi1 = c->phi + n;
   double* phin1 = c->phin + n;
-  // :532-541 (advo carried over from the previous step where the state continues)
-  if (c->verify)
-    fused::weno5_keep(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->uo, c->vo, c->wo, c->adv, c->advo, c->same,
-                      c->wprec, c->wsplit);
-  else if (c->cont)
-    fused::weno5_one(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->adv, c->wprec, c->wsplit);
-  else
-    fused::weno5_both(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->uo, c->vo, c->wo, c->adv, c->advo, c->wprec,
-                      c->wsplit);
-  op::calphat(s, g, c->p, c->po, c->phat);
+  if (!c->forks) advection(c, s);
   fused::explicit_viscous(s, g, dxinv, dyinv, dzinv, c->u, c->v, c->w, c->rmu, c->tau, c->vis, nullptr,
                           c->wprec ? c->wsplit : nullptr);
-  // :545-570 surface tension (sfst carried over from the previous step's sfstn where
-  // the state continues)
-  if (c->verify && fused::csf_supported(g))
-    fused::csf_force(s, g, dxinv, dyinv, dzinv, P.rhol, P.rhog, P.sigma, phi1, c->sfst[0], c->sfst[1], c->sfst[2],
-                     c->mixed, c->rn, c->same + 1);
-  else if (!c->cont || c->verify)
-    csf_one(c, phi1, c->sfst);
-  csf_one(c, phin1, c->sfstn);
+  if (c->forks)
+    join(c, 1);
+  else
+    surface_tension(c, s);
   // :579-603 (cal_av of rho/rhon at :571-573 feeds nothing downstream)
   const double* advp[3] = {c->adv[0], c->adv[1], c->adv[2]};
   const double* advop[3] = {c->advo[0], c->advo[1], c->advo[2]};
@@ -603,10 +652,9 @@ static void seg_pre2(fmf_ctx* c) {
 // The surface tension of one field (the force on the u, v, w points): the fused
 // kernel, or the reference's sequence of subroutines on grids it does not tile (ni
 // not a multiple of 32 or nj not a multiple of 8).
-static void csf_one(fmf_ctx* c, const double* phi, double* const* f) {
+static void csf_one(fmf_ctx* c, cudaStream_t s, const double* phi, double* const* f) {
   const fmf_params& P = c->prm;
   const Grid& g = c->g;
-  cudaStream_t s = c->s;
   const long n = g.n;
   const double dxinv = 1.0 / P.dx, dyinv = 1.0 / P.dy, dzinv = 1.0 / P.dz;
   if (fused::csf_supported(g)) {
@@ -753,7 +801,27 @@ static void seg_small(fmf_ctx* c) {
 }
 // the parts of a step that nothing on the host interrupts, as one segment (one graph)
 static void seg_before(fmf_ctx* c) {
-  seg_pre(c);
+  if (!c->forks) {
+    seg_pre(c);
+    seg_pre2(c);
+    return;
+  }
+  // beside the transport, the advection and phat (0), the wall angles and phi(0)'s ghosts
+  // (1); beside the means and the explicit viscous term, the surface tension (1)
+  // (20 steps of 32x32x16 7.75 -> 7.18 ms, 4 of 256x128x128 32.3 -> 31.3: the plane kernels
+  // and reductions leave most of the chip)
+  branch(c, 0, [&](cudaStream_t s) { advection(c, s); });
+  branch(c, 1, [&](cudaStream_t s) {
+    wall_angles(c, s);
+    phi0_ghosts(c, s);
+  });
+  seg_pre_a(c);
+  transport(c);
+  join(c, 1);
+  phin_ghosts(c);
+  branch(c, 1, [&](cudaStream_t s) { surface_tension(c, s); });
+  means(c);
+  join(c, 0);
   seg_pre2(c);
 }
 static void seg_all(fmf_ctx* c) {
@@ -762,6 +830,14 @@ static void seg_all(fmf_ctx* c) {
   seg_post(c);
 }
 
+// the branches' streams, made once
+static bool branches(fmf_ctx* c) {
+  for (int b = 0; b < 2; ++b)
+    if (!c->br[b] && (!FMF_CUDA(cudaStreamCreateWithFlags(&c->br[b], cudaStreamNonBlocking)) ||
+                      !FMF_CUDA(cudaEventCreateWithFlags(&c->ev_br[b], cudaEventDisableTiming))))
+      return false;
+  return true;
+}
 // Runs one segment: eagerly, or as a CUDA graph captured the first time this
 // segment is met with the current set of rotating buffer pointers and replayed
 // afterwards (the rotation cycles through six pointer sets).
@@ -778,8 +854,10 @@ static void run_segment(fmf_ctx* c, int id, void (*fn)(fmf_ctx*)) {
     const long long l0 = launches();
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
+    c->forks = (id == 7 || id == 8) && !c->verify && branches(c);
     if (!FMF_CUDA(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeRelaxed))) return;
     fn(c);
+    c->forks = false;
     if (!FMF_CUDA(cudaStreamEndCapture(c->s, &graph))) return;
     if (!FMF_CUDA(cudaGraphInstantiate(&exec, graph, 0))) {
       cudaGraphDestroy(graph);
