@@ -139,9 +139,9 @@ __global__ void __launch_bounds__(256) k_src_ab(Grid g, SrcK K, SrcIn in, const 
   after_previous();
   const Tile T = warp_tile(g.ni);
   const int i = 1 + T.x, j = 1 + T.y, k = 1 + (int)blockIdx.z;
-  if (i > g.ni || j > g.nj) return;
+  const bool here = i <= g.ni && j <= g.nj;  // (the count below takes every thread)
   const long X = 1, Y = g.sy, Z = g.sz;
-  const long c = g.at(i, j, k);
+  const long c = here ? g.at(i, j, k) : g.at(1, 1, k);
   auto L = [&](const double* a, long o) { return __ldg(a + c + o); };
   const double r0 = L(in.rho, 0), rx = L(in.rho, X), ry = L(in.rho, Y), rz = L(in.rho, Z);
   const double n0 = L(in.rhon, 0), nx = L(in.rhon, X), ny = L(in.rhon, Y), nz = L(in.rhon, Z);
@@ -153,10 +153,11 @@ __global__ void __launch_bounds__(256) k_src_ab(Grid g, SrcK K, SrcIn in, const 
                     same_bits(m0, xyx, xyy, xz0, xzx) && same_bits(m0, xzz, yz0, yzy, yzz);
   const int f = flat && rb == K.rb[0] && mb == K.mb[0] ? 0 : (flat && rb == K.rb[1] && mb == K.mb[1] ? 1 : -1);
   if (K.fluid) {
-    K.fluid[c] = (unsigned char)(f < 0 ? 2 : f);
-    const int flats = __syncthreads_count(f >= 0);
+    if (here) K.fluid[c] = (unsigned char)(f < 0 ? 2 : f);
+    const int flats = __syncthreads_count(here && f >= 0);
     if (threadIdx.x == 0 && flats) atomicAdd(K.count, flats);
   }
+  if (!here) return;
   double su, sv, sw, Au, Av, Aw;
   if (__any_sync(__activemask(), f < 0)) {
     const double s0 = r0 + n0;
@@ -236,9 +237,9 @@ __global__ void __launch_bounds__(256, 6) k_src_ab_e(Grid g, VPS p, VP pv, Fac<d
   using namespace df;
   const Tile tile = warp_tile(g.ni);
   const int i = 1 + tile.x, j = 1 + tile.y, k = 1 + (int)blockIdx.z;
-  if (i > g.ni || j > g.nj) return;
+  const bool here = i <= g.ni && j <= g.nj;  // (the count below takes every thread)
   const long X = 1, Y = g.sy, Z = g.sz;
-  const long c = g.at(i, j, k);
+  const long c = here ? g.at(i, j, k) : g.at(1, 1, k);
   int f = 2;
   {
     auto V = [&](const double* a, long o) { return __ldg(a + c + o); };
@@ -254,10 +255,11 @@ __global__ void __launch_bounds__(256, 6) k_src_ab_e(Grid g, VPS p, VP pv, Fac<d
     if (flat && rb == FE.rb[0] && mb == FE.mb[0]) f = 0;
   }
   if (FE.fluid) {
-    FE.fluid[c] = (unsigned char)f;
-    const int flats = __syncthreads_count(f != 2);
+    if (here) FE.fluid[c] = (unsigned char)f;
+    const int flats = __syncthreads_count(here && f != 2);
     if (threadIdx.x == 0 && flats) atomicAdd(FE.count, flats);
   }
+  if (!here) return;
   auto L = [&](const double* a, long o) { return split_double(__ldg(a + c + o)); };
   // rho00 * src; the pressure gradient as cal_grad_prs rounds it
   const double p0 = __ldg(in.phat + c);

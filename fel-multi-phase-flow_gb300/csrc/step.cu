@@ -854,8 +854,9 @@ static void run_segment(fmf_ctx* c, int id, void (*fn)(fmf_ctx*)) {
     const long long l0 = launches();
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    c->forks = (id == 7 || id == 8) && !c->verify && branches(c);
+    const bool forks = (id == 7 || id == 8) && !c->verify && branches(c);
     if (!FMF_CUDA(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeRelaxed))) return;
+    c->forks = forks;
     fn(c);
     c->forks = false;
     if (!FMF_CUDA(cudaStreamEndCapture(c->s, &graph))) return;
