@@ -112,6 +112,7 @@ __global__ void __launch_bounds__(64, GRAD ? 10 : 16) k_pair_T(Grid g, SwK K, in
       if (hx) *px = 0.0;
       if (hz) *pz = 0.0;
       if (hx && hz) *pxz = 0.0;
+      l[c] = 0.0;  // also where the images cancel it
     }
   }
   if (m == 0.0) return;
