@@ -1,6 +1,7 @@
 // bits.cuh -- tests on a double's bits.  A double comparison, minimum or maximum takes a
 // slot of the FP64 pipe (64 cycles per warp and quarter SM on GB300); these do not.
 #pragma once
+#include "snap.cuh"
 
 namespace fmf {
 
@@ -31,15 +32,8 @@ __device__ __forceinline__ double clip01(double p) {
   if (b > kOneBits || is_nan(p)) return 1.0;
   return b < 0 ? 0.0 : p;
 }
-// p <= eps gives 0 and 1 - p <= eps gives 1 (solphi_mthinc1.f, solphi_mthinc3.f): eps > 0 as
-// bits, and the smallest double t with 1 - t <= eps as bits (one_minus, below)
-__device__ __forceinline__ double snap01(double p, long long eps, long long one_eps) {
-  const long long b = raw(p);
-  if (is_nan(p)) return p;
-  if (b <= eps) return 0.0;
-  return b >= one_eps ? 1.0 : p;
-}
-
+// the snap of phi outside the band
+__device__ __forceinline__ double snap01(double p, const Snap& s) { return snapped(p, raw(p), s); }
 
 // The point of this thread in a plane of w points a row (from (0, 0); may be past the
 // ends); blockIdx.z is the plane.  A warp takes 8 x 4 points, so that of the warps that

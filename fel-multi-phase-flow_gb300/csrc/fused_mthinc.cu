@@ -24,7 +24,6 @@
 // interior row gets exactly one writer (solphi_mthinc1.f:121-130 zeroes first;
 // faces nobody donates through hold the zero written by k_classify's owner).
 #include <cmath>
-#include <cstring>
 
 #include "bits.cuh"
 #include "fused.cuh"
@@ -38,7 +37,7 @@ struct MC {
   double gp1, gp2, lim, bet, dt, dxi, dyi, dzi;
   double lim2lo, lim2hi;  // lim^2 (1 -/+ 1e-12)
   double dtdx, dtdy, dtdz;  // dt dxinv etc.
-  long long eps, one_eps;   // eps_trunc and the smallest t with 1 - t <= eps_trunc, as bits
+  Snap snap;                // with eps_trunc
 };
 // the constants of solphi_mthinc1.f and solphi_mthinc3.f (dt = 0 for the latter)
 MC make_mc(double dxinv, double dyinv, double dzinv, double dt, double bet) {
@@ -51,12 +50,7 @@ MC make_mc(double dxinv, double dyinv, double dzinv, double dt, double bet) {
   m.lim = bet / (2.0 * (ch * ch)) * dcellinv;
   m.lim2lo = m.lim * m.lim * (1.0 - 1.0e-12);
   m.lim2hi = m.lim * m.lim * (1.0 + 1.0e-12);
-  const double eps = 0.5 * (std::tanh(-bet * 2.5) + 1.0);
-  double t = 1.0 - eps;
-  while (1.0 - t > eps) t = std::nextafter(t, 2.0);
-  while (1.0 - std::nextafter(t, 0.0) <= eps) t = std::nextafter(t, 0.0);
-  std::memcpy(&m.eps, &eps, sizeof(double));
-  std::memcpy(&m.one_eps, &t, sizeof(double));
+  m.snap = make_snap(0.5 * (std::tanh(-bet * 2.5) + 1.0));
   m.bet = bet;
   m.dt = dt;
   m.dxi = dxinv;
@@ -170,7 +164,7 @@ __global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double*
     const int slot = atomicAdd(count, 1);
     list[slot] = (int)c;
   }
-  const double phi00 = band ? 0.0 : snap01(__ldg(phi + c), m.eps, m.one_eps);
+  const double phi00 = band ? 0.0 : snap01(__ldg(phi + c), m.snap);
   // owned faces: east/north/top when the velocity there is >= 0 (this cell donates or
   // the flux is zero), west/south/bottom when < 0; band cells leave the donated
   // faces to k_band but still zero the owned faces they do not donate through.
@@ -476,7 +470,7 @@ __global__ void __launch_bounds__(256) k_snap(Grid g, MC m, const double* __rest
   G8 ax, ay, az;
   const bool graded = (ax.load(gx, c, X, Y, Z) | ay.load(gy, c, X, Y, Z) | az.load(gz, c, X, Y, Z)) != 0;
   double p = phin[c];
-  if (!__any_sync(__activemask(), graded) || outside_band(ax, ay, az, m)) p = snap01(p, m.eps, m.one_eps);
+  if (!__any_sync(__activemask(), graded) || outside_band(ax, ay, az, m)) p = snap01(p, m.snap);
   if (i >= 1 && i <= g.ni && j >= 1 && j <= g.nj && k >= 1 && k <= g.nk) p = clip01(p);
   phin[c] = p;
 }
