@@ -53,6 +53,8 @@ void halo_neumann_periodic(cudaStream_t s, const Grid& g, double* q);
 void mixture_means(cudaStream_t s, const Grid& g, const double* phi0, const double* phin0, double rhol, double rhog,
                    double rmul, double rmug, double* rho, double* rhon, double* rmu, double* rmun);
 
+// whether mthinc_fluxes' FP64 form for this steepness is its fast one (see there)
+bool band_in_y(double bet);
 // solphi_mthinc1 for the faces solphi_mthinc2 reads (every face of rows 1..n in
 // the two directions normal to it, faces 0..n along it); list/count: device scratch
 // of >= (ni+2)(nj+2)(nk+2) ints and one int.  newton (optional, 2 (ni+2)(nj+2)(nk+2)

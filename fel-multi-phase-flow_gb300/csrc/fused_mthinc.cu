@@ -101,8 +101,15 @@ __device__ __forceinline__ double avg8(const double* __restrict__ p, long c, lon
          0.125;
 }
 
+__device__ __forceinline__ double ex(double x) { return exp(x); }
 __device__ __forceinline__ float ex(float x) { return expf(fminf(x, 80.0f)); }
 
+// 1/(1+e) for e >= 0: the division-free reciprocal in double (an overflowed e gives
+// exactly 0, as the quotient does; NaN stays NaN), the quotient in float
+__device__ __forceinline__ double inv1p(double e) {
+  const double a = 1.0 + e;
+  return (__double2hiint(a) == 0x7ff00000 && __double2loint(a) == 0) ? 0.0 : recip_nr(a);
+}
 __device__ __forceinline__ float inv1p(float e) { return 1.0f / (1.0f + e); }
 
 // The sum over the 8 Gauss points t of w/(1+exp(m2b (a_t + d))) (m2b = -2 bet) and,
@@ -121,7 +128,7 @@ __device__ __forceinline__ R sig8f(const R* E, R w, R ed, R* sd) {
     const R e = E[t] * ed;
     const R r = inv1p(e);
     s += r;
-    if (sd) q += e * r * r;
+    if (sd) q += r == (R)0 ? (R)0 : e * r * r;  // (an overflowed e: 0 times infinity)
   }
   if (sd) *sd = q;
   return w * s;
@@ -212,10 +219,13 @@ __global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double*
   if (k == g.nk + 1 && !t_) fz[c] = 0.0;
 }
 
-// The mixed-precision step (normal, band test and the fluxes' storage stay double; the
-// Newton solve and the Gauss-point integrals run in float with the exponent argument
-// clamped to the float range and the Newton regularisation 1e-99 raised to 1e-30).
-__global__ void __launch_bounds__(128) k_band_f32(Grid g, MC m, const double* __restrict__ phi,
+// The ten Newton steps on the offset itself.  R = float: the mixed-precision step (normal,
+// band test and the fluxes' storage stay double; the Newton solve and the Gauss-point
+// integrals run in float with the exponent argument clamped to the float range and the
+// Newton regularisation 1e-99 raised to 1e-30).  R = double: FP64 outside the steepnesses
+// of k_band below (band_in_y).
+template <class R>
+__global__ void __launch_bounds__(128) k_band_ten(Grid g, MC m, const double* __restrict__ phi,
                                               const double* __restrict__ gx, const double* __restrict__ gy,
                                               const double* __restrict__ gz, const double* __restrict__ u,
                                               const double* __restrict__ v, const double* __restrict__ w,
@@ -224,11 +234,10 @@ __global__ void __launch_bounds__(128) k_band_f32(Grid g, MC m, const double* __
                                               const int* __restrict__ count, double* __restrict__ newton,
                                               long cap) {
   after_previous();
-  using R = float;
   const int n = *count;
   const long X = 1, Y = g.sy, Z = g.sz;
   const R m2b = (R)(-2.0 * m.bet), gp1 = (R)m.gp1, gp2 = (R)m.gp2, bet = (R)m.bet, dtt = (R)m.dt;
-  const R reg = (R)1.0e-30;
+  const R reg = sizeof(R) == 8 ? (R)1.0e-99 : (R)1.0e-30;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const long c = list[e];
     double nx = avg8(gx, c, X, Y, Z), ny = avg8(gy, c, X, Y, Z), nz = avg8(gz, c, X, Y, Z);
@@ -248,14 +257,15 @@ __global__ void __launch_bounds__(128) k_band_f32(Grid g, MC m, const double* __
       const R f = sig8f<R>(E, (R)0.125, ex(m2b * ddd), &sd) - ph;
       // df = 0.5 bet sum 0.125/cosh^2 = 0.5 bet * 0.125 * 4 * sum s(1-s)
       const R df = (R)0.25 * bet * sd;
-      step = f * df / (df * df + reg);
+      step = sizeof(R) == 8 ? (R)((double)(f * df) * recip_nr((double)(df * df + reg))) : f * df / (df * df + reg);
       const R dn = ddd - step;
       // once d no longer changes, every remaining iteration recomputes the same
-      // f, df and step; the iterate can dither in its last bit instead, so a step
-      // below float precision ends the loop as well.
+      // f, df and step: stopping here is the ten-step result bit for bit.  In
+      // float the iterate can dither in its last bit instead; there a step below
+      // float precision ends the loop.
       if (dn == ddd) break;
       ddd = dn;
-      if (fabs((double)step) <= 1.0e-7 * (1.0 + fabs((double)ddd))) break;
+      if (sizeof(R) == 4 && fabs((double)step) <= 1.0e-7 * (1.0 + fabs((double)ddd))) break;
     }
     if (newton) {
       newton[e] = (double)ddd;
@@ -502,6 +512,17 @@ static const Exp16& exp16_table() {
   return table;
 }
 
+// Up to bet = 4 the ten Newton steps converge or approach their root from one side, and
+// either form gives the reference's fluxes to rounding.  Beyond, cells with phi near 0 or 1
+// overshoot into the flat tail, where the tenth iterate multiplies every rounding.  Largest
+// difference of phi from the oracle after a step, 786 432 cells of random phi, the ten
+// steps on the offset itself and k_band's form: 7.8e-16 and 7.8e-16 at 4, 3.8e-11 and
+// 1.3e-10 at 6, 9.3e-11 and 3.2e-9 at 8, 1.5e-8 and 2.4e-6 at 12 (cells beyond 1e-13: 64
+// and 100, 260 and 476, 833 and 276 128).  The fluxes of a couette 128x64x64 at 4.01 take 586
+// us in the former, 379 in the latter.  bet <= 0 (a profile the wrong way round) takes the
+// former as well.
+bool band_in_y(double bet) { return bet > 0.0 && bet <= 4.0; }
+
 void mthinc_fluxes(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, double dt, double bet,
                    const double* phi, const double* gx, const double* gy, const double* gz, const double* u,
                    const double* v, const double* w, double* fx, double* fy, double* fz, int* list, int* count,
@@ -511,7 +532,9 @@ void mthinc_fluxes(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
   chain(s, tile_grid(g.ni + 2, g.nj + 2, g.nk + 2, 256), 256, k_classify)(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count);
   const long cap = (long)(g.ni + 2) * (g.nj + 2) * (g.nk + 2);
   if (fp32)
-    chain(s, 152 * 8, 128, k_band_f32)(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
+    chain(s, 152 * 8, 128, k_band_ten<float>)(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
+  else if (!band_in_y(bet))
+    chain(s, 152 * 8, 128, k_band_ten<double>)(g, m, phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
   else
     chain(s, 152 * 16, 64, k_band)(g, m, exp16_table(), phi, gx, gy, gz, u, v, w, fx, fy, fz, list, count, newton, cap);
   count_launch(2);

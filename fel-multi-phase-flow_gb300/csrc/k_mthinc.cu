@@ -94,10 +94,9 @@ void solphi_mthinc1(cudaStream_t s, const Grid& g, double dxinv, double dyinv, d
   });
   // The fused step's kernels (cells outside the band at once, the band's compacted) give
   // the same fluxes to rounding in a twelfth of the time (1109 -> 87 us at 64x32x32)
-  // while the ten Newton steps converge or approach their root from one side.  Beyond bet of
-  // about 4 they overshoot into the flat tail, where the tenth iterate depends on every
-  // rounding: there the reference's operations one by one, as below.
-  if (bet <= 4.0) {
+  // where the Newton steps are well conditioned; elsewhere the reference's operations one
+  // by one, as below.
+  if (fused::band_in_y(bet)) {
     const long nb = (long)(g.ni + 2) * (g.nj + 2) * (g.nk + 2);
     int* band = (int*)scratch(sizeof(int) * (nb + 1), 0);
     if (!band) return;
