@@ -932,13 +932,15 @@ int fmf_dev_csf_fused(int precision, int ni, int nj, int nk, double dx, double d
   const Grid g(ni, nj, nk);
   if (!phi || !fu || !fv || !fw || precision < FMF_FP64 || precision > FMF_FP64E || !fused::csf_supported(g))
     return FMF_ERR_ARG;
-  double* work[4] = {nullptr, nullptr, nullptr, nullptr};
   if (precision == FMF_FP64) {
-    double* w = (double*)scratch(sizeof(double) * 12 * g.n, 8);
-    if (!w) return take_status();
-    for (int q = 0; q < 4; ++q) work[q] = w + 3 * q * g.n;
+    const Workspace ws(sizeof(double) * 12 * g.n, stream());
+    if (!ws.p) return take_status();
+    double* work[4];
+    for (int q = 0; q < 4; ++q) work[q] = (double*)ws.p + 3 * q * g.n;
+    fused::csf_force(stream(), g, 1.0 / dx, 1.0 / dy, 1.0 / dz, rhol, rhog, sigma, phi, fu, fv, fw, precision, work);
+  } else {
+    fused::csf_force(stream(), g, 1.0 / dx, 1.0 / dy, 1.0 / dz, rhol, rhog, sigma, phi, fu, fv, fw, precision, nullptr);
   }
-  fused::csf_force(stream(), g, 1.0 / dx, 1.0 / dy, 1.0 / dz, rhol, rhog, sigma, phi, fu, fv, fw, precision, work);
   FMF_CUDA(cudaGetLastError());
   return take_status();
 }

@@ -35,6 +35,18 @@ bool cuda_ok(cudaError_t e, const char* where);
 void count_launch(int n = 1);
 cudaStream_t stream();
 void* scratch(size_t bytes, int slot);  // per-slot growable device scratch (library owned)
+// Device memory for the kernels one call enqueues on stream s, taken and given back in the
+// order of that stream: calls on several streams or from several threads have their own,
+// and a call that is captured leaves it to the graph (p null and a status where there is
+// none).
+struct Workspace {
+  void* p = nullptr;
+  cudaStream_t s;
+  Workspace(size_t bytes, cudaStream_t stream);
+  ~Workspace();
+  Workspace(const Workspace&) = delete;
+  Workspace& operator=(const Workspace&) = delete;
+};
 
 // Programmatic dependent launch: chain(s, grid, block, kernel, smem)(arguments) is the
 // launch of kernel with these, whose start is set up while the kernel before it in the

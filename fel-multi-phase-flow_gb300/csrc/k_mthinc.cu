@@ -98,8 +98,9 @@ void solphi_mthinc1(cudaStream_t s, const Grid& g, double dxinv, double dyinv, d
   // by one, as below.
   if (fused::band_in_y(bet)) {
     const long nb = (long)(g.ni + 2) * (g.nj + 2) * (g.nk + 2);
-    int* band = (int*)scratch(sizeof(int) * (nb + 1), 0);
-    if (!band) return;
+    const Workspace ws(sizeof(int) * (nb + 1), s);
+    if (!ws.p) return;
+    int* band = (int*)ws.p;
     fused::mthinc_fluxes(s, g, dxinv, dyinv, dzinv, dt, bet, phi, phix, phiy, phiz, u, v, w, flx, fly, flz, band,
                          band + nb);
     return;

@@ -90,6 +90,55 @@ void* scratch(size_t bytes, int slot) {
   return s.p;
 }
 
+// ---- workspace of one call ---------------------------------------------------
+// Up to kPoolKeep bytes stay with the pool between calls (the largest workspace, of the
+// 512x256x256 surface tension, is 3.4 GB), so that a call after a synchronisation does not
+// map its memory again; fmf_reset gives them back.
+constexpr unsigned long long kPoolKeep = 4ull << 30;
+constexpr int kMaxDevices = 64;
+static cudaMemPool_t g_pools[kMaxDevices];
+static std::mutex g_pool_mu;
+static cudaMemPool_t pool_locked(int dev) {
+  if (g_pools[dev]) return g_pools[dev];
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t p = nullptr;
+  // (allowed beside a capture: the pool belongs to none)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  unsigned long long keep = kPoolKeep;
+  int off = 0;  // no stream is made to wait for another's call
+  const bool ok = FMF_CUDA(cudaMemPoolCreate(&p, &props)) &&
+                  FMF_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) &&
+                  FMF_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolReuseAllowInternalDependencies, &off));
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (!ok) return nullptr;
+  return g_pools[dev] = p;
+}
+Workspace::Workspace(size_t bytes, cudaStream_t stream) : s(stream) {
+  int dev = 0;
+  if (!FMF_CUDA(cudaGetDevice(&dev)) || dev >= kMaxDevices) return;
+  cudaMemPool_t pool;
+  {
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    pool = pool_locked(dev);
+  }
+  if (!pool || !FMF_CUDA(cudaMallocFromPoolAsync(&p, bytes, pool, s))) {
+    p = nullptr;
+    set_status(5);
+  }
+}
+Workspace::~Workspace() {
+  if (p) FMF_CUDA(cudaFreeAsync(p, s));
+}
+static void trim_pools() {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  for (cudaMemPool_t p : g_pools)
+    if (p) FMF_CUDA(cudaMemPoolTrimTo(p, 0));
+}
+
 // ---- host-array registry -------------------------------------------------
 // Entries are keyed by host start address and never overlap: a request that
 // overlaps existing mirrors without being contained in one of them merges them
@@ -233,6 +282,7 @@ int reset_registry() {
   FMF_CUDA(cudaStreamSynchronize(stream()));
   for (auto& e : g_reg) FMF_CUDA(cudaFree(e.second.dev));
   g_reg.clear();
+  trim_pools();
   return 0;
 }
 

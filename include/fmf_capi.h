@@ -34,7 +34,7 @@
  * whole of main.f90:473-697 on the GPU.
  *
  * Threading: one host thread drives the library at a time (the reference's
- * single-threaded caller contract).  All work goes to one CUDA stream.
+ * single-threaded caller contract).  All work goes to one CUDA stream (fmf_set_stream).
  */
 #ifndef FMF_CAPI_H
 #define FMF_CAPI_H
@@ -60,12 +60,17 @@ enum { FMF_RESIDENT = 0, FMF_COHERENT = 1 };
 int fmf_last_error(void);                 /* last status, then cleared */
 const char* fmf_error_string(int code);
 int fmf_set_mode(int mode);               /* FMF_RESIDENT or FMF_COHERENT */
-int fmf_set_stream(void* cuda_stream);    /* NULL: the library's own stream */
+/* The stream of the calls that follow (NULL: the library's own).  Nothing waits: earlier
+ * calls go on where they are.  The pressure solve, the reductions and monitors, solu_sor4_
+ * and fmf_dev_weno5_fused in FMF_MIXED and FMF_FP64E share one scratch area, so a caller
+ * waits for the stream it leaves before calling those on another; solphi_mthinc1_ and
+ * fmf_dev_csf_fused have a workspace per call, in stream order, and the rest has none. */
+int fmf_set_stream(void* cuda_stream);
 int fmf_sync_to_host(void* host_ptr);     /* copy one mirrored array back */
 int fmf_sync_to_device(void* host_ptr);   /* re-upload one mirrored array */
 int fmf_sync_all_to_host(void);
 int fmf_forget(void* host_ptr);           /* drop one mirror (host array about to be freed) */
-int fmf_reset(void);                      /* drop every mirror */
+int fmf_reset(void);                      /* drop every mirror and the workspace memory kept between calls */
 int fmf_device_synchronize(void);
 /* kernels this library launched since load (a counter kept by its launch helpers) */
 long long fmf_kernel_launches(void);
@@ -346,7 +351,10 @@ int fmf_dev_weno5_fused(int precision, int ni, int nj, int nk, double dxinv, dou
                         double* adv_u, double* adv_v, double* adv_w);
 /* the CSF force of one phi field, FMF_FP64 and FMF_MIXED as the fused step of that
  * precision forms it, FMF_FP64E in FP32 pairs; interior u, v, w points (ni % 32 == 0,
- * nj % 8 == 0); returns a status */
+ * nj % 8 == 0); returns a status.  FMF_FP64 works in 12 (ni+6)(nj+6)(nk+6) doubles
+ * (3.4 GB at 512x256x256), allocated and freed in the order of the stream: a call
+ * may be captured (the graph owns that memory) and calls on several streams do not
+ * touch each other's; up to 4 GB stay with the library until fmf_reset. */
 int fmf_dev_csf_fused(int precision, int ni, int nj, int nk, double dx, double dy, double dz,
                       double rhol, double rhog, double sigma, const double* phi, double* fu,
                       double* fv, double* fw);
