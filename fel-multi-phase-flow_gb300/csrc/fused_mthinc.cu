@@ -128,7 +128,8 @@ __device__ __forceinline__ R sig8f(const R* E, R w, R ed, R* sd) {
     const R e = E[t] * ed;
     const R r = inv1p(e);
     s += r;
-    if (sd) q += r == (R)0 ? (R)0 : e * r * r;  // (an overflowed e: 0 times infinity)
+    if (sizeof(R) == 8 && r == (R)0) continue;  // an overflowed e: no 0 times infinity
+    if (sd) q += e * r * r;
   }
   if (sd) *sd = q;
   return w * s;
