@@ -182,7 +182,10 @@ __global__ void __launch_bounds__(256, 5) k_classify(Grid g, MC m, const double*
   // under them were issued per set of lanes, 15 slots of the FP64 pipe for 3 products).
   const long long pb = raw(phi00);
   double pdx = 0.0, pdy = 0.0, pdz = 0.0;
-  const bool filled = __any_sync(warp, pb != 0);
+  // (a velocity that is not finite has a flux that is not, where phi is 0 as well)
+  auto size = [](double x) { return __double2hiint(x) & 0x7fffffff; };
+  const int fastest = max(max(max(size(uw), size(ue)), max(size(vs), size(vn))), max(size(wb), size(wt)));
+  const bool filled = __any_sync(warp, pb != 0 || fastest >= 0x7ff00000);
   if (filled) {
     if (__any_sync(warp, pb != 0 && pb != kOneBits)) {
       pdx = phi00 * m.dtdx;
