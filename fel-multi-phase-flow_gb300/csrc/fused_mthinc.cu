@@ -434,8 +434,11 @@ __global__ void __launch_bounds__(64) k_band(Grid g, MC m, __grid_constant__ con
 // point instead of the reference's 27, none in a warp whose points are all flat.
 // NEAR1 (phin before its snap, for the band test alone): eight values within 64 units in
 // the last place below 1 count as flat.  There phin is 1 but for the roundings of
-// solphi_mthinc2; a gradient of 2^-47 dxinv is 1e-12 of the band test's limit, inside
-// which the test falls back on the square root.
+// solphi_mthinc2.  What that drops is a gradient of at most 2^-47 dxinv per vertex, 7e-13 of
+// the band test's limit at bet = 2, 1e-10 at 4, 1e-5 at 8 and more than all of it at 12; but
+// a cell is one of the eight values of each of its vertices, so a cell whose test that can
+// turn is itself within 64 units of 1, and snapped or not it stays there: phin changes by
+// 7.1e-15 at most, whatever bet > 0 is.
 template <bool NEAR1>
 __global__ void __launch_bounds__(128) k_vertex_grad(Grid g, double cx, double cy, double cz,
                                                      const double* __restrict__ q, double* __restrict__ qx,
