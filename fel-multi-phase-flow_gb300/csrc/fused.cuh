@@ -148,8 +148,9 @@ constexpr int kSorCapped = 1 << 20, kSorNonfinite = 1 << 21;
 // sets the rule and empties the log
 void sor_rule(cudaStream_t s, SorLoop* L, double tol, int maxit, double cells);
 // The whole solve of a small grid in one launch, with its stop rule and log entry, where
-// supported: what sor_iteration (sor_iteration_refine) repeated until the rule gives, bit
-// for bit
+// supported: the iterates of sor_iteration (sor_iteration_refine) bit for bit, and the same
+// number of them but where a residual is within its sum's rounding of the tolerance (the
+// squares are added in another order)
 bool solve_small_supported(const Grid& g, bool fp64);
 void solve_small(cudaStream_t s, const Grid& g, double dxinv, double dyinv, double dzinv, const double* mu,
                  double* const* E, double* const* AB, double uwall, const double* wallc, double* un, double* vn,

@@ -1478,21 +1478,32 @@ __device__ __forceinline__ T cluster_pair(const Grid& g, const SolveK<T>& K, con
   }
   return e;
 }
+// A thread's sum over the sweeps, which k_pair's blocks add up in double: in FP32 with the
+// roundings of the additions kept (a conversion per sweep would take the FP64 pipe)
+__device__ __forceinline__ void sweep_sum(double& s, double e) { s += e; }
+__device__ __forceinline__ void sweep_sum(df::D& s, float e) {
+  const df::D t = df::two_sum(s.h, e);
+  s = df::D{t.h, df::fadd(s.l, t.l)};
+}
+__device__ __forceinline__ double sum_of(double s) { return s; }
+__device__ __forceinline__ double sum_of(df::D s) { return (double)s.h + (double)s.l; }
+template <class T>
+using SweepSum = typename std::conditional<std::is_same<T, double>::value, double, df::D>::type;
 template <int COMP, class T, class G, class Sync>
-__device__ __forceinline__ T cluster_component(const Grid& g, const SolveK<T>& K, const G& gh, int me, Sync sync) {
-  T e = cluster_pair<COMP, false>(g, K, gh, 1, 1, 1, me);
+__device__ __forceinline__ void cluster_component(const Grid& g, const SolveK<T>& K, const G& gh, int me, SweepSum<T>& e,
+                                                  Sync sync) {
+  sweep_sum(e, cluster_pair<COMP, false>(g, K, gh, 1, 1, 1, me));
   sync();
   for (int region = 0; region < 3; ++region)
     for (long t = me; t < refresh_tasks(g, region); t += kClusterBlocks * kClusterThreads)
       refresh(g, 1 << COMP, gh, K.un, K.vn, K.wn, region, t);
   sync();
-  e += cluster_pair<COMP, true>(g, K, gh, 1, 1, 2, me);
+  sweep_sum(e, cluster_pair<COMP, true>(g, K, gh, 1, 1, 2, me));
   sync();
-  e += cluster_pair<COMP, true>(g, K, gh, 1, 2, 1, me);
+  sweep_sum(e, cluster_pair<COMP, true>(g, K, gh, 1, 2, 1, me));
   sync();
-  e += cluster_pair<COMP, true>(g, K, gh, 2, 1, 1, me);
+  sweep_sum(e, cluster_pair<COMP, true>(g, K, gh, 2, 1, 1, me));
   sync();
-  return e;
 }
 template <class T, class G>
 __global__ void __launch_bounds__(kClusterThreads) k_solve_cluster(Grid g, SolveK<T> K, G gh, SorLoop* L, int* log) {
@@ -1508,11 +1519,12 @@ __global__ void __launch_bounds__(kClusterThreads) k_solve_cluster(Grid g, Solve
   const int mx = min(max(L->maxit, 1), kSorMax);
   double err0 = 0.0;
   for (int it = 1;; ++it) {
-    T e = cluster_component<0>(g, K, gh, me, sync);
-    e += cluster_component<1>(g, K, gh, me, sync);
-    e += cluster_component<2>(g, K, gh, me, sync);
+    SweepSum<T> e{};
+    cluster_component<0>(g, K, gh, me, e, sync);
+    cluster_component<1>(g, K, gh, me, e, sync);
+    cluster_component<2>(g, K, gh, me, e, sync);
     // every block gets every block's sum and applies the rule to the same total
-    double s = (double)e;
+    double s = sum_of(e);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if ((t & 31) == 0) warps[t >> 5] = s;
     __syncthreads();
