@@ -948,9 +948,10 @@ static int step_once(fmf_ctx* c, const StepHooks* hk = nullptr) {
 // launches after one warm-up launch, on the current state (the state is not
 // advanced: stages write only work arrays).  Stage 0: WENO5 advection of both
 // levels, (u,v,w) and (uo,vo,wo); 1: one outer SOR iteration on copies of the
-// velocity; 2: pressure FFT+TDMA+inverse; 3: MTHINC fluxes; 4: WENO5 advection of
-// (u,v,w) alone (what a step that continues from the previous one runs).  *ms =
-// mean milliseconds per launch of the stage.
+// velocity (small grids: the one-launch solve at a limit of one iteration); 2:
+// pressure FFT+TDMA+inverse; 3: MTHINC fluxes; 4: WENO5 advection of (u,v,w) alone
+// (what a step that continues from the previous one runs).  *ms = mean milliseconds
+// per launch of the stage.
 int fmf_ctx_time_stage(fmf_ctx* c, int stage, int reps, float* ms) {
   if (!c || !ms || reps <= 0 || stage < 0 || stage > 4) return FMF_ERR_ARG;
   ScratchScope scope(c->scr);
@@ -967,11 +968,10 @@ int fmf_ctx_time_stage(fmf_ctx* c, int stage, int reps, float* ms) {
                           c->wprec, c->wsplit);
         break;
       case 1:
-        if (mixed)
-          fused::sor_iteration_refine(s, g, dxinv, dyinv, dzinv, c->rb, c->sorpart, c->red + 8, c->flat);
+        if (c->small)
+          seg_small(c);  // its rule set to one iteration below
         else
-          fused::sor_iteration(s, g, dxinv, dyinv, dzinv, P.harmonic, c->rmun, c->edge, c->ab, P.uwall, c->wallc,
-                               c->un, c->vn, c->wn, c->sorpart, c->red + 8, c->flat);
+          iter_kernels(c);
         break;
       case 2:
         fused::pressure_half(s, g, P.rhog, dxinv, dzinv, c->as_f, c->an_f, c->ap_f, c->div, c->pr, c->pi, c->dp,
@@ -991,6 +991,7 @@ int fmf_ctx_time_stage(fmf_ctx* c, int stage, int reps, float* ms) {
     op::copy(s, n, c->u, c->un);
     op::copy(s, n, c->v, c->vn);
     op::copy(s, n, c->w, c->wn);
+    if (c->small) fused::sor_rule(s, c->loop, c->sor_tol, 1, (double)g.cells());
   }
   run();
   cudaEvent_t e0, e1;
@@ -1005,6 +1006,7 @@ int fmf_ctx_time_stage(fmf_ctx* c, int stage, int reps, float* ms) {
   *ms = t / (float)reps;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if (stage == 1 && c->small) fused::sor_rule(s, c->loop, c->sor_tol, c->sor_max, (double)g.cells());
   return take_status();
 }
 
@@ -1038,16 +1040,30 @@ int fmf_ctx_check_sor(fmf_ctx* c, double* out) {
     return rms(e);
   };
   // the context's own solve (FP32 correction sweeps in the mixed precision)
-  double err0 = 0.0, err = 0.0;
-  int lp;
-  for (lp = 0; lp < c->sor_max && !get_status(); ++lp) {
-    seg_iter(c);
-    err = read_err();
-    if (lp == 0) err0 = err;
-    if (err / err0 <= c->sor_tol) break;
+  if (c->small) {
+    seg_small(c);
+    SorLoop h{};
+    int entry = 0;
+    FMF_CUDA(cudaMemcpyAsync(&h, c->loop, sizeof(SorLoop), cudaMemcpyDeviceToHost, s));
+    FMF_CUDA(cudaMemcpyAsync(&entry, c->sorlog, sizeof(int), cudaMemcpyDeviceToHost, s));
+    chain(s, 1, 1, k_sor_log_reset)(c->loop);
+    count_launch();
+    FMF_CUDA(cudaStreamSynchronize(s));
+    if (entry & kSorNonfinite) set_status(FMF_ERR_NONFINITE);
+    out[0] = (double)(entry & (kSorCapped - 1));
+    out[1] = h.err / h.err0;
+  } else {
+    double err0 = 0.0, err = 0.0;
+    int lp;
+    for (lp = 0; lp < c->sor_max && !get_status(); ++lp) {
+      seg_iter(c);
+      err = read_err();
+      if (lp == 0) err0 = err;
+      if (err / err0 <= c->sor_tol) break;
+    }
+    out[0] = (double)std::min(lp + 1, c->sor_max);
+    out[1] = err / err0;
   }
-  out[0] = (double)std::min(lp + 1, c->sor_max);
-  out[1] = err / err0;
   if (c->mixed) {
     fused::refine_finish(s, g, c->u, c->v, c->w, c->rb, c->un, c->vn, c->wn);
     // the FP64 factors of the same system

@@ -448,7 +448,7 @@ int fmf_ctx_state_device_ptr(fmf_ctx* ctx, int field, void** out);
 long long fmf_ctx_device_bytes(fmf_ctx* ctx);
 /* CUDA-event time of one stage of the step on the context stream (mean ms per
  * launch over reps): 0 WENO5 advection of both velocity levels, 1 one outer SOR
- * iteration, 2 pressure FFT+TDMA, 3 MTHINC fluxes, 4 WENO5 advection of (u, v, w)
+ * iteration (where the step solves in one launch, that launch limited to one), 2 pressure FFT+TDMA, 3 MTHINC fluxes, 4 WENO5 advection of (u, v, w)
  * alone (the level a continuing step computes).  Measurement support; no
  * counterpart in the reference. */
 int fmf_ctx_time_stage(fmf_ctx* ctx, int stage, int reps, float* ms);
