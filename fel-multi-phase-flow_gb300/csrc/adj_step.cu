@@ -559,7 +559,7 @@ int record_step(fmf_adj* a, bool graphs) {
       fused::sor_iteration(s, g, dxi, dyi, dzi, P.harmonic, a->rmun, a->E, a->AB, P.uwall, a->wallc, a->un[0],
                            a->un[1], a->un[2], a->sorpart, a->red + 4, a->flat);
   };
-  if (a->small) {
+  if (a->small && a->sor_max <= fused::kSorMax) {  // (the most one launch runs)
     fused::sor_rule(s, a->loop, a->sor_tol, a->sor_max, (double)g.cells());
     if (a->mixed)
       fused::solve_small_refine(s, g, dxi, dyi, dzi, a->rb, a->loop, a->sorlog);
