@@ -24,7 +24,9 @@
 // interior row gets exactly one writer (solphi_mthinc1.f:121-130 zeroes first;
 // faces nobody donates through hold the zero written by k_classify's owner).
 #include <cmath>
+#include <cstring>
 
+#include "../../include/fmf_capi.h"
 #include "bits.cuh"
 #include "fused.cuh"
 #include "recip.cuh"
@@ -427,6 +429,21 @@ __global__ void __launch_bounds__(64) k_band(Grid g, MC m, __grid_constant__ con
     axis(wb, wt, m.dtdz, b[2], kz0, kz1, fz + c - Z, fz + c);
   }
 }
+// n arguments: spread over [-5, 5] (exp16 hands over to exp at 4), and the same moved to an
+// odd thirty-second, where k turns, give or take a few units in the last place
+__global__ void k_check_exp16(__grid_constant__ const Exp16 T, long n, unsigned long long* worst) {
+  unsigned long long m = 0;
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
+    double z = -5.0 + 10.0 * ((double)t + 0.5) / (double)n;
+    if (t & 1) {
+      z = (2.0 * rint(16.0 * z - 0.5) + 1.0) * 0.03125;
+      z = __longlong_as_double(__double_as_longlong(z) + (t / 2) % 7 - 3);
+    }
+    const double q = exp(z);
+    m = max(m, (unsigned long long)__double_as_longlong(fabs(exp16(T, z) - q) / q));
+  }
+  atomicMax(worst, m);
+}
 // cal_grad_p2a.f:46-60 for the fused step: the vertex gradient at (i+1/2, j+1/2,
 // k+1/2), i, j, k in -2..n+2, from the 8 surrounding points.  Per (i, j) corner the sum s and difference
 // d of the two k planes; with ta = s(+,+) - s(0,0) and tb = s(+,0) - s(0,+) the x sum is
@@ -547,5 +564,25 @@ void mthinc_fluxes(cudaStream_t s, const Grid& g, double dxinv, double dyinv, do
   count_launch(2);
 }
 
+int check_exp16(long n, double* max_rel_err) {
+  unsigned long long* d = nullptr;
+  if (cudaMalloc(&d, sizeof(unsigned long long)) != cudaSuccess) return FMF_ERR_NOMEM;
+  cudaMemset(d, 0, sizeof(unsigned long long));
+  k_check_exp16<<<152 * 4, 256>>>(exp16_table(), n, d);
+  count_launch();
+  unsigned long long h = 0;
+  const cudaError_t e = cudaMemcpy(&h, d, sizeof(h), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e != cudaSuccess || cudaGetLastError() != cudaSuccess) return FMF_ERR_CUDA;
+  std::memcpy(max_rel_err, &h, sizeof(double));
+  return FMF_OK;
+}
+
 }  // namespace fused
 }  // namespace fmf
+
+// The short exponential of the band kernel against exp.  Verification support; no
+// counterpart in the reference.
+extern "C" int fmf_check_exponential(long long n, double* max_rel_err) {
+  return max_rel_err && n > 0 ? fmf::fused::check_exp16((long)n, max_rel_err) : FMF_ERR_ARG;
+}

@@ -6,7 +6,7 @@
 // 8 independent multiply-add chains (enough independent work to fill every FP64
 // pipe), timed with CUDA events after a warm-up launch.  Reads no memory; writes
 // one value per thread so the chains are not removed.  Also here: the error
-// checks of the division-free reciprocal and reciprocal square root (recip.cuh)
+// checks of the division-free reciprocals and reciprocal square root (recip.cuh)
 // against CUDA's own 1.0 / x and 1.0 / sqrt(x).
 #include <cstring>
 
@@ -58,10 +58,11 @@ int measure(int iters, double* tflops) {
   return cudaGetLastError() == cudaSuccess ? FMF_OK : FMF_ERR_CUDA;
 }
 
-// n positive normal doubles spread over exponents 2^-1000 .. 2^1000 with
-// pseudo-random mantissas (a 64-bit mix of the index); the largest relative error
-// of recip_nr (which = 0) against the IEEE quotient 1.0 / x, or of rsqrt_nr
-// (which = 1) against 1.0 / sqrt(x), as ordered bits of a non-negative double.
+// n positive normal doubles spread over exponents 2^-1000 .. 2^1000 with pseudo-random
+// mantissas (a 64-bit mix of the index), every other one with a low word of ones (which the
+// approximate seeds do not read); the largest relative error of recip_nr and recip_h
+// (which = 0) against the IEEE quotient 1.0 / x, or of rsqrt_h (which = 1) against
+// 1.0 / sqrt(x), as ordered bits of a non-negative double.
 __global__ void k_check_recip(long n, int which, unsigned long long* worst) {
   unsigned long long m = 0;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
@@ -69,10 +70,12 @@ __global__ void k_check_recip(long n, int which, unsigned long long* worst) {
     h ^= h >> 31;
     h *= 0xBF58476D1CE4E5B9ull;
     h ^= h >> 29;
+    if (t & 1) h |= 0xFFFFFFFFull;
     const long long e = 1023 + (long long)(t % 2001) - 1000;
     const double x = __longlong_as_double((long long)((e << 52) | (h & 0xFFFFFFFFFFFFFull)));
-    const double q = which ? 1.0 / sqrt(x) : 1.0 / x, r = which ? fmf::rsqrt_nr(x) : fmf::recip_nr(x);
-    const double rel = fabs(r - q) / q;
+    const double q = which ? 1.0 / sqrt(x) : 1.0 / x, r = which ? fmf::rsqrt_h(x) : fmf::recip_h(x);
+    const double s = which ? r : fmf::recip_nr(x);
+    const double rel = fmax(fabs(r - q), fabs(s - q)) / q;
     const unsigned long long b = (unsigned long long)__double_as_longlong(rel);
     m = b > m ? b : m;
   }

@@ -470,14 +470,16 @@ int fmf_ctx_check_sor(fmf_ctx* ctx, double* out);
  * Measurement support; no counterpart in the reference. */
 int fmf_measure_fma_rate(int fp64, double* tflops);
 /* Largest relative error, over n positive normal doubles spread over 2^-1000 ..
- * 2^1000, of the division-free reciprocal the fused WENO5 kernel uses (Newton-
- * Raphson from an approximate reciprocal) against the IEEE quotient 1.0 / x.
- * Verification support; no counterpart in the reference. */
+ * 2^1000, of the division-free reciprocals of the fused kernels (by Newton-Raphson and
+ * by one third-order step, from an approximate reciprocal) against the IEEE quotient
+ * 1.0 / x.  Verification support; no counterpart in the reference. */
 int fmf_check_reciprocal(long long n, double* max_rel_err);
-/* The same for the division-free reciprocal square root of the fused CSF kernel
- * (Newton-Raphson from an approximate reciprocal square root) against
- * 1.0 / sqrt(x). */
+/* The same for the division-free reciprocal square root of the fused kernels (one
+ * third-order step from an approximate reciprocal square root) against 1.0 / sqrt(x). */
 int fmf_check_rsqrt(long long n, double* max_rel_err);
+/* The same for the short exponential of the interface band (a table of sixteenths and
+ * a polynomial) against exp, over n arguments in [-5, 5]. */
+int fmf_check_exponential(long long n, double* max_rel_err);
 /* Largest relative error of the (hi, lo) float pairs the mixed-precision WENO5
  * splits each double into (hi + lo against the double), over n values of both
  * signs spread over 2^-96 .. 2^127.  Verification support; no counterpart in the
