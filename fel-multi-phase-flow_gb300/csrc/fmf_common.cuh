@@ -81,7 +81,7 @@ template <class... P>
 inline Chain<P...> chain(cudaStream_t s, dim3 grid, dim3 block, void (*kernel)(P...), size_t smem = 0) {
   return Chain<P...>{s, grid, block, kernel, smem};
 }
-__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void after_previous() { cudaGridDependencySynchronize(); }
 
 // ---- index-range launcher ------------------------------------------------
 // fn(i,j,k) for i in [i0,i1], j in [j0,j1], k in [k0,k1]; 32x8 threads per block,
