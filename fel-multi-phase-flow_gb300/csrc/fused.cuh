@@ -140,7 +140,7 @@ long sor_parts(const Grid& g);
 // err/err0 <= tol or after maxit iterations (kSorMax at most, whatever this memory
 // holds).  A finished solve's log entry is its iteration count with the two bits.
 struct SorLoop {
-  double tol, cells, err0, err;  // (err: the last of a one-launch solve)
+  double tol, cells, err0, pad;
   int maxit, it, nlog, flags;
 };
 constexpr int kSorLog = 4096, kSorMax = 100000;

@@ -1517,7 +1517,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_solve_cluster(Grid g, Solve
   auto sync = [&] { cl.sync(); };
   const double tol = L->tol, cells = L->cells;
   const int mx = min(max(L->maxit, 1), kSorMax);
-  double err0 = 0.0, err = 0.0;
+  double err0 = 0.0;
   for (int it = 1;; ++it) {
     SweepSum<T> e{};
     cluster_component<0>(g, K, gh, me, e, sync);
@@ -1544,7 +1544,7 @@ __global__ void __launch_bounds__(kClusterThreads) k_solve_cluster(Grid g, Solve
           entry |= kSorNonfinite;
           done = true;
         } else {
-          err = sqrt(s / cells) + 1.0e-99;
+          const double err = sqrt(s / cells) + 1.0e-99;
           if (it == 1) err0 = err;
           if (err / err0 <= tol)
             done = true;
@@ -1560,8 +1560,6 @@ __global__ void __launch_bounds__(kClusterThreads) k_solve_cluster(Grid g, Solve
   if (me == 0) {
     if (L->nlog < kSorLog) log[L->nlog] = verdict;
     L->nlog += 1;
-    L->err0 = err0;
-    L->err = err;
   }
 }
 __global__ void k_to_float(long n, const double* __restrict__ a, float* __restrict__ b) {

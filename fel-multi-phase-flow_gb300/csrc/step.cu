@@ -1040,29 +1040,35 @@ int fmf_ctx_check_sor(fmf_ctx* c, double* out) {
     return rms(e);
   };
   // the context's own solve (FP32 correction sweeps in the mixed precision)
+  double err0 = 0.0, err = 0.0;
+  int lp;
+  for (lp = 0; lp < c->sor_max && !get_status(); ++lp) {
+    seg_iter(c);
+    err = read_err();
+    if (lp == 0) err0 = err;
+    if (err / err0 <= c->sor_tol) break;
+  }
+  out[0] = (double)std::min(lp + 1, c->sor_max);
+  out[1] = err / err0;
   if (c->small) {
+    // the same solve in the step's one launch, again from un = u, which leaves its
+    // iteration count (keeping its residuals there as well costs a step of 32x32x16 0.5 %
+    // in registers)
+    if (c->mixed) {
+      for (int q = 0; q < 3; ++q) FMF_CUDA(cudaMemsetAsync(c->rb.d[q], 0, sizeof(float) * n, s));
+    } else {
+      op::copy(s, n, c->u, c->un);
+      op::copy(s, n, c->v, c->vn);
+      op::copy(s, n, c->w, c->wn);
+    }
     seg_small(c);
-    SorLoop h{};
     int entry = 0;
-    FMF_CUDA(cudaMemcpyAsync(&h, c->loop, sizeof(SorLoop), cudaMemcpyDeviceToHost, s));
     FMF_CUDA(cudaMemcpyAsync(&entry, c->sorlog, sizeof(int), cudaMemcpyDeviceToHost, s));
     chain(s, 1, 1, k_sor_log_reset)(c->loop);
     count_launch();
     FMF_CUDA(cudaStreamSynchronize(s));
     if (entry & kSorNonfinite) set_status(FMF_ERR_NONFINITE);
     out[0] = (double)(entry & (kSorCapped - 1));
-    out[1] = h.err / h.err0;
-  } else {
-    double err0 = 0.0, err = 0.0;
-    int lp;
-    for (lp = 0; lp < c->sor_max && !get_status(); ++lp) {
-      seg_iter(c);
-      err = read_err();
-      if (lp == 0) err0 = err;
-      if (err / err0 <= c->sor_tol) break;
-    }
-    out[0] = (double)std::min(lp + 1, c->sor_max);
-    out[1] = err / err0;
   }
   if (c->mixed) {
     fused::refine_finish(s, g, c->u, c->v, c->w, c->rb, c->un, c->vn, c->wn);

@@ -457,7 +457,8 @@ int fmf_ctx_time_stage(fmf_ctx* ctx, int stage, int reps, float* ms);
  * the carried advection and surface tension).  Runs the step up to the solve and the
  * solve in the context's precision, then FP64 outer iterations on copies:
  *   out[0] outer iterations of the context's solve;
- *   out[1] err/err0 at its last iteration (in FMF_MIXED: of the FP32 correction);
+ *   out[1] err/err0 at its last iteration (in FMF_MIXED: of the FP32 correction; on
+ *          grids solved in one launch, of the same iterations run one by one);
  *   out[2] the RMS change of one FP64 outer iteration from the solve's result over
  *          the FP64 first-iteration change from un = u (the FP64 solve's err0);
  *   out[3] the same from the result of an FP64 solve run to the same rule;
