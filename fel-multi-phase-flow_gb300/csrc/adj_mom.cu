@@ -71,7 +71,7 @@ __device__ __forceinline__ void walk_rev(const Walk& W, double g4, double* la) {
   la[3] = fma(ld2, 0.5, fma(lD3, 0.625, fma(lt1c, -2.0, fma(lt2c, -4.0, lt1b - lt2b))));
   la[4] = fma(lD3, -0.125, lt1c + lt2c);
 }
-// adjoint of  out += wdir(q, c, S, 4 vel, di/24)  given lout: lD[0..5] = the
+// adjoint of  out += |vel| di/6 R(e)  (R above, from the upwind side) given lout: lD[0..5] = the
 // adjoints of the six differences (dm5, dm3, dm1, dp1, dp3, dp5); returns lvel
 __device__ double wline_T(const double* __restrict__ q, long c, long S, double vel, double lout, double di,
                           double* lD) {
