@@ -933,7 +933,7 @@ int fmf_dev_csf_fused(int precision, int ni, int nj, int nk, double dx, double d
   if (!phi || !fu || !fv || !fw || precision < FMF_FP64 || precision > FMF_FP64E || !fused::csf_supported(g))
     return FMF_ERR_ARG;
   if (precision == FMF_FP64) {
-    const Workspace ws(sizeof(double) * 12 * g.n, stream());
+    const Workspace ws(sizeof(double) * 12 * g.n, stream(), 8);
     if (!ws.p) return take_status();
     double* work[4];
     for (int q = 0; q < 4; ++q) work[q] = (double*)ws.p + 3 * q * g.n;

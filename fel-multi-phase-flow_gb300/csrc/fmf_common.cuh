@@ -35,14 +35,16 @@ bool cuda_ok(cudaError_t e, const char* where);
 void count_launch(int n = 1);
 cudaStream_t stream();
 void* scratch(size_t bytes, int slot);  // per-slot growable device scratch (library owned)
-// Device memory for the kernels one call enqueues on stream s, taken and given back in the
-// order of that stream: calls on several streams or from several threads have their own,
-// and a call that is captured leaves it to the graph (p null and a status where there is
-// none).
+// Device memory for the kernels one call enqueues on stream s, held in the order of that
+// stream: calls on several streams or from several threads have their own, and a call that
+// is captured leaves it to the graph (p null and a status where there is none).  slot: of
+// the library-wide scratch, for calls on the library's own stream; no other use of it.
 struct Workspace {
   void* p = nullptr;
   cudaStream_t s;
-  Workspace(size_t bytes, cudaStream_t stream);
+  bool pooled = false;
+  static unsigned slots;  // the slots in use, a bit each
+  Workspace(size_t bytes, cudaStream_t stream, int slot);
   ~Workspace();
   Workspace(const Workspace&) = delete;
   Workspace& operator=(const Workspace&) = delete;

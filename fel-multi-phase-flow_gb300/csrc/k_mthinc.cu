@@ -98,7 +98,7 @@ void solphi_mthinc1(cudaStream_t s, const Grid& g, double dxinv, double dyinv, d
   // by one, as below.
   if (fused::band_in_y(bet)) {
     const long nb = (long)(g.ni + 2) * (g.nj + 2) * (g.nk + 2);
-    const Workspace ws(sizeof(int) * (nb + 1), s);
+    const Workspace ws(sizeof(int) * (nb + 1), s, 0);
     if (!ws.p) return;
     int* band = (int*)ws.p;
     fused::mthinc_fluxes(s, g, dxinv, dyinv, dzinv, dt, bet, phi, phix, phiy, phiz, u, v, w, flx, fly, flz, band,

@@ -12,8 +12,8 @@ namespace fmf {
 // atomic: the adjoint rollout runs a second host thread
 static std::atomic<int> g_status{0};
 static std::atomic<long long> g_launches{0};
-static cudaStream_t g_stream = nullptr;
-static bool g_own_stream = false;
+static cudaStream_t g_stream = nullptr;  // the caller's or g_lib
+static cudaStream_t g_lib = nullptr;     // the library's own, made once
 static int g_mode = 0;  // FMF_RESIDENT
 
 void set_status(int code) {
@@ -32,19 +32,12 @@ long long launches() { return g_launches; }
 
 cudaStream_t stream() {
   if (!g_stream) {
-    if (FMF_CUDA(cudaStreamCreateWithFlags(&g_stream, cudaStreamNonBlocking))) g_own_stream = true;
+    if (!g_lib) FMF_CUDA(cudaStreamCreateWithFlags(&g_lib, cudaStreamNonBlocking));
+    g_stream = g_lib;
   }
   return g_stream;
 }
-void set_stream(cudaStream_t s) {
-  if (s) {
-    g_stream = s;
-    g_own_stream = false;
-  } else {
-    g_stream = nullptr;
-    stream();
-  }
-}
+void set_stream(cudaStream_t s) { g_stream = s; }
 int mode() { return g_mode; }
 void set_mode(int m) { g_mode = m; }
 
@@ -73,8 +66,8 @@ void* scratch_set_use(void* p) {
   g_set = (ScratchSet*)p;
   return old;
 }
-void* scratch(size_t bytes, int slot) {
-  Slot& s = (g_set ? g_set : &g_global_set)->slots[slot];
+static void* scratch_of(ScratchSet* set, size_t bytes, int slot) {
+  Slot& s = set->slots[slot];
   if (s.bytes >= bytes) return s.p;
   if (s.p) {
     FMF_CUDA(cudaStreamSynchronize(stream()));
@@ -89,13 +82,24 @@ void* scratch(size_t bytes, int slot) {
   s.bytes = bytes;
   return s.p;
 }
+void* scratch(size_t bytes, int slot) { return scratch_of(g_set ? g_set : &g_global_set, bytes, slot); }
 
 // ---- workspace of one call ---------------------------------------------------
-// Up to kPoolKeep bytes stay with the pool between calls (the largest workspace, of the
-// 512x256x256 surface tension, is 3.4 GB), so that a call after a synchronisation does not
-// map its memory again; fmf_reset gives them back.
+// On the library's own stream, which nobody else can capture or destroy, the calls are in
+// order and share a slot of the library-wide scratch; on a caller's stream each takes its
+// own from a pool (an allocation and a free in stream order: 1 us on a surface tension of
+// 128x64x256, 1 to 4 on the drop-in subroutines at 64x32x32).  Up to kPoolKeep bytes stay
+// with either between calls (the largest workspace, of the 512x256x256 surface tension, is
+// 3.4 GB), so that a call after a synchronisation does not map its memory again; fmf_reset
+// gives them back.
 constexpr unsigned long long kPoolKeep = 4ull << 30;
 constexpr int kMaxDevices = 64;
+// allocations for no captured stream are allowed while one is captured
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 static cudaMemPool_t g_pools[kMaxDevices];
 static std::mutex g_pool_mu;
 static cudaMemPool_t pool_locked(int dev) {
@@ -105,19 +109,22 @@ static cudaMemPool_t pool_locked(int dev) {
   props.location.type = cudaMemLocationTypeDevice;
   props.location.id = dev;
   cudaMemPool_t p = nullptr;
-  // (allowed beside a capture: the pool belongs to none)
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  cudaThreadExchangeStreamCaptureMode(&mode);
+  const RelaxedCapture relaxed;
   unsigned long long keep = kPoolKeep;
   int off = 0;  // no stream is made to wait for another's call
   const bool ok = FMF_CUDA(cudaMemPoolCreate(&p, &props)) &&
                   FMF_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep)) &&
                   FMF_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolReuseAllowInternalDependencies, &off));
-  cudaThreadExchangeStreamCaptureMode(&mode);
   if (!ok) return nullptr;
   return g_pools[dev] = p;
 }
-Workspace::Workspace(size_t bytes, cudaStream_t stream) : s(stream) {
+Workspace::Workspace(size_t bytes, cudaStream_t stream, int slot) : s(stream) {
+  if (stream == g_lib && bytes <= kPoolKeep) {
+    const RelaxedCapture relaxed;
+    p = scratch_of(&g_global_set, bytes, slot);
+    slots |= 1u << slot;
+    return;
+  }
   int dev = 0;
   if (!FMF_CUDA(cudaGetDevice(&dev)) || dev >= kMaxDevices) return;
   cudaMemPool_t pool;
@@ -129,11 +136,20 @@ Workspace::Workspace(size_t bytes, cudaStream_t stream) : s(stream) {
     p = nullptr;
     set_status(5);
   }
+  pooled = p != nullptr;
 }
 Workspace::~Workspace() {
-  if (p) FMF_CUDA(cudaFreeAsync(p, s));
+  if (pooled) FMF_CUDA(cudaFreeAsync(p, s));
 }
-static void trim_pools() {
+unsigned Workspace::slots = 0;
+static void give_back_workspaces() {
+  if (g_lib) FMF_CUDA(cudaStreamSynchronize(g_lib));
+  for (int q = 0; q < 16; ++q)
+    if (Workspace::slots >> q & 1) {
+      Slot& sl = g_global_set.slots[q];
+      if (sl.p) FMF_CUDA(cudaFree(sl.p));
+      sl = Slot{};
+    }
   std::lock_guard<std::mutex> lk(g_pool_mu);
   for (cudaMemPool_t p : g_pools)
     if (p) FMF_CUDA(cudaMemPoolTrimTo(p, 0));
@@ -282,7 +298,7 @@ int reset_registry() {
   FMF_CUDA(cudaStreamSynchronize(stream()));
   for (auto& e : g_reg) FMF_CUDA(cudaFree(e.second.dev));
   g_reg.clear();
-  trim_pools();
+  give_back_workspaces();
   return 0;
 }
 

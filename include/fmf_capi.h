@@ -64,7 +64,7 @@ int fmf_set_mode(int mode);               /* FMF_RESIDENT or FMF_COHERENT */
  * calls go on where they are.  The pressure solve, the reductions and monitors, solu_sor4_
  * and fmf_dev_weno5_fused in FMF_MIXED and FMF_FP64E share one scratch area, so a caller
  * waits for the stream it leaves before calling those on another; solphi_mthinc1_ and
- * fmf_dev_csf_fused have a workspace per call, in stream order, and the rest has none. */
+ * fmf_dev_csf_fused have a workspace per stream or call, and the rest has none. */
 int fmf_set_stream(void* cuda_stream);
 int fmf_sync_to_host(void* host_ptr);     /* copy one mirrored array back */
 int fmf_sync_to_device(void* host_ptr);   /* re-upload one mirrored array */
@@ -352,9 +352,10 @@ int fmf_dev_weno5_fused(int precision, int ni, int nj, int nk, double dxinv, dou
 /* the CSF force of one phi field, FMF_FP64 and FMF_MIXED as the fused step of that
  * precision forms it, FMF_FP64E in FP32 pairs; interior u, v, w points (ni % 32 == 0,
  * nj % 8 == 0); returns a status.  FMF_FP64 works in 12 (ni+6)(nj+6)(nk+6) doubles
- * (3.4 GB at 512x256x256), allocated and freed in the order of the stream: a call
- * may be captured (the graph owns that memory) and calls on several streams do not
- * touch each other's; up to 4 GB stay with the library until fmf_reset. */
+ * (3.4 GB at 512x256x256): on the library's own stream in its scratch, on a caller's
+ * allocated and freed in the order of the stream, so that a call may be captured (the
+ * graph owns that memory) and calls on several streams do not touch each other's; up
+ * to 4 GB stay with the library until fmf_reset. */
 int fmf_dev_csf_fused(int precision, int ni, int nj, int nk, double dx, double dy, double dz,
                       double rhol, double rhog, double sigma, const double* phi, double* fu,
                       double* fv, double* fw);

@@ -40,8 +40,10 @@ def L(fmf_lib):
     fmf_lib.fmf_reset()
 
 
-def test_csf_on_two_streams(L):
-    """Both streams busy at once: the larger grid's kernels run while the smaller's start."""
+@pytest.mark.parametrize("own", [False, True], ids=["callers", "library"])
+def test_csf_on_two_streams(L, own):
+    """Both streams busy at once (the callers', or the library's own and a caller's): the
+    larger grid's kernels run while the smaller's start."""
     torch = pytest.importorskip("torch")
     sizes = [(128, 128, 128), (64, 64, 64)]
     phis = [_phi(torch, (s[2] + 6, s[1] + 6, s[0] + 6), q) for q, s in enumerate(sizes)]
@@ -54,7 +56,7 @@ def test_csf_on_two_streams(L):
     torch.cuda.synchronize()
     for rep in got:
         for q in (0, 1):
-            L.fmf_set_stream(ctypes.c_void_p(streams[q].cuda_stream))
+            L.fmf_set_stream(None if own and q == 0 else ctypes.c_void_p(streams[q].cuda_stream))
             assert _csf(L, sizes[q], phis[q], rep[q]) == 0
     torch.cuda.synchronize()
     for rep in got:
@@ -62,7 +64,8 @@ def test_csf_on_two_streams(L):
             assert all(torch.equal(x, y) for x, y in zip(a, b))
 
 
-def test_fluxes_on_two_streams(L):
+@pytest.mark.parametrize("own", [False, True], ids=["callers", "library"])
+def test_fluxes_on_two_streams(L, own):
     """solphi_mthinc1_ on host arrays that live on the device, each set on its own stream."""
     torch = pytest.importorskip("torch")
     size = (64, 32, 32)
@@ -93,7 +96,7 @@ def test_fluxes_on_two_streams(L):
     streams = [torch.cuda.Stream() for _ in range(2)]
     for _ in range(10):
         for q in (0, 1):
-            L.fmf_set_stream(ctypes.c_void_p(streams[q].cuda_stream))
+            L.fmf_set_stream(None if own and q == 0 else ctypes.c_void_p(streams[q].cuda_stream))
             call(q)
     torch.cuda.synchronize()
     assert L.fmf_last_error() == 0
@@ -115,7 +118,10 @@ with torch.cuda.graph(graph, stream=s):  # this process's first call
     L.fmf_set_stream(ctypes.c_void_p(s.cuda_stream))
     assert _csf(L, size, phi, out) == 0
 L.fmf_set_stream(None)
-plain = _fields(torch, size)
+plain, aside = [_fields(torch, size) for _ in range(2)]
+with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=s):  # and one beside a capture
+    torch.zeros(1, device="cuda").add_(1)
+    assert _csf(L, size, phi, aside) == 0
 assert _csf(L, size, phi, plain) == 0
 L.fmf_device_synchronize()
 assert _csf(L, larger, _phi(torch, (70, 70, 134), 1), _fields(torch, larger)) == 0
@@ -126,7 +132,8 @@ for _ in range(3):
     torch.cuda.synchronize()
     graph.replay()
     torch.cuda.synchronize()
-    assert all(torch.equal(a, b) for a, b in zip(out, plain)) and bool(out[0].abs().max() > 0)
+    assert all(torch.equal(a, b) and torch.equal(a, c) for a, b, c in zip(out, plain, aside))
+    assert bool(out[0].abs().max() > 0)
 """
 
 
